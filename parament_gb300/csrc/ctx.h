@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include <vector>
+
 #include "parament.h"
 
 namespace pgb {
@@ -48,6 +50,11 @@ struct Ctx {
     bool split_ready = false;
     bool split_herm = false;                     // split stack exactly (anti-)Hermitian per slot
 
+    // Fixed-point form of complex128 contexts (fx.cu): the stack as integers
+    // and the workspace of a propagation.
+    DevBuf fx_stack, fx_ws;
+    bool fx_ready = false;
+
     // Instrumentation: CUDA events around the dominant kernel of the last call
     // and the number of kernels it launched.
     bool timing = false;
@@ -76,7 +83,7 @@ struct Ctx {
     size_t esize() const { return fp64 ? 16 : 8; }
     size_t device_bytes() const {
         return stack.cap + split_stack.cap + carr.cap + out.cap + chunks.cap + work.cap + X.cap + B1.cap + B2.cap +
-               aux.cap + grad.cap + wts.cap + xplanes.cap;
+               aux.cap + grad.cap + wts.cap + xplanes.cap + fx_stack.cap + fx_ws.cap;
     }
     void release_all() {
         stack.release();
@@ -92,6 +99,8 @@ struct Ctx {
         grad.release();
         wts.release();
         xplanes.release();
+        fx_stack.release();
+        fx_ws.release();
     }
 };
 
@@ -114,6 +123,19 @@ int split_order(double hnorm, double h, long long P);
 Parament_ErrorCode run_split(Ctx *c, const void *d_carr, unsigned pts, unsigned amps, double h, int M, long long P,
                              void *d_out, cudaStream_t stream);
 Parament_ErrorCode run_split_large(Ctx *c, const SplitArgs &a, double h, void *d_out, cudaStream_t stream);
+
+// c0 = m_0 - 1 and mu_n = m_n / Hnorm^n of the regrouped polynomial (split.cu).
+void split_coefficients(int M, double x, double hnorm, double *c0, std::vector<double> &mu);
+
+// complex128 by exact sliced products (fx.cu): fx_prepare converts the stack
+// (set_hamiltonian), fx_ensure allocates the workspace of P steps, run_fx
+// propagates (x = Hnorm h).
+struct WeightSpecHost;
+void fx_prepare(Ctx *c);
+bool fx_applies(const Ctx *c, int M);
+bool fx_ensure(Ctx *c, long long P);
+cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double x, int M, long long P, void *d_out,
+                   cudaStream_t stream);
 
 // Adjoint: d/du_k[i] Re Tr(W^H U) for real samples, d <= adj_max_dim.
 int adj_max_dim(bool fp64);

@@ -1,0 +1,788 @@
+// complex128 propagation for d > kFxMinDim on the tensor cores: fixed-point
+// matrices and exact sliced products (fx.cuh).
+//
+// The same X_j, Chebyshev order and Bessel coefficients as the FP64 kernels
+// (step_small.cu, gemm.cu; src/cuda/parament.cpp:486-718).  What changes:
+//
+//   * The polynomial.  For x = Hnorm h <= 1 the Chebyshev-Bessel sum is
+//     evaluated by powers of X (the same polynomial, regrouped as in split.cu;
+//     sum |c_n| |X|^n <= e^x, so no cancellation): Y = X^2 and, for M >= 9,
+//     W = X^3, then Horner's rule in Y or W with coefficients of degree 1 or 2,
+//         M   3  5  7  9  11  13  15
+//         products   2  3  4  4   5   6   6    (Clenshaw: M - 1).
+//     Above x = 1 the Clenshaw recurrence runs as before.  Every coefficient
+//     (-i)^n times a real number is real or imaginary, so an epilogue needs one
+//     64-bit multiply per value and term.
+//   * E_j = U_j - I is what is formed and kept, and the running product of a
+//     chunk of steps is P <- E P + E + P with U_(s1-1) ... U_s0 = I + P: the
+//     unit diagonal never meets the small terms.  The chunk products meet in
+//     the pairwise tree in the same form.
+//   * X_j = sum_m w_jm S_m is itself a product, weights (steps x 1 + Ke) times
+//     the stack (1 + Ke rows of 2 dp^2 numbers), on the same sliced kernel:
+//     one row of weights per step, each with an exponent of its own.
+//
+// d <= 64: one CTA per chunk walks its steps through all products of a step,
+// the matrices in global memory (L2), no launch per product (k_fx_steps).
+// d > 64: the chunks advance together, one launch per product of a round
+// (k_fx_gemm over the chunks' items and their 64 x 64 tiles).
+#include <math.h>
+#include <stdlib.h>
+
+#include <algorithm>
+#include <vector>
+
+#include "common.cuh"
+#include "ctx.h"
+#include "fx.cuh"
+#include "kernels.h"
+
+namespace pgb {
+namespace fx {
+
+// ------------------------------------------------------------------ set-up of the stack
+
+// Largest biased exponent of each stack matrix (emax zeroed before).
+__global__ void k_fx_stack_max(const double2 *src, i64 dd, int *emax) {
+    const double2 *m = src + (size_t)blockIdx.y * dd;
+    int e = 0;
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < dd; i += (i64)gridDim.x * blockDim.x) {
+        const double2 v = m[i];
+        e = max(e, max((__double2hiint(v.x) >> 20) & 0x7FF, (__double2hiint(v.y) >> 20) & 0x7FF));
+    }
+    e = __reduce_max_sync(0xffffffffu, e);
+    if ((threadIdx.x & 31) == 0) atomicMax(&emax[blockIdx.y], e);
+}
+
+// Exponent e with |v| < 2^e for a largest biased exponent.
+__device__ __forceinline__ int exp_of(int biased) { return max(biased, 1) - 1022; }
+
+// The stack as fixed-point items, every matrix at its own exponent.
+__global__ void k_fx_stack(const double2 *src, int d, int dp, const int *emax, i64 *dst) {
+    const int m = blockIdx.y, s = 62 - exp_of(emax[m]);
+    const double2 *a = src + (size_t)m * d * d;
+    i64 *o = dst + (size_t)m * 2 * dp * dp;
+    const i64 n = (i64)dp * dp;
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
+        const int r = (int)(i / dp), c = (int)(i % dp);
+        double2 v = make_double2(0.0, 0.0);
+        if (r < d && c < d) v = a[(size_t)r * d + c];
+        o[i] = __double2ll_rn(scalbn(v.x, s));
+        o[n + i] = __double2ll_rn(scalbn(v.y, s));
+    }
+}
+
+// ------------------------------------------------------------------ weights and X
+
+// P steps in nch chunks of consecutive steps: len + 1 in the first nlong, len in
+// the others, so that the chunks with a step left are always the first ones.
+struct Chunks {
+    i64 len;
+    int nlong, nch;
+    __host__ __device__ __forceinline__ i64 start(i64 c) const { return c * len + (c < nlong ? c : nlong); }
+    __host__ __device__ __forceinline__ i64 steps(i64 c) const { return len + (c < nlong ? 1 : 0); }
+    __host__ __device__ __forceinline__ i64 longest() const { return len + (nlong > 0 ? 1 : 0); }
+};
+
+// Row j of a batch: step i0 + j % per of chunk j / per (none: a zero row).
+struct Rows {
+    Chunks ch;
+    int per;
+    i64 i0;
+    __device__ __forceinline__ i64 step(i64 j) const {
+        const i64 c = j / per, i = i0 + j % per;
+        return (c < ch.nch && i < ch.steps(c)) ? ch.start(c) + i : -1;
+    }
+};
+
+// One warp per row: the step's weights times the stack matrices' scales, as
+// integers at the row's exponent; the exponent of X_j and its length (zero
+// here, kPoison for weights that are not finite).
+__global__ void __launch_bounds__(128) k_fx_weights(const double2 *carr, WeightSpec w, int Ke, const int *emax,
+                                                    Rows rows, i64 nrows, int kpad, int lgk, i64 *W, i64 plane,
+                                                    Info *info) {
+    const i64 j = (i64)blockIdx.x * 4 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (j >= nrows) return;
+    const i64 st = rows.step(j);
+    i64 *re = W + j * kpad, *im = re + plane;
+    if (st < 0) {
+        for (int m = lane; m < kpad; m += 32) re[m] = im[m] = 0;
+        if (lane == 0) info[j] = Info{0, 0};
+        return;
+    }
+    auto weight = [&](int m) {
+        double2 v = m == 0 ? make_double2(1.0, 0.0) : step_weight(carr, w, m - 1, st);
+        const int e = exp_of(emax[m]);
+        return make_double2(scalbn(v.x, e), scalbn(v.y, e));
+    };
+    int be = 0;
+    for (int m = lane; m <= Ke; m += 32) {
+        const double2 v = weight(m);
+        be = max(be, max((__double2hiint(v.x) >> 20) & 0x7FF, (__double2hiint(v.y) >> 20) & 0x7FF));
+    }
+    be = __reduce_max_sync(0xffffffffu, be);
+    const int e = exp_of(be);
+    for (int m = lane; m < kpad; m += 32) {
+        double2 v = make_double2(0.0, 0.0);
+        if (m <= Ke && be < 0x7FF) v = weight(m);
+        re[m] = __double2ll_rn(scalbn(v.x, 62 - e));
+        im[m] = __double2ll_rn(scalbn(v.y, 62 - e));
+    }
+    if (lane == 0) info[j] = Info{e + lgk, be < 0x7FF ? 0 : kPoison};
+}
+
+struct AssembleArgs {
+    const i64 *W, *stack;
+    i64 wplane;
+    i64 *X;
+    Info *info;
+    i64 nrows, item;  // item: 2 dp^2
+    int kpad, kvalid, lgk;
+    int *fault;
+};
+
+// Tile (64 rows, 64 numbers of a plane) of X = W S.
+__global__ void __launch_bounds__(kThreads, 1) k_fx_assemble(const __grid_constant__ AssembleArgs a) {
+    extern __shared__ unsigned char raw[];
+    __shared__ Shared s;
+    Thread t;
+    setup(s, t, raw);
+    const i64 plane = a.item / 2;
+    const i64 rt = (a.nrows + 63) / 64, ct = plane / 64, units = rt * ct;
+    for (i64 u = blockIdx.x; u < units; u += gridDim.x) {
+        const i64 r0 = (u % rt) * 64, n0 = (u / rt) * 64;
+        if (t.tid < 64) s.rowmb[t.tid] = 0;
+        const Operand A{a.W + r0 * a.kpad, a.kpad, a.wplane, 0}, B{a.stack + n0, a.item, plane, 0};
+        i64 v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = 0;
+        if (!product(s, t, A, B, false, a.kpad / kStageK, a.kvalid, 6 + a.lgk, v)) break;
+        const i64 row = r0 + t.r;
+        if (row < a.nrows) {
+            u64 m = 0;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) m |= (u64)(v[j] ^ (v[j] >> 63));
+            atomicMax(&s.rowmb[t.r], bits_of(m));
+            store16(a.X + row * a.item + t.p * plane + n0 + t.c0, v);
+        }
+        __syncthreads();
+        if (t.tid < 64 && r0 + t.tid < a.nrows) atomicMax(&a.info[r0 + t.tid].mb, s.rowmb[t.tid]);
+        __syncthreads();
+    }
+    teardown(s, t, a.fault);
+}
+
+// ------------------------------------------------------------------ d <= 64: whole steps in one launch
+
+enum { kBufX, kBufY, kBufW, kBufR0, kBufR1, kBufE, kBufP, kBufs };
+constexpr int kMaxOps = 64;
+constexpr i64 kItem64 = 2 * 64 * 64;
+
+struct StepsArgs {
+    Op op[kMaxOps];
+    int nops;
+    const i64 *X;
+    const Info *xinfo;
+    i64 *scratch;  // per CTA: Y, W, R0, R1, E
+    i64 *pbuf;     // 2 x nch running products
+    i64 *chunks;   // nch finished products
+    Info *pinfo, *cinfo;
+    Chunks ch;
+    i64 i0;
+    int per, d, nst, lgk;
+    int *fault;
+};
+
+// One product of an item held by this CTA alone: infos in shared memory.
+__device__ __forceinline__ bool run_op(Shared &s, Thread &t, const Op &op, i64 *const (&buf)[kBufs], Info *info, int d,
+                                       int nst, int lgk) {
+    const Info ia = info[op.a], ib = info[op.b];
+    const int ha = headroom(ia), hb = headroom(ib);
+    const Operand A{buf[op.a], 64, 4096, ha}, B{buf[op.b], 64, 4096, hb};
+    const int eT = ia.e - ha + ib.e - hb + lgk;
+    i64 T[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) T[j] = 0;
+    if (!product(s, t, A, B, op.imag != 0, nst, 64, 6 + lgk, T)) return false;
+    const int off = t.r * 64 + t.c0;
+#pragma unroll 1
+    for (int o = 0; o < 2; ++o) {
+        const Out &out = op.out[o];
+        if (out.buf < 0) continue;
+        View w[kTerms];
+        for (int k = 0; k < out.nterm; ++k) w[k] = View{buf[out.term[k].buf] + off, 4096, info[out.term[k].buf]};
+        bool poison = ia.mb == kPoison || ib.mb == kPoison;
+        const int e = out_exponent(out, eT, w, poison);
+        i64 v[16];
+        out_values(out, t, T, eT, e, w, t.r, t.c0, d, v);
+        store16(buf[out.buf] + t.p * 4096 + off, v);
+        const u64 m = warp_or(v);
+        if (t.lane == 0) {
+            atomicOr(&s.orhi[o], (uint32_t)(m >> 32));
+            atomicOr(&s.orlo[o], (uint32_t)m);
+        }
+        __syncthreads();
+        if (t.tid == 0) {
+            info[out.buf] = Info{e, poison ? kPoison : bits_of((u64)s.orhi[o] << 32 | s.orlo[o])};
+            s.orhi[o] = s.orlo[o] = 0;
+        }
+    }
+    __syncthreads();
+    return true;
+}
+
+__global__ void __launch_bounds__(kThreads, 1) k_fx_steps(const __grid_constant__ StepsArgs a) {
+    extern __shared__ unsigned char raw[];
+    __shared__ Shared s;
+    __shared__ Info info[kBufs];
+    Thread t;
+    if (threadIdx.x < 2) s.orhi[threadIdx.x] = s.orlo[threadIdx.x] = 0;
+    setup(s, t, raw);
+    const int c = blockIdx.x;
+    const i64 len = a.ch.steps(c);
+    const i64 last = min(len, a.i0 + a.per);
+    i64 *scratch = a.scratch + (i64)c * 5 * kItem64;
+    i64 *buf[kBufs];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) buf[kBufY + k] = scratch + k * kItem64;
+    if (t.tid == 0 && a.i0 > 0) info[kBufP] = a.pinfo[c];
+    Op run{};
+    run.a = kBufE;
+    run.b = kBufP;
+    run.out[1].buf = -1;
+    run.out[0].buf = kBufX;  // the target's place, set below
+    run.out[0].nterm = 2;
+    const Coef one{1ll << 61, 1, 0};
+    run.out[0].t = one;
+    run.out[0].term[0] = Term{one, kBufE};
+    run.out[0].term[1] = Term{one, kBufP};
+    bool ok = true;
+    for (i64 i = a.i0; i < last && ok; ++i) {
+        const i64 xi = (i64)c * a.per + (i - a.i0);
+        i64 *dst = i == len - 1 ? a.chunks + (i64)c * kItem64 : a.pbuf + ((i & 1) * a.ch.nch + c) * kItem64;
+        buf[kBufX] = const_cast<i64 *>(a.X) + xi * kItem64;
+        buf[kBufP] = a.pbuf + (((i - 1) & 1) * a.ch.nch + c) * kItem64;
+        buf[kBufE] = i == 0 ? dst : scratch + 4 * kItem64;
+        __syncthreads();
+        if (t.tid == 0) info[kBufX] = a.xinfo[xi];
+        __syncthreads();
+        for (int o = 0; o < a.nops && ok; ++o) ok = run_op(s, t, a.op[o], buf, info, a.d, a.nst, a.lgk);
+        if (!ok) break;
+        if (i == 0) {
+            if (t.tid == 0) info[kBufP] = info[kBufE];
+        } else {
+            buf[kBufX] = dst;
+            ok = run_op(s, t, run, buf, info, a.d, a.nst, a.lgk);
+            if (t.tid == 0) info[kBufP] = info[kBufX];
+        }
+    }
+    __syncthreads();
+    if (t.tid == 0 && ok && last > a.i0) (last == len ? a.cinfo : a.pinfo)[c] = info[kBufP];
+    teardown(s, t, a.fault);
+}
+
+// ------------------------------------------------------------------ d > 64 and the tree: one product of many items
+
+struct Buf {
+    i64 *ptr;
+    i64 stride;  // numbers from one item to the next
+    Info *info;
+    int istride;
+};
+struct GemmArgs {
+    Op op;
+    Buf buf[kBufs];
+    int items, nt, dp, d, nst, lgk;
+    int *fault;
+};
+
+__global__ void __launch_bounds__(kThreads, 1) k_fx_gemm(const __grid_constant__ GemmArgs a) {
+    extern __shared__ unsigned char raw[];
+    __shared__ Shared s;
+    Thread t;
+    if (threadIdx.x < 2) s.orhi[threadIdx.x] = s.orlo[threadIdx.x] = 0;
+    setup(s, t, raw);
+    const i64 plane = (i64)a.dp * a.dp;
+    const int tiles = a.nt * a.nt;
+    const i64 units = (i64)a.items * tiles;
+    const Op &op = a.op;
+    for (i64 u = blockIdx.x; u < units; u += gridDim.x) {
+        const i64 it = u / tiles;
+        const int tile = (int)(u % tiles), I = tile / a.nt, J = tile % a.nt;
+        auto view = [&](int b, i64 off) {
+            const Buf &q = a.buf[b];
+            return View{q.ptr + it * q.stride + off, plane, q.info[it * q.istride]};
+        };
+        const View va = view(op.a, (i64)I * 64 * a.dp), vb = view(op.b, J * 64);
+        const int ha = headroom(va.info), hb = headroom(vb.info);
+        const Operand A{va.re, a.dp, plane, ha}, B{vb.re, a.dp, plane, hb};
+        const int eT = va.info.e - ha + vb.info.e - hb + a.lgk;
+        i64 T[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) T[j] = 0;
+        if (!product(s, t, A, B, op.imag != 0, a.nst, a.dp, 6 + a.lgk, T)) break;
+        const int row = I * 64 + t.r, col0 = J * 64 + t.c0;
+        const i64 off = (i64)row * a.dp + col0;
+#pragma unroll 1
+        for (int o = 0; o < 2; ++o) {
+            const Out &out = op.out[o];
+            if (out.buf < 0) continue;
+            View w[kTerms];
+            for (int k = 0; k < out.nterm; ++k) w[k] = view(out.term[k].buf, off);
+            bool poison = va.info.mb == kPoison || vb.info.mb == kPoison;
+            const int e = out_exponent(out, eT, w, poison);
+            i64 v[16];
+            out_values(out, t, T, eT, e, w, row, col0, a.d, v);
+            const Buf &q = a.buf[out.buf];
+            store16(q.ptr + it * q.stride + t.p * plane + off, v);
+            const u64 m = warp_or(v);
+            if (t.lane == 0) {
+                atomicOr(&s.orhi[o], (uint32_t)(m >> 32));
+                atomicOr(&s.orlo[o], (uint32_t)m);
+            }
+            __syncthreads();
+            if (t.tid == 0) {
+                Info *i = &q.info[it * q.istride];
+                if (tile == 0) i->e = e;
+                atomicMax(&i->mb, poison ? kPoison : bits_of((u64)s.orhi[o] << 32 | s.orlo[o]));
+                s.orhi[o] = s.orlo[o] = 0;
+            }
+        }
+        __syncthreads();
+    }
+    teardown(s, t, a.fault);
+}
+
+// I + E as complex128, row-major d x d.
+__global__ void k_fx_out(const i64 *E, const Info *info, int d, int dp, double2 *out) {
+    const Info q = *info;
+    const i64 plane = (i64)dp * dp, n = (i64)d * d;
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
+        const int r = (int)(i / d), c = (int)(i % d);
+        double2 v = make_double2(scalbn((double)E[(i64)r * dp + c], q.e - 62),
+                                 scalbn((double)E[plane + (i64)r * dp + c], q.e - 62));
+        if (q.mb == kPoison) v.x = v.y = __longlong_as_double(0x7FF8000000000000ll);
+        if (r == c) v.x += 1.0;
+        out[i] = v;
+    }
+}
+
+// ------------------------------------------------------------------ host side
+
+static int ceil_log2(i64 n) {
+    int l = 0;
+    while ((1ll << l) < n) ++l;
+    return l;
+}
+
+// A real or imaginary coefficient re + i im (one of them zero).
+static Coef coef(long double re, long double im) {
+    const long double v = im != 0.0L ? im : re;
+    if (v == 0.0L) return Coef{0, 0, 0};
+    int e = 0;
+    const long double f = frexpl(v, &e);
+    return Coef{(i64)ldexpl(f, 62), e, im != 0.0L ? 1 : 0};
+}
+
+static Out plain_out(int buf) {
+    Out o{};
+    o.buf = buf;
+    o.plain = 1;
+    return o;
+}
+static Out no_out() {
+    Out o{};
+    o.buf = -1;
+    return o;
+}
+
+// The products of a step: E from X.  Powers of X for x <= 1, the Clenshaw
+// recurrence above.
+static void build_program(int M, double x, double hnorm, std::vector<Op> &ops) {
+    ops.clear();
+    auto add = [](Out &o, Coef c, int buf) {
+        if (c.m) o.term[o.nterm++] = Term{c, buf};
+    };
+    if (x <= 1.0) {
+        double c0[2];
+        std::vector<double> mu;
+        split_coefficients(M, x, hnorm, c0, mu);
+        // c_0 = p(0) - 1: the orders above M of 1 = J_0 + 2 sum J_2k.  Summed as
+        // J_0 - 1 + ... its rounding (1e-16) would scale U at every step alike:
+        // 3e-14 after 300 steps where the FP64 kernels are at 6e-15.
+        double tail = 0.0;
+        for (int k = M + 21; k > M; k -= 2) tail += jn(k, x);
+        c0[0] = -2.0 * tail;
+        c0[1] = 0.0;
+        auto cf = [&](int n) { return n == 0 ? coef(c0[0], c0[1]) : coef(mu[2 * n], mu[2 * n + 1]); };
+        Op y{kBufX, kBufX, 0, {plain_out(kBufY), no_out()}};
+        ops.push_back(y);
+        // An imaginary factor of a product goes into its operand.
+        // Horner in Y: r = c_M X Y + c_(M-1) Y + c_(M-2) X + c_(M-3), then r Y + c_(k+1) X + c_k.
+        auto horner = [&](int a, int b, Coef tc, int k, int deg, bool fin) {
+            Op o{a, b, tc.imag, {Out{}, no_out()}};
+            tc.imag = 0;
+            Out &r = o.out[0];
+            r.buf = fin ? kBufE : (a == kBufR0 ? kBufR1 : kBufR0);
+            r.t = tc;
+            const int powbuf[3] = {0, kBufX, kBufY};
+            for (int n = 1; n <= deg; ++n) add(r, cf(k + n), powbuf[n]);
+            r.diag = cf(k);
+            ops.push_back(o);
+            return r.buf;
+        };
+        const Coef one = coef(1.0, 0.0);
+        if (M < 9) {
+            int r = horner(kBufX, kBufY, cf(M), M - 3, 2, M == 3);
+            for (int k = M - 5; k >= 0; k -= 2) r = horner(r, kBufY, one, k, 1, k == 0);
+        } else {
+            // W = X Y and, beside it, the top coefficient of the rule in W:
+            // degree 3 (with W itself) where 3 divides M; its c_M is imaginary,
+            // so the buffer then holds i W and r W = -(i r (i W)).
+            const bool three = M % 3 == 0;
+            const int top = three ? M - 3 : M - M % 3;
+            Op w{kBufX, kBufY, three ? 1 : 0, {plain_out(kBufW), Out{}}};
+            Out &r = w.out[1];
+            r.buf = kBufR0;
+            if (three) {
+                r.t = cf(M);
+                r.t.imag = 0;
+            }
+            add(r, cf(top + 1), kBufX);
+            if (M - top >= 2) add(r, cf(top + 2), kBufY);
+            r.diag = cf(top);
+            ops.push_back(w);
+            int cur = kBufR0;
+            Coef f = one;
+            if (three) {
+                f.m = -f.m;
+                f.imag = 1;
+            }
+            for (int k = top - 3; k >= 0; k -= 3) cur = horner(cur, kBufW, f, k, 2, k == 0);
+        }
+        return;
+    }
+    // b_M = J_M, b_(M-1) = s J_M X + J_(M-1), b_k = s b_(k+1) X - b_(k+2) + J_k
+    // with s = 2 / Hnorm; E = s b_1 X - 2 b_2 + J_0 - 1.  b_(M-2) comes from X X
+    // directly: s^2 J_M X^2 + s J_(M-1) X + J_(M-2) - J_M.  s is a coefficient of
+    // 62 bits: rounded into X it would turn every step's phase alike.
+    const long double sc = 2.0L / hnorm;
+    std::vector<double> J(2 * (M + 1));
+    bessel_coeffs(M, x, J.data());
+    // J_0 - 1 from the even orders, for the same reason.
+    long double j0m1 = 0.0L;
+    for (int k = M + 41; k >= 2; k -= 2) j0m1 -= 2.0L * jn(k, x);
+    auto j = [&](int k, long double f) { return coef(f * J[2 * k], f * J[2 * k + 1]); };
+    int prev = -1, cur = -1, n = 0;  // buffers of b_(k+2) and b_(k+1); -1: from X
+    const int rot[3] = {kBufY, kBufW, kBufR0};
+    for (int k = M - 2; k >= 0; --k) {
+        Op o{cur < 0 ? kBufX : cur, kBufX, 0, {Out{}, no_out()}};
+        Out &r = o.out[0];
+        const double beta = k == 0 ? -2.0 : -1.0;
+        long double dr = k == 0 ? j0m1 : J[2 * k], di = J[2 * k + 1];
+        if (cur < 0) {  // k = M - 2
+            r.t = j(M, sc * sc);
+            o.imag = r.t.imag;
+            r.t.imag = 0;
+            add(r, j(M - 1, sc), kBufX);
+            dr += beta * J[2 * M];
+            di += beta * J[2 * M + 1];
+        } else {
+            r.t = coef(sc, 0.0L);
+            if (prev < 0) {  // k = M - 3: b_(M-1) = s J_M X + J_(M-1)
+                add(r, j(M, sc * beta), kBufX);
+                dr += beta * J[2 * (M - 1)];
+                di += beta * J[2 * (M - 1) + 1];
+            } else {
+                add(r, coef(beta, 0.0), prev);
+            }
+        }
+        r.diag = coef(dr, di);
+        r.buf = k == 0 ? kBufE : rot[n++ % 3];
+        prev = cur;
+        cur = r.buf;
+        ops.push_back(o);
+    }
+}
+
+static bool disabled() {
+    static const bool off = [] {
+        const char *v = getenv("PARAMENT_DISABLE_TENSOR_CORES");
+        return v && v[0] && v[0] != '0';
+    }();
+    return off;
+}
+
+static cudaError_t set_smem() {
+    cudaError_t e = cudaSuccess;
+    for (const void *fn : {reinterpret_cast<const void *>(&k_fx_assemble), reinterpret_cast<const void *>(&k_fx_steps),
+                           reinterpret_cast<const void *>(&k_fx_gemm)})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    return e;
+}
+
+// The workspace of a propagation, carved from one allocation.
+struct Plan {
+    int d, dp, nt, kpad, kvalid, nch, per;
+    Chunks ch;
+    i64 item, rows;
+    size_t off_w, off_x, off_s, off_p, off_c, off_t, off_info, bytes;
+    size_t n_info;
+};
+
+static Plan make_plan(int d, int Ke, i64 P, int num_sms) {
+    Plan q{};
+    q.d = d;
+    q.dp = (d + 63) / 64 * 64;
+    q.nt = q.dp / 64;
+    q.item = 2ll * q.dp * q.dp;
+    q.kvalid = 1 + Ke;
+    q.kpad = (q.kvalid + kStageK - 1) / kStageK * kStageK;
+    const int tiles = q.nt * q.nt;
+    if (tiles == 1) {
+        // One chunk per SM; X of up to 32 steps of every chunk at a time (320 MB).
+        q.nch = (int)std::min<i64>(num_sms, P);
+        q.per = (int)std::min<i64>(32, (P + q.nch - 1) / q.nch);
+    } else {
+        // About eight waves of tiles per product, in rounds of equal size.
+        const i64 g0 = std::min<i64>(P, std::max<i64>(1, (8ll * num_sms + tiles - 1) / tiles));
+        const i64 L = (P + g0 - 1) / g0;
+        q.nch = (int)((P + L - 1) / L);
+        q.per = 1;
+    }
+    q.ch = Chunks{P / q.nch, (int)(P % q.nch), q.nch};
+    q.rows = (i64)q.nch * q.per;
+    const i64 rpad = (q.rows + 63) / 64 * 64;
+    size_t o = 0;
+    auto take = [&](size_t n) {
+        const size_t at = o;
+        o += (n + 255) / 256 * 256;
+        return at;
+    };
+    const size_t m = sizeof(i64) * (size_t)q.item;
+    q.off_w = take(sizeof(i64) * 2 * (size_t)rpad * q.kpad);
+    q.off_x = take(m * (size_t)q.rows);
+    q.off_s = take(m * 5 * (size_t)q.nch);
+    q.off_p = take(m * 2 * (size_t)q.nch);
+    q.off_c = take(m * (size_t)q.nch);
+    // X rows; the results of a step's products; P0 P1; finished chunks; the tree's.
+    q.n_info = (size_t)q.rows + (kMaxOps + 5) * (size_t)q.nch;
+    q.off_info = take(sizeof(Info) * q.n_info);
+    q.bytes = o;
+    return q;
+}
+
+// Bytes before the matrices of the fixed-point stack: the largest exponents.
+static size_t stack_head(int n) { return (sizeof(int) * (size_t)n + 255) / 256 * 256; }
+
+static cudaError_t launch_gemm_op(const GemmArgs &a, int num_sms, cudaStream_t st, int *launches) {
+    const i64 units = (i64)a.items * a.nt * a.nt;
+    k_fx_gemm<<<(int)std::min<i64>(units, num_sms), kThreads, kSmem, st>>>(a);
+    ++*launches;
+    return cudaGetLastError();
+}
+
+}  // namespace fx
+
+using namespace fx;
+
+bool fx_applies(const Ctx *c, int M) {
+    return c->fp64 && c->fx_ready && M >= 3 && isfinite(c->hnorm) && c->hnorm > 0.0;
+}
+
+// The context's stack in fixed point, made with the Hamiltonian on the
+// context's stream (the caller waits for it).  Without room for it the FP64
+// kernels serve.
+void fx_prepare(Ctx *c) {
+    c->fx_ready = false;
+    const int d = (int)c->dim, dp = (d + 63) / 64 * 64, n = 1 + (int)c->Ke;
+    if (d < kFxMinDim || disabled()) return;
+    const size_t head = stack_head(n);
+    void *p = nullptr;
+    if (cudaMalloc(&p, head + sizeof(i64) * 2 * (size_t)dp * dp * n) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    c->fx_stack.release();
+    c->fx_stack.ptr = p;
+    c->fx_stack.cap = head + sizeof(i64) * 2 * (size_t)dp * dp * n;
+    int *emax = static_cast<int *>(p);
+    const double2 *src = static_cast<const double2 *>(c->stack.ptr);
+    if (cudaMemsetAsync(emax, 0, sizeof(int) * n, c->stream) != cudaSuccess) return;
+    k_fx_stack_max<<<dim3(std::max(1, std::min(256, d * d / 1024)), n), 256, 0, c->stream>>>(src, (i64)d * d, emax);
+    k_fx_stack<<<dim3(std::max(1, std::min(1024, dp * dp / 512)), n), 256, 0, c->stream>>>(
+        src, d, dp, emax, reinterpret_cast<i64 *>(static_cast<char *>(p) + head));
+    c->fx_ready = cudaGetLastError() == cudaSuccess;
+}
+
+bool fx_ensure(Ctx *c, long long P) {
+    const Plan q = make_plan((int)c->dim, (int)c->Ke, P, c->num_sms);
+    return c->fx_ws.ensure(q.bytes) == cudaSuccess;
+}
+
+cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double x, int M, long long P, void *d_out,
+                   cudaStream_t st) {
+    const int d = (int)c->dim, Ke = (int)c->Ke, n = 1 + Ke;
+    const Plan q = make_plan(d, Ke, P, c->num_sms);
+    int launches = 0;
+    cudaError_t e = set_smem();
+    if (e != cudaSuccess) return e;
+    const size_t head = stack_head(n);
+    const int *emax = static_cast<const int *>(c->fx_stack.ptr);
+    const i64 *stack = reinterpret_cast<const i64 *>(static_cast<const char *>(c->fx_stack.ptr) + head);
+    char *ws = static_cast<char *>(c->fx_ws.ptr);
+    i64 *W = reinterpret_cast<i64 *>(ws + q.off_w), *X = reinterpret_cast<i64 *>(ws + q.off_x);
+    i64 *S = reinterpret_cast<i64 *>(ws + q.off_s), *Pb = reinterpret_cast<i64 *>(ws + q.off_p);
+    i64 *chunks = reinterpret_cast<i64 *>(ws + q.off_c);
+    Info *xinfo = reinterpret_cast<Info *>(ws + q.off_info), *sinfo = xinfo + q.rows;
+    Info *pinfo = sinfo + (kMaxOps + 1) * (size_t)q.nch, *cinfo = pinfo + 2 * (size_t)q.nch, *tinfo = cinfo + q.nch;
+    std::vector<Op> ops;
+    build_program(M, x, c->hnorm, ops);
+    if ((int)ops.size() > kMaxOps) return cudaErrorInvalidValue;  // orders up to 63: 62 products
+    const WeightSpec w{wh.pts, wh.K, wh.amps, wh.mode, wh.magnus, wh.hfac};
+    const i64 rpad = (q.rows + 63) / 64 * 64;
+    const int lgw = std::max(3, ceil_log2(2ll * q.kvalid)), lgk = ceil_log2(2ll * d);
+    const int nst = (d + kStageK - 1) / kStageK;
+    auto assemble = [&](i64 i0, i64 rows, int per) -> cudaError_t {
+        const Rows r{q.ch, per, i0};
+        k_fx_weights<<<(unsigned)((rows + 3) / 4), 128, 0, st>>>(static_cast<const double2 *>(d_carr), w, Ke, emax, r,
+                                                               rows, q.kpad, lgw, W, rpad * q.kpad, xinfo);
+        const AssembleArgs a{W, stack, rpad * q.kpad, X, xinfo, rows, q.item, q.kpad, q.kvalid, lgw, c->d_fault};
+        const i64 units = ((rows + 63) / 64) * (q.item / 128);
+        k_fx_assemble<<<(int)std::min<i64>(units, c->num_sms), kThreads, kSmem, st>>>(a);
+        launches += 2;
+        return cudaGetLastError();
+    };
+    if (c->timing) cudaEventRecord(c->ev_start, st);
+    if (q.nt == 1) {
+        StepsArgs a;
+        for (size_t k = 0; k < ops.size(); ++k) a.op[k] = ops[k];
+        a.nops = (int)ops.size();
+        a.X = X;
+        a.xinfo = xinfo;
+        a.scratch = S;
+        a.pbuf = Pb;
+        a.chunks = chunks;
+        a.pinfo = pinfo;
+        a.cinfo = cinfo;
+        a.ch = q.ch;
+        a.per = q.per;
+        a.d = d;
+        a.nst = nst;
+        a.lgk = lgk;
+        a.fault = c->d_fault;
+        for (i64 i0 = 0; i0 < q.ch.longest(); i0 += q.per) {
+            if ((e = assemble(i0, q.rows, q.per)) != cudaSuccess) return e;
+            a.i0 = i0;
+            k_fx_steps<<<q.nch, kThreads, kSmem, st>>>(a);
+            ++launches;
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        }
+    } else {
+        const i64 longest = q.ch.longest(), mat = q.item, set = mat * q.nch;
+        GemmArgs a{};
+        a.nt = q.nt;
+        a.dp = q.dp;
+        a.d = d;
+        a.nst = nst;
+        a.lgk = lgk;
+        a.fault = c->d_fault;
+        Op run{kBufE, kBufP, 0, {Out{}, no_out()}};
+        const Coef one = coef(1.0, 0.0);
+        run.out[0].buf = kBufX;
+        run.out[0].t = one;
+        run.out[0].nterm = 2;
+        run.out[0].term[0] = Term{one, kBufE};
+        run.out[0].term[1] = Term{one, kBufP};
+        for (i64 i = 0; i < longest; ++i) {
+            const int active = i < q.ch.len ? q.nch : q.ch.nlong;
+            if ((e = assemble(i, active, 1)) != cudaSuccess) return e;
+            for (int b = 0; b < kBufs; ++b) a.buf[b] = Buf{};
+            a.buf[kBufX] = Buf{X, mat, xinfo, 1};
+            for (int b = 0; b < 5; ++b) a.buf[kBufY + b] = Buf{S + b * set, mat, nullptr, 1};
+            Buf dst{Pb + (i & 1) * set, mat, pinfo + (i & 1) * q.nch, 1};
+            a.buf[kBufP] = Buf{Pb + ((i - 1) & 1) * set, mat, pinfo + ((i - 1) & 1) * q.nch, 1};
+            // A buffer may be written more than once in a round: the lengths, which
+            // start at zero, are kept per result.
+            const size_t results = ops.size() + 1;
+            if ((e = cudaMemsetAsync(sinfo, 0, sizeof(Info) * results * q.nch, st)) != cudaSuccess) return e;
+            size_t slot = 0;
+            if ((e = cudaMemsetAsync(dst.info, 0, sizeof(Info) * q.nch, st)) != cudaSuccess) return e;
+            if (i == 0) a.buf[kBufE] = dst;
+            a.items = active;
+            for (const Op &o : ops) {
+                a.op = o;
+                for (const Out &out : o.out)
+                    if (out.buf >= 0 && !(out.buf == kBufE && i == 0)) a.buf[out.buf].info = sinfo + slot++ * q.nch;
+                if ((e = launch_gemm_op(a, c->num_sms, st, &launches)) != cudaSuccess) return e;
+            }
+            if (i > 0) {
+                a.buf[kBufX] = dst;
+                a.op = run;
+                if ((e = launch_gemm_op(a, c->num_sms, st, &launches)) != cudaSuccess) return e;
+            }
+            if (active < q.nch) {
+                // The chunks without a step in this round keep their product.
+                const Buf &prev = a.buf[kBufP];
+                const size_t rest = (size_t)(q.nch - active);
+                e = cudaMemcpyAsync(dst.ptr + active * mat, prev.ptr + active * mat, sizeof(i64) * mat * rest,
+                                    cudaMemcpyDeviceToDevice, st);
+                if (e == cudaSuccess)
+                    e = cudaMemcpyAsync(dst.info + active, prev.info + active, sizeof(Info) * rest,
+                                        cudaMemcpyDeviceToDevice, st);
+                if (e != cudaSuccess) return e;
+            }
+        }
+        chunks = Pb + ((longest - 1) & 1) * set;
+        cinfo = pinfo + ((longest - 1) & 1) * q.nch;
+    }
+    if (c->timing) cudaEventRecord(c->ev_stop, st);
+    // Pairwise tree over the chunk products, later chunks on the left:
+    // E = Ea Eb + Ea + Eb; an odd leftover moves up unchanged.
+    {
+        GemmArgs a{};
+        a.nt = q.nt;
+        a.dp = q.dp;
+        a.d = d;
+        a.nst = nst;
+        a.lgk = lgk;
+        a.fault = c->d_fault;
+        const Coef one = coef(1.0, 0.0);
+        a.op = Op{kBufX, kBufY, 0, {Out{}, no_out()}};
+        Out &o = a.op.out[0];
+        o.buf = kBufW;
+        o.t = one;
+        o.nterm = 2;
+        o.term[0] = Term{one, kBufX};
+        o.term[1] = Term{one, kBufY};
+        i64 *cur = chunks, *nxt = S;
+        Info *ci = cinfo, *ni = tinfo;
+        for (i64 n2 = q.nch; n2 > 1;) {
+            const i64 pairs = n2 / 2;
+            if ((e = cudaMemsetAsync(ni, 0, sizeof(Info) * pairs, st)) != cudaSuccess) return e;
+            a.buf[kBufX] = Buf{cur + q.item, 2 * q.item, ci + 1, 2};
+            a.buf[kBufY] = Buf{cur, 2 * q.item, ci, 2};
+            a.buf[kBufW] = Buf{nxt, q.item, ni, 1};
+            a.items = (int)pairs;
+            if ((e = launch_gemm_op(a, c->num_sms, st, &launches)) != cudaSuccess) return e;
+            if (n2 & 1) {
+                e = cudaMemcpyAsync(nxt + pairs * q.item, cur + 2 * pairs * q.item, sizeof(i64) * q.item,
+                                    cudaMemcpyDeviceToDevice, st);
+                if (e == cudaSuccess)
+                    e = cudaMemcpyAsync(ni + pairs, ci + 2 * pairs, sizeof(Info), cudaMemcpyDeviceToDevice, st);
+                if (e != cudaSuccess) return e;
+            }
+            n2 = pairs + (n2 & 1);
+            std::swap(cur, nxt);
+            std::swap(ci, ni);
+        }
+        const i64 total = (i64)d * d;
+        k_fx_out<<<(int)std::min<i64>((total + 255) / 256, 1024), 256, 0, st>>>(cur, ci, d, q.dp,
+                                                                               static_cast<double2 *>(d_out));
+        ++launches;
+    }
+    c->launches = launches;
+    return cudaGetLastError();
+}
+
+}  // namespace pgb

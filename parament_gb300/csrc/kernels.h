@@ -22,6 +22,8 @@ struct WeightSpecHost {
 // (d <= kSmallMaxDim) writes one ordered product per chunk of consecutive
 // steps into `chunks`.
 constexpr int kSmallMaxDim = 64;
+// complex128 from this dimension on runs as exact sliced products (fx.cu).
+constexpr int kFxMinDim = 17;
 
 struct StepLaunch {
     bool fp64;

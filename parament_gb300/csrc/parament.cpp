@@ -206,6 +206,8 @@ static Parament_ErrorCode set_hamiltonian(Ctx *c, const void *H0, const void *H1
     c->has_h = false;
     c->stack.release();
     c->split_stack.release();
+    c->fx_stack.release();
+    c->fx_ready = false;
     if (use_magnus) {
         c->magnus = true;
         if (quad != PARAMENT_QUADRATURE_SIMPSON) return c->last_error = PARAMENT_STATUS_INVALID_QUADRATURE_SELECTION;
@@ -261,6 +263,9 @@ static Parament_ErrorCode set_hamiltonian(Ctx *c, const void *H0, const void *H1
             for (unsigned j = 0; j < i && e == cudaSuccess; ++j)
                 e = commutator(1 + j, 1 + i, 1 + 2 * amps + i * (i - 1) / 2 + j);
     }
+    c->dim = dim;
+    c->Ke = Ke;
+    if (e == cudaSuccess && c->fp64) fx_prepare(c);
     if (use_magnus) note_call_end(c, c->stream, true);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
@@ -272,9 +277,7 @@ static Parament_ErrorCode set_hamiltonian(Ctx *c, const void *H0, const void *H1
         c->stack.release();
         return c->last_error = PARAMENT_STATUS_KERNEL_TIMEOUT;
     }
-    c->dim = dim;
     c->K = amps;
-    c->Ke = Ke;
     c->hnorm = hn;
     c->has_h = true;
     c->split_ready = false;
@@ -299,6 +302,18 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
     // product per CTA, combined by the double-float tree.  Where the planes
     // (up to 2.3 GB) cannot be allocated, the FP32 SIMT kernel below runs,
     // which needs only the chunk buffers.
+    // complex128: exact sliced products on the tensor cores (fx.cu).  Without
+    // room for their workspace the FP64 kernels below run; of those the cluster
+    // kernel, which needs the least memory, where it applies.
+    bool no_room = false;
+    if (fx_applies(c, M)) {
+        no_room = !fx_ensure(c, P);
+        if (!no_room) {
+            if (run_fx(c, d_carr, w, h * c->hnorm, M, P, d_out, stream) == cudaSuccess) return PARAMENT_STATUS_SUCCESS;
+            cudaGetLastError();
+            return PARAMENT_STATUS_CUBLAS_FAILED;
+        }
+    }
     const int nmax = small_tc_max_chunks(P, c->num_sms);
     if (small_tc_applies(c->fp64, d, (int)c->Ke, M) && c->chunks.ensure(es * dd * nmax) == cudaSuccess &&
         c->work.ensure(16 * dd * nmax) == cudaSuccess && c->X.ensure(16 * dd * ((nmax + 1) / 2)) == cudaSuccess &&
@@ -363,7 +378,7 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
         long long G = std::max<long long>(1, std::min<long long>(P, (long long)((4ULL << 30) / per)));
         G = std::min<long long>(G, 4096);
         const long long nb = (P + G - 1) / G;
-        if (c->X.ensure(es * dd * G) != cudaSuccess || c->B1.ensure(es * dd * G) != cudaSuccess ||
+        if ((no_room && mid_applies(c->fp64, d, (int)c->Ke)) || c->X.ensure(es * dd * G) != cudaSuccess || c->B1.ensure(es * dd * G) != cudaSuccess ||
             c->B2.ensure(es * dd * G) != cudaSuccess || c->chunks.ensure(es * dd * nb) != cudaSuccess ||
             c->work.ensure(es * dd * nb) != cudaSuccess) {
             if (!mid_applies(c->fp64, d, (int)c->Ke)) return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
@@ -452,9 +467,11 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
 
 // Whether an equiprop of this context may launch a kernel with bounded waits
 // (the tensor-core GEMM of complex64 contexts with d > 64, the tensor-core
-// split kernel, the tensor-core plain kernel at d = 64).
+// split kernel, the tensor-core plain kernel at d = 64, the sliced products of
+// complex128 contexts).
 static bool uses_tensor_kernels(const Ctx *c) {
-    return !c->fp64 && (c->dim >= (unsigned)kSmallMaxDim || c->precision == PARAMENT_PRECISION_SPLIT);
+    if (c->fp64) return c->fx_ready;
+    return c->dim >= (unsigned)kSmallMaxDim || c->precision == PARAMENT_PRECISION_SPLIT;
 }
 
 // Checks, order selection and dispatch shared by the host and device entry

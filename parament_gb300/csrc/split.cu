@@ -448,7 +448,7 @@ int split_order(double hnorm, double h, long long P) {
 
 // Monomial coefficients m_n of J_0(x) + 2 sum_(k=1..M) (-i)^k J_k(x) T_k(t);
 // returns mu_n = m_n / Hnorm^n (n >= 1) and c0 = m_0 - 1.
-static void split_coefficients(int M, double x, double hnorm, double *c0, std::vector<double> &mu) {
+void split_coefficients(int M, double x, double hnorm, double *c0, std::vector<double> &mu) {
     std::vector<double> J(2 * (M + 1));
     bessel_coeffs(M, x, J.data());
     std::vector<double> re(M + 1, 0.0), im(M + 1, 0.0);
