@@ -64,10 +64,11 @@ __global__ void k_fx_stack(const double2 *src, int d, int dp, const int *emax, i
     const i64 n = (i64)dp * dp;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
         const int r = (int)(i / dp), c = (int)(i % dp);
+        const i64 k = (i64)(c >> 2) * 4 * dp + 4 * r + (c & 3);
         double2 v = make_double2(0.0, 0.0);
         if (r < d && c < d) v = a[(size_t)r * d + c];
-        o[i] = __double2ll_rn(scalbn(v.x, s));
-        o[n + i] = __double2ll_rn(scalbn(v.y, s));
+        o[k] = __double2ll_rn(scalbn(v.x, s));
+        o[n + k] = __double2ll_rn(scalbn(v.y, s));
     }
 }
 
@@ -141,35 +142,62 @@ struct AssembleArgs {
     int *fault;
 };
 
+// Products a CTA of a grid runs of `units` dealt out in turn.
+__device__ __forceinline__ i64 my_units(i64 units) { return (units - blockIdx.x + gridDim.x - 1) / gridDim.x; }
+
 // Tile (64 rows, 64 numbers of a plane) of X = W S.
+struct AssembleWork {
+    using At = i64;
+    const AssembleArgs &a;
+    Shared &s;
+    Thread &t;
+    i64 rt, units, plane;
+    __device__ __forceinline__ At first() const { return blockIdx.x; }
+    __device__ __forceinline__ At next(At u) const { return u + gridDim.x; }
+    __device__ __forceinline__ bool more(At u) const { return u < units; }
+    __device__ __forceinline__ bool needs(At, At) const { return false; }
+    __device__ __forceinline__ bool operands(At u, Operand &A, Operand &B) const {
+        A = Operand{a.W + (u % rt) * 64 * a.kpad, a.kpad, 4, a.wplane, 0};
+        B = Operand{a.stack + (u / rt) * 64, a.item, 4, plane, 0};
+        return false;
+    }
+    __device__ __forceinline__ bool epilogue(At u, i64 (&v)[kCols], uint32_t n) const {
+        const i64 r0 = (u % rt) * 64, row = r0 + t.r;
+        int *rowmb = s.rowmb[n & 1];
+        if (row < a.nrows) {
+            u64 m = 0;
+#pragma unroll
+            for (int j = 0; j < kCols; ++j) m |= (u64)(v[j] ^ (v[j] >> 63));
+            atomicMax(&rowmb[t.r], bits_of(m));
+            i64 *dst = a.X + row * a.item + t.p * plane + (u / rt) * 64 + t.c0;
+#pragma unroll
+            for (int i = 0; i < kCols / 4; ++i) store4(dst + 4 * i, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
+        if (!(t.ok = wsync_and(t.ok))) return false;
+        if (t.tid < 64) {
+            if (r0 + t.tid < a.nrows) atomicMax(&a.info[r0 + t.tid].mb, rowmb[t.tid]);
+            rowmb[t.tid] = 0;
+        }
+        return true;
+    }
+};
+
 __global__ void __launch_bounds__(kThreads, 1) k_fx_assemble(const __grid_constant__ AssembleArgs a) {
     extern __shared__ unsigned char raw[];
     __shared__ Shared s;
     Thread t;
     setup(s, t, raw);
-    const i64 plane = a.item / 2;
-    const i64 rt = (a.nrows + 63) / 64, ct = plane / 64, units = rt * ct;
-    for (i64 u = blockIdx.x; u < units; u += gridDim.x) {
-        const i64 r0 = (u % rt) * 64, n0 = (u / rt) * 64;
-        if (t.tid < 64) s.rowmb[t.tid] = 0;
-        const Operand A{a.W + r0 * a.kpad, a.kpad, a.wplane, 0}, B{a.stack + n0, a.item, plane, 0};
-        i64 v[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = 0;
-        if (!product(s, t, A, B, false, a.kpad / kStageK, a.kvalid, 6 + a.lgk, v)) break;
-        const i64 row = r0 + t.r;
-        if (row < a.nrows) {
-            u64 m = 0;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) m |= (u64)(v[j] ^ (v[j] >> 63));
-            atomicMax(&s.rowmb[t.r], bits_of(m));
-            store16(a.X + row * a.item + t.p * plane + n0 + t.c0, v);
-        }
-        __syncthreads();
-        if (t.tid < 64 && r0 + t.tid < a.nrows) atomicMax(&a.info[r0 + t.tid].mb, s.rowmb[t.tid]);
-        __syncthreads();
+    const i64 plane = a.item / 2, rt = (a.nrows + 63) / 64, units = rt * (plane / 64);
+    const int nst = a.kpad / kStageK;
+    if (t.warp >= kWorkers / 32) {
+        regs_down<kRegsIssue>();
+        if (t.tid == kWorkers) t.ok = issue_products(s, t.smem, my_units(units), nst);
+    } else {
+        regs_up<kRegsWorker>();
+        AssembleWork w{a, s, t, rt, units, plane};
+        work(s, t, w, nst, a.kvalid, 6 + a.lgk);
     }
-    teardown(s, t, a.fault);
+    teardown(s, t, t.ok, a.fault);
 }
 
 // ------------------------------------------------------------------ d <= 64: whole steps in one launch
@@ -179,11 +207,11 @@ constexpr int kMaxOps = 64;
 constexpr i64 kItem64 = 2 * 64 * 64;
 
 struct StepsArgs {
-    Op op[kMaxOps];
-    int nops;
+    Op op[kMaxOps];  // a step's products, and the running product (into kBufX: its target)
+    int nops;        // without the running product
     const i64 *X;
     const Info *xinfo;
-    i64 *scratch;  // per CTA: Y, W, R0, R1, E
+    i64 *scratch;  // per chunk: Y, W, R0, R1, E
     i64 *pbuf;     // 2 x nch running products
     i64 *chunks;   // nch finished products
     Info *pinfo, *cinfo;
@@ -193,92 +221,119 @@ struct StepsArgs {
     int *fault;
 };
 
-// One product of an item held by this CTA alone: infos in shared memory.
-__device__ __forceinline__ bool run_op(Shared &s, Thread &t, const Op &op, i64 *const (&buf)[kBufs], Info *info, int d,
-                                       int nst, int lgk) {
-    const Info ia = info[op.a], ib = info[op.b];
-    const int ha = headroom(ia), hb = headroom(ib);
-    const Operand A{buf[op.a], 64, 4096, ha}, B{buf[op.b], 64, 4096, hb};
-    const int eT = ia.e - ha + ib.e - hb + lgk;
-    i64 T[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) T[j] = 0;
-    if (!product(s, t, A, B, op.imag != 0, nst, 64, 6 + lgk, T)) return false;
-    const int off = t.r * 64 + t.c0;
-#pragma unroll 1
-    for (int o = 0; o < 2; ++o) {
-        const Out &out = op.out[o];
-        if (out.buf < 0) continue;
-        View w[kTerms];
-        for (int k = 0; k < out.nterm; ++k) w[k] = View{buf[out.term[k].buf] + off, 4096, info[out.term[k].buf]};
-        bool poison = ia.mb == kPoison || ib.mb == kPoison;
-        const int e = out_exponent(out, eT, w, poison);
-        i64 v[16];
-        out_values(out, t, T, eT, e, w, t.r, t.c0, d, v);
-        store16(buf[out.buf] + t.p * 4096 + off, v);
-        const u64 m = warp_or(v);
-        if (t.lane == 0) {
-            atomicOr(&s.orhi[o], (uint32_t)(m >> 32));
-            atomicOr(&s.orlo[o], (uint32_t)m);
-        }
-        __syncthreads();
-        if (t.tid == 0) {
-            info[out.buf] = Info{e, poison ? kPoison : bits_of((u64)s.orhi[o] << 32 | s.orlo[o])};
-            s.orhi[o] = s.orlo[o] = 0;
-        }
+// A CTA walks chunks blockIdx.x and blockIdx.x + gridDim.x (if there is one)
+// step by step, product by product, the two in turn: a product's operands come
+// from the product before the last, so they are cut while the last one is read
+// and finished.  With one chunk every product waits for the one before.
+struct StepsWork {
+    struct At {
+        int i, o, k;  // step of the batch, product, chunk slot
+    };
+    const StepsArgs &a;
+    Shared &s;
+    Thread &t;
+    // Every worker writes the same exponents and lengths after a product's
+    // barrier, so each finds them without another one.
+    Info (*info)[kBufs];
+    int nk, steps;  // chunk slots, steps of the batch
+
+    __device__ __forceinline__ i64 chunk(int k) const { return blockIdx.x + k * gridDim.x; }
+    // Steps of the batch that slot k has (the first slot's chunk is not the shorter one).
+    __device__ __forceinline__ int end(int k) const { return (int)(min(a.ch.steps(chunk(k)), a.i0 + a.per) - a.i0); }
+    __device__ __forceinline__ At first() const { return At{0, 0, 0}; }
+    __device__ __forceinline__ bool more(const At &q) const { return q.i < steps; }
+    __device__ __forceinline__ At next(At q) const {
+        do {
+            if (++q.k == nk) {
+                q.k = 0;
+                if (++q.o == a.nops + (a.i0 + q.i > 0 ? 1 : 0)) {
+                    q.o = 0;
+                    ++q.i;
+                }
+            }
+        } while (q.i < steps && q.i >= end(q.k));
+        return q;
     }
-    __syncthreads();
-    return true;
-}
+    __device__ __forceinline__ bool needs(const At &q, const At &before) const { return q.k == before.k; }
+    __device__ __forceinline__ i64 *item(const At &q, int b, bool out) const {
+        const i64 c = chunk(q.k), i = a.i0 + q.i;
+        i64 *dst = i == a.ch.steps(c) - 1 ? a.chunks + c * kItem64 : a.pbuf + ((i & 1) * a.ch.nch + c) * kItem64;
+        if (b == kBufX) return out ? dst : const_cast<i64 *>(a.X) + (c * a.per + q.i) * kItem64;
+        if (b == kBufP) return a.pbuf + (((i - 1) & 1) * a.ch.nch + c) * kItem64;
+        if (b == kBufE && i == 0) return dst;
+        return a.scratch + (5 * c + b - kBufY) * kItem64;
+    }
+    __device__ __forceinline__ Info info_of(const At &q, int b) const {
+        return b == kBufX ? a.xinfo[chunk(q.k) * a.per + q.i] : info[q.k][b];
+    }
+    __device__ __forceinline__ bool operands(const At &q, Operand &A, Operand &B) const {
+        const Op &op = a.op[q.o];
+        A = Operand{item(q, op.a, false), 4, 256, 4096, headroom(info_of(q, op.a))};
+        B = Operand{item(q, op.b, false), 4, 256, 4096, headroom(info_of(q, op.b))};
+        return op.imag != 0;
+    }
+    __device__ __forceinline__ bool epilogue(const At &q, i64 (&T)[kCols], uint32_t n) const {
+        const Op &op = a.op[q.o];
+        const Info ia = info_of(q, op.a), ib = info_of(q, op.b);
+        const int eT = ia.e - headroom(ia) + ib.e - headroom(ib) + a.lgk, off = t.c0 * 64 + 4 * t.r;
+        const bool bad = ia.mb == kPoison || ib.mb == kPoison;
+        auto view = [&](int b) { return View{item(q, b, false) + off, info_of(q, b)}; };
+        int e0 = 0, e1 = 0;
+        bool p0 = bad, p1 = bad;
+#pragma unroll 1
+        for (int o = 0; o < 2; ++o) {
+            const Out &out = op.out[o];
+            if (out.buf < 0) continue;
+            bool poison = bad;
+            const int e = out_exponent(out, eT, view, poison);
+            merge_or(s, t, n, o, put_out(out, t, T, eT, e, view, 4096, 256, t.r, t.c0, a.d,
+                                         item(q, out.buf, true) + t.p * 4096 + off));
+            if (o == 0)
+                e0 = e, p0 = poison;
+            else
+                e1 = e, p1 = poison;
+        }
+        if (!(t.ok = wsync_and(t.ok))) return false;
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+            const u64 m = read_or(s, t, n, o);
+            const int b = op.out[o].buf;
+            if (b < 0) continue;
+            const Info r{o == 0 ? e0 : e1, (o == 0 ? p0 : p1) ? kPoison : bits_of(m)};
+            // The running product, or the first step's own propagator.
+            if (b == kBufX || (b == kBufE && a.i0 + q.i == 0)) info[q.k][kBufP] = r;
+            if (b != kBufX) info[q.k][b] = r;
+        }
+        return true;
+    }
+};
 
 __global__ void __launch_bounds__(kThreads, 1) k_fx_steps(const __grid_constant__ StepsArgs a) {
     extern __shared__ unsigned char raw[];
     __shared__ Shared s;
-    __shared__ Info info[kBufs];
+    __shared__ Info info[2][kBufs];
     Thread t;
-    if (threadIdx.x < 2) s.orhi[threadIdx.x] = s.orlo[threadIdx.x] = 0;
     setup(s, t, raw);
-    const int c = blockIdx.x;
-    const i64 len = a.ch.steps(c);
-    const i64 last = min(len, a.i0 + a.per);
-    i64 *scratch = a.scratch + (i64)c * 5 * kItem64;
-    i64 *buf[kBufs];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) buf[kBufY + k] = scratch + k * kItem64;
-    if (t.tid == 0 && a.i0 > 0) info[kBufP] = a.pinfo[c];
-    Op run{};
-    run.a = kBufE;
-    run.b = kBufP;
-    run.out[1].buf = -1;
-    run.out[0].buf = kBufX;  // the target's place, set below
-    run.out[0].nterm = 2;
-    const Coef one{1ll << 61, 1, 0};
-    run.out[0].t = one;
-    run.out[0].term[0] = Term{one, kBufE};
-    run.out[0].term[1] = Term{one, kBufP};
-    bool ok = true;
-    for (i64 i = a.i0; i < last && ok; ++i) {
-        const i64 xi = (i64)c * a.per + (i - a.i0);
-        i64 *dst = i == len - 1 ? a.chunks + (i64)c * kItem64 : a.pbuf + ((i & 1) * a.ch.nch + c) * kItem64;
-        buf[kBufX] = const_cast<i64 *>(a.X) + xi * kItem64;
-        buf[kBufP] = a.pbuf + (((i - 1) & 1) * a.ch.nch + c) * kItem64;
-        buf[kBufE] = i == 0 ? dst : scratch + 4 * kItem64;
-        __syncthreads();
-        if (t.tid == 0) info[kBufX] = a.xinfo[xi];
-        __syncthreads();
-        for (int o = 0; o < a.nops && ok; ++o) ok = run_op(s, t, a.op[o], buf, info, a.d, a.nst, a.lgk);
-        if (!ok) break;
-        if (i == 0) {
-            if (t.tid == 0) info[kBufP] = info[kBufE];
-        } else {
-            buf[kBufX] = dst;
-            ok = run_op(s, t, run, buf, info, a.d, a.nst, a.lgk);
-            if (t.tid == 0) info[kBufP] = info[kBufX];
-        }
+    StepsWork w{a, s, t, info, blockIdx.x + gridDim.x < a.ch.nch ? 2 : 1, 0};
+    w.steps = max(0, w.end(0));
+    if (t.warp >= kWorkers / 32) {
+        regs_down<kRegsIssue>();
+        i64 products = 0;
+        for (int k = 0; k < w.nk; ++k)
+            if (w.end(k) > 0) products += (i64)w.end(k) * (a.nops + 1) - (a.i0 == 0 ? 1 : 0);
+        if (t.tid == kWorkers) t.ok = issue_products(s, t.smem, products, a.nst);
+    } else {
+        regs_up<kRegsWorker>();
+        if (a.i0 > 0)
+            for (int k = 0; k < w.nk; ++k) info[k][kBufP] = a.pinfo[w.chunk(k)];
+        work(s, t, w, a.nst, 64, 6 + a.lgk);
+        if (t.tid == 0 && t.ok)
+            for (int k = 0; k < w.nk; ++k) {
+                const i64 c = w.chunk(k);
+                if (w.end(k) > 0) (a.i0 + w.end(k) == a.ch.steps(c) ? a.cinfo : a.pinfo)[c] = info[k][kBufP];
+            }
     }
-    __syncthreads();
-    if (t.tid == 0 && ok && last > a.i0) (last == len ? a.cinfo : a.pinfo)[c] = info[kBufP];
-    teardown(s, t, a.fault);
+    teardown(s, t, t.ok, a.fault);
 }
 
 // ------------------------------------------------------------------ d > 64 and the tree: one product of many items
@@ -296,61 +351,87 @@ struct GemmArgs {
     int *fault;
 };
 
-__global__ void __launch_bounds__(kThreads, 1) k_fx_gemm(const __grid_constant__ GemmArgs a) {
-    extern __shared__ unsigned char raw[];
-    __shared__ Shared s;
-    Thread t;
-    if (threadIdx.x < 2) s.orhi[threadIdx.x] = s.orlo[threadIdx.x] = 0;
-    setup(s, t, raw);
-    const i64 plane = (i64)a.dp * a.dp;
-    const int tiles = a.nt * a.nt;
-    const i64 units = (i64)a.items * tiles;
-    const Op &op = a.op;
-    for (i64 u = blockIdx.x; u < units; u += gridDim.x) {
+struct GemmWork {
+    using At = i64;
+    const GemmArgs &a;
+    Shared &s;
+    Thread &t;
+    int tiles;
+    i64 units, plane, qs;
+    __device__ __forceinline__ At first() const { return blockIdx.x; }
+    __device__ __forceinline__ At next(At u) const { return u + gridDim.x; }
+    __device__ __forceinline__ bool more(At u) const { return u < units; }
+    __device__ __forceinline__ bool needs(At, At) const { return false; }
+    __device__ __forceinline__ View view(int b, i64 it, i64 off) const {
+        const Buf &q = a.buf[b];
+        return View{q.ptr + it * q.stride + off, q.info[it * q.istride]};
+    }
+    __device__ __forceinline__ bool operands(At u, Operand &A, Operand &B) const {
         const i64 it = u / tiles;
         const int tile = (int)(u % tiles), I = tile / a.nt, J = tile % a.nt;
-        auto view = [&](int b, i64 off) {
-            const Buf &q = a.buf[b];
-            return View{q.ptr + it * q.stride + off, plane, q.info[it * q.istride]};
-        };
-        const View va = view(op.a, (i64)I * 64 * a.dp), vb = view(op.b, J * 64);
-        const int ha = headroom(va.info), hb = headroom(vb.info);
-        const Operand A{va.re, a.dp, plane, ha}, B{vb.re, a.dp, plane, hb};
-        const int eT = va.info.e - ha + vb.info.e - hb + a.lgk;
-        i64 T[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) T[j] = 0;
-        if (!product(s, t, A, B, op.imag != 0, a.nst, a.dp, 6 + a.lgk, T)) break;
+        const View va = view(a.op.a, it, I * 256), vb = view(a.op.b, it, (i64)J * 64 * a.dp);
+        A = Operand{va.re, 4, qs, plane, headroom(va.info)};
+        B = Operand{vb.re, 4, qs, plane, headroom(vb.info)};
+        return a.op.imag != 0;
+    }
+    __device__ __forceinline__ bool epilogue(At u, i64 (&T)[kCols], uint32_t n) const {
+        const i64 it = u / tiles;
+        const int tile = (int)(u % tiles), I = tile / a.nt, J = tile % a.nt;
+        const Op &op = a.op;
+        const Info ia = view(op.a, it, 0).info, ib = view(op.b, it, 0).info;
+        const int eT = ia.e - headroom(ia) + ib.e - headroom(ib) + a.lgk;
+        const bool bad = ia.mb == kPoison || ib.mb == kPoison;
         const int row = I * 64 + t.r, col0 = J * 64 + t.c0;
-        const i64 off = (i64)row * a.dp + col0;
+        const i64 off = (i64)col0 * a.dp + 4 * row;
+        auto at = [&](int b) { return view(b, it, off); };
+        int e0 = 0, e1 = 0;
+        bool p0 = bad, p1 = bad;
 #pragma unroll 1
         for (int o = 0; o < 2; ++o) {
             const Out &out = op.out[o];
             if (out.buf < 0) continue;
-            View w[kTerms];
-            for (int k = 0; k < out.nterm; ++k) w[k] = view(out.term[k].buf, off);
-            bool poison = va.info.mb == kPoison || vb.info.mb == kPoison;
-            const int e = out_exponent(out, eT, w, poison);
-            i64 v[16];
-            out_values(out, t, T, eT, e, w, row, col0, a.d, v);
+            bool poison = bad;
+            const int e = out_exponent(out, eT, at, poison);
             const Buf &q = a.buf[out.buf];
-            store16(q.ptr + it * q.stride + t.p * plane + off, v);
-            const u64 m = warp_or(v);
-            if (t.lane == 0) {
-                atomicOr(&s.orhi[o], (uint32_t)(m >> 32));
-                atomicOr(&s.orlo[o], (uint32_t)m);
-            }
-            __syncthreads();
-            if (t.tid == 0) {
+            merge_or(s, t, n, o, put_out(out, t, T, eT, e, at, plane, qs, row, col0, a.d,
+                                         q.ptr + it * q.stride + t.p * plane + off));
+            if (o == 0)
+                e0 = e, p0 = poison;
+            else
+                e1 = e, p1 = poison;
+        }
+        if (!(t.ok = wsync_and(t.ok))) return false;
+        if (t.tid == 0) {
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                const u64 m = read_or(s, t, n, o);
+                if (op.out[o].buf < 0) continue;
+                const Buf &q = a.buf[op.out[o].buf];
                 Info *i = &q.info[it * q.istride];
-                if (tile == 0) i->e = e;
-                atomicMax(&i->mb, poison ? kPoison : bits_of((u64)s.orhi[o] << 32 | s.orlo[o]));
-                s.orhi[o] = s.orlo[o] = 0;
+                if (tile == 0) i->e = o == 0 ? e0 : e1;
+                atomicMax(&i->mb, (o == 0 ? p0 : p1) ? kPoison : bits_of(m));
             }
         }
-        __syncthreads();
+        return true;
     }
-    teardown(s, t, a.fault);
+};
+
+__global__ void __launch_bounds__(kThreads, 1) k_fx_gemm(const __grid_constant__ GemmArgs a) {
+    extern __shared__ unsigned char raw[];
+    __shared__ Shared s;
+    Thread t;
+    setup(s, t, raw);
+    const int tiles = a.nt * a.nt;
+    const i64 units = (i64)a.items * tiles;
+    if (t.warp >= kWorkers / 32) {
+        regs_down<kRegsIssue>();
+        if (t.tid == kWorkers) t.ok = issue_products(s, t.smem, my_units(units), a.nst);
+    } else {
+        regs_up<kRegsWorker>();
+        GemmWork w{a, s, t, tiles, units, (i64)a.dp * a.dp, 4ll * a.dp};
+        work(s, t, w, a.nst, a.dp, 6 + a.lgk);
+    }
+    teardown(s, t, t.ok, a.fault);
 }
 
 // I + E as complex128, row-major d x d.
@@ -359,8 +440,8 @@ __global__ void k_fx_out(const i64 *E, const Info *info, int d, int dp, double2 
     const i64 plane = (i64)dp * dp, n = (i64)d * d;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
         const int r = (int)(i / d), c = (int)(i % d);
-        double2 v = make_double2(scalbn((double)E[(i64)r * dp + c], q.e - 62),
-                                 scalbn((double)E[plane + (i64)r * dp + c], q.e - 62));
+        const i64 k = (i64)(c >> 2) * 4 * dp + 4 * r + (c & 3);
+        double2 v = make_double2(scalbn((double)E[k], q.e - 62), scalbn((double)E[plane + k], q.e - 62));
         if (q.mb == kPoison) v.x = v.y = __longlong_as_double(0x7FF8000000000000ll);
         if (r == c) v.x += 1.0;
         out[i] = v;
@@ -540,9 +621,9 @@ static Plan make_plan(int d, int Ke, i64 P, int num_sms) {
     q.kpad = (q.kvalid + kStageK - 1) / kStageK * kStageK;
     const int tiles = q.nt * q.nt;
     if (tiles == 1) {
-        // One chunk per SM; X of up to 32 steps of every chunk at a time (320 MB).
-        q.nch = (int)std::min<i64>(num_sms, P);
-        q.per = (int)std::min<i64>(32, (P + q.nch - 1) / q.nch);
+        // Two chunks per SM; X of up to 16 steps of every chunk at a time (320 MB).
+        q.nch = (int)std::min<i64>(2ll * num_sms, P);
+        q.per = (int)std::min<i64>(16, (P + q.nch - 1) / q.nch);
     } else {
         // About eight waves of tiles per product, in rounds of equal size.
         const i64 g0 = std::min<i64>(P, std::max<i64>(1, (8ll * num_sms + tiles - 1) / tiles));
@@ -638,10 +719,10 @@ cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double 
     Info *pinfo = sinfo + (kMaxOps + 1) * (size_t)q.nch, *cinfo = pinfo + 2 * (size_t)q.nch, *tinfo = cinfo + q.nch;
     std::vector<Op> ops;
     build_program(M, x, c->hnorm, ops);
-    if ((int)ops.size() > kMaxOps) return cudaErrorInvalidValue;  // orders up to 63: 62 products
+    if ((int)ops.size() >= kMaxOps) return cudaErrorInvalidValue;  // orders up to 63: 62 products
     const WeightSpec w{wh.pts, wh.K, wh.amps, wh.mode, wh.magnus, wh.hfac};
     const i64 rpad = (q.rows + 63) / 64 * 64;
-    const int lgw = std::max(3, ceil_log2(2ll * q.kvalid)), lgk = ceil_log2(2ll * d);
+    const int lgw = std::max(4, ceil_log2(2ll * q.kvalid)), lgk = ceil_log2(2ll * d);
     const int nst = (d + kStageK - 1) / kStageK;
     auto assemble = [&](i64 i0, i64 rows, int per) -> cudaError_t {
         const Rows r{q.ch, per, i0};
@@ -654,9 +735,18 @@ cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double 
         return cudaGetLastError();
     };
     if (c->timing) cudaEventRecord(c->ev_start, st);
+    // The running product of a chunk, into kBufX of its caller: E P + E + P.
+    Op run{kBufE, kBufP, 0, {Out{}, no_out()}};
+    const Coef one = coef(1.0, 0.0);
+    run.out[0].buf = kBufX;
+    run.out[0].t = one;
+    run.out[0].nterm = 2;
+    run.out[0].term[0] = Term{one, kBufE};
+    run.out[0].term[1] = Term{one, kBufP};
     if (q.nt == 1) {
         StepsArgs a;
         for (size_t k = 0; k < ops.size(); ++k) a.op[k] = ops[k];
+        a.op[ops.size()] = run;
         a.nops = (int)ops.size();
         a.X = X;
         a.xinfo = xinfo;
@@ -674,7 +764,7 @@ cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double 
         for (i64 i0 = 0; i0 < q.ch.longest(); i0 += q.per) {
             if ((e = assemble(i0, q.rows, q.per)) != cudaSuccess) return e;
             a.i0 = i0;
-            k_fx_steps<<<q.nch, kThreads, kSmem, st>>>(a);
+            k_fx_steps<<<std::min(q.nch, c->num_sms), kThreads, kSmem, st>>>(a);
             ++launches;
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
@@ -687,13 +777,6 @@ cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double 
         a.nst = nst;
         a.lgk = lgk;
         a.fault = c->d_fault;
-        Op run{kBufE, kBufP, 0, {Out{}, no_out()}};
-        const Coef one = coef(1.0, 0.0);
-        run.out[0].buf = kBufX;
-        run.out[0].t = one;
-        run.out[0].nterm = 2;
-        run.out[0].term[0] = Term{one, kBufE};
-        run.out[0].term[1] = Term{one, kBufP};
         for (i64 i = 0; i < longest; ++i) {
             const int active = i < q.ch.len ? q.nch : q.ch.nlong;
             if ((e = assemble(i, active, 1)) != cudaSuccess) return e;
@@ -747,7 +830,6 @@ cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double 
         a.nst = nst;
         a.lgk = lgk;
         a.fault = c->d_fault;
-        const Coef one = coef(1.0, 0.0);
         a.op = Op{kBufX, kBufY, 0, {Out{}, no_out()}};
         Out &o = a.op.out[0];
         o.buf = kBufW;

@@ -15,6 +15,10 @@
 // 0x8080808080808080 turns the top seven bytes into the digits of
 //     v = sum_s q_s 2^(8 (7 - s)),  q_s in [-128, 127], |q_0| <= 64,
 // (rounded at the eighth byte): byte s minus 128, which fp16 holds exactly.
+// Four columns of a row are one 32-byte piece and the pieces of a column group
+// follow each other row by row: the epilogue's lanes (one row each) and the
+// lanes that cut operands (8 columns of a row each) both move whole lines
+// (row-major items cost 32 passes of the load pipe per access).
 //
 // Products of digits of level L = s + t <= 7 (34 of the 49) accumulate in their
 // own FP32 accumulator of tensor memory, which never rounds: over 64 complex
@@ -29,8 +33,22 @@
 //     [C_r; C_i] = [[A_r, -A_i], [A_i, A_r]] [B_r; B_i].
 // The A digits of one slice are a 128 x 32 K-major tile (64-byte swizzle), the
 // B digits a 32 x 64 MN-major tile (128-byte swizzle) so that the slices of B
-// stack along N (ozaki.cuh).  Two stages of 84 KB: the 512 threads cut stage
-// k + 1 while the tensor core multiplies stage k.
+// stack along N (ozaki.cuh).
+//
+// Eight worker warps cut, read the levels and run the epilogues; a ninth issues
+// the products (sixteen of half the columns would have 120 registers a thread and
+// spill).  They meet on mbarriers only: `full` (a stage is cut), `done` (a stage
+// is multiplied), `drained` (the levels are read).  Two stages of 84 KB: a stage
+// is cut while the one before is multiplied, and the first stage of the next
+// product, if it does not depend on this one, before this one's levels are read.
+//
+// What bounds it: a 64 x 64 x 64 product takes 19 thousand clocks inside a long
+// K and 31 thousand with its epilogue (d = 64), of which the tensor core is busy
+// 9 thousand; the rest is latency of the operands' and the terms' loads (L2) with
+// two worker warps per scheduler.  Against the first form, with row-major items,
+// one warp of the workers issuing and all of them meeting at every stage, 42
+// thousand: d = 64 Magnus, 4096 steps, 3.38 -> 2.57 ms; d = 96, 512 steps, 2.21 ->
+// 1.80 ms; d = 512, 16 steps, 4.16 -> 3.30 ms.
 #pragma once
 
 #include "ozaki.cuh"
@@ -38,7 +56,13 @@
 namespace pgb {
 namespace fx {
 
-constexpr int kThreads = 512;
+constexpr int kWorkers = 256;
+constexpr int kCols = 32;  // columns of a worker thread
+constexpr int kThreads = kWorkers + 128;  // and a warpgroup of which one warp issues
+// Registers: 168 a thread at launch (64,512 in all), then 224 for the two worker
+// warpgroups and 40 for the third (62,464).
+constexpr int kRegsWorker = 224, kRegsIssue = 40;
+static_assert(kWorkers * kRegsWorker + 128 * kRegsIssue <= kThreads * 168, "register split");
 constexpr int kSlices = 7;
 constexpr int kLevels = 8;
 constexpr int kStageK = 16;                                  // complex columns of a stage
@@ -61,21 +85,44 @@ struct Info {
 __device__ __forceinline__ int headroom(Info i) { return i.mb >= 62 ? 0 : 62 - i.mb; }
 
 struct Shared {
-    uint64_t bar[2];
+    uint64_t full[2], done[2], drained;
     uint32_t tmem_base;
-    uint32_t orhi[2], orlo[2];  // running OR of the magnitudes of an item
-    int rowmb[64];
+    uint32_t orhi[4][2], orlo[4][2];  // OR of the magnitudes of a product's results, four products in turn
+    int rowmb[2][64];                 // lengths of a tile's rows, two tiles in turn
 };
 
 // Where a thread sits: tensor-memory lane 32 (warp % 4) + lane, plane p, row r
-// of the 64 x 64 tile, columns c0 .. c0 + 15.
+// of the 64 x 64 tile, columns c0 .. c0 + 31.
 struct Thread {
     int tid, lane, warp, p, r, c0;
     uint32_t tm;      // this thread's lane and first column in tensor memory
     unsigned char *smem;
-    uint32_t ncommit[2];
-    bool ok;
+    uint32_t g;        // stages cut so far; stage g sits in buffer g % 2
+    bool ok;           // no wait gave up (then the remaining ones are skipped)
 };
+
+// Barrier of the workers, alone and with a vote.
+__device__ __forceinline__ void wsync() { asm volatile("bar.sync 1, %0;" ::"n"(kWorkers) : "memory"); }
+__device__ __forceinline__ bool wsync_and(bool p) {
+    int r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.and.pred q, 1, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((int)p), "n"(kWorkers)
+        : "memory");
+    return r != 0;
+}
+template <int N>
+__device__ __forceinline__ void regs_up() {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void regs_down() {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+__device__ __forceinline__ void arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_addr(bar)) : "memory");
+}
 
 __device__ __forceinline__ uint32_t sw64(int row, int k) {
     return (uint32_t)((row >> 3) * 512 + (row & 7) * 64 + ((((k >> 3) ^ (row >> 1)) & 3) << 4) + ((k & 7) << 1));
@@ -95,143 +142,207 @@ __host__ __device__ constexpr uint32_t idesc(int N) {
     return (1u << 4) | (1u << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
-// The MMAs of one stage (one thread).  The slices of B that a slice s of A
-// meets (t <= 7 - s) stack along N, at most four at a time; level s + t sits at
-// tensor-memory columns 64 (s + t).  `fresh` starts the levels: s = 0 starts
+// N = 64 n columns: slices t0 .. t0 + n - 1 of B against slice s of A, at
+// tensor-memory columns 64 (s + t0) on.
+__device__ __forceinline__ void issue_chain(uint32_t tmem, uint64_t da, uint64_t db, int s, int t0, int n,
+                                            uint32_t acc) {
+    const uint64_t a = da + (uint64_t)(s * (int)(kASliceB / 16)), b = db + (uint64_t)(t0 * (int)(kBSliceB / 16));
+    oz::mma_bf16(tmem + 64u * (uint32_t)(s + t0), a, b, idesc(64 * n), acc);
+    oz::mma_bf16(tmem + 64u * (uint32_t)(s + t0), a + 2, b + 128, idesc(64 * n), 1u);
+}
+
+// The MMAs of one stage (one thread): level s + t <= 7, the slices of B that a
+// slice of A meets stacked along N.  `fresh` starts the levels: s = 0 starts
 // levels 0 .. 6, the pair (1, 6) level 7.
-__device__ __forceinline__ void issue_stage(uint32_t tmem, uint32_t sa, uint32_t sb, bool fresh) {
-#pragma unroll
-    for (int s = 0; s < kSlices; ++s) {
-        const int nt = (kLevels - s) < kSlices ? kLevels - s : kSlices;
-        for (int t0 = 0; t0 < nt;) {
-            int n = nt - t0 < 4 ? nt - t0 : 4;
-            uint32_t acc = (fresh && s == 0) ? 0u : 1u;
-            if (fresh && s == 1 && t0 == 4) n = 2;
-            if (fresh && s == 1 && t0 == 6) acc = 0u;
-            const uint32_t d = tmem + 64u * (uint32_t)(s + t0), id = idesc(64 * n);
-            const uint32_t a = sa + (uint32_t)s * kASliceB, b = sb + (uint32_t)t0 * kBSliceB;
-            oz::mma_bf16(d, desc_k_sw64(a), oz::desc_mn_sw128(b, kBSliceB), id, acc);
-            oz::mma_bf16(d, desc_k_sw64(a + 32), oz::desc_mn_sw128(b + 2048, kBSliceB), id, 1u);
-            t0 += n;
+template <bool FRESH>
+__device__ __forceinline__ void issue_stage(uint32_t tmem, uint64_t da, uint64_t db) {
+    issue_chain(tmem, da, db, 0, 0, 4, FRESH ? 0u : 1u);
+    issue_chain(tmem, da, db, 0, 4, 3, FRESH ? 0u : 1u);
+    issue_chain(tmem, da, db, 1, 0, 4, 1u);
+    if (FRESH) {
+        issue_chain(tmem, da, db, 1, 4, 2, 1u);
+        issue_chain(tmem, da, db, 1, 6, 1, 0u);
+    } else {
+        issue_chain(tmem, da, db, 1, 4, 3, 1u);
+    }
+    issue_chain(tmem, da, db, 2, 0, 3, 1u);
+    issue_chain(tmem, da, db, 2, 3, 3, 1u);
+    issue_chain(tmem, da, db, 3, 0, 3, 1u);
+    issue_chain(tmem, da, db, 3, 3, 2, 1u);
+    issue_chain(tmem, da, db, 4, 0, 4, 1u);
+    issue_chain(tmem, da, db, 5, 0, 3, 1u);
+    issue_chain(tmem, da, db, 6, 0, 2, 1u);
+}
+
+// The issuing warp: `products` products of nst stages each.  Returns whether
+// every wait ended.
+__device__ __forceinline__ bool issue_products(Shared &s, const unsigned char *smem, i64 products, int nst) {
+    const uint32_t base = tc::smem_addr(smem);
+    uint32_t g = 0, drains = 0;
+    for (i64 k = 0; k < products; ++k)
+        for (int st = 0; st < nst; ++st, ++g) {
+            const uint32_t b = g & 1;
+            const bool fresh = (st & (kGroup - 1)) == 0;
+            bool ok = tc::mbar_wait(&s.full[b], (g >> 1) & 1, kWait);
+            if (fresh) {
+                ok = ok && (drains == 0 || tc::mbar_wait(&s.drained, (drains - 1) & 1, kWait));
+                ++drains;
+            }
+            if (!ok) {
+                // What was issued finishes before tensor memory is freed.
+                if (g > 0) tc::mbar_wait(&s.done[(g - 1) & 1], ((g - 1) >> 1) & 1, kWait);
+                return false;
+            }
+            tc::fence_after_sync();
+            const uint64_t da = desc_k_sw64(base + b * kStageB);
+            const uint64_t db = oz::desc_mn_sw128(base + b * kStageB + kSlices * kASliceB, kBSliceB);
+            if (fresh)
+                issue_stage<true>(s.tmem_base, da, db);
+            else
+                issue_stage<false>(s.tmem_base, da, db);
+            tc::mma_commit(&s.done[b]);
         }
-    }
+    // The last stages finish before tensor memory is freed.
+    if (g > 0 && !tc::mbar_wait(&s.done[(g - 1) & 1], ((g - 1) >> 1) & 1, kWait)) return false;
+    return true;
 }
 
-// Eight 64-bit values from 32-byte aligned memory.
-__device__ __forceinline__ void load8(const i64 *p, i64 (&v)[8]) {
-    const longlong2 *q = reinterpret_cast<const longlong2 *>(p);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const longlong2 x = q[i];
-        v[2 * i] = x.x;
-        v[2 * i + 1] = x.y;
-    }
+// Four 64-bit values of a 32-byte piece.
+__device__ __forceinline__ void load4(const i64 *p, i64 &a, i64 &b, i64 &c, i64 &d) {
+    asm volatile("ld.global.v4.b64 {%0,%1,%2,%3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p) : "memory");
 }
-
-// Digit s of eight shifted values as fp16: byte 7 - s minus 128, two at a time
-// (0x6400 | byte is 1024 + byte in fp16).
-template <int S>
-__device__ __forceinline__ uint4 digits8(const u64 (&u)[8]) {
-    constexpr uint32_t by = S < 4 ? 3 - S : 7 - S;
-    uint32_t w[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint32_t x = (uint32_t)(S < 4 ? u[2 * i] >> 32 : u[2 * i]);
-        const uint32_t y = (uint32_t)(S < 4 ? u[2 * i + 1] >> 32 : u[2 * i + 1]);
-        const uint32_t b = (__byte_perm(x, y, by | (4 + by) << 8) & 0x00FF00FFu) | 0x64006400u;
-        asm("sub.f16x2 %0, %1, %2;" : "=r"(w[i]) : "r"(b), "r"(0x64806480u));
-    }
-    return make_uint4(w[0], w[1], w[2], w[3]);
+__device__ __forceinline__ void store4(i64 *p, i64 a, i64 b, i64 c, i64 d) {
+    asm volatile("st.global.v4.b64 [%0], {%1,%2,%3,%4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
 }
 
 // One operand of a product: element (row, col) of plane p at
-// ptr + p * plane + row * ld + col, normalised by `shift` bits.
+// ptr + p * plane + row * rs + (col / 4) * qs + col % 4, normalised by `shift`
+// bits.
 struct Operand {
     const i64 *ptr;
-    i64 ld, plane;
+    i64 rs, qs, plane;
     int shift;
 };
 
-// A thread's share of the cutting: eight columns of one row and plane, of A
-// (threads 0 .. 255; the row of a lane is laid out so that the eight lanes of
-// a store phase meet eight different 16-byte banks) or of B (threads 256 ..
-// 511; rows k of the stage).
+// A thread's share of the cutting: eight columns of one row and plane of A (the
+// row of a lane is laid out so that the eight lanes of a store phase meet eight
+// different 16-byte banks) and of B (rows k of the stage).
 struct Cut {
-    const i64 *src;   // stage 0
-    i64 step;         // elements from one stage to the next
-    int k, shift;     // B: row within the stage
-    uint32_t o0, o1;  // byte offsets within a slice (A: the two copies)
-    bool isA, n0, n1;  // A: the copies that are negated
+    const i64 *a, *b;    // stage 0
+    i64 aqs, bqs, brs;   // from one piece to the next; from one row of B to the next
+    int k, ash, bsh;     // B: row within the stage; shifts
+    uint32_t o0, o1, ob;  // byte offsets within a slice (A: the two copies)
+    bool n0, n1;         // A: the copies that are negated
 };
 
 // With `imag` the operand is i A: the product is i A B.
 __device__ __forceinline__ Cut make_cut(const Thread &t, const Operand &A, const Operand &B, bool imag) {
     Cut c;
-    c.isA = t.tid < 256;
-    if (c.isA) {
-        const int l = t.lane, w = t.warp, p = w >> 2;
-        const int row = ((l >> 1) & 1) | ((l >> 2) & 2) | (l & 4) | ((l >> 1) & 8) | ((w & 3) << 4);
-        const int k = 8 * (l & 1);
-        c.src = A.ptr + p * A.plane + row * A.ld + k;
-        c.step = kStageK;
-        c.k = 0;
-        c.shift = A.shift;
-        // A_r: [A_r | .] of the real rows and [. | A_r] of the imaginary rows;
-        // A_i: [A_i | .] of the imaginary rows and [. | -A_i] of the real rows.
-        // (i A: the parts -A_i and A_r in their places.)
-        const int q = imag ? 1 - p : p;
-        c.o0 = sw64(q ? 64 + row : row, k);
-        c.o1 = sw64(q ? row : 64 + row, kStageK + k);
-        c.n0 = imag && p != 0;
-        c.n1 = imag || p != 0;
-    } else {
-        const int w = t.warp - 8, p = w >> 2;
-        c.k = ((w & 3) << 2) | (t.lane >> 3);
-        const int col = 8 * (t.lane & 7);
-        c.src = B.ptr + p * B.plane + c.k * B.ld + col;
-        c.step = kStageK * B.ld;
-        c.shift = B.shift;
-        c.o0 = kSlices * kASliceB + oz::sw(kStageK * p + c.k, col);
-        c.o1 = 0;
-        c.n0 = c.n1 = false;
-    }
+    const int l = t.lane, w = t.warp, p = w >> 2;
+    const int row = ((l >> 1) & 1) | ((l >> 2) & 2) | (l & 4) | ((l >> 1) & 8) | ((w & 3) << 4);
+    const int k = 8 * (l & 1);
+    c.a = A.ptr + p * A.plane + row * A.rs + (k / 4) * A.qs;
+    c.aqs = A.qs;
+    c.ash = A.shift;
+    // A_r: [A_r | .] of the real rows and [. | A_r] of the imaginary rows;
+    // A_i: [A_i | .] of the imaginary rows and [. | -A_i] of the real rows.
+    // (i A: the parts -A_i and A_r in their places.)
+    const int q = imag ? 1 - p : p;
+    c.o0 = sw64(q ? 64 + row : row, k);
+    c.o1 = sw64(q ? row : 64 + row, kStageK + k);
+    c.n0 = imag && p != 0;
+    c.n1 = imag || p != 0;
+    c.k = ((w & 3) << 2) | (l >> 3);
+    const int col = 8 * (l & 7);
+    c.b = B.ptr + p * B.plane + c.k * B.rs + (col / 4) * B.qs;
+    c.bqs = B.qs;
+    c.brs = B.rs;
+    c.bsh = B.shift;
+    c.ob = kSlices * kASliceB + oz::sw(kStageK * p + c.k, col);
     return c;
 }
 
 // Values of stage st; rows of B from kvalid on are zero.
-__device__ __forceinline__ void cut_load(const Cut &c, int st, int kvalid, i64 (&v)[8]) {
-    if (c.isA || st * kStageK + c.k < kvalid) {
-        load8(c.src + st * c.step, v);
+__device__ __forceinline__ void load_a(const Cut &c, int st, i64 (&v)[8]) {
+    const i64 *p = c.a + (i64)st * (kStageK / 4) * c.aqs;
+    load4(p, v[0], v[1], v[2], v[3]);
+    load4(p + c.aqs, v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ void load_b(const Cut &c, int st, int kvalid, i64 (&v)[8]) {
+    if (st * kStageK + c.k < kvalid) {
+        const i64 *p = c.b + (i64)st * kStageK * c.brs;
+        load4(p, v[0], v[1], v[2], v[3]);
+        load4(p + c.bqs, v[4], v[5], v[6], v[7]);
     } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = 0;
     }
 }
 
-template <int S>
-__device__ __forceinline__ void cut_store_slice(const Cut &c, unsigned char *stage, const u64 (&u)[8]) {
-    const uint4 q = digits8<S>(u);
-    if (c.isA) {
-        unsigned char *b = stage + S * kASliceB;
-        const uint4 m = oz::neg8(q);
-        *reinterpret_cast<uint4 *>(b + c.o0) = c.n0 ? m : q;
-        *reinterpret_cast<uint4 *>(b + c.o1) = c.n1 ? m : q;
+// One slice (16 bytes: eight digits) from words that hold the digits of a pair
+// of values in bytes 0 and 2 (LOW) or 1 and 3.  0x6400 | byte is 1024 + byte in
+// fp16; 1152 less is the digit.
+template <bool ISA, int S, bool LOW>
+__device__ __forceinline__ void cut_slice(const Cut &c, unsigned char *stage, const uint32_t (&z)[4]) {
+    uint32_t b[4], q[4], m[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        b[i] = LOW ? (z[i] & 0x00FF00FFu) | 0x64006400u : __byte_perm(z[i], 0x64646464u, 0x4341);
+        asm("sub.f16x2 %0, %1, %2;" : "=r"(q[i]) : "r"(b[i]), "r"(0x64806480u));
+    }
+    const uint4 v = make_uint4(q[0], q[1], q[2], q[3]);
+    if (ISA) {
+        unsigned char *base = stage + S * kASliceB;
+        if (c.n1) {  // (n0 only with n1)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) asm("sub.f16x2 %0, %1, %2;" : "=r"(m[i]) : "r"(0x64806480u), "r"(b[i]));
+            const uint4 n = make_uint4(m[0], m[1], m[2], m[3]);
+            *reinterpret_cast<uint4 *>(base + c.o0) = c.n0 ? n : v;
+            *reinterpret_cast<uint4 *>(base + c.o1) = n;
+        } else {
+            *reinterpret_cast<uint4 *>(base + c.o0) = v;
+            *reinterpret_cast<uint4 *>(base + c.o1) = v;
+        }
     } else {
-        *reinterpret_cast<uint4 *>(stage + S * kBSliceB + c.o0) = q;
+        *reinterpret_cast<uint4 *>(stage + S * kBSliceB + c.ob) = v;
     }
 }
 
-__device__ __forceinline__ void cut_store(const Cut &c, unsigned char *stage, const i64 (&v)[8]) {
-    u64 u[8];
+// Digits of eight values into the stage's slices.  The shift and the digit bias
+// are multiply-adds (the integer pipe for logic and shifts is the busier one);
+// the bytes of a pair of values come together in four words.
+template <bool ISA>
+__device__ __forceinline__ void cut_store(const Cut &c, unsigned char *stage, i64 (&v)[8]) {
+    int h = ISA ? c.ash : c.bsh;
+    if (h >= 32) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) u[j] = ((u64)v[j] << c.shift) + 0x8080808080808080ull;
-    cut_store_slice<0>(c, stage, u);
-    cut_store_slice<1>(c, stage, u);
-    cut_store_slice<2>(c, stage, u);
-    cut_store_slice<3>(c, stage, u);
-    cut_store_slice<4>(c, stage, u);
-    cut_store_slice<5>(c, stage, u);
-    cut_store_slice<6>(c, stage, u);
+        for (int j = 0; j < 8; ++j) v[j] = (i64)((u64)v[j] << 32);
+        h -= 32;
+    }
+    const uint32_t mul = 1u << h;
+    uint32_t z[4][4];  // [bytes 0-1, 2-3 of the low words, of the high words][pair]
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        uint32_t lo[2], hi[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const u64 x = (u64)v[2 * i + k];
+            const u64 w = (u64)(uint32_t)x * mul + 0x8080808080808080ull;
+            lo[k] = (uint32_t)w;
+            hi[k] = (uint32_t)(w >> 32) + (uint32_t)(x >> 32) * mul;
+        }
+        z[0][i] = __byte_perm(lo[0], lo[1], 0x5410);
+        z[1][i] = __byte_perm(lo[0], lo[1], 0x7632);
+        z[2][i] = __byte_perm(hi[0], hi[1], 0x5410);
+        z[3][i] = __byte_perm(hi[0], hi[1], 0x7632);
+    }
+    cut_slice<ISA, 0, false>(c, stage, z[3]);
+    cut_slice<ISA, 1, true>(c, stage, z[3]);
+    cut_slice<ISA, 2, false>(c, stage, z[2]);
+    cut_slice<ISA, 3, true>(c, stage, z[2]);
+    cut_slice<ISA, 4, false>(c, stage, z[1]);
+    cut_slice<ISA, 5, true>(c, stage, z[1]);
+    cut_slice<ISA, 6, false>(c, stage, z[0]);
 }
 
 __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
@@ -245,69 +356,102 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
 }
 
 // An integer of magnitude up to 2^22 held in a float, plus 0x4B400000: one add.
-__device__ __forceinline__ int biased_int(float f) { return __float_as_int(__fadd_rn(f, 12582912.0f)); }
+constexpr uint32_t kIntBias = 0x4B400000u;
+__device__ __forceinline__ uint32_t biased_int(float f) { return __float_as_uint(__fadd_rn(f, 12582912.0f)); }
 
-// Adds sum_L D_L 2^(8 (7 - L)) shifted right by `sh` (9 .. 32, rounded) to the
-// thread's 16 sums.  Levels 0 .. 2 stay within 2^22; the others are converted.
-__device__ __forceinline__ void drain(const Thread &t, int sh, i64 (&acc)[16]) {
-    const int shl = 32 - sh;  // of the high part (levels 0 .. 3, units of 2^32)
-    const int sl = sh - 8;    // of the low part (units of 2^8)
-    const i64 half = 1ll << (sl - 1);
+// Adds sum_L D_L 2^(8 (7 - L)) shifted right by `sh` (10 .. 24) to the thread's
+// 16 sums, every level as an integer times a power of two.  Levels 0 .. 2 stay
+// within 2^22 and convert by an addition, 3 .. 5 by the conversion unit; levels
+// 6 and 7 join in FP32 (their sum is below the last kept bit by then).
+__device__ __forceinline__ void drain(const Thread &t, int sh, i64 (&acc)[kCols]) {
+    const uint32_t m3 = 1u << (32 - sh);                  // level 3 (2^32)
+    const int m4 = 1 << (24 - sh);                        // level 4 (2^24)
+    const int m5 = sh <= 16 ? 1 << (16 - sh) : 0, r5 = sh <= 16 ? 0 : sh - 16;  // level 5 (2^16)
+    const int half5 = r5 ? 1 << (r5 - 1) : 0;
+    const float f6 = __int_as_float((127 + 8 - sh) << 23);  // levels 6, 7: 2^(8 - sh)
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
+    for (int g = 0; g < kCols / 4; ++g) {
         float f[kLevels][4];
 #pragma unroll
         for (int L = 0; L < kLevels; ++L) tmem_ld4(t.tm + 64u * L + 4u * g, f[L]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            constexpr uint32_t B = 0x4B400000u;
-            const int h01 = (int)((uint32_t)biased_int(f[0][j]) * 256u + (uint32_t)biased_int(f[1][j]) - 257u * B);
-            const int h23 = (int)((uint32_t)biased_int(f[2][j]) * 256u - 256u * B) + __float2int_rn(f[3][j]);
-            const i64 hi = (i64)h01 * 65536 + h23;
-            const int l67 = __float2int_rn(f[6][j]) + ((__float2int_rn(f[7][j]) + 128) >> 8);
-            const i64 lo = (i64)__float2int_rn(f[4][j]) * 65536 + (i64)__float2int_rn(f[5][j]) * 256 + l67;
-            acc[4 * g + j] += (hi << shl) + ((lo + half) >> sl);
+            const int h01 = (int)(biased_int(f[0][j]) * 256u + biased_int(f[1][j]) - 257u * kIntBias);
+            const int h23 = (int)(biased_int(f[2][j]) * 256u - 256u * kIntBias) + __float2int_rn(f[3][j]);
+            const float l67 = __fmaf_rn(f[7][j], 0.00390625f, f[6][j]);
+            const int l = (int)(__float_as_uint(__fmaf_rn(l67, f6, 12582912.0f)) - kIntBias);
+            const int i5 = __float2int_rn(f[5][j]);
+            i64 v = (i64)__float2int_rn(f[4][j]) * m4 + acc[4 * g + j];
+            v += r5 ? (i64)(((i5 + half5) >> r5) + l) : (i64)i5 * m5 + l;
+            acc[4 * g + j] = (i64)((u64)((i64)h01 * 65536 + h23) * (u64)m3 + (u64)v);
         }
     }
 }
 
-// acc += A B 2^-sh (i A B with `imag`) over nst stages.  Every thread of the CTA calls it; returns
-// false (in every thread) if a wait gave up.  Ends with all MMAs complete and
-// all levels read, but no barrier.
-__device__ __forceinline__ bool product(Shared &s, Thread &t, const Operand &A, const Operand &B, bool imag, int nst,
-                                        int kvalid, int sh, i64 (&acc)[16]) {
-    const Cut c = make_cut(t, A, B, imag);
-    i64 v[8];
-    cut_load(c, 0, kvalid, v);
-    cut_store(c, t.smem, v);
-    if (nst > 1) cut_load(c, 1, kvalid, v);
-    for (int st = 0; st < nst; ++st) {
-        const int b = st & 1;
-        tc::fence_proxy_async();
-        tc::fence_before_sync();
-        const bool all = __syncthreads_and(t.ok) != 0;
-        tc::fence_after_sync();
-        if (!all) return false;
-        if (t.tid == 0) {
-            const uint32_t sa = tc::smem_addr(t.smem + b * kStageB);
-            issue_stage(s.tmem_base, sa, sa + kSlices * kASliceB, (st & (kGroup - 1)) == 0);
-            tc::mma_commit(&s.bar[b]);
+// Cuts stage st into the next buffer once that has been multiplied.  The loads
+// come first; they and the cutting fit under the stage being multiplied.
+__device__ __forceinline__ void cut_stage(Shared &s, Thread &t, const Cut &c, int st, int kvalid) {
+    const uint32_t b = t.g & 1;
+    i64 va[8], vb[8];
+    load_a(c, st, va);
+    load_b(c, st, kvalid, vb);
+    if (t.g >= 2 && t.ok) t.ok = tc::mbar_wait(&s.done[b], ((t.g >> 1) - 1) & 1, kWait);
+    cut_store<true>(c, t.smem + b * kStageB, va);
+    cut_store<false>(c, t.smem + b * kStageB, vb);
+    tc::fence_proxy_async();
+    __syncwarp();
+    if (t.lane == 0) arrive(&s.full[b]);
+    ++t.g;
+}
+
+// The workers' loop over the products of `w` (one copy of each part: the code of
+// a launch with one product per CTA has to come from L2 first).  `w` deals out
+// products (at, more, next), gives their operands, says whether one needs the
+// result of the product just before, and takes the sums (epilogue; false ends).
+// Stages are cut one ahead of those read, across products where that is allowed.
+template <class W>
+__device__ __forceinline__ void work(Shared &s, Thread &t, W &w, int nst, int kvalid, int sh) {
+    typename W::At cur = w.first(), ahead = cur;
+    Cut c;
+    int sc = 0, sa = 0;    // stage read, stage cut
+    uint32_t read = 0, n = 0;
+    i64 T[kCols];
+#pragma unroll
+    for (int j = 0; j < kCols; ++j) T[j] = 0;
+    while (w.more(cur)) {
+        while (t.g <= read + 1 && w.more(ahead)) {
+            if (sa == 0) {
+                if (t.g > read && w.needs(ahead, cur)) break;
+                Operand A, B;
+                const bool imag = w.operands(ahead, A, B);
+                c = make_cut(t, A, B, imag);
+            }
+            cut_stage(s, t, c, sa, kvalid);
+            if (++sa == nst) {
+                sa = 0;
+                ahead = w.next(ahead);
+            }
         }
-        ++t.ncommit[b];
-        if (st + 1 < nst) {
-            // The other buffer is free once stage st - 1 has been multiplied.
-            if (st > 0) t.ok = tc::mbar_wait(&s.bar[b ^ 1], (t.ncommit[b ^ 1] - 1) & 1, kWait);
-            cut_store(c, t.smem + (b ^ 1) * kStageB, v);
-            if (st + 2 < nst) cut_load(c, st + 2, kvalid, v);
-        }
-        if ((st & (kGroup - 1)) == kGroup - 1 || st + 1 == nst) {
-            t.ok = tc::mbar_wait(&s.bar[b], (t.ncommit[b] - 1) & 1, kWait) && t.ok;
+        const bool end = sc + 1 == nst;
+        if (end || (sc & (kGroup - 1)) == kGroup - 1) {
+            if (t.ok) t.ok = tc::mbar_wait(&s.done[read & 1], (read >> 1) & 1, kWait);
             tc::fence_after_sync();
-            drain(t, sh, acc);
+            drain(t, sh, T);
+            tc::fence_before_sync();
+            __syncwarp();
+            if (t.lane == 0) arrive(&s.drained);
+        }
+        ++read;
+        ++sc;
+        if (end) {
+            if (!w.epilogue(cur, T, n++)) break;
+#pragma unroll
+            for (int j = 0; j < kCols; ++j) T[j] = 0;
+            sc = 0;
+            cur = w.next(cur);
         }
     }
-    return true;
 }
 
 // ------------------------------------------------------------------ epilogue
@@ -338,26 +482,21 @@ struct Op {
     Out out[2];
 };
 
-// An item as the epilogue sees it: this thread's row of the tile.
+// An item as the epilogue sees it: this thread's row and first column.
 struct View {
     const i64 *re;  // plane 0; plane 1 at + plane
-    i64 plane;
     Info info;
 };
 
-__device__ __forceinline__ void st4(i64 *p, i64 a, i64 b, i64 c, i64 d) {
-    asm volatile("st.global.v4.b64 [%0], {%1,%2,%3,%4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
-}
-
 // Exponent of a result: two above the largest of up to four addends.
-__device__ __forceinline__ int out_exponent(const Out &o, int eT, const View *views, bool &poison) {
+template <class V>
+__device__ __forceinline__ int out_exponent(const Out &o, int eT, V view, bool &poison) {
     if (o.plain) return eT;
     int e = -1000000;
     if (o.t.m) e = eT + o.t.e;
-#pragma unroll
-    for (int k = 0; k < kTerms; ++k) {
-        if (k >= o.nterm) break;
-        const Info i = views[k].info;
+#pragma unroll 1
+    for (int k = 0; k < o.nterm; ++k) {
+        const Info i = view(o.term[k].buf).info;
         if (i.mb == kPoison) poison = true;
         e = max(e, i.e - headroom(i) + o.term[k].c.e);
     }
@@ -365,59 +504,103 @@ __device__ __forceinline__ int out_exponent(const Out &o, int eT, const View *vi
     return e + 2;
 }
 
-// The result's values for this thread (16 columns of its row and plane).
-// r, c0: global row and first column; diagonal entries below d only.
-__device__ __forceinline__ void out_values(const Out &o, const Thread &t, const i64 (&T)[16], int eT, int e,
-                                           const View *views, int row, int col0, int d, i64 (&v)[16]) {
-    if (o.plain) {
+// A coefficient and the shift that its product needs, as one factor: the upper
+// half of v * factor is the term in the result's units.  The upper and lower
+// words of the factor are signed.
+struct Factor {
+    int hi, lo, pre;  // pre: left shift of v first (a short item meets a large result)
+};
+__device__ __forceinline__ Factor make_factor(i64 m, int sr, int headroom) {
+    const int s = min(sr, 63) - headroom;
+    Factor f;
+    f.pre = s < 0 ? -s : 0;
+    if (s > 0) m = ((m >> (s - 1)) + 1) >> 1;
+    f.lo = (int)(uint32_t)(u64)m;
+    f.hi = (int)((m - f.lo) >> 32);
+    return f;
+}
+// v * factor / 2^64, rounded (the product of the low words is left out, a
+// quarter of a unit at most).  Rounding down instead would add the same sign to
+// every element at every step.
+__device__ __forceinline__ i64 scaled(i64 v, const Factor &f) {
+    const int lo = (int)(uint32_t)(u64)v;
+    const int hi = (int)(v >> 32) + (int)((uint32_t)lo >> 31);  // with the low word read as signed
+    const i64 mid = (i64)lo * f.hi + ((i64)hi * f.lo + 0x80000000ll);
+    return (i64)hi * f.hi + (int)(mid >> 32);
+}
+
+// One result, for this thread's columns of its row and plane: formed in place
+// of T, stored at dst (pieces qs apart, as those of the terms); returns the OR of
+// the magnitudes (ones' complement for negative values).  row, col0: global row
+// and first column; diagonal entries below d only.  The loads of a term go out
+// together: one wait per term, not one per piece.
+template <class V>
+__device__ __forceinline__ u64 put_out(const Out &o, const Thread &t, i64 (&T)[kCols], int eT, int e, V view,
+                                       i64 plane, i64 qs, int row, int col0, int d, i64 *dst) {
+    if (!o.plain) {
+        // T times its coefficient, then the terms; the first term's loads go
+        // out before the multiplication.
+        const Factor ft = o.t.m ? make_factor(o.t.m, e - eT - o.t.e - 2, 0) : Factor{0, 0, 0};
+#pragma unroll 1
+        for (int k = 0; k < max(1, o.nterm); ++k) {
+            i64 x[kCols];
+            Factor f{0, 0, 0};
+            if (k < o.nterm) {
+                const View w = view(o.term[k].buf);
+                const Coef c = o.term[k].c;
+                const i64 *q = w.re + (c.imag ? 1 - t.p : t.p) * plane;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = T[j];
-        return;
-    }
-    if (o.t.m) {
-        const int sr = min(e - eT - o.t.e - 2, 63);
+                for (int i = 0; i < kCols / 4; ++i)
+                    load4(q + i * qs, x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+                const int hr = headroom(w.info);
+                f = make_factor((c.imag && t.p == 0) ? -c.m : c.m, e - (w.info.e - hr) - c.e - 2, hr);
+            } else {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = __mul64hi(T[j], o.t.m) >> sr;
-    } else {
+                for (int j = 0; j < kCols; ++j) x[j] = 0;
+            }
+            if (k == 0) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = 0;
-    }
-    for (int k = 0; k < o.nterm; ++k) {
-        const View &w = views[k];
-        const Coef c = o.term[k].c;
-        const int hr = headroom(w.info);
-        const int sr = min(e - (w.info.e - hr) - c.e - 2, 63);
-        const int p = c.imag ? 1 - t.p : t.p;
-        const i64 m = (c.imag && t.p == 0) ? -c.m : c.m;
-        const longlong2 *q = reinterpret_cast<const longlong2 *>(w.re + p * w.plane);
+                for (int j = 0; j < kCols; ++j) T[j] = scaled(T[j], ft);
+            }
+            if (f.pre) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const longlong2 x = q[i];
-            v[2 * i] += __mul64hi((i64)((u64)x.x << hr), m) >> sr;
-            v[2 * i + 1] += __mul64hi((i64)((u64)x.y << hr), m) >> sr;
+                for (int j = 0; j < kCols; ++j) x[j] = (i64)((u64)x[j] << f.pre);
+            }
+#pragma unroll
+            for (int j = 0; j < kCols; ++j) T[j] += scaled(x[j], f);
+        }
+        if (o.diag.m && t.p == o.diag.imag && row < d && row >= col0 && row < col0 + kCols) {
+            const i64 x = o.diag.m >> min(e - o.diag.e, 63);
+#pragma unroll
+            for (int j = 0; j < kCols; ++j)
+                if (row == col0 + j) T[j] += x;
         }
     }
-    if (o.diag.m && t.p == o.diag.imag && row < d && row >= col0 && row < col0 + 16) {
-        const i64 x = o.diag.m >> min(e - o.diag.e, 63);
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-            if (row == col0 + j) v[j] += x;
-    }
-}
-
-__device__ __forceinline__ void store16(i64 *dst, const i64 (&v)[16]) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) st4(dst + 4 * i, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-}
-
-// OR of the magnitudes (ones' complement for negative values) over the warp.
-__device__ __forceinline__ u64 warp_or(const i64 (&v)[16]) {
     u64 m = 0;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) m |= (u64)(v[j] ^ (v[j] >> 63));
+    for (int i = 0; i < kCols / 4; ++i) {
+        store4(dst + i * qs, T[4 * i], T[4 * i + 1], T[4 * i + 2], T[4 * i + 3]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) m |= (u64)(T[4 * i + j] ^ (T[4 * i + j] >> 63));
+    }
+    return m;
+}
+
+// OR over the warp into the workers' OR of result o of product n.
+__device__ __forceinline__ void merge_or(Shared &s, const Thread &t, uint32_t n, int o, u64 m) {
     const uint32_t hi = __reduce_or_sync(0xffffffffu, (uint32_t)(m >> 32));
     const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)m);
-    return (u64)hi << 32 | lo;
+    if (t.lane == 0) {
+        atomicOr(&s.orhi[n & 3][o], hi);
+        atomicOr(&s.orlo[n & 3][o], lo);
+    }
+}
+// After the workers' barrier of product n: its result o; clears the place of
+// product n - 1, which every worker has read by then and none fills before n + 3.
+__device__ __forceinline__ u64 read_or(Shared &s, const Thread &t, uint32_t n, int o) {
+    const u64 m = (u64)s.orhi[n & 3][o] << 32 | s.orlo[n & 3][o];
+    if (t.tid == 0) s.orhi[(n - 1) & 3][o] = s.orlo[(n - 1) & 3][o] = 0;
+    return m;
 }
 
 __device__ __forceinline__ int bits_of(u64 m) { return 64 - __clzll((i64)m); }
@@ -430,17 +613,22 @@ __device__ __forceinline__ void setup(Shared &s, Thread &t, unsigned char *raw) 
     const int q4 = t.warp & 3;
     t.p = q4 >> 1;
     t.r = 32 * (q4 & 1) + t.lane;
-    t.c0 = 16 * (t.warp >> 2);
+    t.c0 = kCols * (t.warp >> 2);
     t.smem = raw + ((1024u - (tc::smem_addr(raw) & 1023u)) & 1023u);
-    t.ncommit[0] = t.ncommit[1] = 0;
+    t.g = 0;
     t.ok = true;
+    if (t.tid < 8) s.orhi[t.tid >> 1][t.tid & 1] = s.orlo[t.tid >> 1][t.tid & 1] = 0;
+    if (t.tid < 128) s.rowmb[t.tid >> 6][t.tid & 63] = 0;
     if (t.warp == 0) {
         tc::tmem_alloc(&s.tmem_base, 512);
         tc::tmem_relinquish();
     }
     if (t.tid == 0) {
-        tc::mbar_init(&s.bar[0], 1);
-        tc::mbar_init(&s.bar[1], 1);
+        for (int b = 0; b < 2; ++b) {
+            tc::mbar_init(&s.full[b], kWorkers / 32);
+            tc::mbar_init(&s.done[b], 1);
+        }
+        tc::mbar_init(&s.drained, kWorkers / 32);
         tc::fence_mbar_init();
     }
     tc::fence_before_sync();
@@ -449,16 +637,11 @@ __device__ __forceinline__ void setup(Shared &s, Thread &t, unsigned char *raw) 
     t.tm = s.tmem_base + ((uint32_t)(32 * q4) << 16) + (uint32_t)t.c0;
 }
 
-__device__ __forceinline__ void teardown(Shared &s, Thread &t, int *fault) {
-    const bool ok = __syncthreads_and(t.ok) != 0;
-    if (!ok) {
-        if (t.tid == 0 && fault) atomicAdd(fault, 1);
-        // Products still in flight finish before tensor memory is freed.
-        for (int b = 0; b < 2; ++b)
-            if (t.ncommit[b] > 0) tc::mbar_wait(&s.bar[b], (t.ncommit[b] - 1) & 1, kWait);
-    }
+// The CTA's end; ok: this thread's waits all ended.
+__device__ __forceinline__ void teardown(Shared &s, const Thread &t, bool ok, int *fault) {
     tc::fence_before_sync();
-    __syncthreads();
+    const bool all = __syncthreads_and(ok) != 0;
+    if (!all && t.tid == 0 && fault) atomicAdd(fault, 1);
     if (t.warp == 0) {
         tc::fence_after_sync();
         tc::tmem_dealloc(s.tmem_base, 512);
