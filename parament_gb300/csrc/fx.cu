@@ -173,7 +173,7 @@ struct AssembleWork {
 #pragma unroll
             for (int i = 0; i < kCols / 4; ++i) store4(dst + 4 * i, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
         }
-        if (!(t.ok = wsync_and(t.ok))) return false;
+        if (!(t.ok = fsync_and(t.ok))) return false;
         if (t.tid < 64) {
             if (r0 + t.tid < a.nrows) atomicMax(&a.info[r0 + t.tid].mb, rowmb[t.tid]);
             rowmb[t.tid] = 0;
@@ -189,14 +189,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_fx_assemble(const __grid_consta
     setup(s, t, raw);
     const i64 plane = a.item / 2, rt = (a.nrows + 63) / 64, units = rt * (plane / 64);
     const int nst = a.kpad / kStageK;
-    if (t.warp >= kWorkers / 32) {
-        regs_down<kRegsIssue>();
-        if (t.tid == kWorkers) t.ok = issue_products(s, t.smem, my_units(units), nst);
-    } else {
-        regs_up<kRegsWorker>();
-        AssembleWork w{a, s, t, rt, units, plane};
-        work(s, t, w, nst, a.kvalid, 6 + a.lgk);
-    }
+    const AssembleWork w{a, s, t, rt, units, plane};
+    run(s, t, w, my_units(units), nst, a.kvalid, 6 + a.lgk);
     teardown(s, t, t.ok, a.fault);
 }
 
@@ -223,8 +217,8 @@ struct StepsArgs {
 
 // A CTA walks chunks blockIdx.x and blockIdx.x + gridDim.x (if there is one)
 // step by step, product by product, the two in turn: a product's operands come
-// from the product before the last, so they are cut while the last one is read
-// and finished.  With one chunk every product waits for the one before.
+// from the product before the last, so it is cut and multiplied while the last
+// one is finished.  With one chunk every product waits for the one before.
 struct StepsWork {
     struct At {
         int i, o, k;  // step of the batch, product, chunk slot
@@ -232,8 +226,9 @@ struct StepsWork {
     const StepsArgs &a;
     Shared &s;
     Thread &t;
-    // Every worker writes the same exponents and lengths after a product's
-    // barrier, so each finds them without another one.
+    // Every finisher writes the same exponents and lengths after a product's
+    // barrier, so each finds them without another one; the cutters after
+    // `finished`.
     Info (*info)[kBufs];
     int nk, steps;  // chunk slots, steps of the batch
 
@@ -293,7 +288,7 @@ struct StepsWork {
             else
                 e1 = e, p1 = poison;
         }
-        if (!(t.ok = wsync_and(t.ok))) return false;
+        if (!(t.ok = fsync_and(t.ok))) return false;
 #pragma unroll
         for (int o = 0; o < 2; ++o) {
             const u64 m = read_or(s, t, n, o);
@@ -316,23 +311,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_fx_steps(const __grid_constant_
     setup(s, t, raw);
     StepsWork w{a, s, t, info, blockIdx.x + gridDim.x < a.ch.nch ? 2 : 1, 0};
     w.steps = max(0, w.end(0));
-    if (t.warp >= kWorkers / 32) {
-        regs_down<kRegsIssue>();
-        i64 products = 0;
-        for (int k = 0; k < w.nk; ++k)
-            if (w.end(k) > 0) products += (i64)w.end(k) * (a.nops + 1) - (a.i0 == 0 ? 1 : 0);
-        if (t.tid == kWorkers) t.ok = issue_products(s, t.smem, products, a.nst);
-    } else {
-        regs_up<kRegsWorker>();
-        if (a.i0 > 0)
-            for (int k = 0; k < w.nk; ++k) info[k][kBufP] = a.pinfo[w.chunk(k)];
-        work(s, t, w, a.nst, 64, 6 + a.lgk);
-        if (t.tid == 0 && t.ok)
-            for (int k = 0; k < w.nk; ++k) {
-                const i64 c = w.chunk(k);
-                if (w.end(k) > 0) (a.i0 + w.end(k) == a.ch.steps(c) ? a.cinfo : a.pinfo)[c] = info[k][kBufP];
-            }
-    }
+    i64 products = 0;
+    for (int k = 0; k < w.nk; ++k)
+        if (w.end(k) > 0) products += (i64)w.end(k) * (a.nops + 1) - (a.i0 == 0 ? 1 : 0);
+    if (a.i0 > 0 && t.tid < w.nk) info[t.tid][kBufP] = a.pinfo[w.chunk(t.tid)];
+    __syncthreads();
+    run(s, t, w, products, a.nst, 64, 6 + a.lgk);
+    if (t.tid == 0 && t.ok)
+        for (int k = 0; k < w.nk; ++k) {
+            const i64 c = w.chunk(k);
+            if (w.end(k) > 0) (a.i0 + w.end(k) == a.ch.steps(c) ? a.cinfo : a.pinfo)[c] = info[k][kBufP];
+        }
     teardown(s, t, t.ok, a.fault);
 }
 
@@ -400,7 +389,7 @@ struct GemmWork {
             else
                 e1 = e, p1 = poison;
         }
-        if (!(t.ok = wsync_and(t.ok))) return false;
+        if (!(t.ok = fsync_and(t.ok))) return false;
         if (t.tid == 0) {
 #pragma unroll
             for (int o = 0; o < 2; ++o) {
@@ -423,14 +412,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_fx_gemm(const __grid_constant__
     setup(s, t, raw);
     const int tiles = a.nt * a.nt;
     const i64 units = (i64)a.items * tiles;
-    if (t.warp >= kWorkers / 32) {
-        regs_down<kRegsIssue>();
-        if (t.tid == kWorkers) t.ok = issue_products(s, t.smem, my_units(units), a.nst);
-    } else {
-        regs_up<kRegsWorker>();
-        GemmWork w{a, s, t, tiles, units, (i64)a.dp * a.dp, 4ll * a.dp};
-        work(s, t, w, a.nst, a.dp, 6 + a.lgk);
-    }
+    const GemmWork w{a, s, t, tiles, units, (i64)a.dp * a.dp, 4ll * a.dp};
+    run(s, t, w, my_units(units), a.nst, a.dp, 6 + a.lgk);
     teardown(s, t, t.ok, a.fault);
 }
 
@@ -722,7 +705,7 @@ cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double 
     if ((int)ops.size() >= kMaxOps) return cudaErrorInvalidValue;  // orders up to 63: 62 products
     const WeightSpec w{wh.pts, wh.K, wh.amps, wh.mode, wh.magnus, wh.hfac};
     const i64 rpad = (q.rows + 63) / 64 * 64;
-    const int lgw = std::max(4, ceil_log2(2ll * q.kvalid)), lgk = ceil_log2(2ll * d);
+    const int lgw = std::max(5, ceil_log2(2ll * q.kvalid)), lgk = ceil_log2(2ll * d);
     const int nst = (d + kStageK - 1) / kStageK;
     auto assemble = [&](i64 i0, i64 rows, int per) -> cudaError_t {
         const Rows r{q.ch, per, i0};

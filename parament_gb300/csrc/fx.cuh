@@ -35,20 +35,21 @@
 // B digits a 32 x 64 MN-major tile (128-byte swizzle) so that the slices of B
 // stack along N (ozaki.cuh).
 //
-// Eight worker warps cut, read the levels and run the epilogues; a ninth issues
-// the products (sixteen of half the columns would have 120 registers a thread and
-// spill).  They meet on mbarriers only: `full` (a stage is cut), `done` (a stage
-// is multiplied), `drained` (the levels are read).  Two stages of 84 KB: a stage
-// is cut while the one before is multiplied, and the first stage of the next
-// product, if it does not depend on this one, before this one's levels are read.
+// Three kinds of warps walk the products of a launch, each at its own pace: eight
+// cut operands into stages, one issues the digit products, eight read the levels
+// and run the epilogues.  They meet on mbarriers only: `full` (a stage is cut),
+// `done` (a stage is multiplied), `ready` (a group of stages is), `drained` (its
+// levels are read), `finished` (a product is stored).  Two stages of 84 KB.
 //
-// What bounds it: a 64 x 64 x 64 product takes 19 thousand clocks inside a long
-// K and 31 thousand with its epilogue (d = 64), of which the tensor core is busy
-// 9 thousand; the rest is latency of the operands' and the terms' loads (L2) with
-// two worker warps per scheduler.  Against the first form, with row-major items,
-// one warp of the workers issuing and all of them meeting at every stage, 42
-// thousand: d = 64 Magnus, 4096 steps, 3.38 -> 2.57 ms; d = 96, 512 steps, 2.21 ->
-// 1.80 ms; d = 512, 16 steps, 4.16 -> 3.30 ms.
+// What bounds it: inside a long K, 64 columns take 14 thousand clocks, 8 of them
+// on the tensor core and 5 reading the levels, during which it stands still (its
+// 512 columns hold one product's levels); cutting (4.5) and the operands' loads
+// (6) lie underneath.  Measured: d = 64 Magnus, 4096 steps, 2.36 ms; d = 96, 512
+// steps, 1.71 ms; d = 512, 16 steps, 3.07 ms on the device.  Before, with eight
+// warps that did all but the issuing, and three conversions a value where the
+// levels are read: 2.57, 1.80 and 3.13 ms.  Accumulators for each half of the
+// columns, one read while the other is filled, measured slower (2.84, 2.37, 4.49
+// ms: the 32-column B tiles).
 #pragma once
 
 #include "ozaki.cuh"
@@ -56,13 +57,13 @@
 namespace pgb {
 namespace fx {
 
-constexpr int kWorkers = 256;
-constexpr int kCols = 32;  // columns of a worker thread
-constexpr int kThreads = kWorkers + 128;  // and a warpgroup of which one warp issues
-// Registers: 168 a thread at launch (64,512 in all), then 224 for the two worker
-// warpgroups and 40 for the third (62,464).
-constexpr int kRegsWorker = 224, kRegsIssue = 40;
-static_assert(kWorkers * kRegsWorker + 128 * kRegsIssue <= kThreads * 168, "register split");
+constexpr int kFinishers = 256, kCutters = 256;  // threads; warps 0 .. 7 and 8 .. 15
+constexpr int kThreads = kFinishers + kCutters + 128;  // and a warpgroup of which one thread issues
+constexpr int kIssuer = kFinishers + kCutters;
+constexpr int kCols = 32;  // columns of a finisher
+// Registers: 96 a thread at launch (61,440 in all), then by warpgroup.
+constexpr int kRegsFinish = 136, kRegsCut = 88, kRegsIssue = 32;
+static_assert(kFinishers * kRegsFinish + kCutters * kRegsCut + 128 * kRegsIssue <= kThreads * 96, "register split");
 constexpr int kSlices = 7;
 constexpr int kLevels = 8;
 constexpr int kStageK = 16;                                  // complex columns of a stage
@@ -85,30 +86,28 @@ struct Info {
 __device__ __forceinline__ int headroom(Info i) { return i.mb >= 62 ? 0 : 62 - i.mb; }
 
 struct Shared {
-    uint64_t full[2], done[2], drained;
+    uint64_t full[2], done[2], ready, drained, finished, last;
     uint32_t tmem_base;
     uint32_t orhi[4][2], orlo[4][2];  // OR of the magnitudes of a product's results, four products in turn
     int rowmb[2][64];                 // lengths of a tile's rows, two tiles in turn
 };
 
-// Where a thread sits: tensor-memory lane 32 (warp % 4) + lane, plane p, row r
-// of the 64 x 64 tile, columns c0 .. c0 + 31.
+// Where a thread sits; finishers: tensor-memory lane 32 (warp % 4) + lane, plane
+// p, row r of the 64 x 64 tile, columns c0 .. c0 + 31.
 struct Thread {
     int tid, lane, warp, p, r, c0;
     uint32_t tm;      // this thread's lane and first column in tensor memory
     unsigned char *smem;
-    uint32_t g;        // stages cut so far; stage g sits in buffer g % 2
-    bool ok;           // no wait gave up (then the remaining ones are skipped)
+    bool ok;          // no wait gave up (then the remaining ones are skipped)
 };
 
-// Barrier of the workers, alone and with a vote.
-__device__ __forceinline__ void wsync() { asm volatile("bar.sync 1, %0;" ::"n"(kWorkers) : "memory"); }
-__device__ __forceinline__ bool wsync_and(bool p) {
+// Barrier of the finishers, with a vote.
+__device__ __forceinline__ bool fsync_and(bool p) {
     int r;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.and.pred q, 1, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
         : "=r"(r)
-        : "r"((int)p), "n"(kWorkers)
+        : "r"((int)p), "n"(kFinishers)
         : "memory");
     return r != 0;
 }
@@ -179,20 +178,17 @@ __device__ __forceinline__ void issue_stage(uint32_t tmem, uint64_t da, uint64_t
 __device__ __forceinline__ bool issue_products(Shared &s, const unsigned char *smem, i64 products, int nst) {
     const uint32_t base = tc::smem_addr(smem);
     uint32_t g = 0, drains = 0;
-    for (i64 k = 0; k < products; ++k)
+    bool ok = true;
+    for (i64 k = 0; k < products && ok; ++k)
         for (int st = 0; st < nst; ++st, ++g) {
             const uint32_t b = g & 1;
             const bool fresh = (st & (kGroup - 1)) == 0;
-            bool ok = tc::mbar_wait(&s.full[b], (g >> 1) & 1, kWait);
+            ok = tc::mbar_wait(&s.full[b], (g >> 1) & 1, kWait);
             if (fresh) {
                 ok = ok && (drains == 0 || tc::mbar_wait(&s.drained, (drains - 1) & 1, kWait));
                 ++drains;
             }
-            if (!ok) {
-                // What was issued finishes before tensor memory is freed.
-                if (g > 0) tc::mbar_wait(&s.done[(g - 1) & 1], ((g - 1) >> 1) & 1, kWait);
-                return false;
-            }
+            if (!ok) break;
             tc::fence_after_sync();
             const uint64_t da = desc_k_sw64(base + b * kStageB);
             const uint64_t db = oz::desc_mn_sw128(base + b * kStageB + kSlices * kASliceB, kBSliceB);
@@ -201,10 +197,11 @@ __device__ __forceinline__ bool issue_products(Shared &s, const unsigned char *s
             else
                 issue_stage<false>(s.tmem_base, da, db);
             tc::mma_commit(&s.done[b]);
+            if (st + 1 == nst || (st & (kGroup - 1)) == kGroup - 1) tc::mma_commit(&s.ready);
         }
-    // The last stages finish before tensor memory is freed.
-    if (g > 0 && !tc::mbar_wait(&s.done[(g - 1) & 1], ((g - 1) >> 1) & 1, kWait)) return false;
-    return true;
+    // What was issued finishes before tensor memory is freed.
+    tc::mma_commit(&s.last);
+    return tc::mbar_wait(&s.last, 0, kWait) && ok;
 }
 
 // Four 64-bit values of a 32-byte piece.
@@ -238,7 +235,7 @@ struct Cut {
 // With `imag` the operand is i A: the product is i A B.
 __device__ __forceinline__ Cut make_cut(const Thread &t, const Operand &A, const Operand &B, bool imag) {
     Cut c;
-    const int l = t.lane, w = t.warp, p = w >> 2;
+    const int l = t.lane, w = t.warp & 7, p = w >> 2;
     const int row = ((l >> 1) & 1) | ((l >> 2) & 2) | (l & 4) | ((l >> 1) & 8) | ((w & 3) << 4);
     const int k = 8 * (l & 1);
     c.a = A.ptr + p * A.plane + row * A.rs + (k / 4) * A.qs;
@@ -355,20 +352,28 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
     for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// An integer of magnitude up to 2^22 held in a float, plus 0x4B400000: one add.
+// Integers held in floats, |f| <= 2^22: f + 1.5 2^23 has f in its low bits.
+constexpr float kMagic = 12582912.0f;
 constexpr uint32_t kIntBias = 0x4B400000u;
-__device__ __forceinline__ uint32_t biased_int(float f) { return __float_as_uint(__fadd_rn(f, 12582912.0f)); }
+__device__ __forceinline__ uint32_t biased_int(float f) { return __float_as_uint(__fadd_rn(f, kMagic)); }
+// f = 256 q + r for an integer |f| < 2^24: biased q, and r (|r| <= 128).
+__device__ __forceinline__ uint32_t split8(float f, float &r) {
+    const float q = __fmaf_rn(f, 0.00390625f, kMagic);
+    r = __fmaf_rn(__fsub_rn(q, kMagic), -256.0f, f);
+    return __float_as_uint(q);
+}
 
-// Adds sum_L D_L 2^(8 (7 - L)) shifted right by `sh` (10 .. 24) to the thread's
-// 16 sums, every level as an integer times a power of two.  Levels 0 .. 2 stay
-// within 2^22 and convert by an addition, 3 .. 5 by the conversion unit; levels
-// 6 and 7 join in FP32 (their sum is below the last kept bit by then).
+// Adds sum_L D_L 2^(8 (7 - L)) shifted right by `sh` (11 .. 24) to the thread's
+// sums.  Levels 0 .. 2 stay within 2^22 and convert by an addition; 3 .. 5 split
+// into a multiple of 256 and a rest first (the conversion unit takes eight
+// clocks a warp).  The rests of 4 and 5 and levels 6 and 7 are below 2^22 in the
+// result's units and meet in FP32, good to 2^-2 of its last bit.
 __device__ __forceinline__ void drain(const Thread &t, int sh, i64 (&acc)[kCols]) {
-    const uint32_t m3 = 1u << (32 - sh);                  // level 3 (2^32)
-    const int m4 = 1 << (24 - sh);                        // level 4 (2^24)
-    const int m5 = sh <= 16 ? 1 << (16 - sh) : 0, r5 = sh <= 16 ? 0 : sh - 16;  // level 5 (2^16)
-    const int half5 = r5 ? 1 << (r5 - 1) : 0;
-    const float f6 = __int_as_float((127 + 8 - sh) << 23);  // levels 6, 7: 2^(8 - sh)
+    const uint32_t m3 = 1u << (32 - sh);                    // level 3 (2^32)
+    const int m4 = 1 << (24 - sh);                          // level 4 (2^24)
+    const float f4 = __int_as_float((127 + 24 - sh) << 23);  // the same, 2^(24 - sh)
+    const float f5 = __int_as_float((127 + 16 - sh) << 23);  // level 5 (2^16)
+    const float f6 = __int_as_float((127 + 8 - sh) << 23);   // levels 6, 7 (2^8)
 #pragma unroll
     for (int g = 0; g < kCols / 4; ++g) {
         float f[kLevels][4];
@@ -377,80 +382,96 @@ __device__ __forceinline__ void drain(const Thread &t, int sh, i64 (&acc)[kCols]
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
+            float r3, r4, r5;
+            const uint32_t q3 = split8(f[3][j], r3), q4 = split8(f[4][j], r4), q5 = split8(f[5][j], r5);
             const int h01 = (int)(biased_int(f[0][j]) * 256u + biased_int(f[1][j]) - 257u * kIntBias);
-            const int h23 = (int)(biased_int(f[2][j]) * 256u - 256u * kIntBias) + __float2int_rn(f[3][j]);
-            const float l67 = __fmaf_rn(f[7][j], 0.00390625f, f[6][j]);
-            const int l = (int)(__float_as_uint(__fmaf_rn(l67, f6, 12582912.0f)) - kIntBias);
-            const int i5 = __float2int_rn(f[5][j]);
-            i64 v = (i64)__float2int_rn(f[4][j]) * m4 + acc[4 * g + j];
-            v += r5 ? (i64)(((i5 + half5) >> r5) + l) : (i64)i5 * m5 + l;
+            const int h23 = (int)((biased_int(f[2][j]) + q3) * 256u + biased_int(r3) - 513u * kIntBias);
+            const int q45 = (int)(q4 * 256u + q5 - 257u * kIntBias);
+            float l = __fmaf_rn(__fmaf_rn(f[7][j], 0.00390625f, f[6][j]), f6, kMagic);
+            l = __fadd_rn(__fmaf_rn(r4, f4, __fmul_rn(r5, f5)), l);
+            const i64 v = (i64)q45 * m4 + (int)(__float_as_uint(l) - kIntBias) + acc[4 * g + j];
             acc[4 * g + j] = (i64)((u64)((i64)h01 * 65536 + h23) * (u64)m3 + (u64)v);
         }
     }
 }
 
-// Cuts stage st into the next buffer once that has been multiplied.  The loads
-// come first; they and the cutting fit under the stage being multiplied.
-__device__ __forceinline__ void cut_stage(Shared &s, Thread &t, const Cut &c, int st, int kvalid) {
-    const uint32_t b = t.g & 1;
-    i64 va[8], vb[8];
-    load_a(c, st, va);
-    load_b(c, st, kvalid, vb);
-    if (t.g >= 2 && t.ok) t.ok = tc::mbar_wait(&s.done[b], ((t.g >> 1) - 1) & 1, kWait);
-    cut_store<true>(c, t.smem + b * kStageB, va);
-    cut_store<false>(c, t.smem + b * kStageB, vb);
-    tc::fence_proxy_async();
-    __syncwarp();
-    if (t.lane == 0) arrive(&s.full[b]);
-    ++t.g;
+// Whether the wait ended for every lane (a warp leaves its loop as a whole).
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, kWait)) != 0;
 }
 
-// The workers' loop over the products of `w` (one copy of each part: the code of
-// a launch with one product per CTA has to come from L2 first).  `w` deals out
-// products (at, more, next), gives their operands, says whether one needs the
-// result of the product just before, and takes the sums (epilogue; false ends).
-// Stages are cut one ahead of those read, across products where that is allowed.
+// The cutters' loop over the products of `w`, which deals out products (first,
+// more, next) and gives their operands.  The values of the next stage are on
+// their way while a stage is cut: those of A once A's are used, those of B once
+// B's are.  Before product n is touched, product n - 2 has to be finished, and
+// n - 1 too where `needs` says so.
 template <class W>
-__device__ __forceinline__ void work(Shared &s, Thread &t, W &w, int nst, int kvalid, int sh) {
-    typename W::At cur = w.first(), ahead = cur;
+__device__ __forceinline__ void cutter(Shared &s, Thread &t, const W &w, int nst, int kvalid) {
+    typename W::At at = w.first(), before = at;
+    if (!w.more(at)) return;
+    uint32_t g = 0, n = 0, seen = 0;
+    int st = 0;
     Cut c;
-    int sc = 0, sa = 0;    // stage read, stage cut
-    uint32_t read = 0, n = 0;
-    i64 T[kCols];
-#pragma unroll
-    for (int j = 0; j < kCols; ++j) T[j] = 0;
-    while (w.more(cur)) {
-        while (t.g <= read + 1 && w.more(ahead)) {
-            if (sa == 0) {
-                if (t.g > read && w.needs(ahead, cur)) break;
-                Operand A, B;
-                const bool imag = w.operands(ahead, A, B);
-                c = make_cut(t, A, B, imag);
-            }
-            cut_stage(s, t, c, sa, kvalid);
-            if (++sa == nst) {
-                sa = 0;
-                ahead = w.next(ahead);
-            }
+    i64 va[8], vb[8];
+    auto begin = [&] {
+        const uint32_t until = n == 0 ? 0 : n - (w.needs(at, before) ? 0 : 1);
+        for (; seen < until; ++seen)
+            if (t.ok) t.ok = warp_wait(&s.finished, seen & 1);
+        Operand A, B;
+        const bool imag = w.operands(at, A, B);
+        c = make_cut(t, A, B, imag);
+    };
+    begin();
+    load_a(c, 0, va);
+    load_b(c, 0, kvalid, vb);
+    while (t.ok) {
+        const uint32_t b = g & 1;
+        if (g >= 2) t.ok = warp_wait(&s.done[b], ((g >> 1) - 1) & 1);
+        unsigned char *stage = t.smem + b * kStageB;
+        const bool same = st + 1 < nst;  // the next stage is of this product
+        cut_store<true>(c, stage, va);
+        if (same) load_a(c, st + 1, va);
+        cut_store<false>(c, stage, vb);
+        if (same) load_b(c, st + 1, kvalid, vb);
+        tc::fence_proxy_async();
+        __syncwarp();
+        if (t.lane == 0) arrive(&s.full[b]);
+        ++g;
+        if (same) {
+            ++st;
+            continue;
         }
-        const bool end = sc + 1 == nst;
-        if (end || (sc & (kGroup - 1)) == kGroup - 1) {
-            if (t.ok) t.ok = tc::mbar_wait(&s.done[read & 1], (read >> 1) & 1, kWait);
+        st = 0;
+        before = at;
+        at = w.next(at);
+        if (!w.more(at)) break;
+        ++n;
+        begin();
+        load_a(c, 0, va);
+        load_b(c, 0, kvalid, vb);
+    }
+}
+
+// The finishers' loop: the levels of every group of stages into the sums, then
+// w.epilogue (false ends).
+template <class W>
+__device__ __forceinline__ void finisher(Shared &s, Thread &t, const W &w, int nst, int sh) {
+    uint32_t groups = 0, n = 0;
+    for (typename W::At at = w.first(); w.more(at); at = w.next(at), ++n) {
+        i64 T[kCols];
+#pragma unroll
+        for (int j = 0; j < kCols; ++j) T[j] = 0;
+        for (int st = 0; st < nst; st += kGroup, ++groups) {
+            if (t.ok) t.ok = tc::mbar_wait(&s.ready, groups & 1, kWait);
             tc::fence_after_sync();
             drain(t, sh, T);
             tc::fence_before_sync();
             __syncwarp();
             if (t.lane == 0) arrive(&s.drained);
         }
-        ++read;
-        ++sc;
-        if (end) {
-            if (!w.epilogue(cur, T, n++)) break;
-#pragma unroll
-            for (int j = 0; j < kCols; ++j) T[j] = 0;
-            sc = 0;
-            cur = w.next(cur);
-        }
+        if (!w.epilogue(at, T, n)) break;
+        __syncwarp();
+        if (t.lane == 0) arrive(&s.finished);
     }
 }
 
@@ -538,36 +559,42 @@ template <class V>
 __device__ __forceinline__ u64 put_out(const Out &o, const Thread &t, i64 (&T)[kCols], int eT, int e, V view,
                                        i64 plane, i64 qs, int row, int col0, int d, i64 *dst) {
     if (!o.plain) {
-        // T times its coefficient, then the terms; the first term's loads go
-        // out before the multiplication.
+        // T times its coefficient, then the terms, half of the columns at a time;
+        // the first loads go out before the multiplication.
         const Factor ft = o.t.m ? make_factor(o.t.m, e - eT - o.t.e - 2, 0) : Factor{0, 0, 0};
+        constexpr int H = kCols / 2;
 #pragma unroll 1
         for (int k = 0; k < max(1, o.nterm); ++k) {
-            i64 x[kCols];
             Factor f{0, 0, 0};
+            const i64 *q = nullptr;
             if (k < o.nterm) {
                 const View w = view(o.term[k].buf);
                 const Coef c = o.term[k].c;
-                const i64 *q = w.re + (c.imag ? 1 - t.p : t.p) * plane;
-#pragma unroll
-                for (int i = 0; i < kCols / 4; ++i)
-                    load4(q + i * qs, x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+                q = w.re + (c.imag ? 1 - t.p : t.p) * plane;
                 const int hr = headroom(w.info);
                 f = make_factor((c.imag && t.p == 0) ? -c.m : c.m, e - (w.info.e - hr) - c.e - 2, hr);
-            } else {
-#pragma unroll
-                for (int j = 0; j < kCols; ++j) x[j] = 0;
-            }
-            if (k == 0) {
-#pragma unroll
-                for (int j = 0; j < kCols; ++j) T[j] = scaled(T[j], ft);
-            }
-            if (f.pre) {
-#pragma unroll
-                for (int j = 0; j < kCols; ++j) x[j] = (i64)((u64)x[j] << f.pre);
             }
 #pragma unroll
-            for (int j = 0; j < kCols; ++j) T[j] += scaled(x[j], f);
+            for (int h = 0; h < 2; ++h) {
+                i64 x[H];
+                if (q) {
+#pragma unroll
+                    for (int i = 0; i < H / 4; ++i)
+                        load4(q + (h * H / 4 + i) * qs, x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+                }
+                if (k == 0) {
+#pragma unroll
+                    for (int j = 0; j < H; ++j) T[h * H + j] = scaled(T[h * H + j], ft);
+                }
+                if (q) {
+                    if (f.pre) {
+#pragma unroll
+                        for (int j = 0; j < H; ++j) x[j] = (i64)((u64)x[j] << f.pre);
+                    }
+#pragma unroll
+                    for (int j = 0; j < H; ++j) T[h * H + j] += scaled(x[j], f);
+                }
+            }
         }
         if (o.diag.m && t.p == o.diag.imag && row < d && row >= col0 && row < col0 + kCols) {
             const i64 x = o.diag.m >> min(e - o.diag.e, 63);
@@ -586,7 +613,7 @@ __device__ __forceinline__ u64 put_out(const Out &o, const Thread &t, i64 (&T)[k
     return m;
 }
 
-// OR over the warp into the workers' OR of result o of product n.
+// OR over the warp into the finishers' OR of result o of product n.
 __device__ __forceinline__ void merge_or(Shared &s, const Thread &t, uint32_t n, int o, u64 m) {
     const uint32_t hi = __reduce_or_sync(0xffffffffu, (uint32_t)(m >> 32));
     const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)m);
@@ -595,8 +622,8 @@ __device__ __forceinline__ void merge_or(Shared &s, const Thread &t, uint32_t n,
         atomicOr(&s.orlo[n & 3][o], lo);
     }
 }
-// After the workers' barrier of product n: its result o; clears the place of
-// product n - 1, which every worker has read by then and none fills before n + 3.
+// After the finishers' barrier of product n: its result o; clears the place of
+// product n - 1, which every finisher has read by then and none fills before n + 3.
 __device__ __forceinline__ u64 read_or(Shared &s, const Thread &t, uint32_t n, int o) {
     const u64 m = (u64)s.orhi[n & 3][o] << 32 | s.orlo[n & 3][o];
     if (t.tid == 0) s.orhi[(n - 1) & 3][o] = s.orlo[(n - 1) & 3][o] = 0;
@@ -615,7 +642,6 @@ __device__ __forceinline__ void setup(Shared &s, Thread &t, unsigned char *raw) 
     t.r = 32 * (q4 & 1) + t.lane;
     t.c0 = kCols * (t.warp >> 2);
     t.smem = raw + ((1024u - (tc::smem_addr(raw) & 1023u)) & 1023u);
-    t.g = 0;
     t.ok = true;
     if (t.tid < 8) s.orhi[t.tid >> 1][t.tid & 1] = s.orlo[t.tid >> 1][t.tid & 1] = 0;
     if (t.tid < 128) s.rowmb[t.tid >> 6][t.tid & 63] = 0;
@@ -625,16 +651,34 @@ __device__ __forceinline__ void setup(Shared &s, Thread &t, unsigned char *raw) 
     }
     if (t.tid == 0) {
         for (int b = 0; b < 2; ++b) {
-            tc::mbar_init(&s.full[b], kWorkers / 32);
+            tc::mbar_init(&s.full[b], kCutters / 32);
             tc::mbar_init(&s.done[b], 1);
         }
-        tc::mbar_init(&s.drained, kWorkers / 32);
+        tc::mbar_init(&s.drained, kFinishers / 32);
+        tc::mbar_init(&s.finished, kFinishers / 32);
+        tc::mbar_init(&s.ready, 1);
+        tc::mbar_init(&s.last, 1);
         tc::fence_mbar_init();
     }
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     t.tm = s.tmem_base + ((uint32_t)(32 * q4) << 16) + (uint32_t)t.c0;
+}
+
+// A launch: every role over the products of w (`products` of them for this CTA).
+template <class W>
+__device__ __forceinline__ void run(Shared &s, Thread &t, const W &w, i64 products, int nst, int kvalid, int sh) {
+    if (t.tid >= kIssuer) {
+        regs_down<kRegsIssue>();
+        if (t.tid == kIssuer) t.ok = issue_products(s, t.smem, products, nst);
+    } else if (t.tid >= kFinishers) {
+        regs_down<kRegsCut>();
+        cutter(s, t, w, nst, kvalid);
+    } else {
+        regs_up<kRegsFinish>();
+        finisher(s, t, w, nst, sh);
+    }
 }
 
 // The CTA's end; ok: this thread's waits all ended.
