@@ -63,6 +63,7 @@ struct Ctx {
 
     // Work buffers (grow-only, like src/cuda/parament.cpp:418-474)
     DevBuf carr, out, chunks, work, X, B1, B2, aux, grad, wts, xplanes;
+    DevBuf arrived;  // pair counters of the small groups' tree, zero between launches
 
     // Bounded-wait faults of this context's tensor-core kernels.  The kernels
     // add to a device counter (d_fault, zero at creation, never reset); after
@@ -83,7 +84,8 @@ struct Ctx {
     size_t esize() const { return fp64 ? 16 : 8; }
     size_t device_bytes() const {
         return stack.cap + split_stack.cap + carr.cap + out.cap + chunks.cap + work.cap + X.cap + B1.cap + B2.cap +
-               aux.cap + grad.cap + wts.cap + xplanes.cap + fx_stack.cap + fx_ws.cap;
+               aux.cap + grad.cap + wts.cap + xplanes.cap + fx_stack.cap + fx_ws.cap +
+               arrived.cap;
     }
     void release_all() {
         stack.release();
@@ -101,6 +103,7 @@ struct Ctx {
         xplanes.release();
         fx_stack.release();
         fx_ws.release();
+        arrived.release();
     }
 };
 
@@ -125,7 +128,10 @@ Parament_ErrorCode run_split(Ctx *c, const void *d_carr, unsigned pts, unsigned 
 Parament_ErrorCode run_split_large(Ctx *c, const SplitArgs &a, double h, void *d_out, cudaStream_t stream);
 
 // c0 = m_0 - 1 and mu_n = m_n / Hnorm^n of the regrouped polynomial (split.cu).
-void split_coefficients(int M, double x, double hnorm, double *c0, std::vector<double> &mu);
+void power_coefficients(int M, double x, double hnorm, double *c0, std::vector<double> &mu);
+// The same polynomial with the FP32 coefficients of the complex64 contexts;
+// returns J_0, which c_0 = p(0) - J_0 leaves out.
+double plain_coefficients(int M, double x, double hnorm, std::vector<double> &c);
 
 // complex128 by exact sliced products (fx.cu): fx_prepare converts the stack
 // (set_hamiltonian), fx_ensure allocates the workspace of P steps, run_fx

@@ -470,14 +470,7 @@ static void build_program(int M, double x, double hnorm, std::vector<Op> &ops) {
     if (x <= 1.0) {
         double c0[2];
         std::vector<double> mu;
-        split_coefficients(M, x, hnorm, c0, mu);
-        // c_0 = p(0) - 1: the orders above M of 1 = J_0 + 2 sum J_2k.  Summed as
-        // J_0 - 1 + ... its rounding (1e-16) would scale U at every step alike:
-        // 3e-14 after 300 steps where the FP64 kernels are at 6e-15.
-        double tail = 0.0;
-        for (int k = M + 21; k > M; k -= 2) tail += jn(k, x);
-        c0[0] = -2.0 * tail;
-        c0[1] = 0.0;
+        power_coefficients(M, x, hnorm, c0, mu);
         auto cf = [&](int n) { return n == 0 ? coef(c0[0], c0[1]) : coef(mu[2 * n], mu[2 * n + 1]); };
         Op y{kBufX, kBufX, 0, {plain_out(kBufY), no_out()}};
         ops.push_back(y);
@@ -533,7 +526,7 @@ static void build_program(int M, double x, double hnorm, std::vector<Op> &ops) {
     const long double sc = 2.0L / hnorm;
     std::vector<double> J(2 * (M + 1));
     bessel_coeffs(M, x, J.data());
-    // J_0 - 1 from the even orders, for the same reason.
+    // J_0 - 1 from the even orders (power_coefficients says why).
     long double j0m1 = 0.0L;
     for (int k = M + 41; k >= 2; k -= 2) j0m1 -= 2.0L * jn(k, x);
     auto j = [&](int k, long double f) { return coef(f * J[2 * k], f * J[2 * k + 1]); };

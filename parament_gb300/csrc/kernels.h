@@ -46,6 +46,14 @@ int small_chunk_count(bool fp64, int d, int Ke, long long P, int num_sms);
 size_t small_smem_bytes(bool fp64, int d, int Ke);
 cudaError_t launch_small_steps(const StepLaunch &a);
 
+// A whole propagation with d <= 8 and x = Hnorm h <= 1 in one launch of groups of 16
+// threads (step_group.cu): the result in `out` (context precision); `nodes` holds
+// nchunks d x d nodes of 16 bytes, `arrived` nchunks zeros (zero again after it).
+bool group_applies(int d, int M, double x);
+int group_chunk_count(bool fp64, int d, int Ke, long long P, int num_sms);  // 0: does not fit
+cudaError_t launch_group_steps(const StepLaunch &l, double x, double hnorm, int num_sms, void *nodes, int *arrived,
+                               void *out);
+
 // The same plain complex64 propagation at d = 64 on the tcgen05 tensor cores
 // (small_tc.cu): per batch of up to 65536 steps, the X planes of the batch
 // (xplanes: small_tc_xplane_bytes(P)) and then one CTA per SM over the batch.

@@ -340,6 +340,34 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
                             static_cast<float2 *>(d_out), stream, &levels);
         const long long batches = (P + 65535) / 65536;
         c->launches = 2 * (int)batches + levels;
+    } else if (const int ngr = group_applies(d, M, h * c->hnorm)
+                                   ? group_chunk_count(c->fp64, d, (int)c->Ke, P, c->num_sms)
+                                   : 0) {
+        const size_t count = sizeof(int) * (size_t)ngr;
+        if (c->work.ensure(16 * dd * ngr) != cudaSuccess) return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
+        e = cudaSuccess;
+        if (c->arrived.cap < count) {
+            if (c->arrived.ensure(count) != cudaSuccess) return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
+            // The next call may come on another stream.
+            e = cudaMemsetAsync(c->arrived.ptr, 0, c->arrived.cap, stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        }
+        StepLaunch l{};
+        l.fp64 = c->fp64;
+        l.d = d;
+        l.Ke = (int)c->Ke;
+        l.w = w;
+        l.M = M;
+        l.stack = c->stack.ptr;
+        l.carr = d_carr;
+        l.P = P;
+        l.stream = stream;
+        if (c->timing) cudaEventRecord(c->ev_start, stream);
+        if (e == cudaSuccess)
+            e = launch_group_steps(l, h * c->hnorm, c->hnorm, c->num_sms, c->work.ptr,
+                                   static_cast<int *>(c->arrived.ptr), d_out);
+        if (c->timing) cudaEventRecord(c->ev_stop, stream);
+        c->launches = 1;
     } else if (d <= kSmallMaxDim) {
         const int nch = small_chunk_count(c->fp64, d, (int)c->Ke, P, c->num_sms);
         // complex64: the chunk products are combined by the double-float tree

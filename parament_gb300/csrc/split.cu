@@ -448,7 +448,7 @@ int split_order(double hnorm, double h, long long P) {
 
 // Monomial coefficients m_n of J_0(x) + 2 sum_(k=1..M) (-i)^k J_k(x) T_k(t);
 // returns mu_n = m_n / Hnorm^n (n >= 1) and c0 = m_0 - 1.
-void split_coefficients(int M, double x, double hnorm, double *c0, std::vector<double> &mu) {
+static void split_coefficients(int M, double x, double hnorm, double *c0, std::vector<double> &mu) {
     std::vector<double> J(2 * (M + 1));
     bessel_coeffs(M, x, J.data());
     std::vector<double> re(M + 1, 0.0), im(M + 1, 0.0);
@@ -483,6 +483,41 @@ void split_coefficients(int M, double x, double hnorm, double *c0, std::vector<d
         mu[2 * n] = re[n] * scale;
         mu[2 * n + 1] = im[n] * scale;
     }
+}
+
+// The same with c0 = p(0) - 1 summed without cancellation: the orders above M of
+// 1 = J_0 + 2 sum J_2k.  As J_0 - 1 + ... its rounding (1e-16) would scale U at
+// every step alike: 3e-14 after 300 complex128 steps where FP64 sums are at 6e-15.
+void power_coefficients(int M, double x, double hnorm, double *c0, std::vector<double> &mu) {
+    split_coefficients(M, x, hnorm, c0, mu);
+    double tail = 0.0;
+    for (int k = M + 21; k > M; k -= 2) tail += jn(k, x);
+    c0[0] = -2.0 * tail;
+    c0[1] = 0.0;
+}
+
+// The polynomial of the complex64 contexts by powers of X, c_n real for even n and
+// imaginary for odd n: from the coefficients J_k(x) and 2 / Hnorm as these
+// contexts hold them, rounded to FP32 -- U_j is that of the Clenshaw kernels.  c_0
+// without J_0(x), which is returned: the sum of both would round once more, at
+// every step alike.
+double plain_coefficients(int M, double x, double hnorm, std::vector<double> &c) {
+    std::vector<double> J(2 * (M + 1)), a(M + 2, 0.0), b(M + 2, 0.0), t(M + 2, 0.0);
+    bessel_coeffs(M, x, J.data());
+    c.assign(M + 1, 0.0);
+    a[0] = 1.0;  // T_(k-1)
+    b[1] = 1.0;  // T_k
+    for (int k = 1; k <= M; ++k) {
+        const double j = (float)J[2 * k + (k & 1)];
+        for (int n = k & 1; n <= k; n += 2) c[n] += 2.0 * j * b[n];
+        for (int n = 0; n <= k + 1 && n <= M; ++n) t[n] = (n > 0 ? 2.0 * b[n - 1] : 0.0) - a[n];
+        a = b;
+        b = t;
+    }
+    const double s = 0.5 * (double)(float)(2.0 / hnorm);
+    double f = 1.0;
+    for (int n = 1; n <= M; ++n) c[n] *= (f *= s);
+    return (float)J[0];
 }
 
 // Builds the split form's stack: the complex64 inputs (exact), and the Magnus
