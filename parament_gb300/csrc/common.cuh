@@ -76,38 +76,43 @@ struct WeightSpec {
 // for step s.  Slots: [0,K) controls, [K,2K) commutators [H0,H_k],
 // [2K, 2K+K(K-1)/2) pair commutators [H_j,H_i], j<i, at slot 2K+i(i-1)/2+j.
 // Follows src/cuda/control_expansion.cu:27-170 with the pair slot re-indexed.
-template <class C>
-__device__ __forceinline__ C step_weight(const C *__restrict__ carr, const WeightSpec &w, int m, long long s) {
-    using R = decltype(C().x);
-    C zero = mk<C>(0.0, 0.0);
+// Formed in the arithmetic of A from samples of type C.
+template <class A, class C>
+__device__ __forceinline__ A step_weight_as(const C *__restrict__ carr, const WeightSpec &w, int m, long long s) {
+    using R = decltype(A().x);
+    const A zero = mk<A>(0.0, 0.0);
     const size_t pts = w.pts;
+    auto at = [&](int k, long long i) {
+        const C v = carr[(size_t)k * pts + i];
+        return mk<A>(v.x, v.y);
+    };
     if (m < w.K) {
         if (m >= w.amps) return zero;
-        const C *u = carr + (size_t)m * pts;
         if (w.magnus || w.mode == kQuadSimpson) {
-            C a = u[2 * s], b = u[2 * s + 1], c = u[2 * s + 2];
-            C t = cadd(cadd(a, cscale(b, (R)4)), c);
-            return mk<C>(t.x / (R)6, t.y / (R)6);
+            A a = at(m, 2 * s), b = at(m, 2 * s + 1), c = at(m, 2 * s + 2);
+            A t = cadd(cadd(a, cscale(b, (R)4)), c);
+            return mk<A>(t.x / (R)6, t.y / (R)6);
         }
-        if (w.mode == kQuadMidpoint) return cscale(cadd(u[s], u[s + 1]), (R)0.5);
-        return u[s];
+        if (w.mode == kQuadMidpoint) return cscale(cadd(at(m, s), at(m, s + 1)), (R)0.5);
+        return at(m, s);
     }
-    const C f = mk<C>(0.0, w.hfac);
+    const A f = mk<A>(0.0, w.hfac);
     if (m < 2 * w.K) {
         int k = m - w.K;
         if (k >= w.amps) return zero;
-        const C *u = carr + (size_t)k * pts;
-        return cmul(csub(u[2 * s + 2], u[2 * s]), f);
+        return cmul(csub(at(k, 2 * s + 2), at(k, 2 * s)), f);
     }
     int p = m - 2 * w.K;
     int i = 1;
     while ((i + 1) * i / 2 <= p) ++i;
     int j = p - i * (i - 1) / 2;
     if (i >= w.amps) return zero;
-    const C *ui = carr + (size_t)i * pts;
-    const C *uj = carr + (size_t)j * pts;
-    C t = csub(cmul(uj[2 * s], ui[2 * s + 2]), cmul(uj[2 * s + 2], ui[2 * s]));
+    A t = csub(cmul(at(j, 2 * s), at(i, 2 * s + 2)), cmul(at(j, 2 * s + 2), at(i, 2 * s)));
     return cmul(t, f);
+}
+template <class C>
+__device__ __forceinline__ C step_weight(const C *__restrict__ carr, const WeightSpec &w, int m, long long s) {
+    return step_weight_as<C>(carr, w, m, s);
 }
 
 // acc[i][j] = sum_k A[r_i][k] B[k][c_j] (plus A2[r_i][k] B2[k][c_j] when A2 is

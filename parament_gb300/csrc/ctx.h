@@ -50,10 +50,10 @@ struct Ctx {
     bool split_ready = false;
     bool split_herm = false;                     // split stack exactly (anti-)Hermitian per slot
 
-    // Fixed-point form of complex128 contexts (fx.cu): the stack as integers
+    // Fixed-point form (fx.cu): the stack as integers, that of the split form,
     // and the workspace of a propagation.
-    DevBuf fx_stack, fx_ws;
-    bool fx_ready = false;
+    DevBuf fx_stack, fx_split, fx_ws;
+    bool fx_ready = false, fx_split_ready = false;
 
     // Instrumentation: CUDA events around the dominant kernel of the last call
     // and the number of kernels it launched.
@@ -84,7 +84,7 @@ struct Ctx {
     size_t esize() const { return fp64 ? 16 : 8; }
     size_t device_bytes() const {
         return stack.cap + split_stack.cap + carr.cap + out.cap + chunks.cap + work.cap + X.cap + B1.cap + B2.cap +
-               aux.cap + grad.cap + wts.cap + xplanes.cap + fx_stack.cap + fx_ws.cap +
+               aux.cap + grad.cap + wts.cap + xplanes.cap + fx_stack.cap + fx_split.cap + fx_ws.cap +
                arrived.cap;
     }
     void release_all() {
@@ -102,6 +102,7 @@ struct Ctx {
         wts.release();
         xplanes.release();
         fx_stack.release();
+        fx_split.release();
         fx_ws.release();
         arrived.release();
     }
@@ -133,15 +134,17 @@ void power_coefficients(int M, double x, double hnorm, double *c0, std::vector<d
 // returns J_0, which c_0 = p(0) - J_0 leaves out.
 double plain_coefficients(int M, double x, double hnorm, std::vector<double> &c);
 
-// complex128 by exact sliced products (fx.cu): fx_prepare converts the stack
-// (set_hamiltonian), fx_ensure allocates the workspace of P steps, run_fx
-// propagates (x = Hnorm h).
+// Exact sliced products (fx.cu): fx_prepare / fx_prepare_split convert the stack
+// (set_hamiltonian; the split form's first call), fx_ensure allocates the
+// workspace of P steps, run_fx propagates (x = Hnorm h).
 struct WeightSpecHost;
+enum class FxForm { kFp64, kPlain32, kSplit32 };
 void fx_prepare(Ctx *c);
-bool fx_applies(const Ctx *c, int M);
+void fx_prepare_split(Ctx *c);
+bool fx_applies(const Ctx *c, FxForm form, int M, double x);
 bool fx_ensure(Ctx *c, long long P);
-cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double x, int M, long long P, void *d_out,
-                   cudaStream_t stream);
+cudaError_t run_fx(Ctx *c, FxForm form, const void *d_carr, const WeightSpecHost &wh, double x, int M, long long P,
+                   void *d_out, cudaStream_t stream);
 
 // Adjoint: d/du_k[i] Re Tr(W^H U) for real samples, d <= adj_max_dim.
 int adj_max_dim(bool fp64);

@@ -1,5 +1,7 @@
-// complex128 propagation for d > kFxMinDim on the tensor cores: fixed-point
-// matrices and exact sliced products (fx.cuh).
+// Propagation on fixed-point matrices and exact sliced products on the tensor cores
+// (fx.cuh): complex128 from d = kFxMinDim on (seven digits), and complex64 with d >
+// 64, where the 3xTF32 kernel does not serve, in the plain form (four digits) and
+// the split form (five).
 //
 // The same X_j, Chebyshev order and Bessel coefficients as the FP64 kernels
 // (step_small.cu, gemm.cu; src/cuda/parament.cpp:486-718).  What changes:
@@ -17,6 +19,9 @@
 //     chunk of steps is P <- E P + E + P with U_(s1-1) ... U_s0 = I + P: the
 //     unit diagonal never meets the small terms.  The chunk products meet in
 //     the pairwise tree in the same form.
+//   * The plain complex64 form keeps the FP32 coefficients of the other complex64
+//     kernels and rounds 1 + the diagonal of E_j to FP32, so U_j is the one those
+//     form (rounded otherwise, results drift apart by 1e-8 a step).
 //   * X_j = sum_m w_jm S_m is itself a product, weights (steps x 1 + Ke) times
 //     the stack (1 + Ke rows of 2 dp^2 numbers), on the same sliced kernel:
 //     one row of weights per step, each with an exponent of its own.
@@ -42,11 +47,12 @@ namespace fx {
 // ------------------------------------------------------------------ set-up of the stack
 
 // Largest biased exponent of each stack matrix (emax zeroed before).
-__global__ void k_fx_stack_max(const double2 *src, i64 dd, int *emax) {
-    const double2 *m = src + (size_t)blockIdx.y * dd;
+template <class C>
+__global__ void k_fx_stack_max(const C *src, i64 dd, int *emax) {
+    const C *m = src + (size_t)blockIdx.y * dd;
     int e = 0;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < dd; i += (i64)gridDim.x * blockDim.x) {
-        const double2 v = m[i];
+        const double2 v = make_double2(m[i].x, m[i].y);
         e = max(e, max((__double2hiint(v.x) >> 20) & 0x7FF, (__double2hiint(v.y) >> 20) & 0x7FF));
     }
     e = __reduce_max_sync(0xffffffffu, e);
@@ -57,16 +63,17 @@ __global__ void k_fx_stack_max(const double2 *src, i64 dd, int *emax) {
 __device__ __forceinline__ int exp_of(int biased) { return max(biased, 1) - 1022; }
 
 // The stack as fixed-point items, every matrix at its own exponent.
-__global__ void k_fx_stack(const double2 *src, int d, int dp, const int *emax, i64 *dst) {
+template <class C>
+__global__ void k_fx_stack(const C *src, int d, int dp, const int *emax, i64 *dst) {
     const int m = blockIdx.y, s = 62 - exp_of(emax[m]);
-    const double2 *a = src + (size_t)m * d * d;
+    const C *a = src + (size_t)m * d * d;
     i64 *o = dst + (size_t)m * 2 * dp * dp;
     const i64 n = (i64)dp * dp;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
         const int r = (int)(i / dp), c = (int)(i % dp);
         const i64 k = (i64)(c >> 2) * 4 * dp + 4 * r + (c & 3);
         double2 v = make_double2(0.0, 0.0);
-        if (r < d && c < d) v = a[(size_t)r * d + c];
+        if (r < d && c < d) v = make_double2(a[(size_t)r * d + c].x, a[(size_t)r * d + c].y);
         o[k] = __double2ll_rn(scalbn(v.x, s));
         o[n + k] = __double2ll_rn(scalbn(v.y, s));
     }
@@ -98,9 +105,14 @@ struct Rows {
 // One warp per row: the step's weights times the stack matrices' scales, as
 // integers at the row's exponent; the exponent of X_j and its length (zero
 // here, kPoison for weights that are not finite).
-__global__ void __launch_bounds__(128) k_fx_weights(const double2 *carr, WeightSpec w, int Ke, const int *emax,
+// A: the arithmetic of the weights (complex64 samples in FP64 for the split form).
+template <class A, class C>
+__global__ void __launch_bounds__(128) k_fx_weights(const C *carr, WeightSpec w, int Ke, const int *emax,
                                                     Rows rows, i64 nrows, int kpad, int lgk, i64 *W, i64 plane,
-                                                    Info *info) {
+                                                    Info *info, Info *zero0, Info *zero1, i64 n0, i64 n1) {
+    // The infos of the round's results start at zero.
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n0 + n1; i += (i64)gridDim.x * blockDim.x)
+        (i < n0 ? zero0[i] : zero1[i - n0]) = Info{0, 0};
     const i64 j = (i64)blockIdx.x * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (j >= nrows) return;
@@ -112,7 +124,8 @@ __global__ void __launch_bounds__(128) k_fx_weights(const double2 *carr, WeightS
         return;
     }
     auto weight = [&](int m) {
-        double2 v = m == 0 ? make_double2(1.0, 0.0) : step_weight(carr, w, m - 1, st);
+        const A q = m == 0 ? mk<A>(1.0, 0.0) : step_weight_as<A>(carr, w, m - 1, st);
+        const double2 v = make_double2(q.x, q.y);
         const int e = exp_of(emax[m]);
         return make_double2(scalbn(v.x, e), scalbn(v.y, e));
     };
@@ -182,6 +195,7 @@ struct AssembleWork {
     }
 };
 
+template <int S>
 __global__ void __launch_bounds__(kThreads, 1) k_fx_assemble(const __grid_constant__ AssembleArgs a) {
     extern __shared__ unsigned char raw[];
     __shared__ Shared s;
@@ -190,7 +204,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_fx_assemble(const __grid_consta
     const i64 plane = a.item / 2, rt = (a.nrows + 63) / 64, units = rt * (plane / 64);
     const int nst = a.kpad / kStageK;
     const AssembleWork w{a, s, t, rt, units, plane};
-    run(s, t, w, my_units(units), nst, a.kvalid, 6 + a.lgk);
+    run<S>(s, t, w, my_units(units), nst, a.kvalid, 6 + a.lgk);
     teardown(s, t, t.ok, a.fault);
 }
 
@@ -316,7 +330,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_fx_steps(const __grid_constant_
         if (w.end(k) > 0) products += (i64)w.end(k) * (a.nops + 1) - (a.i0 == 0 ? 1 : 0);
     if (a.i0 > 0 && t.tid < w.nk) info[t.tid][kBufP] = a.pinfo[w.chunk(t.tid)];
     __syncthreads();
-    run(s, t, w, products, a.nst, 64, 6 + a.lgk);
+    run<7>(s, t, w, products, a.nst, 64, 6 + a.lgk);
     if (t.tid == 0 && t.ok)
         for (int k = 0; k < w.nk; ++k) {
             const i64 c = w.chunk(k);
@@ -405,6 +419,7 @@ struct GemmWork {
     }
 };
 
+template <int S>
 __global__ void __launch_bounds__(kThreads, 1) k_fx_gemm(const __grid_constant__ GemmArgs a) {
     extern __shared__ unsigned char raw[];
     __shared__ Shared s;
@@ -413,12 +428,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_fx_gemm(const __grid_constant__
     const int tiles = a.nt * a.nt;
     const i64 units = (i64)a.items * tiles;
     const GemmWork w{a, s, t, tiles, units, (i64)a.dp * a.dp, 4ll * a.dp};
-    run(s, t, w, my_units(units), a.nst, a.dp, 6 + a.lgk);
+    run<S>(s, t, w, my_units(units), a.nst, a.dp, 6 + a.lgk);
     teardown(s, t, t.ok, a.fault);
 }
 
-// I + E as complex128, row-major d x d.
-__global__ void k_fx_out(const i64 *E, const Info *info, int d, int dp, double2 *out) {
+// I + E in the context's precision, row-major d x d.
+template <class C>
+__global__ void k_fx_out(const i64 *E, const Info *info, int d, int dp, C *out) {
     const Info q = *info;
     const i64 plane = (i64)dp * dp, n = (i64)d * d;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
@@ -427,7 +443,7 @@ __global__ void k_fx_out(const i64 *E, const Info *info, int d, int dp, double2 
         double2 v = make_double2(scalbn((double)E[k], q.e - 62), scalbn((double)E[plane + k], q.e - 62));
         if (q.mb == kPoison) v.x = v.y = __longlong_as_double(0x7FF8000000000000ll);
         if (r == c) v.x += 1.0;
-        out[i] = v;
+        out[i] = mk<C>(v.x, v.y);
     }
 }
 
@@ -462,16 +478,26 @@ static Out no_out() {
 
 // The products of a step: E from X.  Powers of X for x <= 1, the Clenshaw
 // recurrence above.
-static void build_program(int M, double x, double hnorm, std::vector<Op> &ops) {
+static void build_program(FxForm form, int M, double x, double hnorm, std::vector<Op> &ops) {
     ops.clear();
     auto add = [](Out &o, Coef c, int buf) {
         if (c.m) o.term[o.nterm++] = Term{c, buf};
     };
     if (x <= 1.0) {
-        double c0[2];
-        std::vector<double> mu;
-        power_coefficients(M, x, hnorm, c0, mu);
-        auto cf = [&](int n) { return n == 0 ? coef(c0[0], c0[1]) : coef(mu[2 * n], mu[2 * n + 1]); };
+        std::vector<Coef> cs(M + 1);
+        if (form == FxForm::kPlain32) {
+            std::vector<double> c;
+            const double j0 = plain_coefficients(M, x, hnorm, c);
+            cs[0] = coef((long double)j0 - 1.0L + c[0], 0.0L);
+            for (int n = 1; n <= M; ++n) cs[n] = coef(n % 2 ? 0.0L : c[n], n % 2 ? c[n] : 0.0L);
+        } else {
+            double c0[2];
+            std::vector<double> mu;
+            power_coefficients(M, x, hnorm, c0, mu);
+            cs[0] = coef(c0[0], c0[1]);
+            for (int n = 1; n <= M; ++n) cs[n] = coef(mu[2 * n], mu[2 * n + 1]);
+        }
+        auto cf = [&](int n) { return cs[n]; };
         Op y{kBufX, kBufX, 0, {plain_out(kBufY), no_out()}};
         ops.push_back(y);
         // An imaginary factor of a product goes into its operand.
@@ -481,6 +507,7 @@ static void build_program(int M, double x, double hnorm, std::vector<Op> &ops) {
             tc.imag = 0;
             Out &r = o.out[0];
             r.buf = fin ? kBufE : (a == kBufR0 ? kBufR1 : kBufR0);
+            r.grid = fin && form == FxForm::kPlain32;
             r.t = tc;
             const int powbuf[3] = {0, kBufX, kBufY};
             for (int n = 1; n <= deg; ++n) add(r, cf(k + n), powbuf[n]);
@@ -570,11 +597,14 @@ static bool disabled() {
     return off;
 }
 
+template <int S>
 static cudaError_t set_smem() {
     cudaError_t e = cudaSuccess;
-    for (const void *fn : {reinterpret_cast<const void *>(&k_fx_assemble), reinterpret_cast<const void *>(&k_fx_steps),
-                           reinterpret_cast<const void *>(&k_fx_gemm)})
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    for (const void *fn : {reinterpret_cast<const void *>(&k_fx_assemble<S>),
+                           reinterpret_cast<const void *>(&k_fx_gemm<S>),
+                           S == 7 ? reinterpret_cast<const void *>(&k_fx_steps) : nullptr})
+        if (e == cudaSuccess && fn)
+            e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Digits<S>::smem);
     return e;
 }
 
@@ -601,8 +631,9 @@ static Plan make_plan(int d, int Ke, i64 P, int num_sms) {
         q.nch = (int)std::min<i64>(2ll * num_sms, P);
         q.per = (int)std::min<i64>(16, (P + q.nch - 1) / q.nch);
     } else {
-        // About eight waves of tiles per product, in rounds of equal size.
-        const i64 g0 = std::min<i64>(P, std::max<i64>(1, (8ll * num_sms + tiles - 1) / tiles));
+        // About sixteen waves of tiles per product, in rounds of equal size (eight: 5 to
+        // 10 % slower at d = 128 and 200, two: a quarter).
+        const i64 g0 = std::min<i64>(P, std::max<i64>(1, (16ll * num_sms + tiles - 1) / tiles));
         const i64 L = (P + g0 - 1) / g0;
         q.nch = (int)((P + L - 1) / L);
         q.per = 1;
@@ -632,9 +663,10 @@ static Plan make_plan(int d, int Ke, i64 P, int num_sms) {
 // Bytes before the matrices of the fixed-point stack: the largest exponents.
 static size_t stack_head(int n) { return (sizeof(int) * (size_t)n + 255) / 256 * 256; }
 
+template <int S>
 static cudaError_t launch_gemm_op(const GemmArgs &a, int num_sms, cudaStream_t st, int *launches) {
     const i64 units = (i64)a.items * a.nt * a.nt;
-    k_fx_gemm<<<(int)std::min<i64>(units, num_sms), kThreads, kSmem, st>>>(a);
+    k_fx_gemm<S><<<(int)std::min<i64>(units, num_sms), kThreads, Digits<S>::smem, st>>>(a);
     ++*launches;
     return cudaGetLastError();
 }
@@ -643,33 +675,54 @@ static cudaError_t launch_gemm_op(const GemmArgs &a, int num_sms, cudaStream_t s
 
 using namespace fx;
 
-bool fx_applies(const Ctx *c, int M) {
-    return c->fp64 && c->fx_ready && M >= 3 && isfinite(c->hnorm) && c->hnorm > 0.0;
+bool fx_applies(const Ctx *c, FxForm form, int M, double x) {
+    if (M < 3 || !isfinite(c->hnorm) || c->hnorm <= 0.0) return false;
+    if (form == FxForm::kFp64) return c->fx_ready;
+    return x <= 1.0 && (form == FxForm::kPlain32 ? c->fx_ready : c->fx_split_ready);
 }
 
-// The context's stack in fixed point, made with the Hamiltonian on the
-// context's stream (the caller waits for it).  Without room for it the FP64
-// kernels serve.
+// Whether a context's Hamiltonian gets a fixed-point stack: complex64 from 65 on
+// (below, the step kernels of one launch are faster: a product's epilogue takes
+// longer here than its digits), and the plain form not where the 3xTF32 kernel runs.
+static bool fx_serves(FxForm form, int d) {
+    if (disabled()) return false;
+    if (form == FxForm::kFp64) return d >= kFxMinDim;
+    return d > 64 && (form == FxForm::kSplit32 || d < 256 || d % 128 != 0);
+}
+
+// A stack in fixed point, on the context's stream (the caller waits for it).
+// Without room for it the other kernels serve.
+template <class C>
+static bool convert_stack(Ctx *c, const void *stack, DevBuf &buf) {
+    const int d = (int)c->dim, dp = (d + 63) / 64 * 64, n = 1 + (int)c->Ke;
+    const size_t head = stack_head(n), bytes = head + sizeof(i64) * 2 * (size_t)dp * dp * n;
+    void *p = nullptr;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    buf.release();
+    buf.ptr = p;
+    buf.cap = bytes;
+    int *emax = static_cast<int *>(p);
+    const C *src = static_cast<const C *>(stack);
+    if (cudaMemsetAsync(emax, 0, sizeof(int) * n, c->stream) != cudaSuccess) return false;
+    k_fx_stack_max<C><<<dim3(std::max(1, std::min(256, d * d / 1024)), n), 256, 0, c->stream>>>(src, (i64)d * d, emax);
+    k_fx_stack<C><<<dim3(std::max(1, std::min(1024, dp * dp / 512)), n), 256, 0, c->stream>>>(
+        src, d, dp, emax, reinterpret_cast<i64 *>(static_cast<char *>(p) + head));
+    return cudaGetLastError() == cudaSuccess;
+}
+
 void fx_prepare(Ctx *c) {
     c->fx_ready = false;
-    const int d = (int)c->dim, dp = (d + 63) / 64 * 64, n = 1 + (int)c->Ke;
-    if (d < kFxMinDim || disabled()) return;
-    const size_t head = stack_head(n);
-    void *p = nullptr;
-    if (cudaMalloc(&p, head + sizeof(i64) * 2 * (size_t)dp * dp * n) != cudaSuccess) {
-        cudaGetLastError();
-        return;
-    }
-    c->fx_stack.release();
-    c->fx_stack.ptr = p;
-    c->fx_stack.cap = head + sizeof(i64) * 2 * (size_t)dp * dp * n;
-    int *emax = static_cast<int *>(p);
-    const double2 *src = static_cast<const double2 *>(c->stack.ptr);
-    if (cudaMemsetAsync(emax, 0, sizeof(int) * n, c->stream) != cudaSuccess) return;
-    k_fx_stack_max<<<dim3(std::max(1, std::min(256, d * d / 1024)), n), 256, 0, c->stream>>>(src, (i64)d * d, emax);
-    k_fx_stack<<<dim3(std::max(1, std::min(1024, dp * dp / 512)), n), 256, 0, c->stream>>>(
-        src, d, dp, emax, reinterpret_cast<i64 *>(static_cast<char *>(p) + head));
-    c->fx_ready = cudaGetLastError() == cudaSuccess;
+    if (!fx_serves(c->fp64 ? FxForm::kFp64 : FxForm::kPlain32, (int)c->dim)) return;
+    c->fx_ready = c->fp64 ? convert_stack<double2>(c, c->stack.ptr, c->fx_stack)
+                          : convert_stack<float2>(c, c->stack.ptr, c->fx_stack);
+}
+
+void fx_prepare_split(Ctx *c) {
+    c->fx_split_ready =
+        fx_serves(FxForm::kSplit32, (int)c->dim) && convert_stack<float2>(c, c->split_stack.ptr, c->fx_split);
 }
 
 bool fx_ensure(Ctx *c, long long P) {
@@ -677,36 +730,40 @@ bool fx_ensure(Ctx *c, long long P) {
     return c->fx_ws.ensure(q.bytes) == cudaSuccess;
 }
 
-cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double x, int M, long long P, void *d_out,
-                   cudaStream_t st) {
+template <int S, class A, class C>
+static cudaError_t run_fx_t(Ctx *c, FxForm form, const void *d_carr, const WeightSpecHost &wh, double x, int M,
+                            long long P, void *d_out, cudaStream_t st) {
+    const DevBuf &sb = form == FxForm::kSplit32 ? c->fx_split : c->fx_stack;
     const int d = (int)c->dim, Ke = (int)c->Ke, n = 1 + Ke;
     const Plan q = make_plan(d, Ke, P, c->num_sms);
     int launches = 0;
-    cudaError_t e = set_smem();
+    cudaError_t e = set_smem<S>();
     if (e != cudaSuccess) return e;
     const size_t head = stack_head(n);
-    const int *emax = static_cast<const int *>(c->fx_stack.ptr);
-    const i64 *stack = reinterpret_cast<const i64 *>(static_cast<const char *>(c->fx_stack.ptr) + head);
+    const int *emax = static_cast<const int *>(sb.ptr);
+    const i64 *stack = reinterpret_cast<const i64 *>(static_cast<const char *>(sb.ptr) + head);
     char *ws = static_cast<char *>(c->fx_ws.ptr);
     i64 *W = reinterpret_cast<i64 *>(ws + q.off_w), *X = reinterpret_cast<i64 *>(ws + q.off_x);
-    i64 *S = reinterpret_cast<i64 *>(ws + q.off_s), *Pb = reinterpret_cast<i64 *>(ws + q.off_p);
+    i64 *scr = reinterpret_cast<i64 *>(ws + q.off_s), *Pb = reinterpret_cast<i64 *>(ws + q.off_p);
     i64 *chunks = reinterpret_cast<i64 *>(ws + q.off_c);
     Info *xinfo = reinterpret_cast<Info *>(ws + q.off_info), *sinfo = xinfo + q.rows;
     Info *pinfo = sinfo + (kMaxOps + 1) * (size_t)q.nch, *cinfo = pinfo + 2 * (size_t)q.nch, *tinfo = cinfo + q.nch;
     std::vector<Op> ops;
-    build_program(M, x, c->hnorm, ops);
+    build_program(form, M, x, c->hnorm, ops);
     if ((int)ops.size() >= kMaxOps) return cudaErrorInvalidValue;  // orders up to 63: 62 products
     const WeightSpec w{wh.pts, wh.K, wh.amps, wh.mode, wh.magnus, wh.hfac};
     const i64 rpad = (q.rows + 63) / 64 * 64;
     const int lgw = std::max(5, ceil_log2(2ll * q.kvalid)), lgk = ceil_log2(2ll * d);
     const int nst = (d + kStageK - 1) / kStageK;
-    auto assemble = [&](i64 i0, i64 rows, int per) -> cudaError_t {
+    auto assemble = [&](i64 i0, i64 rows, int per, Info *zero0 = nullptr, i64 n0 = 0, Info *zero1 = nullptr,
+                        i64 n1 = 0) -> cudaError_t {
         const Rows r{q.ch, per, i0};
-        k_fx_weights<<<(unsigned)((rows + 3) / 4), 128, 0, st>>>(static_cast<const double2 *>(d_carr), w, Ke, emax, r,
-                                                               rows, q.kpad, lgw, W, rpad * q.kpad, xinfo);
+        k_fx_weights<A><<<(unsigned)((rows + 3) / 4), 128, 0, st>>>(static_cast<const C *>(d_carr), w, Ke, emax, r,
+                                                                  rows, q.kpad, lgw, W, rpad * q.kpad, xinfo, zero0,
+                                                                  zero1, n0, n1);
         const AssembleArgs a{W, stack, rpad * q.kpad, X, xinfo, rows, q.item, q.kpad, q.kvalid, lgw, c->d_fault};
         const i64 units = ((rows + 63) / 64) * (q.item / 128);
-        k_fx_assemble<<<(int)std::min<i64>(units, c->num_sms), kThreads, kSmem, st>>>(a);
+        k_fx_assemble<S><<<(int)std::min<i64>(units, c->num_sms), kThreads, Digits<S>::smem, st>>>(a);
         launches += 2;
         return cudaGetLastError();
     };
@@ -726,7 +783,7 @@ cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double 
         a.nops = (int)ops.size();
         a.X = X;
         a.xinfo = xinfo;
-        a.scratch = S;
+        a.scratch = scr;
         a.pbuf = Pb;
         a.chunks = chunks;
         a.pinfo = pinfo;
@@ -740,7 +797,7 @@ cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double 
         for (i64 i0 = 0; i0 < q.ch.longest(); i0 += q.per) {
             if ((e = assemble(i0, q.rows, q.per)) != cudaSuccess) return e;
             a.i0 = i0;
-            k_fx_steps<<<std::min(q.nch, c->num_sms), kThreads, kSmem, st>>>(a);
+            k_fx_steps<<<std::min(q.nch, c->num_sms), kThreads, Digits<7>::smem, st>>>(a);
             ++launches;
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
@@ -755,30 +812,28 @@ cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double 
         a.fault = c->d_fault;
         for (i64 i = 0; i < longest; ++i) {
             const int active = i < q.ch.len ? q.nch : q.ch.nlong;
-            if ((e = assemble(i, active, 1)) != cudaSuccess) return e;
             for (int b = 0; b < kBufs; ++b) a.buf[b] = Buf{};
             a.buf[kBufX] = Buf{X, mat, xinfo, 1};
-            for (int b = 0; b < 5; ++b) a.buf[kBufY + b] = Buf{S + b * set, mat, nullptr, 1};
+            for (int b = 0; b < 5; ++b) a.buf[kBufY + b] = Buf{scr + b * set, mat, nullptr, 1};
             Buf dst{Pb + (i & 1) * set, mat, pinfo + (i & 1) * q.nch, 1};
             a.buf[kBufP] = Buf{Pb + ((i - 1) & 1) * set, mat, pinfo + ((i - 1) & 1) * q.nch, 1};
             // A buffer may be written more than once in a round: the lengths, which
             // start at zero, are kept per result.
             const size_t results = ops.size() + 1;
-            if ((e = cudaMemsetAsync(sinfo, 0, sizeof(Info) * results * q.nch, st)) != cudaSuccess) return e;
+            if ((e = assemble(i, active, 1, sinfo, (i64)results * q.nch, dst.info, q.nch)) != cudaSuccess) return e;
             size_t slot = 0;
-            if ((e = cudaMemsetAsync(dst.info, 0, sizeof(Info) * q.nch, st)) != cudaSuccess) return e;
             if (i == 0) a.buf[kBufE] = dst;
             a.items = active;
             for (const Op &o : ops) {
                 a.op = o;
                 for (const Out &out : o.out)
                     if (out.buf >= 0 && !(out.buf == kBufE && i == 0)) a.buf[out.buf].info = sinfo + slot++ * q.nch;
-                if ((e = launch_gemm_op(a, c->num_sms, st, &launches)) != cudaSuccess) return e;
+                if ((e = launch_gemm_op<S>(a, c->num_sms, st, &launches)) != cudaSuccess) return e;
             }
             if (i > 0) {
                 a.buf[kBufX] = dst;
                 a.op = run;
-                if ((e = launch_gemm_op(a, c->num_sms, st, &launches)) != cudaSuccess) return e;
+                if ((e = launch_gemm_op<S>(a, c->num_sms, st, &launches)) != cudaSuccess) return e;
             }
             if (active < q.nch) {
                 // The chunks without a step in this round keep their product.
@@ -813,7 +868,7 @@ cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double 
         o.nterm = 2;
         o.term[0] = Term{one, kBufX};
         o.term[1] = Term{one, kBufY};
-        i64 *cur = chunks, *nxt = S;
+        i64 *cur = chunks, *nxt = scr;
         Info *ci = cinfo, *ni = tinfo;
         for (i64 n2 = q.nch; n2 > 1;) {
             const i64 pairs = n2 / 2;
@@ -822,7 +877,7 @@ cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double 
             a.buf[kBufY] = Buf{cur, 2 * q.item, ci, 2};
             a.buf[kBufW] = Buf{nxt, q.item, ni, 1};
             a.items = (int)pairs;
-            if ((e = launch_gemm_op(a, c->num_sms, st, &launches)) != cudaSuccess) return e;
+            if ((e = launch_gemm_op<S>(a, c->num_sms, st, &launches)) != cudaSuccess) return e;
             if (n2 & 1) {
                 e = cudaMemcpyAsync(nxt + pairs * q.item, cur + 2 * pairs * q.item, sizeof(i64) * q.item,
                                     cudaMemcpyDeviceToDevice, st);
@@ -836,11 +891,18 @@ cudaError_t run_fx(Ctx *c, const void *d_carr, const WeightSpecHost &wh, double 
         }
         const i64 total = (i64)d * d;
         k_fx_out<<<(int)std::min<i64>((total + 255) / 256, 1024), 256, 0, st>>>(cur, ci, d, q.dp,
-                                                                               static_cast<double2 *>(d_out));
+                                                                               static_cast<C *>(d_out));
         ++launches;
     }
     c->launches = launches;
     return cudaGetLastError();
+}
+
+cudaError_t run_fx(Ctx *c, FxForm form, const void *d_carr, const WeightSpecHost &wh, double x, int M, long long P,
+                   void *d_out, cudaStream_t st) {
+    if (form == FxForm::kFp64) return run_fx_t<7, double2, double2>(c, form, d_carr, wh, x, M, P, d_out, st);
+    if (form == FxForm::kPlain32) return run_fx_t<4, float2, float2>(c, form, d_carr, wh, x, M, P, d_out, st);
+    return run_fx_t<5, double2, float2>(c, form, d_carr, wh, x, M, P, d_out, st);
 }
 
 }  // namespace pgb

@@ -39,17 +39,20 @@
 // cut operands into stages, one issues the digit products, eight read the levels
 // and run the epilogues.  They meet on mbarriers only: `full` (a stage is cut),
 // `done` (a stage is multiplied), `ready` (a group of stages is), `drained` (its
-// levels are read), `finished` (a product is stored).  Two stages of 84 KB.
+// levels are read), `finished` (a product is stored).
 //
-// What bounds it: inside a long K, 64 columns take 14 thousand clocks, 8 of them
-// on the tensor core and 5 reading the levels, during which it stands still (its
-// 512 columns hold one product's levels); cutting (4.5) and the operands' loads
-// (6) lie underneath.  Measured: d = 64 Magnus, 4096 steps, 2.36 ms; d = 96, 512
-// steps, 1.71 ms; d = 512, 16 steps, 3.07 ms on the device.  Before, with eight
-// warps that did all but the issuing, and three conversions a value where the
-// levels are read: 2.57, 1.80 and 3.13 ms.  Accumulators for each half of the
-// columns, one read while the other is filled, measured slower (2.84, 2.37, 4.49
-// ms: the 32-column B tiles).
+// What bounds it: inside a long K with seven digits, 64 columns take 13 thousand
+// clocks, 8 of them on the tensor core and 5 reading the levels, during which it
+// stands still (its 512 columns hold one product's levels); cutting (4.5) and the
+// operands' loads (6) lie underneath.  At d <= 128 the loads' latency and the
+// epilogues (64-bit multiplies) weigh as much; with four or five digits they are
+// all of it.  Measured: d = 64 Magnus, 4096 steps, 2.04 ms; d = 96, 512 steps, 1.58
+// ms; d = 512, 16 steps, 2.96 ms on the device; complex64, d = 128, 4096 steps, 7.9
+// ms (FP32 kernel: 11.2).  With the finishers' sums spilled (136 registers) the
+// first three took 2.36, 1.71 and 3.07; with eight warps that did all but the
+// issuing 2.57, 1.80 and 3.13.  Accumulators for each half of the columns, one
+// read while the other is filled, measured slower (2.84, 2.37, 4.49: the 32-column
+// B tiles).
 #pragma once
 
 #include "ozaki.cuh"
@@ -61,20 +64,29 @@ constexpr int kFinishers = 256, kCutters = 256;  // threads; warps 0 .. 7 and 8 
 constexpr int kThreads = kFinishers + kCutters + 128;  // and a warpgroup of which one thread issues
 constexpr int kIssuer = kFinishers + kCutters;
 constexpr int kCols = 32;  // columns of a finisher
-// Registers: 96 a thread at launch (61,440 in all), then by warpgroup.
-constexpr int kRegsFinish = 136, kRegsCut = 88, kRegsIssue = 32;
+// Registers: 96 a thread at launch (61,440 in all), then by warpgroup.  The
+// finishers must not spill: with this little L1 a spilled sum comes back from L2.
+constexpr int kRegsFinish = 144, kRegsCut = 80, kRegsIssue = 24;
 static_assert(kFinishers * kRegsFinish + kCutters * kRegsCut + 128 * kRegsIssue <= kThreads * 96, "register split");
-constexpr int kSlices = 7;
-constexpr int kLevels = 8;
-constexpr int kStageK = 16;                                  // complex columns of a stage
-constexpr int kGroup = 4;                                    // stages per exact accumulation
-constexpr uint32_t kASliceB = 128 * 64;                      // 8 KB
-constexpr uint32_t kBSliceB = 32 * 128;                      // 4 KB
-constexpr uint32_t kStageB = kSlices * (kASliceB + kBSliceB);  // 84 KB
-constexpr size_t kSmem = 2 * (size_t)kStageB + 1024;
+constexpr int kStageK = 16;                       // complex columns of a stage
+constexpr int kGroup = 4;                         // stages per exact accumulation
+constexpr uint32_t kASliceB = 128 * 64;           // 8 KB
+constexpr uint32_t kBSliceB = 32 * 128;           // 4 KB
+constexpr int kMaxStages = 4;
+// S digits per operand: 7 for complex128, 4 for the complex64 form, 5 for its split
+// form.  The levels kept, the stages that fit and the accumulators: two sets where
+// they fit into tensor memory, one read while the other is filled.
+template <int S>
+struct Digits {
+    static constexpr int levels = S == 7 ? 8 : S;
+    static constexpr uint32_t stage_bytes = S * (kASliceB + kBSliceB);  // 84, 48, 60 KB
+    static constexpr int stages = S == 7 ? 2 : S == 5 ? 3 : 4;
+    static constexpr int sets = levels <= 4 ? 2 : 1;
+    static constexpr size_t smem = stages * (size_t)stage_bytes + 1024;
+    static_assert(smem <= 232448 - 4096 && stages <= kMaxStages, "shared memory of the fx kernels");
+};
 constexpr uint32_t kWait = 1u << 24;
 constexpr int kPoison = 127;  // measured length of an item that holds infinities or NaN
-static_assert(kSmem <= 232448 - 4096, "shared memory of the fx kernels");
 
 typedef long long i64;
 typedef unsigned long long u64;
@@ -86,7 +98,7 @@ struct Info {
 __device__ __forceinline__ int headroom(Info i) { return i.mb >= 62 ? 0 : 62 - i.mb; }
 
 struct Shared {
-    uint64_t full[2], done[2], ready, drained, finished, last;
+    uint64_t full[kMaxStages], done[kMaxStages], ready[2], drained[2], finished, last;
     uint32_t tmem_base;
     uint32_t orhi[4][2], orlo[4][2];  // OR of the magnitudes of a product's results, four products in turn
     int rowmb[2][64];                 // lengths of a tile's rows, two tiles in turn
@@ -150,54 +162,57 @@ __device__ __forceinline__ void issue_chain(uint32_t tmem, uint64_t da, uint64_t
     oz::mma_bf16(tmem + 64u * (uint32_t)(s + t0), a + 2, b + 128, idesc(64 * n), 1u);
 }
 
-// The MMAs of one stage (one thread): level s + t <= 7, the slices of B that a
-// slice of A meets stacked along N.  `fresh` starts the levels: s = 0 starts
-// levels 0 .. 6, the pair (1, 6) level 7.
-template <bool FRESH>
+// The MMAs of slice s of A (and, recursively, of the slices after it): the slices
+// of B that it meets (level s + t kept) stacked along N in chains of at most four.
+// FRESH starts the levels: s = 0 starts levels 0 .. S - 1; with one level more than
+// slices the pair (1, S - 1) starts that one.
+template <int S, bool FRESH, int s = 0>
 __device__ __forceinline__ void issue_stage(uint32_t tmem, uint64_t da, uint64_t db) {
-    issue_chain(tmem, da, db, 0, 0, 4, FRESH ? 0u : 1u);
-    issue_chain(tmem, da, db, 0, 4, 3, FRESH ? 0u : 1u);
-    issue_chain(tmem, da, db, 1, 0, 4, 1u);
-    if (FRESH) {
-        issue_chain(tmem, da, db, 1, 4, 2, 1u);
-        issue_chain(tmem, da, db, 1, 6, 1, 0u);
-    } else {
-        issue_chain(tmem, da, db, 1, 4, 3, 1u);
+    constexpr int levels = Digits<S>::levels;
+    constexpr int nt = levels - s < S ? levels - s : S;
+    constexpr int first = nt <= 4 ? nt : nt == 7 ? 4 : 3;
+    constexpr uint32_t acc = FRESH && s == 0 ? 0u : 1u;
+    issue_chain(tmem, da, db, s, 0, first, acc);
+    if constexpr (nt > first) {
+        if constexpr (FRESH && s == 1 && (levels > S)) {
+            issue_chain(tmem, da, db, s, first, nt - first - 1, 1u);
+            issue_chain(tmem, da, db, s, nt - 1, 1, 0u);
+        } else {
+            issue_chain(tmem, da, db, s, first, nt - first, acc);
+        }
     }
-    issue_chain(tmem, da, db, 2, 0, 3, 1u);
-    issue_chain(tmem, da, db, 2, 3, 3, 1u);
-    issue_chain(tmem, da, db, 3, 0, 3, 1u);
-    issue_chain(tmem, da, db, 3, 3, 2, 1u);
-    issue_chain(tmem, da, db, 4, 0, 4, 1u);
-    issue_chain(tmem, da, db, 5, 0, 3, 1u);
-    issue_chain(tmem, da, db, 6, 0, 2, 1u);
+    if constexpr (s + 1 < S) issue_stage<S, FRESH, s + 1>(tmem, da, db);
 }
 
 // The issuing warp: `products` products of nst stages each.  Returns whether
 // every wait ended.
+template <int S>
 __device__ __forceinline__ bool issue_products(Shared &s, const unsigned char *smem, i64 products, int nst) {
+    using D = Digits<S>;
     const uint32_t base = tc::smem_addr(smem);
-    uint32_t g = 0, drains = 0;
+    uint32_t b = 0, round = 0, groups = 0;  // buffer, times round the buffers
     bool ok = true;
     for (i64 k = 0; k < products && ok; ++k)
-        for (int st = 0; st < nst; ++st, ++g) {
-            const uint32_t b = g & 1;
+        for (int st = 0; st < nst; ++st) {
             const bool fresh = (st & (kGroup - 1)) == 0;
-            ok = tc::mbar_wait(&s.full[b], (g >> 1) & 1, kWait);
-            if (fresh) {
-                ok = ok && (drains == 0 || tc::mbar_wait(&s.drained, (drains - 1) & 1, kWait));
-                ++drains;
-            }
+            const uint32_t set = groups % D::sets, turn = groups / D::sets;
+            ok = tc::mbar_wait(&s.full[b], round & 1, kWait);
+            if (fresh && turn > 0) ok = ok && tc::mbar_wait(&s.drained[set], (turn - 1) & 1, kWait);
             if (!ok) break;
             tc::fence_after_sync();
-            const uint64_t da = desc_k_sw64(base + b * kStageB);
-            const uint64_t db = oz::desc_mn_sw128(base + b * kStageB + kSlices * kASliceB, kBSliceB);
+            const uint64_t da = desc_k_sw64(base + b * D::stage_bytes);
+            const uint64_t db = oz::desc_mn_sw128(base + b * D::stage_bytes + S * kASliceB, kBSliceB);
+            const uint32_t tmem = s.tmem_base + set * 64u * D::levels;
             if (fresh)
-                issue_stage<true>(s.tmem_base, da, db);
+                issue_stage<S, true>(tmem, da, db);
             else
-                issue_stage<false>(s.tmem_base, da, db);
+                issue_stage<S, false>(tmem, da, db);
             tc::mma_commit(&s.done[b]);
-            if (st + 1 == nst || (st & (kGroup - 1)) == kGroup - 1) tc::mma_commit(&s.ready);
+            if (st + 1 == nst || (st & (kGroup - 1)) == kGroup - 1) {
+                tc::mma_commit(&s.ready[set]);
+                ++groups;
+            }
+            if (++b == D::stages) b = 0, ++round;
         }
     // What was issued finishes before tensor memory is freed.
     tc::mma_commit(&s.last);
@@ -233,6 +248,7 @@ struct Cut {
 };
 
 // With `imag` the operand is i A: the product is i A B.
+template <int S>
 __device__ __forceinline__ Cut make_cut(const Thread &t, const Operand &A, const Operand &B, bool imag) {
     Cut c;
     const int l = t.lane, w = t.warp & 7, p = w >> 2;
@@ -255,7 +271,7 @@ __device__ __forceinline__ Cut make_cut(const Thread &t, const Operand &A, const
     c.bqs = B.qs;
     c.brs = B.rs;
     c.bsh = B.shift;
-    c.ob = kSlices * kASliceB + oz::sw(kStageK * p + c.k, col);
+    c.ob = S * kASliceB + oz::sw(kStageK * p + c.k, col);
     return c;
 }
 
@@ -279,7 +295,7 @@ __device__ __forceinline__ void load_b(const Cut &c, int st, int kvalid, i64 (&v
 // One slice (16 bytes: eight digits) from words that hold the digits of a pair
 // of values in bytes 0 and 2 (LOW) or 1 and 3.  0x6400 | byte is 1024 + byte in
 // fp16; 1152 less is the digit.
-template <bool ISA, int S, bool LOW>
+template <bool ISA, int K, bool LOW>
 __device__ __forceinline__ void cut_slice(const Cut &c, unsigned char *stage, const uint32_t (&z)[4]) {
     uint32_t b[4], q[4], m[4];
 #pragma unroll
@@ -289,7 +305,7 @@ __device__ __forceinline__ void cut_slice(const Cut &c, unsigned char *stage, co
     }
     const uint4 v = make_uint4(q[0], q[1], q[2], q[3]);
     if (ISA) {
-        unsigned char *base = stage + S * kASliceB;
+        unsigned char *base = stage + K * kASliceB;
         if (c.n1) {  // (n0 only with n1)
 #pragma unroll
             for (int i = 0; i < 4; ++i) asm("sub.f16x2 %0, %1, %2;" : "=r"(m[i]) : "r"(0x64806480u), "r"(b[i]));
@@ -301,15 +317,17 @@ __device__ __forceinline__ void cut_slice(const Cut &c, unsigned char *stage, co
             *reinterpret_cast<uint4 *>(base + c.o1) = v;
         }
     } else {
-        *reinterpret_cast<uint4 *>(stage + S * kBSliceB + c.ob) = v;
+        *reinterpret_cast<uint4 *>(stage + K * kBSliceB + c.ob) = v;
     }
 }
 
 // Digits of eight values into the stage's slices.  The shift and the digit bias
 // are multiply-adds (the integer pipe for logic and shifts is the busier one);
 // the bytes of a pair of values come together in four words.
-template <bool ISA>
+template <int S, bool ISA>
 __device__ __forceinline__ void cut_store(const Cut &c, unsigned char *stage, i64 (&v)[8]) {
+    // The digit bias of the S bytes and half a unit of the next.
+    constexpr u64 kBias = 0x8080808080808080ull << (8 * (7 - S));
     int h = ISA ? c.ash : c.bsh;
     if (h >= 32) {
 #pragma unroll
@@ -324,12 +342,12 @@ __device__ __forceinline__ void cut_store(const Cut &c, unsigned char *stage, i6
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             const u64 x = (u64)v[2 * i + k];
-            const u64 w = (u64)(uint32_t)x * mul + 0x8080808080808080ull;
+            const u64 w = (u64)(uint32_t)x * mul + kBias;
             lo[k] = (uint32_t)w;
             hi[k] = (uint32_t)(w >> 32) + (uint32_t)(x >> 32) * mul;
         }
-        z[0][i] = __byte_perm(lo[0], lo[1], 0x5410);
-        z[1][i] = __byte_perm(lo[0], lo[1], 0x7632);
+        if (S > 6) z[0][i] = __byte_perm(lo[0], lo[1], 0x5410);
+        if (S > 4) z[1][i] = __byte_perm(lo[0], lo[1], 0x7632);
         z[2][i] = __byte_perm(hi[0], hi[1], 0x5410);
         z[3][i] = __byte_perm(hi[0], hi[1], 0x7632);
     }
@@ -337,9 +355,9 @@ __device__ __forceinline__ void cut_store(const Cut &c, unsigned char *stage, i6
     cut_slice<ISA, 1, true>(c, stage, z[3]);
     cut_slice<ISA, 2, false>(c, stage, z[2]);
     cut_slice<ISA, 3, true>(c, stage, z[2]);
-    cut_slice<ISA, 4, false>(c, stage, z[1]);
-    cut_slice<ISA, 5, true>(c, stage, z[1]);
-    cut_slice<ISA, 6, false>(c, stage, z[0]);
+    if constexpr (S > 4) cut_slice<ISA, 4, false>(c, stage, z[1]);
+    if constexpr (S > 5) cut_slice<ISA, 5, true>(c, stage, z[1]);
+    if constexpr (S > 6) cut_slice<ISA, 6, false>(c, stage, z[0]);
 }
 
 __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
@@ -363,33 +381,45 @@ __device__ __forceinline__ uint32_t split8(float f, float &r) {
     return __float_as_uint(q);
 }
 
-// Adds sum_L D_L 2^(8 (7 - L)) shifted right by `sh` (11 .. 24) to the thread's
-// sums.  Levels 0 .. 2 stay within 2^22 and convert by an addition; 3 .. 5 split
-// into a multiple of 256 and a rest first (the conversion unit takes eight
-// clocks a warp).  The rests of 4 and 5 and levels 6 and 7 are below 2^22 in the
-// result's units and meet in FP32, good to 2^-2 of its last bit.
-__device__ __forceinline__ void drain(const Thread &t, int sh, i64 (&acc)[kCols]) {
-    const uint32_t m3 = 1u << (32 - sh);                    // level 3 (2^32)
-    const int m4 = 1 << (24 - sh);                          // level 4 (2^24)
-    const float f4 = __int_as_float((127 + 24 - sh) << 23);  // the same, 2^(24 - sh)
-    const float f5 = __int_as_float((127 + 16 - sh) << 23);  // level 5 (2^16)
-    const float f6 = __int_as_float((127 + 8 - sh) << 23);   // levels 6, 7 (2^8)
+// Adds sum_L D_L 2^(-8 L) in the units of the thread's sums, of which a product of
+// two items of scale 2^-62 has 2^(56 - sh) in level 0 (sh = 11 .. 24).
+//
+// Levels 0 .. 2 stay within 2^22 and convert by an addition; 3 .. 5 split into a
+// multiple of 256 and a rest first (the conversion unit takes eight clocks a
+// warp).  Of eight levels the rests of 4 and 5 and levels 6 and 7 are below 2^22 in
+// the result's units and meet in FP32, good to 2^-2 of its last bit.
+template <int S>
+__device__ __forceinline__ void drain(const Thread &t, uint32_t set, int sh, i64 (&acc)[kCols]) {
+    constexpr int levels = Digits<S>::levels;
+    const uint32_t m3 = 1u << (32 - sh);                     // level 3
+    const int m4 = 1 << (24 - sh);                           // level 4
+    const float f4 = __int_as_float((127 + 24 - sh) << 23);  // the same
+    const float f5 = __int_as_float((127 + 16 - sh) << 23);  // level 5
+    const float f6 = __int_as_float((127 + 8 - sh) << 23);   // level 6
+    const uint32_t tm = t.tm + set * 64u * levels;
 #pragma unroll
     for (int g = 0; g < kCols / 4; ++g) {
-        float f[kLevels][4];
+        float f[8][4];
 #pragma unroll
-        for (int L = 0; L < kLevels; ++L) tmem_ld4(t.tm + 64u * L + 4u * g, f[L]);
+        for (int L = 0; L < levels; ++L) tmem_ld4(tm + 64u * L + 4u * g, f[L]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            float r3, r4, r5;
-            const uint32_t q3 = split8(f[3][j], r3), q4 = split8(f[4][j], r4), q5 = split8(f[5][j], r5);
+            float r3;
+            const uint32_t q3 = split8(f[3][j], r3);
             const int h01 = (int)(biased_int(f[0][j]) * 256u + biased_int(f[1][j]) - 257u * kIntBias);
             const int h23 = (int)((biased_int(f[2][j]) + q3) * 256u + biased_int(r3) - 513u * kIntBias);
-            const int q45 = (int)(q4 * 256u + q5 - 257u * kIntBias);
-            float l = __fmaf_rn(__fmaf_rn(f[7][j], 0.00390625f, f[6][j]), f6, kMagic);
-            l = __fadd_rn(__fmaf_rn(r4, f4, __fmul_rn(r5, f5)), l);
-            const i64 v = (i64)q45 * m4 + (int)(__float_as_uint(l) - kIntBias) + acc[4 * g + j];
+            i64 v = acc[4 * g + j];
+            if constexpr (levels == 8) {
+                float r4, r5;
+                const uint32_t q4 = split8(f[4][j], r4), q5 = split8(f[5][j], r5);
+                const int q45 = (int)(q4 * 256u + q5 - 257u * kIntBias);
+                float l = __fmaf_rn(__fmaf_rn(f[7][j], 0.00390625f, f[6][j]), f6, kMagic);
+                l = __fadd_rn(__fmaf_rn(r4, f4, __fmul_rn(r5, f5)), l);
+                v += (i64)q45 * m4 + (int)(__float_as_uint(l) - kIntBias);
+            } else if constexpr (levels == 5) {
+                v += (i64)__float2int_rn(f[4][j]) * m4;
+            }
             acc[4 * g + j] = (i64)((u64)((i64)h01 * 65536 + h23) * (u64)m3 + (u64)v);
         }
     }
@@ -405,11 +435,12 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) {
 // their way while a stage is cut: those of A once A's are used, those of B once
 // B's are.  Before product n is touched, product n - 2 has to be finished, and
 // n - 1 too where `needs` says so.
-template <class W>
+template <int S, class W>
 __device__ __forceinline__ void cutter(Shared &s, Thread &t, const W &w, int nst, int kvalid) {
+    using D = Digits<S>;
     typename W::At at = w.first(), before = at;
     if (!w.more(at)) return;
-    uint32_t g = 0, n = 0, seen = 0;
+    uint32_t b = 0, round = 0, n = 0, seen = 0;
     int st = 0;
     Cut c;
     i64 va[8], vb[8];
@@ -419,24 +450,23 @@ __device__ __forceinline__ void cutter(Shared &s, Thread &t, const W &w, int nst
             if (t.ok) t.ok = warp_wait(&s.finished, seen & 1);
         Operand A, B;
         const bool imag = w.operands(at, A, B);
-        c = make_cut(t, A, B, imag);
+        c = make_cut<S>(t, A, B, imag);
     };
     begin();
     load_a(c, 0, va);
     load_b(c, 0, kvalid, vb);
     while (t.ok) {
-        const uint32_t b = g & 1;
-        if (g >= 2) t.ok = warp_wait(&s.done[b], ((g >> 1) - 1) & 1);
-        unsigned char *stage = t.smem + b * kStageB;
+        if (round > 0) t.ok = warp_wait(&s.done[b], (round - 1) & 1);
+        unsigned char *stage = t.smem + b * D::stage_bytes;
         const bool same = st + 1 < nst;  // the next stage is of this product
-        cut_store<true>(c, stage, va);
+        cut_store<S, true>(c, stage, va);
         if (same) load_a(c, st + 1, va);
-        cut_store<false>(c, stage, vb);
+        cut_store<S, false>(c, stage, vb);
         if (same) load_b(c, st + 1, kvalid, vb);
         tc::fence_proxy_async();
         __syncwarp();
         if (t.lane == 0) arrive(&s.full[b]);
-        ++g;
+        if (++b == D::stages) b = 0, ++round;
         if (same) {
             ++st;
             continue;
@@ -454,20 +484,22 @@ __device__ __forceinline__ void cutter(Shared &s, Thread &t, const W &w, int nst
 
 // The finishers' loop: the levels of every group of stages into the sums, then
 // w.epilogue (false ends).
-template <class W>
+template <int S, class W>
 __device__ __forceinline__ void finisher(Shared &s, Thread &t, const W &w, int nst, int sh) {
+    using D = Digits<S>;
     uint32_t groups = 0, n = 0;
     for (typename W::At at = w.first(); w.more(at); at = w.next(at), ++n) {
         i64 T[kCols];
 #pragma unroll
         for (int j = 0; j < kCols; ++j) T[j] = 0;
         for (int st = 0; st < nst; st += kGroup, ++groups) {
-            if (t.ok) t.ok = tc::mbar_wait(&s.ready, groups & 1, kWait);
+            const uint32_t set = groups % D::sets;
+            if (t.ok) t.ok = tc::mbar_wait(&s.ready[set], (groups / D::sets) & 1, kWait);
             tc::fence_after_sync();
-            drain(t, sh, T);
+            drain<S>(t, set, sh, T);
             tc::fence_before_sync();
             __syncwarp();
-            if (t.lane == 0) arrive(&s.drained);
+            if (t.lane == 0) arrive(&s.drained[set]);
         }
         if (!w.epilogue(at, T, n)) break;
         __syncwarp();
@@ -493,6 +525,7 @@ constexpr int kTerms = 3;
 struct Out {
     int buf;  // -1: none
     int plain, nterm;
+    int grid;  // E of complex64: 1 + the diagonal's real parts rounded to FP32
     Coef t;
     Term term[kTerms];
     Coef diag;
@@ -527,14 +560,17 @@ __device__ __forceinline__ int out_exponent(const Out &o, int eT, V view, bool &
 
 // A coefficient and the shift that its product needs, as one factor: the upper
 // half of v * factor is the term in the result's units.  The upper and lower
-// words of the factor are signed.
+// words of the factor are signed.  A coefficient of one is a shift alone.
 struct Factor {
     int hi, lo, pre;  // pre: left shift of v first (a short item meets a large result)
+    int sh;           // > 0: v >> sh, rounded
 };
+constexpr i64 kOne = 1ll << 61;
 __device__ __forceinline__ Factor make_factor(i64 m, int sr, int headroom) {
     const int s = min(sr, 63) - headroom;
     Factor f;
     f.pre = s < 0 ? -s : 0;
+    f.sh = m == kOne && s + 3 < 32 ? max(s, 0) + 3 : 0;
     if (s > 0) m = ((m >> (s - 1)) + 1) >> 1;
     f.lo = (int)(uint32_t)(u64)m;
     f.hi = (int)((m - f.lo) >> 32);
@@ -549,6 +585,17 @@ __device__ __forceinline__ i64 scaled(i64 v, const Factor &f) {
     const i64 mid = (i64)lo * f.hi + ((i64)hi * f.lo + 0x80000000ll);
     return (i64)hi * f.hi + (int)(mid >> 32);
 }
+template <int N>
+__device__ __forceinline__ void scale_add(const Factor &f, const i64 (&x)[N], i64 *acc, bool add) {
+    if (f.sh) {
+        const i64 half = 1ll << (f.sh - 1);
+#pragma unroll
+        for (int j = 0; j < N; ++j) acc[j] = ((x[j] + half) >> f.sh) + (add ? acc[j] : 0);
+    } else {
+#pragma unroll
+        for (int j = 0; j < N; ++j) acc[j] = scaled(x[j], f) + (add ? acc[j] : 0);
+    }
+}
 
 // One result, for this thread's columns of its row and plane: formed in place
 // of T, stored at dst (pieces qs apart, as those of the terms); returns the OR of
@@ -559,13 +606,13 @@ template <class V>
 __device__ __forceinline__ u64 put_out(const Out &o, const Thread &t, i64 (&T)[kCols], int eT, int e, V view,
                                        i64 plane, i64 qs, int row, int col0, int d, i64 *dst) {
     if (!o.plain) {
-        // T times its coefficient, then the terms, half of the columns at a time;
+        // T times its coefficient, then the terms, a quarter of the columns at a time;
         // the first loads go out before the multiplication.
-        const Factor ft = o.t.m ? make_factor(o.t.m, e - eT - o.t.e - 2, 0) : Factor{0, 0, 0};
-        constexpr int H = kCols / 2;
+        const Factor ft = o.t.m ? make_factor(o.t.m, e - eT - o.t.e - 2, 0) : Factor{0, 0, 0, 0};
+        constexpr int H = kCols / 4;
 #pragma unroll 1
         for (int k = 0; k < max(1, o.nterm); ++k) {
-            Factor f{0, 0, 0};
+            Factor f{0, 0, 0, 0};
             const i64 *q = nullptr;
             if (k < o.nterm) {
                 const View w = view(o.term[k].buf);
@@ -575,7 +622,7 @@ __device__ __forceinline__ u64 put_out(const Out &o, const Thread &t, i64 (&T)[k
                 f = make_factor((c.imag && t.p == 0) ? -c.m : c.m, e - (w.info.e - hr) - c.e - 2, hr);
             }
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            for (int h = 0; h < 4; ++h) {
                 i64 x[H];
                 if (q) {
 #pragma unroll
@@ -583,16 +630,17 @@ __device__ __forceinline__ u64 put_out(const Out &o, const Thread &t, i64 (&T)[k
                         load4(q + (h * H / 4 + i) * qs, x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
                 }
                 if (k == 0) {
+                    i64 v[H];
 #pragma unroll
-                    for (int j = 0; j < H; ++j) T[h * H + j] = scaled(T[h * H + j], ft);
+                    for (int j = 0; j < H; ++j) v[j] = T[h * H + j];
+                    scale_add<H>(ft, v, T + h * H, false);
                 }
                 if (q) {
                     if (f.pre) {
 #pragma unroll
                         for (int j = 0; j < H; ++j) x[j] = (i64)((u64)x[j] << f.pre);
                     }
-#pragma unroll
-                    for (int j = 0; j < H; ++j) T[h * H + j] += scaled(x[j], f);
+                    scale_add<H>(f, x, T + h * H, true);
                 }
             }
         }
@@ -601,6 +649,14 @@ __device__ __forceinline__ u64 put_out(const Out &o, const Thread &t, i64 (&T)[k
 #pragma unroll
             for (int j = 0; j < kCols; ++j)
                 if (row == col0 + j) T[j] += x;
+        }
+        if (o.grid && t.p == 0 && row < d && row >= col0 && row < col0 + kCols) {
+#pragma unroll
+            for (int j = 0; j < kCols; ++j)
+                if (row == col0 + j) {
+                    const float u = (float)(1.0 + scalbn((double)T[j], e - 62));
+                    T[j] = __double2ll_rn(scalbn((double)u - 1.0, 62 - e));
+                }
         }
     }
     u64 m = 0;
@@ -650,13 +706,15 @@ __device__ __forceinline__ void setup(Shared &s, Thread &t, unsigned char *raw) 
         tc::tmem_relinquish();
     }
     if (t.tid == 0) {
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < kMaxStages; ++b) {
             tc::mbar_init(&s.full[b], kCutters / 32);
             tc::mbar_init(&s.done[b], 1);
         }
-        tc::mbar_init(&s.drained, kFinishers / 32);
+        for (int b = 0; b < 2; ++b) {
+            tc::mbar_init(&s.ready[b], 1);
+            tc::mbar_init(&s.drained[b], kFinishers / 32);
+        }
         tc::mbar_init(&s.finished, kFinishers / 32);
-        tc::mbar_init(&s.ready, 1);
         tc::mbar_init(&s.last, 1);
         tc::fence_mbar_init();
     }
@@ -667,17 +725,17 @@ __device__ __forceinline__ void setup(Shared &s, Thread &t, unsigned char *raw) 
 }
 
 // A launch: every role over the products of w (`products` of them for this CTA).
-template <class W>
+template <int S, class W>
 __device__ __forceinline__ void run(Shared &s, Thread &t, const W &w, i64 products, int nst, int kvalid, int sh) {
     if (t.tid >= kIssuer) {
         regs_down<kRegsIssue>();
-        if (t.tid == kIssuer) t.ok = issue_products(s, t.smem, products, nst);
+        if (t.tid == kIssuer) t.ok = issue_products<S>(s, t.smem, products, nst);
     } else if (t.tid >= kFinishers) {
         regs_down<kRegsCut>();
-        cutter(s, t, w, nst, kvalid);
+        cutter<S>(s, t, w, nst, kvalid);
     } else {
         regs_up<kRegsFinish>();
-        finisher(s, t, w, nst, sh);
+        finisher<S>(s, t, w, nst, sh);
     }
 }
 

@@ -207,7 +207,8 @@ static Parament_ErrorCode set_hamiltonian(Ctx *c, const void *H0, const void *H1
     c->stack.release();
     c->split_stack.release();
     c->fx_stack.release();
-    c->fx_ready = false;
+    c->fx_split.release();
+    c->fx_ready = c->fx_split_ready = false;
     if (use_magnus) {
         c->magnus = true;
         if (quad != PARAMENT_QUADRATURE_SIMPSON) return c->last_error = PARAMENT_STATUS_INVALID_QUADRATURE_SELECTION;
@@ -265,7 +266,7 @@ static Parament_ErrorCode set_hamiltonian(Ctx *c, const void *H0, const void *H1
     }
     c->dim = dim;
     c->Ke = Ke;
-    if (e == cudaSuccess && c->fp64) fx_prepare(c);
+    if (e == cudaSuccess) fx_prepare(c);
     if (use_magnus) note_call_end(c, c->stream, true);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
@@ -302,14 +303,15 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
     // product per CTA, combined by the double-float tree.  Where the planes
     // (up to 2.3 GB) cannot be allocated, the FP32 SIMT kernel below runs,
     // which needs only the chunk buffers.
-    // complex128: exact sliced products on the tensor cores (fx.cu).  Without
-    // room for their workspace the FP64 kernels below run; of those the cluster
-    // kernel, which needs the least memory, where it applies.
+    // Exact sliced products on the tensor cores (fx.cu).  Without room for their
+    // workspace the kernels below run; of those the cluster kernel, which needs
+    // the least memory, where it applies.
     bool no_room = false;
-    if (fx_applies(c, M)) {
+    const FxForm form = c->fp64 ? FxForm::kFp64 : FxForm::kPlain32;
+    if (fx_applies(c, form, M, h * c->hnorm)) {
         no_room = !fx_ensure(c, P);
         if (!no_room) {
-            if (run_fx(c, d_carr, w, h * c->hnorm, M, P, d_out, stream) == cudaSuccess) return PARAMENT_STATUS_SUCCESS;
+            if (run_fx(c, form, d_carr, w, h * c->hnorm, M, P, d_out, stream) == cudaSuccess) return PARAMENT_STATUS_SUCCESS;
             cudaGetLastError();
             return PARAMENT_STATUS_CUBLAS_FAILED;
         }

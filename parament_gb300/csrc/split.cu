@@ -566,6 +566,7 @@ static Parament_ErrorCode prepare_split_stack(Ctx *c) {
         k_split_stack<<<512, 256, 0, c->stream>>>(s64, static_cast<float2 *>(c->split_stack.ptr), (long long)n);
         e = cudaGetLastError();
     }
+    if (e == cudaSuccess) fx_prepare_split(c);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     tmp.release();
     // Exact (anti-)Hermitian symmetry of the complex64 stack: H_0 and H_k
@@ -605,6 +606,13 @@ Parament_ErrorCode run_split(Ctx *c, const void *d_carr, unsigned pts, unsigned 
     if (M > kSplitMaxOrder || c->hnorm * h > kSplitMaxX) return PARAMENT_STATUS_SELECT_SMALLER_DT;
     Parament_ErrorCode r = prepare_split_stack(c);
     if (r != PARAMENT_STATUS_SUCCESS) return r;
+    if (fx_applies(c, FxForm::kSplit32, M, c->hnorm * h) && fx_ensure(c, P)) {
+        const WeightSpecHost w{pts, (int)c->K, (int)amps, c->quad, c->magnus ? 1 : 0, h / 12.0};
+        if (run_fx(c, FxForm::kSplit32, d_carr, w, c->hnorm * h, M, P, d_out, stream) == cudaSuccess)
+            return PARAMENT_STATUS_SUCCESS;
+        cudaGetLastError();
+        return PARAMENT_STATUS_CUBLAS_FAILED;
+    }
     SplitArgs a;
     double c0[2];
     std::vector<double> mu;

@@ -1,4 +1,4 @@
-"""complex128 by exact sliced products (fx.cu), d >= 17, against the oracle's
+"""Exact sliced products (fx.cu): complex128, d >= 17 (and complex64, d > 64, below), against the oracle's
 FP64 arithmetic: tile edges (17, 63, 64, 65, 128, 129), chunk counts around the
 number of SMs and the batch length, every evaluation of the polynomial (powers
 in X^2 and X^3, Clenshaw above x = 1, manual orders), non-Hermitian matrices and
@@ -128,3 +128,63 @@ def test_device_entry_point_and_reuse(built_lib):
             U = ctx.equiprop_device(1e-3, x, stream=st)
             ctx.synchronize()
             assert relerr(U.cpu().numpy(), oracle.equiprop(H0, H1, u[:, :P], 1e-3)[0]) < tol(P)
+
+
+# ------------------------------------------------------------------ complex64, d > 64
+
+def c64(*arrays):
+    return [np.asarray(a).astype(np.complex64).astype(np.complex128) for a in arrays]
+
+
+def propagate32(H0, H1, u, dt, magnus=False, quad="none", cycles=None, form="plain"):
+    import parament_gb300 as parament
+    with parament.Parament("fp32") as ctx:
+        ctx.set_precision_mode(form)
+        ctx.set_hamiltonian(H0, *H1, use_magnus=magnus, quadrature_mode=quad)
+        if cycles:
+            ctx.set_iteration_cycles_manually(cycles)
+        U = ctx.equiprop(dt, *u)
+        return U.astype(np.complex128), ctx.last_iteration_cycles
+
+
+@pytest.mark.parametrize("d", [65, 96, 128, 129, 200, 300])
+@pytest.mark.parametrize("P,quad,magnus", [(1, "none", False), (2, "midpoint", False), (21, "simpson", True)])
+@pytest.mark.parametrize("form", ["plain", "split"])
+def test_complex64_forms_above_64(built_lib, d, P, quad, magnus, form):
+    """The plain form within 1e-5 of the oracle at the complex64 order, the split
+    form within 1e-6 of the FP64 oracle at its order (the bars of these forms)."""
+    n = 2 * P + 1 if quad == "simpson" else P + (quad == "midpoint")
+    H0, H1, u = c64(*problem(d, 2, n, 4.0))
+    U, M = propagate32(H0, H1, u, 1e-3, magnus, quad, form=form)
+    mode = {"none": oracle.NONE, "midpoint": oracle.MIDPOINT, "simpson": oracle.SIMPSON}[quad]
+    Uo, Mo = oracle.equiprop(H0, H1, u, 1e-3, magnus=magnus, mode=mode, single=form == "plain",
+                             M=M if form == "split" else 0)[:2]
+    assert M == Mo
+    assert relerr(U, Uo) < (1e-5 if form == "plain" else 1e-6)
+
+
+@pytest.mark.parametrize("dt,cycles", [(1e-5, None), (1e-3, None), (1e-2, None), (4e-2, None), (0.1, None),
+                                       (1e-3, 3), (1e-3, 7), (1e-3, 9), (1e-3, 15)])
+def test_complex64_orders_above_64(built_lib, dt, cycles):
+    """Powers of X up to x = 1, the Clenshaw kernels above."""
+    H0, H1, u = c64(*problem(80, 2, 5, 3.0))
+    U, M = propagate32(H0, H1, u / 2, dt, cycles=cycles)
+    Uo, Mo = oracle.equiprop(H0, H1, u / 2, dt, single=True, M=cycles or 0)[:2]
+    assert M == Mo
+    assert relerr(U, Uo) < 1e-5
+
+
+@pytest.mark.parametrize("form", ["plain", "split"])
+def test_complex64_general_matrices_and_complex_controls(built_lib, form):
+    H0, H1, u = problem(90, 18, 17, 2.0, hermitian=False)
+    H0, H1, u = c64(H0, H1, (u + 1j * np.roll(u, 1, axis=1)) / 20)
+    U, M = propagate32(H0, H1, u, 1e-4, form=form)
+    Uo = oracle.equiprop(H0, H1, u, 1e-4, single=form == "plain", M=M)[0]
+    assert relerr(U, Uo) < (1e-5 if form == "plain" else 1e-6)
+
+
+@pytest.mark.parametrize("form", ["plain", "split"])
+def test_complex64_samples_that_are_not_finite(built_lib, form):
+    H0, H1, u = c64(*problem(70, 2, 9, 2.0))
+    u[1, 4] = np.nan
+    assert np.isnan(propagate32(H0, H1, u, 1e-3, form=form)[0]).all()
