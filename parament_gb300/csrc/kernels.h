@@ -33,6 +33,7 @@ struct StepLaunch {
     int M;                    // odd Chebyshev order
     const double *J;          // 2*(M+1) doubles: (-i)^k J_k(x), k=0..M
     double s;                 // 2 / Hnorm
+    double x;                 // Hnorm h, where the polynomial may run by powers of X (0: by Clenshaw)
     const void *stack;        // (1+Ke) d x d matrices, context precision
     const void *carr;         // amps x pts samples, context precision
     void *chunks;             // nchunks d x d products (output)

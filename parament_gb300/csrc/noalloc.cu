@@ -157,6 +157,7 @@ extern "C" Parament_ErrorCode Parament_equipropNoAlloc_fp64(Parament_Context_f64
     l.M = M;
     l.J = J.data();
     l.s = 2.0 / c->hnorm;
+    l.x = h * c->hnorm;
     l.stack = c->stack.ptr;
     l.carr = d_carr;
     l.chunks = chunks;

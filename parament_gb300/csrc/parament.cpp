@@ -390,6 +390,7 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
         l.chunks = c->chunks.ptr;
         l.P = P;
         l.nchunks = nch;
+        l.x = h * c->hnorm;
         l.stream = stream;
         if (c->timing) cudaEventRecord(c->ev_start, stream);
         e = launch_small_steps(l);

@@ -9,9 +9,20 @@
 // batched Clenshaw GEMMs plus diagonal adds (src/cuda/parament.cpp:569-652,
 // src/cuda/diagonal_add.cu:21-51) and the lower levels of the tree product
 // (src/cuda/parament.cpp:657-718).
+//
+// For x = Hnorm h <= 1 and orders from 5 on the polynomial is evaluated by powers
+// of X (as in step_group.cu, with the same coefficients),
+//     Y = X^2,  r = c_M X Y + c_(M-1) Y + c_(M-2) X + c_(M-3),
+//     r <- r Y + c_(k+1) X + c_k,
+// (M + 1) / 2 products instead of M - 1; at order 3 both take two.  The products are
+// what the kernel spends its time on (the FP64 pipe in complex128, shared-memory
+// loads and FMAs in complex64): d = 16, K = 2, 4096 steps in complex128 (order 5),
+// 777 -> 640 us.
 #include <algorithm>
+#include <vector>
 
 #include "common.cuh"
+#include "ctx.h"
 #include "kernels.h"
 
 namespace pgb {
@@ -19,6 +30,7 @@ namespace pgb {
 template <class R>
 struct SmallArgs {
     cplx_t<R> J[kMaxOrder + 1];
+    R c[kMaxOrder + 1];  // by powers: c_n (odd n: times i); c_0 of E (complex128) or of U - J_0
     const cplx_t<R> *stack;
     const cplx_t<R> *carr;
     cplx_t<R> *chunks;
@@ -30,7 +42,7 @@ struct SmallArgs {
 };
 
 // Complex64 instances keep to 128 registers so that two CTAs share an SM.
-template <class R, int TM>
+template <class R, int TM, bool POWERS>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_small_steps(const __grid_constant__ SmallArgs<R> a) {
     using C = cplx_t<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -62,51 +74,116 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_small_steps(con
     for (long long st = s0; st < s1; ++st) {
         for (int m = tid; m < a.Ke; m += blockDim.x) ws[m] = step_weight(a.carr, a.w, m, st);
         __syncthreads();
-        // X = H0 + sum_m w_m H_m (own elements), straight from the L2-resident
-        // stack; b_M = J[M] I and b_(M-1) = s J[M] X + J[M-1] I need only the
-        // thread's own elements, so they are formed in the same pass.
+        if constexpr (POWERS) {
+            // complex64 forms U, adding J_0 last, as the recurrence below does;
+            // complex128 forms E = U - I.
+            constexpr bool kHasU = sizeof(R) == 4;
+            C x[TM][TM];
 #pragma unroll
-        for (int i = 0; i < TM; ++i)
+            for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int j = 0; j < TM; ++j) {
-                if (!own[i][j]) continue;
-                const int e = eo[i][j];
-                const int ge = (ty + 16 * i) * d + tx + 16 * j;
-                C v = a.stack[ge];
-                for (int m = 0; m < a.Ke; ++m) cfma(v, ws[m], a.stack[(size_t)(m + 1) * dd + ge]);
-                Xs[e] = v;
-                C bm1 = cscale(cmul(a.J[M], v), s);
-                if (diag[i][j]) bm1 = cadd(bm1, a.J[M - 1]);
-                if (M == 1) {
-                    acc[i][j] = bm1;  // U = s J[1] X + J[0] I, since b_2 = 0
-                } else {
-                    b2[i][j] = diag[i][j] ? a.J[M] : mk<C>(0.0, 0.0);
-                    Bs[e] = bm1;
+                for (int j = 0; j < TM; ++j) {
+                    if (!own[i][j]) continue;
+                    const int ge = (ty + 16 * i) * d + tx + 16 * j;
+                    C v = a.stack[ge];
+                    for (int m = 0; m < a.Ke; ++m) cfma(v, ws[m], a.stack[(size_t)(m + 1) * dd + ge]);
+                    x[i][j] = v;
+                    Xs[eo[i][j]] = v;
                 }
-            }
-        if (M > 1) {
             __syncthreads();
-            for (int k = M - 2; k >= 0; --k) {
-                tile_gemm<C, TM>(acc, Bs, Xs, d, ld, ty, tx);
+            tile_gemm<C, TM>(acc, Xs, Xs, d, ld, ty, tx);
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TM; ++j)
+                    if (own[i][j]) Bs[eo[i][j]] = b2[i][j] = acc[i][j];  // Y
+            __syncthreads();
+            tile_gemm<C, TM>(acc, Xs, Bs, d, ld, ty, tx);
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TM; ++j) {
+                    if (!own[i][j]) continue;
+                    const C q = acc[i][j], y = b2[i][j], v = x[i][j];
+                    C r;
+                    r.x = fma(a.c[M - 1], y.x, -a.c[M] * q.y) - a.c[M - 2] * v.y;
+                    r.y = fma(a.c[M - 1], y.y, a.c[M] * q.x) + a.c[M - 2] * v.x;
+                    if (diag[i][j]) r.x += a.c[M - 3];
+                    acc[i][j] = r;
+                }
+            for (int k = M - 5; k >= 0; k -= 2) {
                 __syncthreads();
-                const R beta = (k == 0) ? (R)-2 : (R)-1;
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TM; ++j)
+                        if (own[i][j]) Xs[eo[i][j]] = acc[i][j];
+                __syncthreads();
+                tile_gemm<C, TM>(acc, Xs, Bs, d, ld, ty, tx);
 #pragma unroll
                 for (int i = 0; i < TM; ++i)
 #pragma unroll
                     for (int j = 0; j < TM; ++j) {
                         if (!own[i][j]) continue;
-                        C v = cscale(acc[i][j], s);
-                        v.x += beta * b2[i][j].x;
-                        v.y += beta * b2[i][j].y;
-                        if (diag[i][j]) v = cadd(v, a.J[k]);
-                        if (k > 0) {
-                            b2[i][j] = Bs[eo[i][j]];
-                            Bs[eo[i][j]] = v;
-                        } else {
-                            acc[i][j] = v;  // U_j
+                        C r = acc[i][j];
+                        r.x = fma(-a.c[k + 1], x[i][j].y, r.x);
+                        r.y = fma(a.c[k + 1], x[i][j].x, r.y);
+                        if (diag[i][j]) {
+                            r.x += a.c[k];
+                            if (kHasU && k == 0) r.x += a.J[0].x;
+                            if (!kHasU && k == 0 && st == s0) r.x += (R)1;  // the first step's P
                         }
+                        acc[i][j] = r;
                     }
-                if (k > 0) __syncthreads();
+            }
+            __syncthreads();
+        } else {
+            // X = H0 + sum_m w_m H_m (own elements), straight from the L2-resident
+            // stack; b_M = J[M] I and b_(M-1) = s J[M] X + J[M-1] I need only the
+            // thread's own elements, so they are formed in the same pass.
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TM; ++j) {
+                    if (!own[i][j]) continue;
+                    const int e = eo[i][j];
+                    const int ge = (ty + 16 * i) * d + tx + 16 * j;
+                    C v = a.stack[ge];
+                    for (int m = 0; m < a.Ke; ++m) cfma(v, ws[m], a.stack[(size_t)(m + 1) * dd + ge]);
+                    Xs[e] = v;
+                    C bm1 = cscale(cmul(a.J[M], v), s);
+                    if (diag[i][j]) bm1 = cadd(bm1, a.J[M - 1]);
+                    if (M == 1) {
+                        acc[i][j] = bm1;  // U = s J[1] X + J[0] I, since b_2 = 0
+                    } else {
+                        b2[i][j] = diag[i][j] ? a.J[M] : mk<C>(0.0, 0.0);
+                        Bs[e] = bm1;
+                    }
+                }
+            if (M > 1) {
+                __syncthreads();
+                for (int k = M - 2; k >= 0; --k) {
+                    tile_gemm<C, TM>(acc, Bs, Xs, d, ld, ty, tx);
+                    __syncthreads();
+                    const R beta = (k == 0) ? (R)-2 : (R)-1;
+#pragma unroll
+                    for (int i = 0; i < TM; ++i)
+#pragma unroll
+                        for (int j = 0; j < TM; ++j) {
+                            if (!own[i][j]) continue;
+                            C v = cscale(acc[i][j], s);
+                            v.x += beta * b2[i][j].x;
+                            v.y += beta * b2[i][j].y;
+                            if (diag[i][j]) v = cadd(v, a.J[k]);
+                            if (k > 0) {
+                                b2[i][j] = Bs[eo[i][j]];
+                                Bs[eo[i][j]] = v;
+                            } else {
+                                acc[i][j] = v;  // U_j
+                            }
+                        }
+                    if (k > 0) __syncthreads();
+                }
             }
         }
         // Chunk product P <- U_j P (later step on the left).
@@ -128,7 +205,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_small_steps(con
                 for (int j = 0; j < TM; ++j)
                     if (own[i][j]) {
                         C u = acc[i][j];
-                        if (diag[i][j]) u.x -= (R)1;
+                        if (diag[i][j] && !(POWERS && sizeof(R) == 8)) u.x -= (R)1;
                         Bs[eo[i][j]] = u;
                     }
             __syncthreads();
@@ -154,30 +231,34 @@ size_t small_smem_bytes(bool fp64, int d, int Ke) {
 }
 
 template <class R, int TM>
-static const void *small_kernel_ptr() {
-    return reinterpret_cast<const void *>(&k_small_steps<R, TM>);
+static const void *small_kernel_ptr(bool powers) {
+    return powers ? reinterpret_cast<const void *>(&k_small_steps<R, TM, true>)
+                  : reinterpret_cast<const void *>(&k_small_steps<R, TM, false>);
 }
 
-static const void *pick_small(bool fp64, int d) {
+static const void *pick_small(bool fp64, int d, bool powers) {
     int tm = (d + 15) / 16;
     if (fp64) {
         switch (tm) {
-            case 1: return small_kernel_ptr<double, 1>();
-            case 2: return small_kernel_ptr<double, 2>();
-            case 3: return small_kernel_ptr<double, 3>();
-            default: return small_kernel_ptr<double, 4>();
+            case 1: return small_kernel_ptr<double, 1>(powers);
+            case 2: return small_kernel_ptr<double, 2>(powers);
+            case 3: return small_kernel_ptr<double, 3>(powers);
+            default: return small_kernel_ptr<double, 4>(powers);
         }
     }
     switch (tm) {
-        case 1: return small_kernel_ptr<float, 1>();
-        case 2: return small_kernel_ptr<float, 2>();
-        case 3: return small_kernel_ptr<float, 3>();
-        default: return small_kernel_ptr<float, 4>();
+        case 1: return small_kernel_ptr<float, 1>(powers);
+        case 2: return small_kernel_ptr<float, 2>(powers);
+        case 3: return small_kernel_ptr<float, 3>(powers);
+        default: return small_kernel_ptr<float, 4>(powers);
     }
 }
 
+// The polynomial by powers of X: l.x is set, and it saves products.
+static bool small_powers(const StepLaunch &l) { return l.x > 0.0 && l.x <= 1.0 && l.M >= 5; }
+
 int small_chunk_count(bool fp64, int d, int Ke, long long P, int num_sms) {
-    const void *fn = pick_small(fp64, d);
+    const void *fn = pick_small(fp64, d, true);
     size_t smem = small_smem_bytes(fp64, d, Ke);
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int per_sm = 0;
@@ -202,7 +283,19 @@ static cudaError_t launch_small_t(const StepLaunch &l) {
     a.s = (R)l.s;
     a.w = WeightSpec{l.w.pts, l.w.K, l.w.amps, l.w.mode, l.w.magnus, l.w.hfac};
     size_t smem = small_smem_bytes(l.fp64, l.d, l.Ke);
-    const void *fn = pick_small(l.fp64, l.d);
+    const bool powers = small_powers(l);
+    if (powers && l.fp64) {
+        double c0[2];
+        std::vector<double> mu;
+        power_coefficients(l.M, l.x, 2.0 / l.s, c0, mu);
+        a.c[0] = (R)c0[0];
+        for (int n = 1; n <= l.M; ++n) a.c[n] = (R)mu[2 * n + (n & 1)];
+    } else if (powers) {
+        std::vector<double> c;
+        plain_coefficients(l.M, l.x, 2.0 / l.s, c);
+        for (int n = 0; n <= l.M; ++n) a.c[n] = (R)c[n];
+    }
+    const void *fn = pick_small(l.fp64, l.d, powers);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     void *args[] = {&a};
