@@ -332,6 +332,7 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
         l.carr = d_carr;
         l.chunks = c->chunks.ptr;
         l.P = P;
+        l.x = h * c->hnorm;
         l.stream = stream;
         int nch = 0;
         e = launch_small_tc(l, c->num_sms, static_cast<float *>(c->xplanes.ptr), c->d_fault, &nch,

@@ -25,6 +25,14 @@
 //     hands the product to the tensor core and forms b_k from its levels in
 //     FP32.  U_j - I and P then make the chunk product; P stays in tensor
 //     memory.  The planes of step j + 1 arrive by bulk copy while step j runs.
+// For x = Hnorm h <= 1 and orders from 5 on the polynomial runs by powers of X with
+// the coefficients of the other complex64 step kernels (step_group.cu):
+//     Y = X X,  r = c_M X Y + c_(M-1) Y + c_(M-2) X + c_(M-3),  r <- r Y + c_(k+1) X + c_k,
+// U_j = r: (M + 1) / 2 products instead of M - 1, and the slices of Y stay in place
+// as the B operand of all but the first.  The odd coefficients are imaginary: i X Y
+// comes from the product itself (its i A B form), i X from the other plane of X.
+// d = 64 Magnus, order 5, 8192 steps: 1.43 -> 1.22 ms.
+//
 // Each thread keeps one plane of 16 columns of one row (tc_slice.cuh), so the
 // Clenshaw updates work plane by plane: s is real and J_k I touches the
 // diagonal only.  Every wait is bounded; a wait that runs out stops the CTA and
@@ -32,8 +40,10 @@
 #include <stdlib.h>
 
 #include <algorithm>
+#include <vector>
 
 #include "common.cuh"
+#include "ctx.h"
 #include "kernels.h"
 #include "tc_slice.cuh"
 
@@ -54,6 +64,8 @@ static_assert(kStcXBytes % 16 == 0 && (kStcSA + kStcSB) % 1024 == 0, "plane buff
 
 struct SmallTcArgs {
     float2 J[kMaxOrder + 1];  // (-i)^k J_k(x) in complex64
+    float c[kMaxOrder + 1];   // by powers: c_n (odd n: times i), c_0 without J_0
+    int powers;
     const float *xplanes;     // planes of the batch's steps, kSmallXStride floats apart
     float2 *chunks;           // nchunks products, row-major complex64
     long long P;              // steps of the batch
@@ -205,30 +217,81 @@ __global__ void __launch_bounds__(kTcdThreads, 1) k_small_tc(const __grid_consta
                 }
             }
         }
-        // Every thread has read the planes (the barrier in reduce_max), so the
-        // copy of step i + 1 may overwrite them.
-        tc::fence_proxy_async();
-        reduce_max<true, false>(sh, t, nb, X, X);
-        if (i + 1 < n) issue_x(i + 1);
-        store_a<kStcSlices, false>(sh, SA, t, nb, X, X);
-        nb ^= 1;
         bool live = true;
-        for (int k = M - 2; k >= 0; --k) {
-            reduce_max<false, true>(sh, t, nb, X, b1);
-            store_b<kStcSlices, false>(SB, t, sh.bmax[nb], b1, b1, sh.colmul);
+        if (a.powers) {
+            // b1: r; b2: Y, then i X of this plane.
+            {
+                const float4 *oth =
+                    reinterpret_cast<const float4 *>(XP + (1 - t.p) * kStcPlane + t.r * kStcPlaneLd + t.c0);
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    const float4 y = oth[g];
+                    b2[4 * g] = sgn * y.x;
+                    b2[4 * g + 1] = sgn * y.y;
+                    b2[4 * g + 2] = sgn * y.z;
+                    b2[4 * g + 3] = sgn * y.w;
+                }
+            }
+            tc::fence_proxy_async();
+            reduce_max<true, true>(sh, t, nb, X, X);
+            if (i + 1 < n) issue_x(i + 1);
+            store_a<kStcSlices, false>(sh, SA, t, nb, X, X);
+            store_b<kStcSlices, false>(SB, t, sh.bmax[nb], X, X, sh.colmul);
             nb ^= 1;
-            if (!(live = run_product(sh, t, SA, SB, kStcSlices, kStcSlices, kStcSlices - 1, false, ncommit, ok)))
-                break;
-            float D[16];
-            epilogue_f<kStcSlices - 1>(sh, t, D);
-            const float beta = k == 0 ? -2.0f : -1.0f, jk = jp(k);
+            if (!run_product(sh, t, SA, SB, kStcSlices, kStcSlices, kStcSlices - 1, false, ncommit, ok)) break;
+            epilogue_f<kStcSlices - 1>(sh, t, X);  // Y
+            reduce_max<false, true>(sh, t, nb, X, X);
+            store_b<kStcSlices, false>(SB, t, sh.bmax[nb], X, X, sh.colmul);
+            nb ^= 1;
+            if (!run_product(sh, t, SA, SB, kStcSlices, kStcSlices, kStcSlices - 1, true, ncommit, ok)) break;
+            epilogue_f<kStcSlices - 1>(sh, t, b1);  // i X Y
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-                float v = D[j] * s;
-                v += beta * b2[j];
-                if (t.c0 + j == t.r) v += jk;
-                b2[j] = b1[j];
-                b1[j] = v;  // k = 0: U_j
+                const bool dg = t.p == 0 && t.c0 + j == t.r;
+                b1[j] = fmaf(a.c[M - 1], X[j], a.c[M] * b1[j]) + fmaf(a.c[M - 2], b2[j], dg ? a.c[M - 3] : 0.0f);
+            }
+            for (int k = M - 5; k >= 0; k -= 2) {
+                reduce_max<true, false>(sh, t, nb, b1, b1);
+                store_a<kStcSlices, false>(sh, SA, t, nb, b1, b1);
+                nb ^= 1;
+                if (!(live = run_product(sh, t, SA, SB, kStcSlices, kStcSlices, kStcSlices - 1, false, ncommit, ok)))
+                    break;
+                epilogue_f<kStcSlices - 1>(sh, t, b1);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    float v = fmaf(a.c[k + 1], b2[j], b1[j]);
+                    if (t.p == 0 && t.c0 + j == t.r) {
+                        v += a.c[k];
+                        if (k == 0) v += a.J[0].x;
+                    }
+                    b1[j] = v;
+                }
+            }
+        } else {
+            // Every thread has read the planes (the barrier in reduce_max), so the
+            // copy of step i + 1 may overwrite them.
+            tc::fence_proxy_async();
+            reduce_max<true, false>(sh, t, nb, X, X);
+            if (i + 1 < n) issue_x(i + 1);
+            store_a<kStcSlices, false>(sh, SA, t, nb, X, X);
+            nb ^= 1;
+            for (int k = M - 2; k >= 0; --k) {
+                reduce_max<false, true>(sh, t, nb, X, b1);
+                store_b<kStcSlices, false>(SB, t, sh.bmax[nb], b1, b1, sh.colmul);
+                nb ^= 1;
+                if (!(live = run_product(sh, t, SA, SB, kStcSlices, kStcSlices, kStcSlices - 1, false, ncommit, ok)))
+                    break;
+                float D[16];
+                epilogue_f<kStcSlices - 1>(sh, t, D);
+                const float beta = k == 0 ? -2.0f : -1.0f, jk = jp(k);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    float v = D[j] * s;
+                    v += beta * b2[j];
+                    if (t.c0 + j == t.r) v += jk;
+                    b2[j] = b1[j];
+                    b1[j] = v;  // k = 0: U_j
+                }
             }
         }
         if (!live) break;
@@ -308,6 +371,12 @@ cudaError_t launch_small_tc(const StepLaunch &l, int num_sms, float *xplanes, in
     a.xplanes = xplanes;
     a.M = l.M;
     a.s = (float)l.s;
+    a.powers = l.x > 0.0 && l.x <= 1.0 && l.M >= 5;
+    if (a.powers) {
+        std::vector<double> c;
+        plain_coefficients(l.M, l.x, 2.0 / l.s, c);
+        for (int n = 0; n <= l.M; ++n) a.c[n] = (float)c[n];
+    }
     a.fault = fault;
     const WeightSpec w{l.w.pts, l.w.K, l.w.amps, l.w.mode, l.w.magnus, l.w.hfac};
     const float2 *stack = static_cast<const float2 *>(l.stack);
