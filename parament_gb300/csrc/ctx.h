@@ -52,7 +52,8 @@ struct Ctx {
 
     // Fixed-point form (fx.cu): the stack as integers, that of the split form,
     // and the workspace of a propagation.
-    DevBuf fx_stack, fx_split, fx_ws;
+    void *fx_stack = nullptr;  // behind the matrices of `stack`, in its allocation
+    DevBuf fx_split, fx_ws;
     bool fx_ready = false, fx_split_ready = false;
 
     // Instrumentation: CUDA events around the dominant kernel of the last call
@@ -64,6 +65,10 @@ struct Ctx {
     // Work buffers (grow-only, like src/cuda/parament.cpp:418-474)
     DevBuf carr, out, chunks, work, X, B1, B2, aux, grad, wts, xplanes;
     DevBuf arrived;  // pair counters of the small groups' tree, zero between launches
+
+    // Pinned memory that kernels reach directly: samples and result of small
+    // host-buffer calls.
+    void *h_stage = nullptr, *d_stage = nullptr;
 
     // Bounded-wait faults of this context's tensor-core kernels.  The kernels
     // add to a device counter (d_fault, zero at creation, never reset); after
@@ -84,7 +89,7 @@ struct Ctx {
     size_t esize() const { return fp64 ? 16 : 8; }
     size_t device_bytes() const {
         return stack.cap + split_stack.cap + carr.cap + out.cap + chunks.cap + work.cap + X.cap + B1.cap + B2.cap +
-               aux.cap + grad.cap + wts.cap + xplanes.cap + fx_stack.cap + fx_split.cap + fx_ws.cap +
+               aux.cap + grad.cap + wts.cap + xplanes.cap + fx_split.cap + fx_ws.cap +
                arrived.cap;
     }
     void release_all() {
@@ -101,7 +106,6 @@ struct Ctx {
         grad.release();
         wts.release();
         xplanes.release();
-        fx_stack.release();
         fx_split.release();
         fx_ws.release();
         arrived.release();
@@ -139,6 +143,7 @@ double plain_coefficients(int M, double x, double hnorm, std::vector<double> &c)
 // workspace of P steps, run_fx propagates (x = Hnorm h).
 struct WeightSpecHost;
 enum class FxForm { kFp64, kPlain32, kSplit32 };
+size_t fx_stack_bytes(const Ctx *c, unsigned dim, unsigned Ke);  // 0: none is kept
 void fx_prepare(Ctx *c);
 void fx_prepare_split(Ctx *c);
 bool fx_applies(const Ctx *c, FxForm form, int M, double x);

@@ -690,39 +690,50 @@ static bool fx_serves(FxForm form, int d) {
     return d > 64 && (form == FxForm::kSplit32 || d < 256 || d % 128 != 0);
 }
 
-// A stack in fixed point, on the context's stream (the caller waits for it).
-// Without room for it the other kernels serve.
+static size_t fixed_bytes(unsigned dim, unsigned Ke) {
+    const size_t dp = (dim + 63) / 64 * 64, n = 1 + (size_t)Ke;
+    return stack_head((int)n) + sizeof(i64) * 2 * dp * dp * n;
+}
+
+// A stack in fixed point at dst, on the context's stream (the caller waits for it).
 template <class C>
-static bool convert_stack(Ctx *c, const void *stack, DevBuf &buf) {
+static bool convert_stack(Ctx *c, const void *stack, void *dst) {
     const int d = (int)c->dim, dp = (d + 63) / 64 * 64, n = 1 + (int)c->Ke;
-    const size_t head = stack_head(n), bytes = head + sizeof(i64) * 2 * (size_t)dp * dp * n;
-    void *p = nullptr;
-    if (cudaMalloc(&p, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    buf.release();
-    buf.ptr = p;
-    buf.cap = bytes;
-    int *emax = static_cast<int *>(p);
+    int *emax = static_cast<int *>(dst);
     const C *src = static_cast<const C *>(stack);
     if (cudaMemsetAsync(emax, 0, sizeof(int) * n, c->stream) != cudaSuccess) return false;
     k_fx_stack_max<C><<<dim3(std::max(1, std::min(256, d * d / 1024)), n), 256, 0, c->stream>>>(src, (i64)d * d, emax);
     k_fx_stack<C><<<dim3(std::max(1, std::min(1024, dp * dp / 512)), n), 256, 0, c->stream>>>(
-        src, d, dp, emax, reinterpret_cast<i64 *>(static_cast<char *>(p) + head));
+        src, d, dp, emax, reinterpret_cast<i64 *>(static_cast<char *>(dst) + stack_head(n)));
     return cudaGetLastError() == cudaSuccess;
 }
 
+size_t fx_stack_bytes(const Ctx *c, unsigned dim, unsigned Ke) {
+    return fx_serves(c->fp64 ? FxForm::kFp64 : FxForm::kPlain32, (int)dim) ? fixed_bytes(dim, Ke) : 0;
+}
+
+// The plain form's stack, at c->fx_stack (null: the other kernels serve).
 void fx_prepare(Ctx *c) {
     c->fx_ready = false;
-    if (!fx_serves(c->fp64 ? FxForm::kFp64 : FxForm::kPlain32, (int)c->dim)) return;
+    if (!c->fx_stack) return;
     c->fx_ready = c->fp64 ? convert_stack<double2>(c, c->stack.ptr, c->fx_stack)
                           : convert_stack<float2>(c, c->stack.ptr, c->fx_stack);
 }
 
 void fx_prepare_split(Ctx *c) {
-    c->fx_split_ready =
-        fx_serves(FxForm::kSplit32, (int)c->dim) && convert_stack<float2>(c, c->split_stack.ptr, c->fx_split);
+    c->fx_split_ready = false;
+    if (!fx_serves(FxForm::kSplit32, (int)c->dim)) return;
+    // A set-up allocation, not counted by the allocation-failure injection.
+    const size_t bytes = fixed_bytes(c->dim, c->Ke);
+    c->fx_split.release();
+    void *p = nullptr;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    c->fx_split.ptr = p;
+    c->fx_split.cap = bytes;
+    c->fx_split_ready = convert_stack<float2>(c, c->split_stack.ptr, p);
 }
 
 bool fx_ensure(Ctx *c, long long P) {
@@ -733,15 +744,15 @@ bool fx_ensure(Ctx *c, long long P) {
 template <int S, class A, class C>
 static cudaError_t run_fx_t(Ctx *c, FxForm form, const void *d_carr, const WeightSpecHost &wh, double x, int M,
                             long long P, void *d_out, cudaStream_t st) {
-    const DevBuf &sb = form == FxForm::kSplit32 ? c->fx_split : c->fx_stack;
+    const void *sb = form == FxForm::kSplit32 ? c->fx_split.ptr : c->fx_stack;
     const int d = (int)c->dim, Ke = (int)c->Ke, n = 1 + Ke;
     const Plan q = make_plan(d, Ke, P, c->num_sms);
     int launches = 0;
     cudaError_t e = set_smem<S>();
     if (e != cudaSuccess) return e;
     const size_t head = stack_head(n);
-    const int *emax = static_cast<const int *>(sb.ptr);
-    const i64 *stack = reinterpret_cast<const i64 *>(static_cast<const char *>(sb.ptr) + head);
+    const int *emax = static_cast<const int *>(sb);
+    const i64 *stack = reinterpret_cast<const i64 *>(static_cast<const char *>(sb) + head);
     char *ws = static_cast<char *>(c->fx_ws.ptr);
     i64 *W = reinterpret_cast<i64 *>(ws + q.off_w), *X = reinterpret_cast<i64 *>(ws + q.off_x);
     i64 *scr = reinterpret_cast<i64 *>(ws + q.off_s), *Pb = reinterpret_cast<i64 *>(ws + q.off_p);

@@ -183,7 +183,8 @@ cudaError_t tree_product(bool fp64, int d, void *in, long long n, void *work, vo
         remain = pairs + remain % 2;
         std::swap(cur, nxt);
     }
-    if (out != cur) return cudaMemcpyAsync(out, cur, dd * es, cudaMemcpyDeviceToDevice, stream);
+    // (The result may lie in pinned host memory.)
+    if (out != cur) return cudaMemcpyAsync(out, cur, dd * es, cudaMemcpyDefault, stream);
     return cudaSuccess;
 }
 

@@ -142,6 +142,10 @@ bool new_faults(Ctx *c, bool wait) {
 
 // ------------------------------------------------------------------ life cycle
 
+// Small host-buffer calls go through pinned memory that the kernels read and write
+// themselves (half of it each): two copies less between the launches.
+constexpr size_t kStageBytes = 32 << 10;
+
 static Parament_ErrorCode ctx_create(Ctx **out, bool fp64) {
     Ctx *c = new (std::nothrow) Ctx();
     *out = c;
@@ -175,6 +179,12 @@ static Parament_ErrorCode ctx_create(Ctx **out, bool fp64) {
         return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
     }
     *c->h_fault = 0;
+    if (cudaHostAlloc(&c->h_stage, kStageBytes, cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(&c->d_stage, c->h_stage, 0) != cudaSuccess) {
+        cudaGetLastError();  // calls go without it
+        if (c->h_stage) cudaFreeHost(c->h_stage);
+        c->h_stage = c->d_stage = nullptr;
+    }
     c->last_error = PARAMENT_STATUS_SUCCESS;
     return PARAMENT_STATUS_SUCCESS;
 }
@@ -192,6 +202,7 @@ static Parament_ErrorCode ctx_destroy(Ctx *c) {
     cudaEventDestroy(c->ev_fault);
     cudaFree(c->d_fault);
     cudaFreeHost(c->h_fault);
+    if (c->h_stage) cudaFreeHost(c->h_stage);
     cudaStreamDestroy(c->stream);
     delete c;
     return PARAMENT_STATUS_SUCCESS;
@@ -206,7 +217,7 @@ static Parament_ErrorCode set_hamiltonian(Ctx *c, const void *H0, const void *H1
     c->has_h = false;
     c->stack.release();
     c->split_stack.release();
-    c->fx_stack.release();
+    c->fx_stack = nullptr;
     c->fx_split.release();
     c->fx_ready = c->fx_split_ready = false;
     if (use_magnus) {
@@ -223,7 +234,12 @@ static Parament_ErrorCode set_hamiltonian(Ctx *c, const void *H0, const void *H1
     if (dim == 0 || !H0 || (amps > 0 && !H1)) return c->last_error = PARAMENT_STATUS_INVALID_VALUE;
     const size_t es = c->esize(), dd = (size_t)dim * dim;
     const unsigned Ke = use_magnus ? 2 * amps + amps * (amps - 1) / 2 : amps;
-    if (c->stack.ensure(es * dd * (1 + Ke)) != cudaSuccess) return c->last_error = PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
+    // The stack and, where the sliced products serve, its fixed-point copy behind it.
+    const size_t sbytes = (es * dd * (1 + Ke) + 255) / 256 * 256, fx = fx_stack_bytes(c, dim, Ke);
+    if (fx && c->stack.ensure(sbytes + fx) == cudaSuccess)
+        c->fx_stack = static_cast<char *>(c->stack.ptr) + sbytes;
+    else if (c->stack.ensure(sbytes) != cudaSuccess)
+        return c->last_error = PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
     char *st = static_cast<char *>(c->stack.ptr);
     cudaError_t e = cudaMemcpyAsync(st, H0, es * dd, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess && amps)
@@ -547,6 +563,24 @@ static Parament_ErrorCode equiprop_host(Ctx *c, const void *carr, double dt, uns
     if (!out || (amps > 0 && !carr)) return c->last_error = PARAMENT_STATUS_INVALID_VALUE;
     const size_t es = c->esize(), dd = (size_t)c->dim * c->dim;
     const size_t cbytes = es * (size_t)amps * pts;
+    // Small calls: a qubit's 100 steps take 48 us with the two copies, 41
+    // us without.  Up to 16 KB of samples the kernels' own reads are no slower than
+    // the copy in front of them.
+    if (c->h_stage && cbytes <= kStageBytes / 2 && es * dd <= kStageBytes / 2) {
+        char *hs = static_cast<char *>(c->h_stage), *ds = static_cast<char *>(c->d_stage);
+        if (cbytes) memcpy(hs, carr, cbytes);
+        Parament_ErrorCode r = equiprop_device(c, ds, dt, pts, amps, ds + kStageBytes / 2, c->stream);
+        if (r == PARAMENT_STATUS_SUCCESS) note_call_end(c, c->stream, uses_tensor_kernels(c));
+        const cudaError_t e = cudaStreamSynchronize(c->stream);
+        if (r != PARAMENT_STATUS_SUCCESS) return c->last_error = r;
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return c->last_error = PARAMENT_STATUS_CUBLAS_FAILED;
+        }
+        if (new_faults(c, true)) return c->last_error = PARAMENT_STATUS_KERNEL_TIMEOUT;
+        memcpy(out, hs + kStageBytes / 2, es * dd);
+        return c->last_error = PARAMENT_STATUS_SUCCESS;
+    }
     if (c->carr.ensure(std::max<size_t>(cbytes, 16)) != cudaSuccess || c->out.ensure(es * dd) != cudaSuccess)
         return c->last_error = PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
     // Transfer of the samples (src/cuda/parament.cpp:477).
