@@ -24,7 +24,7 @@
 //      nc about one per SM, so that the chunk boundaries -- the checkpoints --
 //      come every P / nc steps (about sqrt(P) steps at the gradient workload,
 //      16384 steps in 152 chunks);
-//   2. exclusive prefix/suffix products of the chunks (Hillis-Steele scans):
+//   2. exclusive prefix/suffix products of the chunks (scans):
 //      R at every chunk start and L at every chunk end;
 //   3. one CTA per chunk sweeps its steps backward carrying M_j = W^H L_j and
 //      recomputing the rest: U_j from X_j, R_j = U_j^H R_(j+1) from the
@@ -624,6 +624,102 @@ static const void *pick_adj(bool fp64, int d, bool sweep) {
     }
 }
 
+// The same scans in three launches, for products that one CTA forms in a
+// microsecond or two: segments of about sqrt(nc) chunks, their products (phase 0),
+// exclusive prefixes and suffixes of those (phase 1, one CTA each), and from them
+// the chunks' (phase 2).  prod, pre_s, suf_s: one matrix per segment.  A factor S
+// enters as P + (S - I) P, without its unit diagonal.  The two Hillis-Steele scans
+// take 40 launches at 608 chunks; a gradient of 281 steps at d = 11 spends its time
+// launching, 917 us before and 804 now (d = 32, 16384 steps: 2.79 and 2.64 ms).
+template <class R, int TM>
+__global__ void __launch_bounds__(256) k_adj_scan(const cplx_t<R> *S, int nc, int seg, int ns, int d, int phase,
+                                                  cplx_t<R> *prod, cplx_t<R> *pre_s, cplx_t<R> *suf_s,
+                                                  cplx_t<R> *pre, cplx_t<R> *suf) {
+    using C = cplx_t<R>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int dd = d * d, ld = d + 1, sz = d * ld;
+    C *As = reinterpret_cast<C *>(smem_raw), *Ps = As + sz;
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    auto each = [&](auto f) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TM; ++j) {
+                const int r = ty + 16 * i, c = tx + 16 * j;
+                if (r < d && c < d) f(i, j, r, c, r * ld + c);
+            }
+    };
+    // P <- S P (left) or P S.
+    auto multiply = [&](const C *s, bool left) {
+        each([&](int, int, int r, int c, int o) {
+            C v = s[r * d + c];
+            if (r == c) v.x -= (R)1;
+            As[o] = v;
+        });
+        __syncthreads();
+        C acc[TM][TM];
+        if (left)
+            tile_gemm<C, TM>(acc, As, Ps, d, ld, ty, tx);
+        else
+            tile_gemm<C, TM>(acc, Ps, As, d, ld, ty, tx);
+        __syncthreads();
+        each([&](int i, int j, int, int, int o) { Ps[o] = cadd(Ps[o], acc[i][j]); });
+    };
+    auto load = [&](const C *s) {
+        each([&](int, int, int r, int c, int o) {
+            Ps[o] = s ? s[r * d + c] : mk<C>(r == c ? 1.0 : 0.0, 0.0);
+        });
+    };
+    auto store = [&](C *dst) {
+        each([&](int, int, int r, int c, int o) { dst[r * d + c] = Ps[o]; });
+    };
+    const bool prefix = blockIdx.y == 0;
+    if (phase == 0) {
+        const int c0 = blockIdx.x * seg, c1 = min(nc, c0 + seg);
+        load(S + (size_t)c0 * dd);
+        for (int c = c0 + 1; c < c1; ++c) multiply(S + (size_t)c * dd, true);
+        store(prod + (size_t)blockIdx.x * dd);
+    } else if (phase == 1) {
+        load(nullptr);
+        for (int i = 0; i < ns; ++i) {
+            const int k = prefix ? i : ns - 1 - i;
+            store((prefix ? pre_s : suf_s) + (size_t)k * dd);
+            if (i + 1 < ns) multiply(prod + (size_t)k * dd, prefix);
+        }
+    } else {
+        const int c0 = blockIdx.x * seg, c1 = min(nc, c0 + seg);
+        load((prefix ? pre_s : suf_s) + (size_t)blockIdx.x * dd);
+        for (int i = 0; i < c1 - c0; ++i) {
+            const int c = prefix ? c0 + i : c1 - 1 - i;
+            store((prefix ? pre : suf) + (size_t)c * dd);
+            if (i + 1 < c1 - c0) multiply(S + (size_t)c * dd, prefix);
+        }
+    }
+}
+
+// Where k_adj_scan is the faster one: a product within two microseconds.
+static bool short_scan(bool fp64, int d) { return fp64 ? d <= 8 : d <= 32; }
+
+template <class R, int TM>
+static cudaError_t launch_scan_t(int d, const void *S, int nc, void *pre, void *suf, void *t1, void *t2,
+                                 cudaStream_t st) {
+    using C = cplx_t<R>;
+    int seg = 1;
+    while (seg * seg < nc) ++seg;
+    const int ns = (nc + seg - 1) / seg;
+    // t1: nc matrices, t2: nc + 2 (three per segment in all).
+    C *prod = static_cast<C *>(t1), *ps = static_cast<C *>(t2), *ss = ps + (size_t)ns * d * d;
+    const size_t smem = 2 * sizeof(C) * (size_t)d * (d + 1);
+    for (int phase = 0; phase < 3; ++phase) {
+        k_adj_scan<R, TM><<<dim3(phase == 1 ? 1 : ns, phase == 0 ? 1 : 2), 256, smem, st>>>(
+            static_cast<const C *>(S), nc, seg, ns, d, phase, prod, ps, ss, static_cast<C *>(pre),
+            static_cast<C *>(suf));
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 // Hillis-Steele scans over nc chunk products (all d x d, later on the left).
 // prefix: out[c] = S_(c-1) ... S_0 (out[0] = I); suffix: out[c] = S_(nc-1) ... S_(c+1).
 static cudaError_t chunk_scan(bool fp64, int d, const void *S, long long nc, void *out, void *t1, void *t2,
@@ -696,8 +792,13 @@ static cudaError_t launch_adj_t(Ctx *c, const void *d_carr, unsigned pts, unsign
     l.stream = st;
     cudaError_t e = launch_small_steps(l);
     // 2. scans
-    if (e == cudaSuccess) e = chunk_scan(l.fp64, d, chunks, nc, pre, t1, t2, true, st, c->num_sms);
-    if (e == cudaSuccess) e = chunk_scan(l.fp64, d, chunks, nc, suf, t1, t2, false, st, c->num_sms);
+    if (e == cudaSuccess && short_scan(l.fp64, d)) {
+        e = d <= 16 ? launch_scan_t<R, 1>(d, chunks, nc, pre, suf, t1, t2, st)
+                    : launch_scan_t<R, 2>(d, chunks, nc, pre, suf, t1, t2, st);
+    } else {
+        if (e == cudaSuccess) e = chunk_scan(l.fp64, d, chunks, nc, pre, t1, t2, true, st, c->num_sms);
+        if (e == cudaSuccess) e = chunk_scan(l.fp64, d, chunks, nc, suf, t1, t2, false, st, c->num_sms);
+    }
     if (e != cudaSuccess) return e;
     // 3. per-chunk sweeps
     AdjArgs<R> a;
@@ -778,7 +879,7 @@ Parament_ErrorCode run_vjp(Ctx *c, const void *d_carr, double dt, unsigned pts, 
     // The order tables keep the truncation of every step exponential below
     // the working precision, so U_j^H inverts U_j; a manual order may not.
     const bool reversible = !c->manual;
-    if (c->chunks.ensure(es * dd * nc) != cudaSuccess || c->work.ensure(4 * es * dd * nc) != cudaSuccess ||
+    if (c->chunks.ensure(es * dd * nc) != cudaSuccess || c->work.ensure(es * dd * (4 * (size_t)nc + 2)) != cudaSuccess ||
         (!reversible && c->X.ensure(es * dd * (size_t)P) != cudaSuccess) ||
         c->aux.ensure(es * (size_t)P * std::max(1u, c->Ke)) != cudaSuccess)
         return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
