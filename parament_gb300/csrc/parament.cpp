@@ -116,8 +116,16 @@ long long num_steps(int quad, bool magnus, unsigned pts) {
     return pts;
 }
 
+// The fault counter's copy and event stay out of a graph that is being captured
+// on the stream: its calls may not query events.  The counter keeps what the
+// graph's replays add to it.
+static bool capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(stream, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
+}
+
 void note_call_end(Ctx *c, cudaStream_t stream, bool tensor_kernels) {
-    if (tensor_kernels &&
+    if (tensor_kernels && !capturing(stream) &&
         cudaMemcpyAsync(c->h_fault, c->d_fault, sizeof(int), cudaMemcpyDeviceToHost, stream) == cudaSuccess &&
         cudaEventRecord(c->ev_fault, stream) == cudaSuccess)
         c->fault_recorded = true;
@@ -613,8 +621,8 @@ static Ctx *as_ctx(void *p) { return static_cast<Ctx *>(p); }
 static Parament_ErrorCode equiprop_device_call(Ctx *c, const void *d_carr, double dt, unsigned pts, unsigned amps,
                                                void *d_out, void *stream_p) {
     cudaSetDevice(c->device);
-    if (new_faults(c, false)) return c->last_error = PARAMENT_STATUS_KERNEL_TIMEOUT;
     cudaStream_t stream = stream_p ? static_cast<cudaStream_t>(stream_p) : c->stream;
+    if (!capturing(stream) && new_faults(c, false)) return c->last_error = PARAMENT_STATUS_KERNEL_TIMEOUT;
     Parament_ErrorCode r = equiprop_device(c, d_carr, dt, pts, amps, d_out, stream);
     if (r == PARAMENT_STATUS_SUCCESS) note_call_end(c, stream, uses_tensor_kernels(c));
     return c->last_error = r;
@@ -825,8 +833,8 @@ static Parament_ErrorCode vjp_host(Ctx *c, const void *carr, double dt, unsigned
 static Parament_ErrorCode vjp_device_call(Ctx *c, const void *d_carr, double dt, unsigned pts, unsigned amps,
                                           const void *d_W, void *d_grad, void *stream_p) {
     cudaSetDevice(c->device);
-    if (new_faults(c, false)) return c->last_error = PARAMENT_STATUS_KERNEL_TIMEOUT;
     cudaStream_t stream = stream_p ? static_cast<cudaStream_t>(stream_p) : c->stream;
+    if (!capturing(stream) && new_faults(c, false)) return c->last_error = PARAMENT_STATUS_KERNEL_TIMEOUT;
     Parament_ErrorCode r = run_vjp(c, d_carr, dt, pts, amps, d_W, d_grad, stream);
     if (r == PARAMENT_STATUS_SUCCESS) note_call_end(c, stream, false);
     return c->last_error = r;
