@@ -13,13 +13,13 @@
 // product per chunk; two more launches multiply each problem's chunk products
 // in order, first within segments of about the square root of their number, then
 // the segments (one launch over all chunks of a problem lasted as long as its
-// longest chain).  The classes' kernels are branches of the graph, so that a class
-// starts while the last chunks of another run.  All, with the counter reset, are
-// captured in a CUDA graph.  Both changes, samples to results: 512 complex64
-// problems 36.5 -> 32.4 ms, 64 of them 8.7 -> 5.7, 40 complex128 problems of up to
-// 1000 steps 42.7 -> 20.3, 32 short ones 1.50 -> 0.43.  The chunk length per class
-// comes from an autotuner that times a few candidate granularities on the actual
-// ensemble.
+// longest chain).  All, with the counter reset, are captured in a CUDA graph.
+// Samples to results: 512 complex64 problems 36.5 -> 33.0 ms, 64 of them
+// 8.7 -> 6.2, 40 complex128 problems of up to 1000 steps 42.7 -> 20.3, 32 short ones
+// 1.50 -> 0.45.  The classes run one after another: as parallel branches of the
+// graph they gained 1.5 per cent (5 for 64 problems) and gave wrong d = 16 products.
+// The chunk length per class comes from an autotuner that times a few candidate
+// granularities on the actual ensemble.
 #include <math.h>
 #include <string.h>
 
@@ -344,8 +344,6 @@ struct Ensemble {
     std::vector<int> cls;  // class of each problem
     long long carr_elems = 0, out_elems = 0;
     DevBuf d_probs, d_items, d_bundles, d_segs, d_counter, d_stack, d_carr, d_J, d_chunks, d_out;
-    cudaStream_t branch[kEnsClasses - 1] = {nullptr};  // capture branches of the smaller classes
-    cudaEvent_t fork = nullptr, join[kEnsClasses - 1] = {nullptr};
     int nsegs = 0;
     void *h_carr = nullptr, *h_out = nullptr;  // pinned staging
     int nbundles = 0;
@@ -439,22 +437,11 @@ static Parament_ErrorCode build_work(Ensemble *E, double gran) {
 template <class R, int TM, int D, int GROUPS, int MINB>
 static cudaError_t launch_class(Ensemble *E, const EnsArgs<R> &a, int c) {
     if (E->cls_count[c] == 0) return cudaSuccess;
-    // The largest class stays on the stream itself, the others branch off it.
-    const cudaStream_t st = c < kEnsClasses - 1 ? E->branch[c] : E->stream;
-    if (c < kEnsClasses - 1) {
-        const cudaError_t e = cudaStreamWaitEvent(st, E->fork, 0);
-        if (e != cudaSuccess) return e;
-    }
     const int grid = std::max(1, std::min(E->cls_slots[c], E->cls_count[c]));
     int *counter = static_cast<int *>(E->d_counter.ptr) + c;
-    k_ensemble_class<R, TM, D, GROUPS, MINB><<<grid, 256, ens_smem(E->fp64, c), st>>>(
+    k_ensemble_class<R, TM, D, GROUPS, MINB><<<grid, 256, ens_smem(E->fp64, c), E->stream>>>(
         a, E->cls_first[c], E->cls_count[c], counter);
-    cudaError_t e = cudaGetLastError();
-    if (c < kEnsClasses - 1) {
-        if (e == cudaSuccess) e = cudaEventRecord(E->join[c], st);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(E->stream, E->join[c], 0);
-    }
-    return e;
+    return cudaGetLastError();
 }
 
 template <class R>
@@ -483,7 +470,6 @@ static cudaError_t enqueue_t(Ensemble *E) {
     a.carr = static_cast<const C *>(E->d_carr.ptr);
     a.J = static_cast<const C *>(E->d_J.ptr);
     a.chunks = static_cast<C *>(E->d_chunks.ptr);
-    if ((e = cudaEventRecord(E->fork, E->stream)) != cudaSuccess) return e;
     // Largest dimension first: its bundles are the longest.
     e = launch_class<R, 4, 64, 1, sizeof(R) == 4 ? 2 : 1>(E, a, 4);
     if (e == cudaSuccess) e = launch_class<R, 2, 32, 1, sizeof(R) == 4 ? 3 : 2>(E, a, 3);
@@ -573,15 +559,6 @@ Parament_ErrorCode Parament_ensembleCreate(Parament_Ensemble **out, int fp64, un
     }
     cudaEventCreate(&E->ev0);
     cudaEventCreate(&E->ev1);
-    bool branches = cudaEventCreateWithFlags(&E->fork, cudaEventDisableTiming) == cudaSuccess;
-    for (int c = 0; c < kEnsClasses - 1 && branches; ++c)
-        branches = cudaStreamCreateWithFlags(&E->branch[c], cudaStreamNonBlocking) == cudaSuccess &&
-                   cudaEventCreateWithFlags(&E->join[c], cudaEventDisableTiming) == cudaSuccess;
-    if (!branches) {
-        cudaGetLastError();
-        Parament_ensembleDestroy(reinterpret_cast<Parament_Ensemble *>(E));
-        return PARAMENT_STATUS_CUBLAS_INIT_FAILED;
-    }
     const size_t es = E->fp64 ? 16 : 8;
     long long stack_elems = 0, carr_elems = 0, out_elems = 0;
     std::vector<double> J;
@@ -766,11 +743,6 @@ Parament_ErrorCode Parament_ensembleDestroy(Parament_Ensemble *ens) {
     if (E->h_out) cudaFreeHost(E->h_out);
     if (E->ev0) cudaEventDestroy(E->ev0);
     if (E->ev1) cudaEventDestroy(E->ev1);
-    if (E->fork) cudaEventDestroy(E->fork);
-    for (int c = 0; c < kEnsClasses - 1; ++c) {
-        if (E->join[c]) cudaEventDestroy(E->join[c]);
-        if (E->branch[c]) cudaStreamDestroy(E->branch[c]);
-    }
     if (E->stream) cudaStreamDestroy(E->stream);
     delete E;
     return PARAMENT_STATUS_SUCCESS;
