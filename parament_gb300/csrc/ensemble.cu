@@ -46,6 +46,7 @@ struct EnsProblem {
     double s;
     long long stack_off, carr_off, out_off, chunk_off;
     int j_off, nchunks, rseg;  // rseg: chunks of a segment of the reduction
+    int c_off;                 // coefficients of the powers of X, or -1: Clenshaw
 };
 struct EnsItem {
     int prob, slot;
@@ -67,6 +68,7 @@ struct EnsArgs {
     int nbundles;
     int *counter;
     const cplx_t<R> *stack, *carr, *J;
+    const double *c;  // by powers of X: c_n (odd n: times i), c_0 of E = U - I
     cplx_t<R> *chunks;
 };
 
@@ -78,6 +80,28 @@ __device__ __forceinline__ void group_sync(int g) {
         asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(64) : "memory");
     } else {
         __syncthreads();
+    }
+}
+
+// The thread's elements of A B (d x d, rows of ld elements), T threads to a side.
+template <class R, int TM, int T>
+__device__ __forceinline__ void ens_gemm(cplx_t<R> (&acc)[TM][TM], const cplx_t<R> *A, const cplx_t<R> *B, int d,
+                                         int ld, int ty, int tx) {
+    using C = cplx_t<R>;
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TM; ++j) acc[i][j] = mk<C>(0.0, 0.0);
+    for (int q = 0; q < d; ++q) {
+        C av[TM], bv[TM];
+#pragma unroll
+        for (int i = 0; i < TM; ++i) av[i] = A[min(ty + T * i, d - 1) * ld + q];
+#pragma unroll
+        for (int j = 0; j < TM; ++j) bv[j] = B[q * ld + min(tx + T * j, d - 1)];
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TM; ++j) cfma(acc[i][j], av[i], bv[j]);
     }
 }
 
@@ -97,6 +121,11 @@ __device__ void ens_chunk(const EnsArgs<R> &a, const EnsProblem &p, const EnsIte
     const R s = (R)p.s;
     WeightSpec w{p.pts, p.K, p.K, p.mode, 0, 0.0};
     const C *carr = a.carr + p.carr_off;
+    // Powers of X in complex128 only: compiled into the complex64 kernels as well they
+    // slow order 3, which these mostly run, by 2 per cent.
+    constexpr bool kPowers = sizeof(R) == 8;
+    const bool powers = kPowers && p.c_off >= 0;
+    const double *pc = a.c + max(p.c_off, 0);
     C b2[TM][TM], acc[TM][TM];
     // The expansion matrices do not change from step to step: for TM <= 2 and
     // up to kEnsRegK controls each thread keeps its own elements of them in
@@ -143,6 +172,10 @@ __device__ void ens_chunk(const EnsArgs<R> &a, const EnsProblem &p, const EnsIte
                     for (int m = 0; m < p.K; ++m) cfma(v, ws[m], stack[(size_t)(m + 1) * dd + r * d + c]);
                 }
                 Xs[r * ld + c] = v;
+                if (powers) {
+                    b2[i][j] = v;
+                    continue;
+                }
                 C bm1 = cscale(cmul(J[M], v), s);
                 if (r == c) bm1 = cadd(bm1, J[M - 1]);
                 if (M == 1) {
@@ -152,25 +185,69 @@ __device__ void ens_chunk(const EnsArgs<R> &a, const EnsProblem &p, const EnsIte
                     Bs[r * ld + c] = bm1;
                 }
             }
-        if (M > 1) {
-            group_sync<D>(g);
-            for (int k = M - 2; k >= 0; --k) {
-                // acc = Bs Xs
+        if constexpr (kPowers) {
+            if (powers) {
+                // E = U - I by powers of X, Y = X X: (M + 1) / 2 products, the recurrence
+                // below has M - 1.  40 problems of up to 1000 steps 20.3 -> 16.7 ms, 64 of
+                // up to 2000 83.2 -> 63.1 ms.
+                group_sync<D>(g);
+                ens_gemm<R, TM, T>(acc, Xs, Xs, d, ld, ty, tx);
 #pragma unroll
                 for (int i = 0; i < TM; ++i)
 #pragma unroll
-                    for (int j = 0; j < TM; ++j) acc[i][j] = mk<C>(0.0, 0.0);
-                for (int q = 0; q < d; ++q) {
-                    C av[TM], bv[TM];
+                    for (int j = 0; j < TM; ++j) {
+                        const int r = ty + T * i, c = tx + T * j;
+                        if (r < d && c < d) Bs[r * ld + c] = acc[i][j];
+                    }
+                group_sync<D>(g);
+                ens_gemm<R, TM, T>(acc, Xs, Bs, d, ld, ty, tx);
 #pragma unroll
-                    for (int i = 0; i < TM; ++i) av[i] = Bs[min(ty + T * i, d - 1) * ld + q];
+                for (int i = 0; i < TM; ++i)
 #pragma unroll
-                    for (int j = 0; j < TM; ++j) bv[j] = Xs[q * ld + min(tx + T * j, d - 1)];
+                    for (int j = 0; j < TM; ++j) {
+                        const int r = ty + T * i, c = tx + T * j;
+                        if (r >= d || c >= d) continue;
+                        const C q = acc[i][j], y = Bs[r * ld + c], x = b2[i][j];
+                        C v;
+                        v.x = fma(pc[M - 1], y.x, -pc[M] * q.y) - pc[M - 2] * x.y;
+                        v.y = fma(pc[M - 1], y.y, pc[M] * q.x) + pc[M - 2] * x.x;
+                        if (r == c) v.x += pc[M - 3];
+                        acc[i][j] = v;
+                    }
+                for (int k = M - 5; k >= 0; k -= 2) {
+                    group_sync<D>(g);
 #pragma unroll
                     for (int i = 0; i < TM; ++i)
 #pragma unroll
-                        for (int j = 0; j < TM; ++j) cfma(acc[i][j], av[i], bv[j]);
+                        for (int j = 0; j < TM; ++j) {
+                            const int r = ty + T * i, c = tx + T * j;
+                            if (r < d && c < d) Xs[r * ld + c] = acc[i][j];
+                        }
+                    group_sync<D>(g);
+                    ens_gemm<R, TM, T>(acc, Xs, Bs, d, ld, ty, tx);
+#pragma unroll
+                    for (int i = 0; i < TM; ++i)
+#pragma unroll
+                        for (int j = 0; j < TM; ++j) {
+                            const int r = ty + T * i, c = tx + T * j;
+                            if (r >= d || c >= d) continue;
+                            C v = acc[i][j];
+                            v.x = fma(-pc[k + 1], b2[i][j].y, v.x);
+                            v.y = fma(pc[k + 1], b2[i][j].x, v.y);
+                            if (r == c) {
+                                v.x += pc[k];
+                                if (k == 0 && st == it.s0) v.x += (R)1;  // the first step's P
+                            }
+                            acc[i][j] = v;
+                        }
                 }
+                group_sync<D>(g);
+            }
+        }
+        if (!powers && M > 1) {
+            group_sync<D>(g);
+            for (int k = M - 2; k >= 0; --k) {
+                ens_gemm<R, TM, T>(acc, Bs, Xs, d, ld, ty, tx);
                 group_sync<D>(g);
                 const R beta = (k == 0) ? (R)-2 : (R)-1;
 #pragma unroll
@@ -211,25 +288,11 @@ __device__ void ens_chunk(const EnsArgs<R> &a, const EnsProblem &p, const EnsIte
                     const int r = ty + T * i, c = tx + T * j;
                     if (r >= d || c >= d) continue;
                     C u = acc[i][j];
-                    if (r == c) u.x -= (R)1;
+                    if (r == c && !powers) u.x -= (R)1;
                     Bs[r * ld + c] = u;
                 }
             group_sync<D>(g);
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TM; ++j) acc[i][j] = mk<C>(0.0, 0.0);
-            for (int q = 0; q < d; ++q) {
-                C av[TM], bv[TM];
-#pragma unroll
-                for (int i = 0; i < TM; ++i) av[i] = Bs[min(ty + T * i, d - 1) * ld + q];
-#pragma unroll
-                for (int j = 0; j < TM; ++j) bv[j] = Ps[q * ld + min(tx + T * j, d - 1)];
-#pragma unroll
-                for (int i = 0; i < TM; ++i)
-#pragma unroll
-                    for (int j = 0; j < TM; ++j) cfma(acc[i][j], av[i], bv[j]);
-            }
+            ens_gemm<R, TM, T>(acc, Bs, Ps, d, ld, ty, tx);
             group_sync<D>(g);
 #pragma unroll
             for (int i = 0; i < TM; ++i)
@@ -343,7 +406,7 @@ struct Ensemble {
     std::vector<EnsProblem> probs;
     std::vector<int> cls;  // class of each problem
     long long carr_elems = 0, out_elems = 0;
-    DevBuf d_probs, d_items, d_bundles, d_segs, d_counter, d_stack, d_carr, d_J, d_chunks, d_out;
+    DevBuf d_probs, d_items, d_bundles, d_segs, d_counter, d_stack, d_carr, d_J, d_c, d_chunks, d_out;
     int nsegs = 0;
     void *h_carr = nullptr, *h_out = nullptr;  // pinned staging
     int nbundles = 0;
@@ -373,7 +436,10 @@ static size_t ens_smem(bool fp64, int cls) {
 // 32^3 product for the dependent load/synchronise chain every step pays
 // (weights, assembly, barriers) -- for d <= 16 that latency, not the
 // arithmetic, sets the step time, so small problems are cut into more chunks.
-static double step_cost(const EnsProblem &p) { return (double)p.M * ((double)p.d * p.d * p.d + 32768.0) / 256.0; }
+static double step_cost(const EnsProblem &p) {
+    const int products = p.c_off >= 0 ? (p.M + 3) / 2 : p.M;
+    return products * ((double)p.d * p.d * p.d + 32768.0) / 256.0;
+}
 
 // Work list for a given granularity: chunk lengths chosen so that each
 // bundle costs about total / (slots * granularity).
@@ -469,6 +535,7 @@ static cudaError_t enqueue_t(Ensemble *E) {
     a.stack = static_cast<const C *>(E->d_stack.ptr);
     a.carr = static_cast<const C *>(E->d_carr.ptr);
     a.J = static_cast<const C *>(E->d_J.ptr);
+    a.c = static_cast<const double *>(E->d_c.ptr);
     a.chunks = static_cast<C *>(E->d_chunks.ptr);
     // Largest dimension first: its bundles are the longest.
     e = launch_class<R, 4, 64, 1, sizeof(R) == 4 ? 2 : 1>(E, a, 4);
@@ -561,7 +628,7 @@ Parament_ErrorCode Parament_ensembleCreate(Parament_Ensemble **out, int fp64, un
     cudaEventCreate(&E->ev1);
     const size_t es = E->fp64 ? 16 : 8;
     long long stack_elems = 0, carr_elems = 0, out_elems = 0;
-    std::vector<double> J;
+    std::vector<double> J, pc;
     Parament_ErrorCode r = PARAMENT_STATUS_SUCCESS;
     for (unsigned i = 0; i < nprob && r == PARAMENT_STATUS_SUCCESS; ++i) {
         EnsProblem p{};
@@ -592,6 +659,17 @@ Parament_ErrorCode Parament_ensembleCreate(Parament_Ensemble **out, int fp64, un
         std::vector<double> Jp(2 * (p.M + 1));
         bessel_coeffs(p.M, h * hn, Jp.data());
         J.insert(J.end(), Jp.begin(), Jp.end());
+        // Order 3 has two products either way; above x = 1 the powers' coefficients
+        // cancel.
+        p.c_off = -1;
+        if (E->fp64 && p.M >= 5 && h * hn <= 1.0) {
+            double c0[2];
+            std::vector<double> mu;
+            power_coefficients(p.M, h * hn, hn, c0, mu);
+            p.c_off = (int)pc.size();
+            pc.push_back(c0[0]);
+            for (int n = 1; n <= p.M; ++n) pc.push_back(mu[2 * n + (n & 1)]);
+        }
         p.stack_off = stack_elems;
         stack_elems += (long long)dd * (1 + p.K);
         p.carr_off = carr_elems;
@@ -603,7 +681,9 @@ Parament_ErrorCode Parament_ensembleCreate(Parament_Ensemble **out, int fp64, un
     }
     if (r == PARAMENT_STATUS_SUCCESS) {
         if (E->d_stack.ensure(es * stack_elems) != cudaSuccess || E->d_carr.ensure(es * std::max(1LL, carr_elems)) != cudaSuccess ||
-            E->d_J.ensure(es * (J.size() / 2)) != cudaSuccess || E->d_out.ensure(es * out_elems) != cudaSuccess ||
+            E->d_J.ensure(es * (J.size() / 2)) != cudaSuccess ||
+            E->d_c.ensure(sizeof(double) * std::max<size_t>(1, pc.size())) != cudaSuccess ||
+            E->d_out.ensure(es * out_elems) != cudaSuccess ||
             E->d_counter.ensure(sizeof(int) * kEnsClasses) != cudaSuccess ||
             cudaMallocHost(&E->h_carr, es * std::max(1LL, carr_elems)) != cudaSuccess ||
             cudaMallocHost(&E->h_out, es * out_elems) != cudaSuccess)
@@ -628,7 +708,9 @@ Parament_ErrorCode Parament_ensembleCreate(Parament_Ensemble **out, int fp64, un
                 memcpy(hj.data() + 8 * k, v, 8);
             }
         }
-        if (cudaMemcpy(E->d_stack.ptr, hs.data(), hs.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+        if ((!pc.empty() && cudaMemcpy(E->d_c.ptr, pc.data(), sizeof(double) * pc.size(), cudaMemcpyHostToDevice) !=
+                                cudaSuccess) ||
+            cudaMemcpy(E->d_stack.ptr, hs.data(), hs.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
             cudaMemcpy(E->d_J.ptr, hj.data(), hj.size(), cudaMemcpyHostToDevice) != cudaSuccess)
             r = PARAMENT_FAIL;
     }
@@ -736,7 +818,7 @@ Parament_ErrorCode Parament_ensembleDestroy(Parament_Ensemble *ens) {
     cudaSetDevice(E->device);
     if (E->stream) cudaStreamSynchronize(E->stream);
     if (E->graph) cudaGraphExecDestroy(E->graph);
-    for (DevBuf *b : {&E->d_probs, &E->d_items, &E->d_bundles, &E->d_segs, &E->d_counter, &E->d_stack, &E->d_carr, &E->d_J,
+    for (DevBuf *b : {&E->d_probs, &E->d_items, &E->d_bundles, &E->d_segs, &E->d_counter, &E->d_stack, &E->d_carr, &E->d_J, &E->d_c,
                       &E->d_chunks, &E->d_out})
         b->release();
     if (E->h_carr) cudaFreeHost(E->h_carr);
