@@ -224,7 +224,7 @@ def split_slice_products(M):
 
 
 # The step kernel each form of the d=64 workload runs.
-FORM_KERNELS = {"plain_c128": "k_small_steps<double> (FP64 pipe)",
+FORM_KERNELS = {"plain_c128": "k_fx_steps (tcgen05, exact products of seven 8-bit digits)",
                 "plain_c64": "k_small_tc (tcgen05, exact four-slice bf16 products; FP32 Clenshaw)",
                 "split_c64": "k_split_tc (tcgen05, exact bf16 slices; double-float E and running product)"}
 
@@ -459,7 +459,7 @@ def large_dense_block(torch, parament, K_steps, W_steps, flush, stream, err_step
         flops = steps * (M + 1) * 8.0 * 512 ** 3
         res[form] = {"M": M, "ms": round(ms, 3), "steps_per_s": round(steps / (ms * 1e-3), 1),
                      "kernel": ("k_tc_cgemm (tcgen05 kind::tf32, 3xTF32 split products)" if form == "plain_c64"
-                                else "k_oz_cgemm (tcgen05 kind::f16, exact 6-bit bf16 slices) + k_sl_* elementwise"),
+                                else "k_fx_gemm (tcgen05 kind::f16, exact products of five 8-bit digits)"),
                      "algorithmic_tflops": round(flops / (ms * 1e-3) / 1e12, 2),
                      "complex_products_per_step": nprod,
                      "rel_err_vs_oracle_prefix": oracle_prefix_error(parament, w, "fp32", err_steps,
@@ -483,8 +483,8 @@ def large_dense_block(torch, parament, K_steps, W_steps, flush, stream, err_step
 
 def large_dense_c128_block(torch, parament, K_steps, W_steps, stream, steps=4, err_steps=3):
     """Large dense complex128 workload, d=1024, K=4, ||H0|| = 20: the first
-    `steps` of its 2048 steps (all of them for steps = 2048) on the FP64 GEMM
-    path (k_gemm, FP64 pipe); a prefix is checked against the oracle."""
+    `steps` of its 2048 steps (all of them for steps = 2048) on the
+    sliced tensor-core products (k_fx_gemm); a prefix is checked against the oracle."""
     from parament_gb300 import workloads
     w = workloads.large_dense(d=1024, K=4, steps=steps)
     ctx = parament.Parament("fp64")
@@ -497,7 +497,7 @@ def large_dense_c128_block(torch, parament, K_steps, W_steps, stream, steps=4, e
     flops = steps * (M + 1) * 8.0 * 1024 ** 3
     return {"workload": f"large_dense d=1024 K=4 complex128, {steps} of 2048 steps", "M": M,
             "ms": round(ms, 3), "steps_per_s": round(steps / (ms * 1e-3), 2),
-            "algorithmic_tflops": round(flops / (ms * 1e-3) / 1e12, 3), "kernel": "k_gemm (FP64 pipe)",
+            "algorithmic_tflops": round(flops / (ms * 1e-3) / 1e12, 3), "kernel": "k_fx_gemm (tcgen05, exact products of seven 8-bit digits)",
             "rel_err_vs_oracle_prefix": oracle_prefix_error(parament, w, "fp64", min(err_steps, steps)),
             "rel_err_prefix_steps": min(err_steps, steps)}
 
@@ -573,7 +573,7 @@ def mid_block(torch, parament, K_steps, W_steps, flush, stream, steps=16384):
             "M": M, "ms": round(ms, 3), "steps_per_s": round(steps / (ms * 1e-3), 1),
             "algorithmic_tflops": round(fl / (ms * 1e-3) / 1e12, 2), "launches": launches,
             "rel_err_vs_oracle_prefix": oracle_prefix_error(parament, w, prec, 64), "rel_err_prefix_steps": 64}
-    out["workload"] = (f"K=3 NONE ||H0||=8, {steps} steps; the default path for 64 < d <= 128 (batched GEMMs; "
+    out["workload"] = (f"K=3 NONE ||H0||=8, {steps} steps; the default path for 64 < d <= 128 (k_fx_steps, k_fx_gemm; "
                        f"the cluster-resident k_mid_steps serves when the batch buffers cannot be allocated)")
     return out
 
