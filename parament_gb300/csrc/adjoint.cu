@@ -771,7 +771,7 @@ static cudaError_t launch_adj_t(Ctx *c, const void *d_carr, unsigned pts, unsign
     const int d = (int)c->dim;
     const size_t es = sizeof(C), dd = (size_t)d * d;
     WeightSpecHost wh{pts, (int)c->K, (int)amps, c->quad, c->magnus ? 1 : 0,
-                      sizeof(R) == 8 ? h / 12.0 : (double)(float)h / 12.0};
+                      sizeof(R) == 8 ? c->held_step(h) / 12.0 : (double)(float)c->held_step(h) / 12.0};
     char *chunks = static_cast<char *>(c->chunks.ptr);
     char *scan = static_cast<char *>(c->work.ptr);  // pre | suf | t1 | t2
     char *pre = scan, *suf = scan + nc * dd * es, *t1 = suf + nc * dd * es, *t2 = t1 + nc * dd * es;
@@ -783,7 +783,7 @@ static cudaError_t launch_adj_t(Ctx *c, const void *d_carr, unsigned pts, unsign
     l.w = wh;
     l.M = M;
     l.J = J;
-    l.s = 2.0 / c->hnorm;
+    l.s = 2.0 / c->held_norm();
     l.stack = c->stack.ptr;
     l.carr = d_carr;
     l.chunks = chunks;
@@ -817,18 +817,18 @@ static cudaError_t launch_adj_t(Ctx *c, const void *d_carr, unsigned pts, unsign
     a.d = d;
     a.Ke = (int)c->Ke;
     a.M = M;
-    a.s = (R)(2.0 / c->hnorm);
+    a.s = (R)(2.0 / c->held_norm());
     a.w = WeightSpec{wh.pts, wh.K, wh.amps, wh.mode, wh.magnus, wh.hfac};
     const double x = h * c->hnorm;
     if (sweep && l.fp64) {
         double c0[2];
         std::vector<double> mu;
-        power_coefficients(M, x, c->hnorm, c0, mu);
+        power_coefficients(M, x, c->held_norm(), c0, mu);
         a.c[0] = (R)c0[0];
         for (int n = 1; n <= M; ++n) a.c[n] = (R)mu[2 * n + (n & 1)];
     } else if (sweep) {
         std::vector<double> cs;
-        plain_coefficients(M, x, c->hnorm, cs);
+        plain_coefficients(M, x, c->held_norm(), cs);
         for (int n = 0; n <= M; ++n) a.c[n] = (R)cs[n];
     }
     const void *fn = pick_adj(l.fp64, d, sweep);

@@ -7,6 +7,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stddef.h>
 
 #include <vector>
@@ -37,7 +38,14 @@ struct Ctx {
     bool magnus = true;                          // defaults as src/cuda/parament.cpp:72-75
     int quad = PARAMENT_QUADRATURE_SIMPSON;
     double hnorm = 0.0;
+    // The stack is held in units of 2^hexp, hexp = ilogb(hnorm): exact, and powers of
+    // X and their coefficients stay within the range of FP32 for Hamiltonians in any
+    // units (rad/s: with h = 1e-10 s, c_5 = h^5/5! is zero in FP32, and X^3
+    // overflows from norms of 1e13 on).
+    int hexp = 0;
     DevBuf stack;                                // (1+Ke) d x d, context precision
+    double held_norm() const { return ldexp(hnorm, -hexp); }
+    double held_step(double h) const { return ldexp(h, hexp); }
 
     // Chebyshev order control (src/cuda/parament_context.hpp:72-73)
     unsigned mmax = 11;
@@ -132,7 +140,8 @@ Parament_ErrorCode run_split(Ctx *c, const void *d_carr, unsigned pts, unsigned 
                              void *d_out, cudaStream_t stream);
 Parament_ErrorCode run_split_large(Ctx *c, const SplitArgs &a, double h, void *d_out, cudaStream_t stream);
 
-// c0 = m_0 - 1 and mu_n = m_n / Hnorm^n of the regrouped polynomial (split.cu).
+// c0 = m_0 - 1 and mu_n = m_n / Hnorm^n of the regrouped polynomial (split.cu); here and
+// below hnorm is the norm of the stack as it is held.
 void power_coefficients(int M, double x, double hnorm, double *c0, std::vector<double> &mu);
 // The same polynomial with the FP32 coefficients of the complex64 contexts;
 // returns J_0, which c_0 = p(0) - J_0 leaves out.

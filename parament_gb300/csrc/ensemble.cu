@@ -45,6 +45,7 @@ struct EnsProblem {
     long long P;
     double s;
     long long stack_off, carr_off, out_off, chunk_off;
+    int hexp;  // the stack is held in units of 2^hexp (as a context's, ctx.h)
     int j_off, nchunks, rseg;  // rseg: chunks of a segment of the reduction
     int c_off;                 // coefficients of the powers of X, or -1: Clenshaw
 };
@@ -419,6 +420,14 @@ struct Ensemble {
     int slots = 0;
 };
 
+// The n numbers at a times 2^e, by two factors that FP64 holds.
+template <class R>
+static void scale_pow2(R *a, size_t n, int e) {
+    if (e == 0) return;
+    const double f = ldexp(1.0, e / 2), g = ldexp(1.0, e - e / 2);
+    for (size_t i = 0; i < n; ++i) a[i] = (R)((double)a[i] * f * g);
+}
+
 static int class_of(int d) {
     for (int c = 0; c < kEnsClasses; ++c)
         if (d <= kClassDim[c]) return c;
@@ -654,7 +663,8 @@ Parament_ErrorCode Parament_ensembleCreate(Parament_Ensemble **out, int fp64, un
             r = PARAMENT_STATUS_SELECT_SMALLER_DT;
             break;
         }
-        p.s = 2.0 / hn;
+        p.hexp = isfinite(hn) ? ilogb(hn) : 0;
+        p.s = 2.0 / ldexp(hn, -p.hexp);
         p.j_off = (int)(J.size() / 2);
         std::vector<double> Jp(2 * (p.M + 1));
         bessel_coeffs(p.M, h * hn, Jp.data());
@@ -665,7 +675,7 @@ Parament_ErrorCode Parament_ensembleCreate(Parament_Ensemble **out, int fp64, un
         if (E->fp64 && p.M >= 5 && h * hn <= 1.0) {
             double c0[2];
             std::vector<double> mu;
-            power_coefficients(p.M, h * hn, hn, c0, mu);
+            power_coefficients(p.M, h * hn, ldexp(hn, -p.hexp), c0, mu);
             p.c_off = (int)pc.size();
             pc.push_back(c0[0]);
             for (int n = 1; n <= p.M; ++n) pc.push_back(mu[2 * n + (n & 1)]);
@@ -697,6 +707,10 @@ Parament_ErrorCode Parament_ensembleCreate(Parament_Ensemble **out, int fp64, un
             const size_t dd = (size_t)p.d * p.d;
             memcpy(hs.data() + es * p.stack_off, H0s[i], es * dd);
             if (p.K) memcpy(hs.data() + es * (p.stack_off + dd), H1s[i], es * dd * p.K);
+            if (E->fp64)
+                scale_pow2(reinterpret_cast<double *>(hs.data()) + 2 * p.stack_off, 2 * dd * (1 + p.K), -p.hexp);
+            else
+                scale_pow2(reinterpret_cast<float *>(hs.data()) + 2 * p.stack_off, 2 * dd * (1 + p.K), -p.hexp);
         }
         std::vector<char> hj(es * (J.size() / 2));
         for (size_t k = 0; k < J.size() / 2; ++k) {

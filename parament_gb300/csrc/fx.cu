@@ -760,7 +760,7 @@ static cudaError_t run_fx_t(Ctx *c, FxForm form, const void *d_carr, const Weigh
     Info *xinfo = reinterpret_cast<Info *>(ws + q.off_info), *sinfo = xinfo + q.rows;
     Info *pinfo = sinfo + (kMaxOps + 1) * (size_t)q.nch, *cinfo = pinfo + 2 * (size_t)q.nch, *tinfo = cinfo + q.nch;
     std::vector<Op> ops;
-    build_program(form, M, x, c->hnorm, ops);
+    build_program(form, M, x, c->held_norm(), ops);
     if ((int)ops.size() >= kMaxOps) return cudaErrorInvalidValue;  // orders up to 63: 62 products
     const WeightSpec w{wh.pts, wh.K, wh.amps, wh.mode, wh.magnus, wh.hfac};
     const i64 rpad = (q.rows + 63) / 64 * 64;

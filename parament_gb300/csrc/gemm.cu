@@ -305,6 +305,25 @@ __global__ void k_convert(const S *src, D *dst, long long n) {
     }
 }
 
+template <class C>
+__global__ void k_scale(C *m, long long n, int e) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        C v = m[i];
+        v.x = scalbn(v.x, e);
+        v.y = scalbn(v.y, e);
+        m[i] = v;
+    }
+}
+
+cudaError_t scale_complex(bool fp64, void *m, long long n, int e, cudaStream_t stream) {
+    const int blocks = (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 4096));
+    if (fp64)
+        k_scale<<<blocks, 256, 0, stream>>>(static_cast<double2 *>(m), n, e);
+    else
+        k_scale<<<blocks, 256, 0, stream>>>(static_cast<float2 *>(m), n, e);
+    return cudaGetLastError();
+}
+
 cudaError_t convert_complex(bool to_fp64, const void *src, void *dst, long long n, cudaStream_t stream) {
     const int blocks = (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 4096));
     if (to_fp64)

@@ -133,6 +133,8 @@ cudaError_t launch_mid_steps(const StepLaunch &l);
 
 // n complex numbers converted between complex64 and complex128 (to_fp64:
 // complex64 -> complex128).
+// The n complex numbers at m times 2^e.
+cudaError_t scale_complex(bool fp64, void *m, long long n, int e, cudaStream_t stream);
 cudaError_t convert_complex(bool to_fp64, const void *src, void *dst, long long n, cudaStream_t stream);
 
 // Ordered product of n complex64 chunk products (d <= 64) into the complex64

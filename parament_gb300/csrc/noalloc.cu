@@ -153,10 +153,10 @@ extern "C" Parament_ErrorCode Parament_equipropNoAlloc_fp64(Parament_Context_f64
     l.fp64 = true;
     l.d = d;
     l.Ke = (int)c->Ke;
-    l.w = WeightSpecHost{pts, (int)c->K, (int)amps, c->quad, c->magnus ? 1 : 0, h / 12.0};
+    l.w = WeightSpecHost{pts, (int)c->K, (int)amps, c->quad, c->magnus ? 1 : 0, c->held_step(h) / 12.0};
     l.M = M;
     l.J = J.data();
-    l.s = 2.0 / c->hnorm;
+    l.s = 2.0 / c->held_norm();
     l.x = h * c->hnorm;
     l.stack = c->stack.ptr;
     l.carr = d_carr;

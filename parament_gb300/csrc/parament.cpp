@@ -260,6 +260,8 @@ static Parament_ErrorCode set_hamiltonian(Ctx *c, const void *H0, const void *H1
     double hn = onenorm_host(H0, dim, c->fp64);
     for (unsigned k = 0; k < amps; ++k)
         hn += onenorm_host(static_cast<const char *>(H1) + es * dd * k, dim, c->fp64);
+    c->hexp = hn > 0.0 && isfinite(hn) ? ilogb(hn) : 0;
+    if (c->hexp != 0) e = scale_complex(c->fp64, st, (long long)dd * (1 + amps), -c->hexp, c->stream);
     // Magnus commutators (src/cuda/parament.cpp:289-359; pair slots triangular).
     auto commutator = [&](size_t a, size_t b, size_t dst) -> cudaError_t {
         GemmLaunch g{};
@@ -319,8 +321,8 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
     std::vector<double> J(2 * (M + 1));
     bessel_coeffs(M, h * c->hnorm, J.data());
     WeightSpecHost w{pts, (int)c->K, (int)amps, c->quad, c->magnus ? 1 : 0,
-                     c->fp64 ? h / 12.0 : (double)(float)h / 12.0};
-    const double s = 2.0 / c->hnorm;
+                     c->fp64 ? c->held_step(h) / 12.0 : (double)(float)c->held_step(h) / 12.0};
+    const double s = 2.0 / c->held_norm();
     cudaError_t e;
     // complex64 at d = 64: the same scheme with the products on the tensor
     // cores (small_tc.cu); X planes per batch of steps, one complex64 chunk
@@ -391,7 +393,7 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
         l.stream = stream;
         if (c->timing) cudaEventRecord(c->ev_start, stream);
         if (e == cudaSuccess)
-            e = launch_group_steps(l, h * c->hnorm, c->hnorm, c->num_sms, c->work.ptr,
+            e = launch_group_steps(l, h * c->hnorm, c->held_norm(), c->num_sms, c->work.ptr,
                                    static_cast<int *>(c->arrived.ptr), d_out);
         if (c->timing) cudaEventRecord(c->ev_stop, stream);
         c->launches = 1;

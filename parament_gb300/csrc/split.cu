@@ -607,7 +607,7 @@ Parament_ErrorCode run_split(Ctx *c, const void *d_carr, unsigned pts, unsigned 
     Parament_ErrorCode r = prepare_split_stack(c);
     if (r != PARAMENT_STATUS_SUCCESS) return r;
     if (fx_applies(c, FxForm::kSplit32, M, c->hnorm * h) && fx_ensure(c, P)) {
-        const WeightSpecHost w{pts, (int)c->K, (int)amps, c->quad, c->magnus ? 1 : 0, h / 12.0};
+        const WeightSpecHost w{pts, (int)c->K, (int)amps, c->quad, c->magnus ? 1 : 0, c->held_step(h) / 12.0};
         if (run_fx(c, FxForm::kSplit32, d_carr, w, c->hnorm * h, M, P, d_out, stream) == cudaSuccess)
             return PARAMENT_STATUS_SUCCESS;
         cudaGetLastError();
@@ -616,7 +616,7 @@ Parament_ErrorCode run_split(Ctx *c, const void *d_carr, unsigned pts, unsigned 
     SplitArgs a;
     double c0[2];
     std::vector<double> mu;
-    split_coefficients(M, h * c->hnorm, c->hnorm, c0, mu);
+    split_coefficients(M, h * c->hnorm, c->held_norm(), c0, mu);
     a.c0 = make_double2(c0[0], c0[1]);
     for (int n = 0; n <= kSplitMaxOrder; ++n)
         a.mu[n] = (n >= 1 && n <= M) ? make_double2(mu[2 * n], mu[2 * n + 1]) : make_double2(0, 0);
@@ -631,7 +631,7 @@ Parament_ErrorCode run_split(Ctx *c, const void *d_carr, unsigned pts, unsigned 
     a.amps = (int)amps;
     a.mode = c->quad;
     a.magnus = c->magnus ? 1 : 0;
-    a.hfac = h / 12.0;
+    a.hfac = c->held_step(h) / 12.0;
     a.fault = c->d_fault;
     // PARAMENT_SPLIT_HERMITIAN=0 turns the Hermitian-step shortcut of the
     // tensor-core kernel off (a test hook: the results are bit-identical).
@@ -641,7 +641,7 @@ Parament_ErrorCode run_split(Ctx *c, const void *d_carr, unsigned pts, unsigned 
     a.xplanes = nullptr;
     a.chunks = nullptr;
     a.nchunks = 0;
-    if (d > kSmallMaxDim) return run_split_large(c, a, h, d_out, stream);
+    if (d > kSmallMaxDim) return run_split_large(c, a, c->held_step(h), d_out, stream);
     const size_t dd = (size_t)d * d;
     const bool tensor = split_tc_applies(d, (int)c->Ke, M);
     const void *fn = pick_split(d);
