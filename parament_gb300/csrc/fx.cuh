@@ -39,7 +39,7 @@
 // cut operands into stages, one issues the digit products, eight read the levels
 // and run the epilogues.  They meet on mbarriers only: `full` (a stage is cut),
 // `done` (a stage is multiplied), `ready` (a group of stages is), `drained` (its
-// levels are read), `finished` (a product is stored).
+// levels are read), `finished` (a product is stored: two in turn, fx_turns.h).
 //
 // What bounds it: inside a long K with seven digits, 64 columns take 13 thousand
 // clocks, 8 of them on the tensor core and 5 reading the levels, during which it
@@ -55,6 +55,7 @@
 // B tiles).
 #pragma once
 
+#include "fx_turns.h"
 #include "ozaki.cuh"
 
 namespace pgb {
@@ -98,7 +99,7 @@ struct Info {
 __device__ __forceinline__ int headroom(Info i) { return i.mb >= 62 ? 0 : 62 - i.mb; }
 
 struct Shared {
-    uint64_t full[kMaxStages], done[kMaxStages], ready[2], drained[2], finished, last;
+    uint64_t full[kMaxStages], done[kMaxStages], ready[2], drained[2], finished[kFinishedBars], last;
     uint32_t tmem_base;
     uint32_t orhi[4][2], orlo[4][2];  // OR of the magnitudes of a product's results, four products in turn
     int rowmb[2][64];                 // lengths of a tile's rows, two tiles in turn
@@ -445,9 +446,9 @@ __device__ __forceinline__ void cutter(Shared &s, Thread &t, const W &w, int nst
     Cut c;
     i64 va[8], vb[8];
     auto begin = [&] {
-        const uint32_t until = n == 0 ? 0 : n - (w.needs(at, before) ? 0 : 1);
+        const uint32_t until = finished_before(n, w.needs(at, before));
         for (; seen < until; ++seen)
-            if (t.ok) t.ok = warp_wait(&s.finished, seen & 1);
+            if (t.ok) t.ok = warp_wait(&s.finished[finished_bar(seen)], finished_parity(seen));
         Operand A, B;
         const bool imag = w.operands(at, A, B);
         c = make_cut<S>(t, A, B, imag);
@@ -503,7 +504,7 @@ __device__ __forceinline__ void finisher(Shared &s, Thread &t, const W &w, int n
         }
         if (!w.epilogue(at, T, n)) break;
         __syncwarp();
-        if (t.lane == 0) arrive(&s.finished);
+        if (t.lane == 0) arrive(&s.finished[finished_bar(n)]);
     }
 }
 
@@ -714,7 +715,7 @@ __device__ __forceinline__ void setup(Shared &s, Thread &t, unsigned char *raw) 
             tc::mbar_init(&s.ready[b], 1);
             tc::mbar_init(&s.drained[b], kFinishers / 32);
         }
-        tc::mbar_init(&s.finished, kFinishers / 32);
+        for (uint32_t b = 0; b < kFinishedBars; ++b) tc::mbar_init(&s.finished[b], kFinishers / 32);
         tc::mbar_init(&s.last, 1);
         tc::fence_mbar_init();
     }
