@@ -833,7 +833,7 @@ static cudaError_t launch_adj_t(Ctx *c, const void *d_carr, unsigned pts, unsign
     }
     const void *fn = pick_adj(l.fp64, d, sweep);
     const size_t smem = adj_smem_bytes(l.fp64, d, (int)c->Ke);
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_smem(fn);
     if (e != cudaSuccess) return e;
     void *args[] = {&a};
     if (c->timing) cudaEventRecord(c->ev_start, st);
@@ -869,7 +869,7 @@ Parament_ErrorCode run_vjp(Ctx *c, const void *d_carr, double dt, unsigned pts, 
     const void *fn = pick_adj(c->fp64, d, sweep);
     const size_t smem = adj_smem_bytes(c->fp64, d, (int)c->Ke);
     int per_sm = 0;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    if (allow_smem(fn) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, smem) != cudaSuccess || per_sm < 1) {
         cudaGetLastError();
         return PARAMENT_STATUS_CUBLAS_FAILED;

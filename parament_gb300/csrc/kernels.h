@@ -47,13 +47,27 @@ int small_chunk_count(bool fp64, int d, int Ke, long long P, int num_sms);
 size_t small_smem_bytes(bool fp64, int d, int Ke);
 cudaError_t launch_small_steps(const StepLaunch &a);
 
+// Lets a kernel ask for all the dynamic shared memory of a CTA, less the `statics`
+// bytes that it declares.  The limit belongs to the function, not to a launch: always
+// the same value, since one that followed the size at hand could be lowered by another
+// thread's call before this one's launch.
+constexpr size_t kMaxSmem = 232448;
+inline cudaError_t allow_smem(const void *fn, size_t statics = 0) {
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMaxSmem - statics));
+}
+
 // A whole propagation with d <= 8 and x = Hnorm h <= 1 in one launch of groups of 16
 // threads (step_group.cu): the result in `out` (context precision); `nodes` holds
 // nchunks d x d nodes of 16 bytes, `arrived` nchunks zeros (zero again after it).
+struct GroupPlan {
+    const void *fn;
+    int groups, ld, stack_smem, nchunks, grid;  // groups of a CTA, chunks and CTAs of the launch
+    size_t smem;
+};
 bool group_applies(int d, int M, double x);
-int group_chunk_count(bool fp64, int d, int Ke, long long P, int num_sms);  // 0: does not fit
-cudaError_t launch_group_steps(const StepLaunch &l, double x, double hnorm, int num_sms, void *nodes, int *arrived,
-                               void *out);
+bool group_plan(bool fp64, int d, int Ke, long long P, int num_sms, GroupPlan &q);  // false: does not fit
+cudaError_t launch_group_steps(const StepLaunch &l, const GroupPlan &q, double x, double hnorm, void *nodes,
+                               int *arrived, void *out);
 
 // The same plain complex64 propagation at d = 64 on the tcgen05 tensor cores
 // (small_tc.cu): per batch of up to 65536 steps, the X planes of the batch

@@ -343,6 +343,7 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
         }
     }
     const int nmax = small_tc_max_chunks(P, c->num_sms);
+    GroupPlan gp;
     if (small_tc_applies(c->fp64, d, (int)c->Ke, M) && c->chunks.ensure(es * dd * nmax) == cudaSuccess &&
         c->work.ensure(16 * dd * nmax) == cudaSuccess && c->X.ensure(16 * dd * ((nmax + 1) / 2)) == cudaSuccess &&
         c->xplanes.ensure(small_tc_xplane_bytes(P)) == cudaSuccess) {
@@ -369,11 +370,9 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
                             static_cast<float2 *>(d_out), stream, &levels);
         const long long batches = (P + 65535) / 65536;
         c->launches = 2 * (int)batches + levels;
-    } else if (const int ngr = group_applies(d, M, h * c->hnorm)
-                                   ? group_chunk_count(c->fp64, d, (int)c->Ke, P, c->num_sms)
-                                   : 0) {
-        const size_t count = sizeof(int) * (size_t)ngr;
-        if (c->work.ensure(16 * dd * ngr) != cudaSuccess) return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
+    } else if (group_applies(d, M, h * c->hnorm) && group_plan(c->fp64, d, (int)c->Ke, P, c->num_sms, gp)) {
+        const size_t count = sizeof(int) * (size_t)gp.nchunks;
+        if (c->work.ensure(16 * dd * gp.nchunks) != cudaSuccess) return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
         e = cudaSuccess;
         if (c->arrived.cap < count) {
             if (c->arrived.ensure(count) != cudaSuccess) return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
@@ -393,7 +392,7 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
         l.stream = stream;
         if (c->timing) cudaEventRecord(c->ev_start, stream);
         if (e == cudaSuccess)
-            e = launch_group_steps(l, h * c->hnorm, c->held_norm(), c->num_sms, c->work.ptr,
+            e = launch_group_steps(l, gp, h * c->hnorm, c->held_norm(), c->work.ptr,
                                    static_cast<int *>(c->arrived.ptr), d_out);
         if (c->timing) cudaEventRecord(c->ev_stop, stream);
         c->launches = 1;

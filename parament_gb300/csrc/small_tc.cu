@@ -385,8 +385,7 @@ cudaError_t launch_small_tc(const StepLaunch &l, int num_sms, float *xplanes, in
     const void *asm_fn = asm_reg ? reinterpret_cast<const void *>(&k_plain_assemble<kPlainAsmRegKe>)
                                  : reinterpret_cast<const void *>(&k_plain_assemble<0>);
     const size_t hs_bytes = asm_reg ? 0 : sizeof(float4) * 128 * (size_t)(l.Ke + 1);
-    if ((e = cudaFuncSetAttribute(asm_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs_bytes)) != cudaSuccess)
-        return e;
+    if ((e = allow_smem(asm_fn, sizeof(float2) * kPlainAsmSteps * kStcMaxKe)) != cudaSuccess) return e;
     int total = 0;
     for (long long b0 = 0; b0 < l.P; b0 += kSmallXBatch) {
         const long long nb = std::min<long long>(kSmallXBatch, l.P - b0);

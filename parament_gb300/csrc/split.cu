@@ -661,7 +661,7 @@ Parament_ErrorCode run_split(Ctx *c, const void *d_carr, unsigned pts, unsigned 
             return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
         a.wts = static_cast<const float4 *>(c->wts.ptr);
     } else {
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = allow_smem(fn, sizeof(float2) * (kSplitMaxOrder + 1));
         int per_sm = 0;
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, smem);
         if (e != cudaSuccess || per_sm < 1) {

@@ -684,7 +684,7 @@ cudaError_t launch_split_tc(const SplitArgs &a, int num_sms, float *xplanes, int
     const void *asm_fn = asm_reg ? reinterpret_cast<const void *>(&k_split_assemble<kAsmRegKe>)
                                  : reinterpret_cast<const void *>(&k_split_assemble<0>);
     const size_t hs_bytes = sizeof(float4) * ((asm_reg ? 0 : 128 * (size_t)(a.Ke + 1)) + (size_t)kAsmSteps * a.Ke) + 16;
-    e = cudaFuncSetAttribute(asm_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs_bytes);
+    e = allow_smem(asm_fn, sizeof(int) * kAsmSteps);
     if (e != cudaSuccess) return e;
     if (a.Ke > 0) {
         const long long n = a.P * a.Ke;

@@ -336,15 +336,9 @@ __global__ void __launch_bounds__(384) k_group_steps(const __grid_constant__ Gro
 
 bool group_applies(int d, int M, double x) { return d <= 2 * kGroupSide && M >= 3 && x <= 1.0; }
 
-struct GroupShape {
-    const void *fn;
-    int groups, ld, stack_smem, nchunks, grid;
-    size_t smem;
-};
-
 // Groups per CTA and chunks: as many groups as shared memory and 384 threads
 // hold (an SM's share if there are fewer), one chunk per resident group at most.
-static bool group_shape(bool fp64, int d, int Ke, long long P, int num_sms, GroupShape &q) {
+bool group_plan(bool fp64, int d, int Ke, long long P, int num_sms, GroupPlan &q) {
     if (fp64)
         q.fn = d <= 4 ? reinterpret_cast<const void *>(&k_group_steps<double, 1>)
                       : reinterpret_cast<const void *>(&k_group_steps<double, 2>);
@@ -364,7 +358,7 @@ static bool group_shape(bool fp64, int d, int Ke, long long P, int num_sms, Grou
     q.groups = (int)groups;
     q.smem = stack + per * groups;
     int per_sm = 0;
-    if (cudaFuncSetAttribute(q.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)q.smem) != cudaSuccess ||
+    if (allow_smem(q.fn) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, q.fn, kGroupThreads * q.groups, q.smem) !=
             cudaSuccess ||
         per_sm < 1) {
@@ -376,17 +370,10 @@ static bool group_shape(bool fp64, int d, int Ke, long long P, int num_sms, Grou
     return true;
 }
 
-int group_chunk_count(bool fp64, int d, int Ke, long long P, int num_sms) {
-    GroupShape q{};
-    return group_shape(fp64, d, Ke, P, num_sms, q) ? q.nchunks : 0;
-}
-
 template <class R>
-static cudaError_t launch_group_t(const StepLaunch &l, double x, double hnorm, int num_sms, void *nodes, int *arrived,
-                                  void *out) {
+static cudaError_t launch_group_t(const StepLaunch &l, const GroupPlan &q, double x, double hnorm, void *nodes,
+                                  int *arrived, void *out) {
     using C = cplx_t<R>;
-    GroupShape q{};
-    if (!group_shape(l.fp64, l.d, l.Ke, l.P, num_sms, q)) return cudaErrorInvalidValue;
     GroupArgs<R> a;
     a.j0 = (R)0;
     if (l.fp64) {
@@ -417,10 +404,10 @@ static cudaError_t launch_group_t(const StepLaunch &l, double x, double hnorm, i
     return cudaLaunchKernel(q.fn, dim3(q.grid), dim3(kGroupThreads * q.groups), args, q.smem, l.stream);
 }
 
-cudaError_t launch_group_steps(const StepLaunch &l, double x, double hnorm, int num_sms, void *nodes, int *arrived,
-                               void *out) {
-    return l.fp64 ? launch_group_t<double>(l, x, hnorm, num_sms, nodes, arrived, out)
-                  : launch_group_t<float>(l, x, hnorm, num_sms, nodes, arrived, out);
+cudaError_t launch_group_steps(const StepLaunch &l, const GroupPlan &q, double x, double hnorm, void *nodes,
+                               int *arrived, void *out) {
+    return l.fp64 ? launch_group_t<double>(l, q, x, hnorm, nodes, arrived, out)
+                  : launch_group_t<float>(l, q, x, hnorm, nodes, arrived, out);
 }
 
 }  // namespace pgb

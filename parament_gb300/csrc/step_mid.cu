@@ -276,7 +276,7 @@ static cudaError_t launch_mid_t(const StepLaunch &l) {
     a.w = WeightSpec{l.w.pts, l.w.K, l.w.amps, l.w.mode, l.w.magnus, l.w.hfac};
     const size_t smem = mid_smem_bytes(l.fp64, l.d, l.Ke);
     const void *fn = reinterpret_cast<const void *>(&k_mid_steps<R>);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(fn);
     if (e != cudaSuccess) return e;
     void *args[] = {&a};
     return cudaLaunchKernel(fn, dim3(kMidCluster * l.nchunks), dim3(256), args, smem, l.stream);

@@ -260,7 +260,7 @@ static bool small_powers(const StepLaunch &l) { return l.x > 0.0 && l.x <= 1.0 &
 int small_chunk_count(bool fp64, int d, int Ke, long long P, int num_sms) {
     const void *fn = pick_small(fp64, d, true);
     size_t smem = small_smem_bytes(fp64, d, Ke);
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(fn);
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
     long long n = (long long)per_sm * num_sms;
@@ -296,7 +296,7 @@ static cudaError_t launch_small_t(const StepLaunch &l) {
         for (int n = 0; n <= l.M; ++n) a.c[n] = (R)c[n];
     }
     const void *fn = pick_small(l.fp64, l.d, powers);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(fn);
     if (e != cudaSuccess) return e;
     void *args[] = {&a};
     return cudaLaunchKernel(fn, dim3(l.nchunks), dim3(256), args, smem, l.stream);
