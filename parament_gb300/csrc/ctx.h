@@ -63,6 +63,7 @@ struct Ctx {
     void *fx_stack = nullptr;  // behind the matrices of `stack`, in its allocation
     DevBuf fx_split, fx_ws;
     bool fx_ready = false, fx_split_ready = false;
+    bool fx_ran = false;  // by the last equiprop
 
     // Instrumentation: CUDA events around the dominant kernel of the last call
     // and the number of kernels it launched.
@@ -155,7 +156,7 @@ enum class FxForm { kFp64, kPlain32, kSplit32 };
 size_t fx_stack_bytes(const Ctx *c, unsigned dim, unsigned Ke);  // 0: none is kept
 void fx_prepare(Ctx *c);
 void fx_prepare_split(Ctx *c);
-bool fx_applies(const Ctx *c, FxForm form, int M, double x);
+bool fx_applies(const Ctx *c, FxForm form, int M, double x, long long P);
 bool fx_ensure(Ctx *c, long long P);
 cudaError_t run_fx(Ctx *c, FxForm form, const void *d_carr, const WeightSpecHost &wh, double x, int M, long long P,
                    void *d_out, cudaStream_t stream);

@@ -675,10 +675,34 @@ static cudaError_t launch_gemm_op(const GemmArgs &a, int num_sms, cudaStream_t s
 
 using namespace fx;
 
-bool fx_applies(const Ctx *c, FxForm form, int M, double x) {
+// Whether these kernels are the faster ones for P steps of order M.  A product takes
+// them about as long at any d up to 64 and has a latency of some 20 us; the other
+// kernels' products are short at small d and take turns with fewer launches.  Measured
+// against those, times here over times there:
+//   complex64, plain   d = 96 M = 3  1.96 (16 steps) 1.31 (2048)   M = 7  1.62, 0.81
+//                      d = 128       1.61, 0.95                           1.15, 0.60
+//                      d = 200       1.13, 0.87                           0.74, 0.59
+//                      d = 500       0.62 (1 step: 1.26)                  0.45 (0.71)
+//   The line: the FP32 kernels' time per step goes as tiles d M, that of these as the
+//   tiles; of 780 pairs from d = 65 to 500 and orders 3 to 9 it leaves 5 per cent at most
+//   where they are the slower ones and 1 per cent of the time on the whole.
+//   split form         d = 65 M = 7  1.66 (1 step) 1.12 (8) 0.90 (16)
+//                      d = 128       1.63, 0.75, 0.50;  d = 300: 1.61, 0.57 (2 steps)
+//   complex128         d = 17 M = 5  1.15 (16 steps) 1.25 (152) 0.97 (200) 0.62 (3000)
+//                      d = 22        1.01, 1.17, 0.87, 0.50;  d = 32: 0.84, 0.99, 0.71, 0.35
+//   (one step per SM at most is one product after the other in either kernel).
+static bool fx_faster(FxForm form, int d, int M, long long P, int num_sms) {
+    const long long nt = (d + 63) / 64, tiles = nt * nt;
+    if (form == FxForm::kFp64) return P > num_sms || M > 7 || d > (M > 3 ? 20 : kFxSimtDim);
+    if (form == FxForm::kSplit32) return P >= 2 && P * d * d >= 80000;
+    return P * tiles * ((long long)d * M - 420) >= 155000;
+}
+
+bool fx_applies(const Ctx *c, FxForm form, int M, double x, long long P) {
     if (M < 3 || !isfinite(c->hnorm) || c->hnorm <= 0.0) return false;
-    if (form == FxForm::kFp64) return c->fx_ready;
-    return x <= 1.0 && (form == FxForm::kPlain32 ? c->fx_ready : c->fx_split_ready);
+    if (form != FxForm::kFp64 && x > 1.0) return false;
+    return (form == FxForm::kSplit32 ? c->fx_split_ready : c->fx_ready) &&
+           fx_faster(form, (int)c->dim, M, P, c->num_sms);
 }
 
 // Whether a context's Hamiltonian gets a fixed-point stack: complex64 from 65 on
@@ -911,6 +935,7 @@ static cudaError_t run_fx_t(Ctx *c, FxForm form, const void *d_carr, const Weigh
 
 cudaError_t run_fx(Ctx *c, FxForm form, const void *d_carr, const WeightSpecHost &wh, double x, int M, long long P,
                    void *d_out, cudaStream_t st) {
+    c->fx_ran = true;
     if (form == FxForm::kFp64) return run_fx_t<7, double2, double2>(c, form, d_carr, wh, x, M, P, d_out, st);
     if (form == FxForm::kPlain32) return run_fx_t<4, float2, float2>(c, form, d_carr, wh, x, M, P, d_out, st);
     return run_fx_t<5, double2, float2>(c, form, d_carr, wh, x, M, P, d_out, st);

@@ -24,6 +24,8 @@ struct WeightSpecHost {
 constexpr int kSmallMaxDim = 64;
 // complex128 from this dimension on runs as exact sliced products (fx.cu).
 constexpr int kFxMinDim = 17;
+// Up to here a few steps of a low order may run on the FP64 pipe (fx.cu, fx_faster).
+constexpr int kFxSimtDim = 32;
 
 struct StepLaunch {
     bool fp64;

@@ -334,7 +334,7 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
     // the least memory, where it applies.
     bool no_room = false;
     const FxForm form = c->fp64 ? FxForm::kFp64 : FxForm::kPlain32;
-    if (fx_applies(c, form, M, h * c->hnorm)) {
+    if (fx_applies(c, form, M, h * c->hnorm, P)) {
         no_room = !fx_ensure(c, P);
         if (!no_room) {
             if (run_fx(c, form, d_carr, w, h * c->hnorm, M, P, d_out, stream) == cudaSuccess) return PARAMENT_STATUS_SUCCESS;
@@ -524,10 +524,10 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
 
 // Whether an equiprop of this context may launch a kernel with bounded waits
 // (the tensor-core GEMM of complex64 contexts with d > 64, the tensor-core
-// split kernel, the tensor-core plain kernel at d = 64, the sliced products of
-// complex128 contexts).
+// split kernel, the tensor-core plain kernel at d = 64), or has launched one (the
+// sliced products of complex128 contexts).
 static bool uses_tensor_kernels(const Ctx *c) {
-    if (c->fp64) return c->fx_ready;
+    if (c->fp64) return c->fx_ran;
     return c->dim >= (unsigned)kSmallMaxDim || c->precision == PARAMENT_PRECISION_SPLIT;
 }
 
@@ -552,6 +552,7 @@ static Parament_ErrorCode equiprop_device(Ctx *c, const void *d_carr, double dt,
         M = select_cycles(c->fp64, c->hnorm, h);
         if (M < 3) return PARAMENT_STATUS_SELECT_SMALLER_DT;
     }
+    c->fx_ran = false;
     if (c->hnorm == 0.0 || dt == 0.0) {
         // exp(0) = I for every step: the product is the identity.
         cudaError_t e = fill_identity(c->fp64, d_out, (int)c->dim, 1, 1.0, 0.0, stream);
