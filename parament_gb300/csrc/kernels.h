@@ -66,7 +66,7 @@ struct GroupPlan {
     int groups, ld, stack_smem, nchunks, grid;  // groups of a CTA, chunks and CTAs of the launch
     size_t smem;
 };
-bool group_applies(int d, int M, double x);
+bool group_applies(bool fp64, int d, int M, double x, long long P);
 bool group_plan(bool fp64, int d, int Ke, long long P, int num_sms, GroupPlan &q);  // false: does not fit
 cudaError_t launch_group_steps(const StepLaunch &l, const GroupPlan &q, double x, double hnorm, void *nodes,
                                int *arrived, void *out);

@@ -370,7 +370,7 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
                             static_cast<float2 *>(d_out), stream, &levels);
         const long long batches = (P + 65535) / 65536;
         c->launches = 2 * (int)batches + levels;
-    } else if (group_applies(d, M, h * c->hnorm) && group_plan(c->fp64, d, (int)c->Ke, P, c->num_sms, gp)) {
+    } else if (group_applies(c->fp64, d, M, h * c->hnorm, P) && group_plan(c->fp64, d, (int)c->Ke, P, c->num_sms, gp)) {
         const size_t count = sizeof(int) * (size_t)gp.nchunks;
         if (c->work.ensure(16 * dd * gp.nchunks) != cudaSuccess) return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
         e = cudaSuccess;

@@ -76,3 +76,23 @@ def test_line(switched_off, i):
         assert M == Mo
         bar = {"plain": 1e-5 if precision == "fp32" else 1e-10, "split": 1e-6}[form]
         assert np.linalg.norm(U - Uo) / np.linalg.norm(Uo) < bar
+
+
+@pytest.mark.parametrize("precision,d,steps,launches", [
+    ("fp64", 8, 1, 0), ("fp64", 5, 8, 0), ("fp64", 8, 9, 1), ("fp64", 4, 2, 1), ("fp32", 8, 2, 1)])
+@pytest.mark.parametrize("x", [1e-4, 0.6])
+def test_small_groups(built_lib, precision, d, steps, launches, x):
+    """d <= 8: one launch in all, or (complex128, d > 4, up to eight steps) the step
+    kernel and the tree, as many as a call above x = 1 takes."""
+    import parament_gb300 as parament
+    H0, H1, u, dt = problem(precision, d, steps, x)
+    with parament.Parament(precision) as ctx:
+        ctx.set_hamiltonian(H0, *H1)
+        count = ctx._fn("Parament_lastLaunchCount")
+        ctx.equiprop(dt / x * 1.5, *u)
+        above = int(count(ctx._handle))
+        U = ctx.equiprop(dt, *u)
+        assert int(count(ctx._handle)) == (launches or above)
+    c = [a.astype(np.complex128) for a in (H0, H1, u)]
+    Uo = oracle.equiprop(*c, dt, single=precision == "fp32")[0]
+    assert np.linalg.norm(U - Uo) / np.linalg.norm(Uo) < (1e-5 if precision == "fp32" else 1e-14)
