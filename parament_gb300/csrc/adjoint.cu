@@ -875,11 +875,19 @@ Parament_ErrorCode run_vjp(Ctx *c, const void *d_carr, double dt, unsigned pts, 
         return PARAMENT_STATUS_CUBLAS_FAILED;
     }
     const int nc = (int)std::max<long long>(1, std::min<long long>((long long)per_sm * c->num_sms, P));
+    // Buffers for either sweep's chunks: a call at another step length may come in a
+    // capture.
+    int per_other = 0;
+    const void *other = pick_adj(c->fp64, d, !sweep);
+    if (allow_smem(other) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_other, other, 256, smem) != cudaSuccess)
+        cudaGetLastError();
+    const size_t ncb = (size_t)std::max<long long>(nc, std::min<long long>((long long)per_other * c->num_sms, P));
     const size_t es = c->esize(), dd = (size_t)d * d;
     // The order tables keep the truncation of every step exponential below
     // the working precision, so U_j^H inverts U_j; a manual order may not.
     const bool reversible = !c->manual;
-    if (c->chunks.ensure(es * dd * nc) != cudaSuccess || c->work.ensure(es * dd * (4 * (size_t)nc + 2)) != cudaSuccess ||
+    if (c->chunks.ensure(es * dd * ncb) != cudaSuccess || c->work.ensure(es * dd * (4 * ncb + 2)) != cudaSuccess ||
         (!reversible && c->X.ensure(es * dd * (size_t)P) != cudaSuccess) ||
         c->aux.ensure(es * (size_t)P * std::max(1u, c->Ke)) != cudaSuccess)
         return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;

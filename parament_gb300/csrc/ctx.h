@@ -17,6 +17,8 @@
 namespace pgb {
 
 bool fault_inject_alloc();
+// Whether calls on `stream` go into a graph: nothing is allocated or waited for then.
+bool capturing(cudaStream_t stream);
 
 struct DevBuf {
     void *ptr = nullptr;
@@ -150,14 +152,14 @@ double plain_coefficients(int M, double x, double hnorm, std::vector<double> &c)
 
 // Exact sliced products (fx.cu): fx_prepare / fx_prepare_split convert the stack
 // (set_hamiltonian; the split form's first call), fx_ensure allocates the
-// workspace of P steps, run_fx propagates (x = Hnorm h).
+// workspace of P steps (not into a capture: what is there has to do), run_fx propagates (x = Hnorm h).
 struct WeightSpecHost;
 enum class FxForm { kFp64, kPlain32, kSplit32 };
 size_t fx_stack_bytes(const Ctx *c, unsigned dim, unsigned Ke);  // 0: none is kept
 void fx_prepare(Ctx *c);
 void fx_prepare_split(Ctx *c);
 bool fx_applies(const Ctx *c, FxForm form, int M, double x, long long P);
-bool fx_ensure(Ctx *c, long long P);
+bool fx_ensure(Ctx *c, long long P, cudaStream_t stream);
 cudaError_t run_fx(Ctx *c, FxForm form, const void *d_carr, const WeightSpecHost &wh, double x, int M, long long P,
                    void *d_out, cudaStream_t stream);
 

@@ -760,8 +760,9 @@ void fx_prepare_split(Ctx *c) {
     c->fx_split_ready = convert_stack<float2>(c, c->split_stack.ptr, p);
 }
 
-bool fx_ensure(Ctx *c, long long P) {
+bool fx_ensure(Ctx *c, long long P, cudaStream_t stream) {
     const Plan q = make_plan((int)c->dim, (int)c->Ke, P, c->num_sms);
+    if (c->fx_ws.cap < q.bytes && capturing(stream)) return false;
     return c->fx_ws.ensure(q.bytes) == cudaSuccess;
 }
 

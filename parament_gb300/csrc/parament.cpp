@@ -119,7 +119,7 @@ long long num_steps(int quad, bool magnus, unsigned pts) {
 // The fault counter's copy and event stay out of a graph that is being captured
 // on the stream: its calls may not query events.  The counter keeps what the
 // graph's replays add to it.
-static bool capturing(cudaStream_t stream) {
+bool capturing(cudaStream_t stream) {
     cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(stream, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
 }
@@ -335,8 +335,15 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
     bool no_room = false;
     const FxForm form = c->fp64 ? FxForm::kFp64 : FxForm::kPlain32;
     if (fx_applies(c, form, M, h * c->hnorm, P)) {
-        no_room = !fx_ensure(c, P);
-        if (!no_room) {
+        const bool room = fx_ensure(c, P, stream);
+        no_room = !room && !capturing(stream);
+        if (room) {
+            // Fewer steps, which the FP64 kernels take here, find their buffers too
+            // (they may come in a capture).
+            if (c->fp64 && d <= kFxSimtDim && !capturing(stream) &&
+                (c->chunks.ensure(es * dd * c->num_sms) != cudaSuccess ||
+                 c->work.ensure(16 * dd * c->num_sms) != cudaSuccess))
+                return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
             if (run_fx(c, form, d_carr, w, h * c->hnorm, M, P, d_out, stream) == cudaSuccess) return PARAMENT_STATUS_SUCCESS;
             cudaGetLastError();
             return PARAMENT_STATUS_CUBLAS_FAILED;
@@ -370,15 +377,20 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
                             static_cast<float2 *>(d_out), stream, &levels);
         const long long batches = (P + 65535) / 65536;
         c->launches = 2 * (int)batches + levels;
-    } else if (group_applies(c->fp64, d, M, h * c->hnorm, P) && group_plan(c->fp64, d, (int)c->Ke, P, c->num_sms, gp)) {
+    } else if (group_applies(c->fp64, d, M, h * c->hnorm, P) && group_plan(c->fp64, d, (int)c->Ke, P, c->num_sms, gp) &&
+               ((c->arrived.cap >= sizeof(int) * (size_t)gp.nchunks && c->work.cap >= 16 * dd * gp.nchunks) ||
+                !capturing(stream))) {
         const size_t count = sizeof(int) * (size_t)gp.nchunks;
         if (c->work.ensure(16 * dd * gp.nchunks) != cudaSuccess) return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
         e = cudaSuccess;
         if (c->arrived.cap < count) {
-            if (c->arrived.ensure(count) != cudaSuccess) return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
-            // The next call may come on another stream.
+            // And the buffers of the step kernel, for calls above x = 1 (they may come in a capture).
+            const int nch = small_chunk_count(c->fp64, d, (int)c->Ke, P, c->num_sms);
+            if (c->arrived.ensure(count) != cudaSuccess || c->chunks.ensure(es * dd * nch) != cudaSuccess ||
+                c->work.ensure(16 * dd * nch) != cudaSuccess ||
+                (!c->fp64 && c->X.ensure(16 * dd * ((nch + 1) / 2)) != cudaSuccess))
+                return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
             e = cudaMemsetAsync(c->arrived.ptr, 0, c->arrived.cap, stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         }
         StepLaunch l{};
         l.fp64 = c->fp64;

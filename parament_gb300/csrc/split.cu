@@ -606,7 +606,7 @@ Parament_ErrorCode run_split(Ctx *c, const void *d_carr, unsigned pts, unsigned 
     if (M > kSplitMaxOrder || c->hnorm * h > kSplitMaxX) return PARAMENT_STATUS_SELECT_SMALLER_DT;
     Parament_ErrorCode r = prepare_split_stack(c);
     if (r != PARAMENT_STATUS_SUCCESS) return r;
-    if (fx_applies(c, FxForm::kSplit32, M, c->hnorm * h, P) && fx_ensure(c, P)) {
+    if (fx_applies(c, FxForm::kSplit32, M, c->hnorm * h, P) && fx_ensure(c, P, stream)) {
         const WeightSpecHost w{pts, (int)c->K, (int)amps, c->quad, c->magnus ? 1 : 0, c->held_step(h) / 12.0};
         if (run_fx(c, FxForm::kSplit32, d_carr, w, c->hnorm * h, M, P, d_out, stream) == cudaSuccess)
             return PARAMENT_STATUS_SUCCESS;
