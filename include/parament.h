@@ -241,7 +241,9 @@ PARAMENT_API Parament_ErrorCode Parament_equipropNoAlloc_fp64(Parament_Context_f
  * report (that call's result is then not valid), PARAMENT_STATUS_SUCCESS
  * otherwise.  Such a give-up is also reported by the host-buffer entry point
  * that ran the kernel, and by the next device-buffer call on the context once
- * it is known (that call then queues nothing). */
+ * it is known (that call then queues nothing).  Calls captured into a graph
+ * record nothing; for what its replays met, wait for them, then call
+ * Parament_synchronize. */
 PARAMENT_API Parament_ErrorCode Parament_synchronize(Parament_Context_f32 *handle);
 PARAMENT_API Parament_ErrorCode Parament_synchronize_fp64(Parament_Context_f64 *handle);
 /* Bytes of device memory the context's buffers hold (Hamiltonian and work

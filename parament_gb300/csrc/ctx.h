@@ -88,7 +88,8 @@ struct Ctx {
     // there.  A count above faults_seen is reported as
     // PARAMENT_STATUS_KERNEL_TIMEOUT by the call itself (host-buffer entry
     // points), by Parament_synchronize, or by the next device-buffer call on
-    // the context.
+    // the context.  Calls that go into a graph leave copy and events out; once
+    // there was one (`captured`), Parament_synchronize copies the counter itself.
     int *d_fault = nullptr;
     int *h_fault = nullptr;
     int faults_seen = 0;
@@ -96,6 +97,7 @@ struct Ctx {
     bool fault_recorded = false;
     cudaEvent_t ev_done = nullptr;   // end of the last call's work
     bool done_recorded = false;
+    bool captured = false;
 
     size_t esize() const { return fp64 ? 16 : 8; }
     size_t device_bytes() const {

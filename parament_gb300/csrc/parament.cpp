@@ -64,6 +64,18 @@ bool fault_inject_alloc() {
     return false;
 }
 
+// PARAMENT_FAIL_WAIT_AFTER=n makes the (n+1)-th call of this process that may launch a
+// kernel with bounded waits (and only that one) count a wait that gave up, by a memset
+// on the call's stream, so that the reports can be tested without a kernel that waits
+// in vain.
+static bool fault_inject_wait() {
+    static long long budget = [] {
+        const char *v = getenv("PARAMENT_FAIL_WAIT_AFTER");
+        return v ? atoll(v) : -1LL;
+    }();
+    return budget >= 0 && budget-- == 0;
+}
+
 double onenorm_host(const void *m, unsigned d, bool fp64) {
     double best = 0.0;
     for (unsigned i = 0; i < d; ++i) {
@@ -116,16 +128,20 @@ long long num_steps(int quad, bool magnus, unsigned pts) {
     return pts;
 }
 
-// The fault counter's copy and event stay out of a graph that is being captured
-// on the stream: its calls may not query events.  The counter keeps what the
-// graph's replays add to it.
 bool capturing(cudaStream_t stream) {
     cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(stream, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
 }
 
 void note_call_end(Ctx *c, cudaStream_t stream, bool tensor_kernels) {
-    if (tensor_kernels && !capturing(stream) &&
+    if (tensor_kernels && fault_inject_wait()) cudaMemsetAsync(c->d_fault, 1, 1, stream);
+    // No copy and no event into a graph that is being captured: the events of a capture
+    // can be neither queried nor waited for.  The counter keeps what replays add to it.
+    if (capturing(stream)) {
+        c->captured = c->captured || tensor_kernels;
+        return;
+    }
+    if (tensor_kernels &&
         cudaMemcpyAsync(c->h_fault, c->d_fault, sizeof(int), cudaMemcpyDeviceToHost, stream) == cudaSuccess &&
         cudaEventRecord(c->ev_fault, stream) == cudaSuccess)
         c->fault_recorded = true;
@@ -911,6 +927,11 @@ static Parament_ErrorCode ctx_synchronize(Ctx *c) {
     cudaSetDevice(c->device);
     cudaError_t e = cudaSuccess;
     if (c->done_recorded) e = cudaEventSynchronize(c->ev_done);
+    if (e == cudaSuccess && c->captured) {
+        e = cudaMemcpyAsync(c->h_fault, c->d_fault, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = cudaEventRecord(c->ev_fault, c->stream);
+        if (e == cudaSuccess) c->fault_recorded = true;
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
