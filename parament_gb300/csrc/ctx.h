@@ -75,7 +75,8 @@ struct Ctx {
 
     // Work buffers (grow-only, like src/cuda/parament.cpp:418-474)
     DevBuf carr, out, chunks, work, X, B1, B2, aux, grad, wts, xplanes;
-    DevBuf arrived;  // pair counters of the small groups' tree, zero between launches
+    DevBuf arrived;  // arrivals at the pairs of the small groups' tree (step_group.cu)
+    unsigned group_turn = 0;  // of the last launch of small groups
 
     // Pinned memory that kernels reach directly: samples and result of small
     // host-buffer calls.

@@ -60,7 +60,8 @@ inline cudaError_t allow_smem(const void *fn, size_t statics = 0) {
 
 // A whole propagation with d <= 8 and x = Hnorm h <= 1 in one launch of groups of 16
 // threads (step_group.cu): the result in `out` (context precision); `nodes` holds
-// nchunks d x d nodes of 16 bytes, `arrived` nchunks zeros (zero again after it).
+// nchunks d x d nodes of 16 bytes; `arrived` has nchunks numbers other than `turn`,
+// which is not zero (other than `turn` again after it).
 struct GroupPlan {
     const void *fn;
     int groups, ld, stack_smem, nchunks, grid;  // groups of a CTA, chunks and CTAs of the launch
@@ -69,7 +70,7 @@ struct GroupPlan {
 bool group_applies(bool fp64, int d, int M, double x, long long P);
 bool group_plan(bool fp64, int d, int Ke, long long P, int num_sms, GroupPlan &q);  // false: does not fit
 cudaError_t launch_group_steps(const StepLaunch &l, const GroupPlan &q, double x, double hnorm, void *nodes,
-                               int *arrived, void *out);
+                               unsigned *arrived, unsigned turn, void *out);
 
 // The same plain complex64 propagation at d = 64 on the tcgen05 tensor cores
 // (small_tc.cu): per batch of up to 65536 steps, the X planes of the batch

@@ -394,9 +394,9 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
         const long long batches = (P + 65535) / 65536;
         c->launches = 2 * (int)batches + levels;
     } else if (group_applies(c->fp64, d, M, h * c->hnorm, P) && group_plan(c->fp64, d, (int)c->Ke, P, c->num_sms, gp) &&
-               ((c->arrived.cap >= sizeof(int) * (size_t)gp.nchunks && c->work.cap >= 16 * dd * gp.nchunks) ||
+               ((c->arrived.cap >= sizeof(unsigned) * (size_t)gp.nchunks && c->work.cap >= 16 * dd * gp.nchunks) ||
                 !capturing(stream))) {
-        const size_t count = sizeof(int) * (size_t)gp.nchunks;
+        const size_t count = sizeof(unsigned) * (size_t)gp.nchunks;
         if (c->work.ensure(16 * dd * gp.nchunks) != cudaSuccess) return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
         e = cudaSuccess;
         if (c->arrived.cap < count) {
@@ -407,7 +407,11 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
                 (!c->fp64 && c->X.ensure(16 * dd * ((nch + 1) / 2)) != cudaSuccess))
                 return PARAMENT_STATUS_DEVICE_ALLOC_FAILED;
             e = cudaMemsetAsync(c->arrived.ptr, 0, c->arrived.cap, stream);
+        } else if (capturing(stream)) {
+            // A graph's launches have one turn for all replays.
+            e = cudaMemsetAsync(c->arrived.ptr, 0, count, stream);
         }
+        if (++c->group_turn == 0) c->group_turn = 1;
         StepLaunch l{};
         l.fp64 = c->fp64;
         l.d = d;
@@ -421,7 +425,7 @@ static Parament_ErrorCode run_plain(Ctx *c, const void *d_carr, unsigned pts, un
         if (c->timing) cudaEventRecord(c->ev_start, stream);
         if (e == cudaSuccess)
             e = launch_group_steps(l, gp, h * c->hnorm, c->held_norm(), c->work.ptr,
-                                   static_cast<int *>(c->arrived.ptr), d_out);
+                                   static_cast<unsigned *>(c->arrived.ptr), c->group_turn, d_out);
         if (c->timing) cudaEventRecord(c->ev_stop, stream);
         c->launches = 1;
     } else if (d <= kSmallMaxDim) {

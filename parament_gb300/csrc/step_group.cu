@@ -45,7 +45,10 @@ struct GroupArgs {
     R j0;                // complex64: J_0, added last
     const cplx_t<R> *stack, *carr;
     void *nodes;         // nodes of the tree, float4 (double-float) or double2
-    int *arrived;        // arrivals at a pair, zero between launches
+    // A pair's first arrival leaves the launch's turn there, the second finds it and
+    // leaves zero.  What launches that overlapped on one context may leave behind has
+    // another turn and counts for nothing.
+    unsigned *arrived, turn;
     cplx_t<R> *out;
     long long P;
     int nchunks, d, Ke, M, ld, stack_smem;
@@ -308,9 +311,9 @@ __global__ void __launch_bounds__(384) k_group_steps(const __grid_constant__ Gro
         __threadfence();
         group_sync(g);
         if (gt == 0) {
-            const int before = atomicAdd(&a.arrived[hi], 1);
-            if (before) a.arrived[hi] = 0;
-            *flag = before;
+            const bool second = atomicExch(&a.arrived[hi], a.turn) == a.turn;
+            if (second) a.arrived[hi] = 0;
+            *flag = second;
         }
         group_sync(g);
         if (*flag == 0) return;  // the partner's group takes the pair
@@ -377,7 +380,7 @@ bool group_plan(bool fp64, int d, int Ke, long long P, int num_sms, GroupPlan &q
 
 template <class R>
 static cudaError_t launch_group_t(const StepLaunch &l, const GroupPlan &q, double x, double hnorm, void *nodes,
-                                  int *arrived, void *out) {
+                                  unsigned *arrived, unsigned turn, void *out) {
     using C = cplx_t<R>;
     GroupArgs<R> a;
     a.j0 = (R)0;
@@ -396,6 +399,7 @@ static cudaError_t launch_group_t(const StepLaunch &l, const GroupPlan &q, doubl
     a.carr = static_cast<const C *>(l.carr);
     a.nodes = nodes;
     a.arrived = arrived;
+    a.turn = turn;
     a.out = static_cast<C *>(out);
     a.P = l.P;
     a.nchunks = q.nchunks;
@@ -410,9 +414,9 @@ static cudaError_t launch_group_t(const StepLaunch &l, const GroupPlan &q, doubl
 }
 
 cudaError_t launch_group_steps(const StepLaunch &l, const GroupPlan &q, double x, double hnorm, void *nodes,
-                               int *arrived, void *out) {
-    return l.fp64 ? launch_group_t<double>(l, q, x, hnorm, nodes, arrived, out)
-                  : launch_group_t<float>(l, q, x, hnorm, nodes, arrived, out);
+                               unsigned *arrived, unsigned turn, void *out) {
+    return l.fp64 ? launch_group_t<double>(l, q, x, hnorm, nodes, arrived, turn, out)
+                  : launch_group_t<float>(l, q, x, hnorm, nodes, arrived, turn, out);
 }
 
 }  // namespace pgb
