@@ -17,7 +17,10 @@
 // Samples to results: 512 complex64 problems 36.5 -> 33.0 ms, 64 of them
 // 8.7 -> 6.2, 40 complex128 problems of up to 1000 steps 42.7 -> 20.3, 32 short ones
 // 1.50 -> 0.45.  The classes run one after another: as parallel branches of the
-// graph they gained 1.5 per cent (5 for 64 problems) and gave wrong d = 16 products.
+// graph they gained 1.5 per cent (5 for 64 problems) and some replays gave wrong d = 16
+// products beside the classes of d <= 8.  The cause was not found: no access of these
+// kernels leaves its chunk, and ensembles of such classes that run beside each other from
+// several threads give the bits that each gives alone.
 // The chunk length per class comes from an autotuner that times a few candidate
 // granularities on the actual ensemble.
 #include <math.h>
