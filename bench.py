@@ -225,7 +225,7 @@ def split_slice_products(M):
 
 # The step kernel each form of the d=64 workload runs.
 FORM_KERNELS = {"plain_c128": "k_fx_steps (tcgen05, exact products of seven 8-bit digits)",
-                "plain_c64": "k_small_tc (tcgen05, exact four-slice bf16 products; FP32 Clenshaw)",
+                "plain_c64": "k_small_tc (tcgen05, exact four-slice bf16 products; FP32 polynomial)",
                 "split_c64": "k_split_tc (tcgen05, exact bf16 slices; double-float E and running product)"}
 
 
@@ -455,7 +455,8 @@ def large_dense_block(torch, parament, K_steps, W_steps, flush, stream, err_step
         M = ctx.last_iteration_cycles
         Us[form] = out.cpu().numpy().astype(np.complex128)
         ctx.destroy()
-        nprod = (M + 1) if form == "plain_c64" else (M - 3) // 2 + 3
+        # Split form: powers of X (fx.cu) and the running product.
+        nprod = (M + 1) if form == "plain_c64" else {3: 2, 5: 3, 7: 4, 9: 4, 11: 5, 13: 6, 15: 6}[M] + 1
         flops = steps * (M + 1) * 8.0 * 512 ** 3
         res[form] = {"M": M, "ms": round(ms, 3), "steps_per_s": round(steps / (ms * 1e-3), 1),
                      "kernel": ("k_tc_cgemm (tcgen05 kind::tf32, 3xTF32 split products)" if form == "plain_c64"
@@ -465,8 +466,8 @@ def large_dense_block(torch, parament, K_steps, W_steps, flush, stream, err_step
                      "rel_err_vs_oracle_prefix": oracle_prefix_error(parament, w, "fp32", err_steps,
                                                                     split=(form == "split_c64")),
                      "rel_err_prefix_steps": err_steps}
-    res["split_c64"]["scheme"] = ("split form: E = c0 + a1 Z (double-float) + Horner GEMMs, double-float chunk "
-                                  "running products, FP64 tree; GEMMs on the exact sliced tensor-core kernel")
+    res["split_c64"]["scheme"] = ("split form: E by powers of X on 64-bit fixed-point matrices, products of five "
+                                  "8-bit digits exact on the tensor cores, running products and tree in the same form")
     res["plain_c64"]["scheme"] = "the reference's plain complex64 scheme (fp32 order table)"
     if fp64_check:
         ctx = parament.Parament("fp64")
@@ -573,7 +574,7 @@ def mid_block(torch, parament, K_steps, W_steps, flush, stream, steps=16384):
             "M": M, "ms": round(ms, 3), "steps_per_s": round(steps / (ms * 1e-3), 1),
             "algorithmic_tflops": round(fl / (ms * 1e-3) / 1e12, 2), "launches": launches,
             "rel_err_vs_oracle_prefix": oracle_prefix_error(parament, w, prec, 64), "rel_err_prefix_steps": 64}
-    out["workload"] = (f"K=3 NONE ||H0||=8, {steps} steps; the default path for 64 < d <= 128 (k_fx_steps, k_fx_gemm; "
+    out["workload"] = (f"K=3 NONE ||H0||=8, {steps} steps; the default path for 64 < d <= 128 (k_fx_gemm; "
                        f"the cluster-resident k_mid_steps serves when the batch buffers cannot be allocated)")
     return out
 

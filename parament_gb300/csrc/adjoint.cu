@@ -697,7 +697,10 @@ __global__ void __launch_bounds__(256) k_adj_scan(const cplx_t<R> *S, int nc, in
     }
 }
 
-// Where k_adj_scan is the faster one: a product within two microseconds.
+// k_adj_scan where a product takes a microsecond or two.  600 steps, with it and by
+// Hillis-Steele: complex64 d = 16 93 and 216 us, d = 32 205 and 348; complex128 d = 8
+// 378 and 541.  (It would still be ahead at d = 40, 372 and 516, and in complex128 at
+// d = 12, 534 and 647, not at d = 24, 3186 and 2946.)
 static bool short_scan(bool fp64, int d) { return fp64 ? d <= 8 : d <= 32; }
 
 template <class R, int TM>

@@ -1,7 +1,8 @@
 // Propagation on fixed-point matrices and exact sliced products on the tensor cores
 // (fx.cuh): complex128 from d = kFxMinDim on (seven digits), and complex64 with d >
 // 64, where the 3xTF32 kernel does not serve, in the plain form (four digits) and
-// the split form (five).
+// the split form (five).  Few steps of a low order stay with the FP32 and FP64 kernels
+// (fx_faster).
 //
 // The same X_j, Chebyshev order and Bessel coefficients as the FP64 kernels
 // (step_small.cu, gemm.cu; src/cuda/parament.cpp:486-718).  What changes:
@@ -707,7 +708,8 @@ bool fx_applies(const Ctx *c, FxForm form, int M, double x, long long P) {
 
 // Whether a context's Hamiltonian gets a fixed-point stack: complex64 from 65 on
 // (below, the step kernels of one launch are faster: a product's epilogue takes
-// longer here than its digits), and the plain form not where the 3xTF32 kernel runs.
+// longer here than its digits), and the plain form not where the 3xTF32 kernel runs: d
+// = 512, 64 steps of order 7 take 2.45 ms there and 5.96 here, d = 256 0.62 and 1.01.
 static bool fx_serves(FxForm form, int d) {
     if (disabled()) return false;
     if (form == FxForm::kFp64) return d >= kFxMinDim;
@@ -720,6 +722,8 @@ static size_t fixed_bytes(unsigned dim, unsigned Ke) {
 }
 
 // A stack in fixed point at dst, on the context's stream (the caller waits for it).
+// More than 65535 matrices do not fit the launch grid and fail here: the other kernels
+// then serve, and drain's shift (6 and the bits of twice as many) stays below 24.
 template <class C>
 static bool convert_stack(Ctx *c, const void *stack, void *dst) {
     const int d = (int)c->dim, dp = (d + 63) / 64 * 64, n = 1 + (int)c->Ke;

@@ -21,7 +21,7 @@
 //
 // What bounds it: latency.  A qubit's 100 steps took 71 us with host buffers, ten
 // launches (256 threads per chunk, a launch per level of the tree) between two
-// copies; they take 46 us with one.  Above d = 8 the pair of a level takes one
+// copies; they take 40 us with one.  Above d = 8 the pair of a level takes one
 // group longer than a launch over several SMs, and groups of 64 threads with 4 x
 // 4 tiles (d = 27: 217 us against 195) or 2 x 2 in complex128 (d = 16: 833 against
 // 775) were no faster than 256 threads per chunk.
