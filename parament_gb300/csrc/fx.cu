@@ -554,9 +554,13 @@ static void build_program(FxForm form, int M, double x, double hnorm, std::vecto
     const long double sc = 2.0L / hnorm;
     std::vector<double> J(2 * (M + 1));
     bessel_coeffs(M, x, J.data());
-    // J_0 - 1 from the even orders (power_coefficients says why).
-    long double j0m1 = 0.0L;
-    for (int k = M + 41; k >= 2; k -= 2) j0m1 -= 2.0L * jn(k, x);
+    // J_0 - 1 from the even orders (power_coefficients says why); where x is large (a
+    // manual order may be far below it) they do not end at M + 41, and J_0 is far from 1.
+    long double j0m1 = (long double)jn(0, x) - 1.0L;
+    if (x <= 8.0) {
+        j0m1 = 0.0L;
+        for (int k = M + 41; k >= 2; k -= 2) j0m1 -= 2.0L * jn(k, x);
+    }
     auto j = [&](int k, long double f) { return coef(f * J[2 * k], f * J[2 * k + 1]); };
     int prev = -1, cur = -1, n = 0;  // buffers of b_(k+2) and b_(k+1); -1: from X
     const int rot[3] = {kBufY, kBufW, kBufR0};
