@@ -16,10 +16,11 @@
 //     Above x = 1 the Clenshaw recurrence runs as before.  Every coefficient
 //     (-i)^n times a real number is real or imaginary, so an epilogue needs one
 //     64-bit multiply per value and term.
-//   * E_j = U_j - I is what is formed and kept, and the running product of a
-//     chunk of steps is P <- E P + E + P with U_(s1-1) ... U_s0 = I + P: the
-//     unit diagonal never meets the small terms.  The chunk products meet in
-//     the pairwise tree in the same form.
+//   * E_j = U_j - I is what is formed, and the running product of a chunk of steps is
+//     U <- U + E_j U: the unit diagonal never meets the small terms, and a product
+//     that decays keeps its digits (held as U - I, a lossy propagator of size 1e-10
+//     came out good to 1e-5 of itself).  The pairwise tree holds both U and E = U - I
+//     of its nodes and multiplies by the smaller of a left operand: b + E b or U b.
 //   * The plain complex64 form keeps the FP32 coefficients of the other complex64
 //     kernels and rounds 1 + the diagonal of E_j to FP32, so U_j is the one those
 //     form (rounded otherwise, results drift apart by 1e-8 a step).
@@ -62,6 +63,22 @@ __global__ void k_fx_stack_max(const C *src, i64 dd, int *emax) {
 
 // Exponent e with |v| < 2^e for a largest biased exponent.
 __device__ __forceinline__ int exp_of(int biased) { return max(biased, 1) - 1022; }
+
+// Row norm of each stack matrix in units of its 2^e (rnorm zeroed before): a warp a row.
+template <class C>
+__global__ void k_fx_stack_norms(const C *src, int d, const int *emax, float *rnorm) {
+    const C *m = src + (size_t)blockIdx.y * d * d;
+    const int s = -exp_of(emax[blockIdx.y]), lane = threadIdx.x & 31;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < d; i += (gridDim.x * blockDim.x) >> 5) {
+        double t = 0.0;
+        for (int j = lane; j < d; j += 32) {
+            const C v = m[(size_t)i * d + j];
+            t += hypot(scalbn((double)v.x, s), scalbn((double)v.y, s));
+        }
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) atomicMax(reinterpret_cast<int *>(&rnorm[blockIdx.y]), __float_as_int((float)t * 1.0001f));
+    }
+}
 
 // The stack as fixed-point items, every matrix at its own exponent.
 template <class C>
@@ -109,11 +126,11 @@ struct Rows {
 // A: the arithmetic of the weights (complex64 samples in FP64 for the split form).
 template <class A, class C>
 __global__ void __launch_bounds__(128) k_fx_weights(const C *carr, WeightSpec w, int Ke, const int *emax,
-                                                    Rows rows, i64 nrows, int kpad, int lgk, i64 *W, i64 plane,
+                                                    const float *rnorm, Rows rows, i64 nrows, int kpad, int lgk, i64 *W, i64 plane,
                                                     Info *info, Info *zero0, Info *zero1, i64 n0, i64 n1) {
     // The infos of the round's results start at zero.
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n0 + n1; i += (i64)gridDim.x * blockDim.x)
-        (i < n0 ? zero0[i] : zero1[i - n0]) = Info{0, 0};
+        (i < n0 ? zero0[i] : zero1[i - n0]) = Info{0, 0, 0.0f};
     const i64 j = (i64)blockIdx.x * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (j >= nrows) return;
@@ -121,7 +138,7 @@ __global__ void __launch_bounds__(128) k_fx_weights(const C *carr, WeightSpec w,
     i64 *re = W + j * kpad, *im = re + plane;
     if (st < 0) {
         for (int m = lane; m < kpad; m += 32) re[m] = im[m] = 0;
-        if (lane == 0) info[j] = Info{0, 0};
+        if (lane == 0) info[j] = Info{0, 0, 0.0f};
         return;
     }
     auto weight = [&](int m) {
@@ -137,13 +154,17 @@ __global__ void __launch_bounds__(128) k_fx_weights(const C *carr, WeightSpec w,
     }
     be = __reduce_max_sync(0xffffffffu, be);
     const int e = exp_of(be);
+    float r = 0.0f;  // the row norm of X_j, in units of 2^e
     for (int m = lane; m < kpad; m += 32) {
         double2 v = make_double2(0.0, 0.0);
         if (m <= Ke && be < 0x7FF) v = weight(m);
-        re[m] = __double2ll_rn(scalbn(v.x, 62 - e));
-        im[m] = __double2ll_rn(scalbn(v.y, 62 - e));
+        const double2 u = make_double2(scalbn(v.x, -e), scalbn(v.y, -e));
+        if (m <= Ke) r += ((float)fabs(u.x) + (float)fabs(u.y)) * rnorm[m];
+        re[m] = __double2ll_rn(scalbn(u.x, 62));
+        im[m] = __double2ll_rn(scalbn(u.y, 62));
     }
-    if (lane == 0) info[j] = Info{e + lgk, be < 0x7FF ? 0 : kPoison};
+    for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    if (lane == 0) info[j] = Info{e + lgk, be < 0x7FF ? 0 : kPoison, 1.0001f * r * pow2f(-lgk)};
 }
 
 struct AssembleArgs {
@@ -170,6 +191,7 @@ struct AssembleWork {
     __device__ __forceinline__ At next(At u) const { return u + gridDim.x; }
     __device__ __forceinline__ bool more(At u) const { return u < units; }
     __device__ __forceinline__ bool needs(At, At) const { return false; }
+    __device__ __forceinline__ int head(At) const { return a.lgk; }
     __device__ __forceinline__ bool operands(At u, Operand &A, Operand &B) const {
         A = Operand{a.W + (u % rt) * 64 * a.kpad, a.kpad, 4, a.wplane, 0};
         B = Operand{a.stack + (u / rt) * 64, a.item, 4, plane, 0};
@@ -205,7 +227,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_fx_assemble(const __grid_consta
     const i64 plane = a.item / 2, rt = (a.nrows + 63) / 64, units = rt * (plane / 64);
     const int nst = a.kpad / kStageK;
     const AssembleWork w{a, s, t, rt, units, plane};
-    run<S>(s, t, w, my_units(units), nst, a.kvalid, 6 + a.lgk);
+    run<S>(s, t, w, my_units(units), nst, a.kvalid);
     teardown(s, t, t.ok, a.fault);
 }
 
@@ -226,7 +248,8 @@ struct StepsArgs {
     Info *pinfo, *cinfo;
     Chunks ch;
     i64 i0;
-    int per, d, nst, lgk;
+    int per, d, nst;
+    float cap;  // sqrt(2) d
     int *fault;
 };
 
@@ -269,13 +292,13 @@ struct StepsWork {
         const i64 c = chunk(q.k), i = a.i0 + q.i;
         i64 *dst = i == a.ch.steps(c) - 1 ? a.chunks + c * kItem64 : a.pbuf + ((i & 1) * a.ch.nch + c) * kItem64;
         if (b == kBufX) return out ? dst : const_cast<i64 *>(a.X) + (c * a.per + q.i) * kItem64;
-        if (b == kBufP) return a.pbuf + (((i - 1) & 1) * a.ch.nch + c) * kItem64;
-        if (b == kBufE && i == 0) return dst;
+        if (b == kBufP) return out ? dst : a.pbuf + (((i - 1) & 1) * a.ch.nch + c) * kItem64;
         return a.scratch + (5 * c + b - kBufY) * kItem64;
     }
     __device__ __forceinline__ Info info_of(const At &q, int b) const {
         return b == kBufX ? a.xinfo[chunk(q.k) * a.per + q.i] : info[q.k][b];
     }
+    __device__ __forceinline__ int head(const At &q) const { return product_of(info_of(q, a.op[q.o].a), a.cap).head; }
     __device__ __forceinline__ bool operands(const At &q, Operand &A, Operand &B) const {
         const Op &op = a.op[q.o];
         A = Operand{item(q, op.a, false), 4, 256, 4096, headroom(info_of(q, op.a))};
@@ -285,36 +308,44 @@ struct StepsWork {
     __device__ __forceinline__ bool epilogue(const At &q, i64 (&T)[kCols], uint32_t n) const {
         const Op &op = a.op[q.o];
         const Info ia = info_of(q, op.a), ib = info_of(q, op.b);
-        const int eT = ia.e - headroom(ia) + ib.e - headroom(ib) + a.lgk, off = t.c0 * 64 + 4 * t.r;
+        const Product p = product_of(ia, a.cap);
+        Sum S{ia.e - headroom(ia) + ib.e - headroom(ib) + p.head, p.head - p.bits,
+              row_norm(ia, a.cap) * row_norm(ib, a.cap) * pow2f(-p.head)};
+        const int off = t.c0 * 64 + 4 * t.r;
         const bool bad = ia.mb == kPoison || ib.mb == kPoison;
         auto view = [&](int b) { return View{item(q, b, false) + off, info_of(q, b)}; };
-        int e0 = 0, e1 = 0;
-        bool p0 = bad, p1 = bad;
+        Info r0{}, r1{};
 #pragma unroll 1
         for (int o = 0; o < 2; ++o) {
             const Out &out = op.out[o];
-            if (out.buf < 0) continue;
+            if (absent(q, out)) continue;
             bool poison = bad;
-            const int e = out_exponent(out, eT, view, poison);
-            merge_or(s, t, n, o, put_out(out, t, T, eT, e, view, 4096, 256, t.r, t.c0, a.d,
+            Info r;
+            r.e = out_exponent(out, S, a.cap, view, poison, r.r);
+            r.mb = poison ? kPoison : 0;
+            merge_or(s, t, n, o, put_out(out, t, T, S, r.e, view, 4096, 256, t.r, t.c0, a.d,
                                          item(q, out.buf, true) + t.p * 4096 + off));
+            if (!out.plain) S = Sum{r.e, 0, r.r};
             if (o == 0)
-                e0 = e, p0 = poison;
+                r0 = r;
             else
-                e1 = e, p1 = poison;
+                r1 = r;
         }
         if (!(t.ok = fsync_and(t.ok))) return false;
 #pragma unroll
         for (int o = 0; o < 2; ++o) {
             const u64 m = read_or(s, t, n, o);
-            const int b = op.out[o].buf;
-            if (b < 0) continue;
-            const Info r{o == 0 ? e0 : e1, (o == 0 ? p0 : p1) ? kPoison : bits_of(m)};
-            // The running product, or the first step's own propagator.
-            if (b == kBufX || (b == kBufE && a.i0 + q.i == 0)) info[q.k][kBufP] = r;
-            if (b != kBufX) info[q.k][b] = r;
+            if (absent(q, op.out[o])) continue;
+            Info r = o == 0 ? r0 : r1;
+            r.mb = max(r.mb, bits_of(m));
+            // The running product stands in X's place as a result.
+            info[q.k][op.out[o].buf == kBufX ? kBufP : op.out[o].buf] = r;
         }
         return true;
+    }
+    // A step's last product gives the running product too, I + E, in the first step.
+    __device__ __forceinline__ bool absent(const At &q, const Out &o) const {
+        return o.buf < 0 || (o.buf == kBufP && a.i0 + q.i > 0);
     }
 };
 
@@ -331,7 +362,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_fx_steps(const __grid_constant_
         if (w.end(k) > 0) products += (i64)w.end(k) * (a.nops + 1) - (a.i0 == 0 ? 1 : 0);
     if (a.i0 > 0 && t.tid < w.nk) info[t.tid][kBufP] = a.pinfo[w.chunk(t.tid)];
     __syncthreads();
-    run<7>(s, t, w, products, a.nst, 64, 6 + a.lgk);
+    run<7>(s, t, w, products, a.nst, 64);
     if (t.tid == 0 && t.ok)
         for (int k = 0; k < w.nk; ++k) {
             const i64 c = w.chunk(k);
@@ -350,8 +381,11 @@ struct Buf {
 };
 struct GemmArgs {
     Op op;
+    Op alt;      // instead of op where its left operand is the smaller one
+    int tree;    // with alt, and the row norms of the results measured
     Buf buf[kBufs];
-    int items, nt, dp, d, nst, lgk;
+    int items, nt, dp, d, nst;
+    float cap;  // sqrt(2) d
     int *fault;
 };
 
@@ -370,50 +404,83 @@ struct GemmWork {
         const Buf &q = a.buf[b];
         return View{q.ptr + it * q.stride + off, q.info[it * q.istride]};
     }
+    __device__ __forceinline__ const Op &op_of(i64 it) const {
+        if (!a.tree) return a.op;
+        const Info x = view(a.op.a, it, 0).info, y = view(a.alt.a, it, 0).info;
+        return y.e - headroom(y) < x.e - headroom(x) ? a.alt : a.op;
+    }
+    __device__ __forceinline__ int head(At u) const {
+        const i64 it = u / tiles;
+        return product_of(view(op_of(it).a, it, 0).info, a.cap).head;
+    }
     __device__ __forceinline__ bool operands(At u, Operand &A, Operand &B) const {
         const i64 it = u / tiles;
         const int tile = (int)(u % tiles), I = tile / a.nt, J = tile % a.nt;
-        const View va = view(a.op.a, it, I * 256), vb = view(a.op.b, it, (i64)J * 64 * a.dp);
+        const Op &op = op_of(it);
+        const View va = view(op.a, it, I * 256), vb = view(op.b, it, (i64)J * 64 * a.dp);
         A = Operand{va.re, 4, qs, plane, headroom(va.info)};
         B = Operand{vb.re, 4, qs, plane, headroom(vb.info)};
-        return a.op.imag != 0;
+        return op.imag != 0;
     }
     __device__ __forceinline__ bool epilogue(At u, i64 (&T)[kCols], uint32_t n) const {
         const i64 it = u / tiles;
         const int tile = (int)(u % tiles), I = tile / a.nt, J = tile % a.nt;
-        const Op &op = a.op;
+        const Op &op = op_of(it);
         const Info ia = view(op.a, it, 0).info, ib = view(op.b, it, 0).info;
-        const int eT = ia.e - headroom(ia) + ib.e - headroom(ib) + a.lgk;
+        const Product p = product_of(ia, a.cap);
+        Sum S{ia.e - headroom(ia) + ib.e - headroom(ib) + p.head, p.head - p.bits,
+              row_norm(ia, a.cap) * row_norm(ib, a.cap) * pow2f(-p.head)};
         const bool bad = ia.mb == kPoison || ib.mb == kPoison;
         const int row = I * 64 + t.r, col0 = J * 64 + t.c0;
         const i64 off = (i64)col0 * a.dp + 4 * row;
         auto at = [&](int b) { return view(b, it, off); };
-        int e0 = 0, e1 = 0;
-        bool p0 = bad, p1 = bad;
+        Info r0{}, r1{};
 #pragma unroll 1
         for (int o = 0; o < 2; ++o) {
             const Out &out = op.out[o];
             if (out.buf < 0) continue;
             bool poison = bad;
-            const int e = out_exponent(out, eT, at, poison);
+            Info r;
+            r.e = out_exponent(out, S, a.cap, at, poison, r.r);
+            r.mb = poison ? kPoison : 0;
             const Buf &q = a.buf[out.buf];
-            merge_or(s, t, n, o, put_out(out, t, T, eT, e, at, plane, qs, row, col0, a.d,
-                                         q.ptr + it * q.stride + t.p * plane + off));
+            merge_or(s, t, n, o, put_out(out, t, T, S, r.e, at, plane, qs, row, col0, a.d,
+                                         q.ptr + it * q.stride + t.p * plane + off,
+                                         a.tree ? &s.rows[n & 1][o][t.r] : nullptr));
+            if (!out.plain) S = Sum{r.e, 0, r.r};
             if (o == 0)
-                e0 = e, p0 = poison;
+                r0 = r;
             else
-                e1 = e, p1 = poison;
+                r1 = r;
         }
         if (!(t.ok = fsync_and(t.ok))) return false;
+        if (a.tree && t.tid < 64) {
+            // The norm: as many tiles as a row has, times the largest sum over one (bounds
+            // from the operands' norms grow from level to level; what the sums then
+            // leave unused cost 6e-15 at d = 32, x = 0.5).
+            for (int o = 0; o < 2; ++o) {
+                if (op.out[o].buf < 0) continue;
+                const uint32_t r = __reduce_max_sync(0xffffffffu, s.rows[n & 1][o][t.tid]);
+                s.rows[n & 1][o][t.tid] = 0;
+                const Buf &q = a.buf[op.out[o].buf];
+                if (t.lane == 0)
+                    atomicMax(reinterpret_cast<int *>(&q.info[it * q.istride].r),
+                              __float_as_int(1.001f * (float)a.nt * (float)r * pow2f(-24)));
+            }
+        }
         if (t.tid == 0) {
 #pragma unroll
             for (int o = 0; o < 2; ++o) {
                 const u64 m = read_or(s, t, n, o);
                 if (op.out[o].buf < 0) continue;
                 const Buf &q = a.buf[op.out[o].buf];
+                const Info r = o == 0 ? r0 : r1;
                 Info *i = &q.info[it * q.istride];
-                if (tile == 0) i->e = o == 0 ? e0 : e1;
-                atomicMax(&i->mb, (o == 0 ? p0 : p1) ? kPoison : bits_of(m));
+                if (tile == 0) {
+                    i->e = r.e;
+                    if (!a.tree) i->r = r.r;
+                }
+                atomicMax(&i->mb, max(r.mb, bits_of(m)));
             }
         }
         return true;
@@ -429,21 +496,81 @@ __global__ void __launch_bounds__(kThreads, 1) k_fx_gemm(const __grid_constant__
     const int tiles = a.nt * a.nt;
     const i64 units = (i64)a.items * tiles;
     const GemmWork w{a, s, t, tiles, units, (i64)a.dp * a.dp, 4ll * a.dp};
-    run<S>(s, t, w, my_units(units), a.nst, a.dp, 6 + a.lgk);
+    run<S>(s, t, w, my_units(units), a.nst, a.dp);
     teardown(s, t, t.ok, a.fault);
 }
 
-// I + E in the context's precision, row-major d x d.
+// E = U - I beside the chunk products U, and the row norms of both, for the tree (the
+// infos zeroed before).  A warp takes 32 rows of an item, eight warps its columns.
+__global__ void __launch_bounds__(256) k_fx_less_one(const i64 *U, const Info *in, i64 *E, Info *einfo, Info *uinfo,
+                                                     int d, int dp) {
+    __shared__ float sums[2][8][32];
+    const Info u = in[blockIdx.y];
+    const int h = headroom(u), lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = blockIdx.x * 32 + lane;
+    const int e = max(u.e - h, 0) + 1, left = u.e - e;  // |E| <= 1 + 2^(u.e - h)
+    const i64 plane = (i64)dp * dp, one = e <= 62 ? 1ll << (62 - e) : 0;
+    const i64 *src = U + 2 * plane * blockIdx.y;
+    i64 *dst = E + 2 * plane * blockIdx.y;
+    auto scale = [&](i64 v) {
+        if (left >= 0) return (i64)((u64)v << min(left, 63));
+        return left < -62 ? 0ll : (v + (1ll << (-left - 1))) >> -left;
+    };
+    u64 bits = 0;
+    float su = 0.0f, se = 0.0f;
+    for (int q = warp; q < dp / 4; q += 8) {
+        const i64 at = (i64)q * 4 * dp + 4 * row;
+        i64 x[4], y[4];
+        load4(src + at, x[0], x[1], x[2], x[3]);
+        load4(src + plane + at, y[0], y[1], y[2], y[3]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            su += hypotf((float)x[j], (float)y[j]);
+            x[j] = scale(x[j]) - (4 * q + j == row && row < d ? one : 0);
+            y[j] = scale(y[j]);
+            se += hypotf((float)x[j], (float)y[j]);
+            bits |= (u64)(x[j] ^ (x[j] >> 63)) | (u64)(y[j] ^ (y[j] >> 63));
+        }
+        store4(dst + at, x[0], x[1], x[2], x[3]);
+        store4(dst + plane + at, y[0], y[1], y[2], y[3]);
+    }
+    sums[0][warp][lane] = su;
+    sums[1][warp][lane] = se;
+    const int mb = __reduce_max_sync(0xffffffffu, bits_of(bits));
+    if (lane == 0) atomicMax(&einfo[blockIdx.y].mb, u.mb == kPoison ? kPoison : mb);
+    __syncthreads();
+    if (warp < 2) {
+        float s = 0.0f;
+        for (int k = 0; k < 8; ++k) s += sums[warp][k][lane];
+        Info *o = &(warp == 0 ? uinfo : einfo)[blockIdx.y];
+        atomicMax(reinterpret_cast<int *>(&o->r), __float_as_int(1.001f * s * pow2f(-62)));
+        if (lane == 0 && blockIdx.x == 0) o->e = warp == 0 ? u.e : e;
+        if (lane == 0 && warp == 0 && blockIdx.x == 0) o->mb = u.mb;
+    }
+}
+
+// An odd leftover of a level: an item and its info, E and U.
+__global__ void __launch_bounds__(256) k_fx_carry(const i64 *e0, const i64 *u0, i64 *e1, i64 *u1, const Info *ei0,
+                                                  const Info *ui0, Info *ei1, Info *ui1, i64 n) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *ei1 = *ei0, *ui1 = *ui0;
+    for (i64 i = 4 * ((i64)blockIdx.x * blockDim.x + threadIdx.x); i < n; i += 4ll * gridDim.x * blockDim.x) {
+        i64 a, b, c, d;
+        load4(e0 + i, a, b, c, d);
+        store4(e1 + i, a, b, c, d);
+        load4(u0 + i, a, b, c, d);
+        store4(u1 + i, a, b, c, d);
+    }
+}
+
+// The result in the context's precision, row-major d x d.
 template <class C>
-__global__ void k_fx_out(const i64 *E, const Info *info, int d, int dp, C *out) {
+__global__ void k_fx_out(const i64 *U, const Info *info, int d, int dp, C *out) {
     const Info q = *info;
     const i64 plane = (i64)dp * dp, n = (i64)d * d;
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
         const int r = (int)(i / d), c = (int)(i % d);
         const i64 k = (i64)(c >> 2) * 4 * dp + 4 * r + (c & 3);
-        double2 v = make_double2(scalbn((double)E[k], q.e - 62), scalbn((double)E[plane + k], q.e - 62));
+        double2 v = make_double2(scalbn((double)U[k], q.e - 62), scalbn((double)U[plane + k], q.e - 62));
         if (q.mb == kPoison) v.x = v.y = __longlong_as_double(0x7FF8000000000000ll);
-        if (r == c) v.x += 1.0;
         out[i] = mk<C>(v.x, v.y);
     }
 }
@@ -658,15 +785,16 @@ static Plan make_plan(int d, int Ke, i64 P, int num_sms) {
     q.off_s = take(m * 5 * (size_t)q.nch);
     q.off_p = take(m * 2 * (size_t)q.nch);
     q.off_c = take(m * (size_t)q.nch);
-    // X rows; the results of a step's products; P0 P1; finished chunks; the tree's.
-    q.n_info = (size_t)q.rows + (kMaxOps + 5) * (size_t)q.nch;
+    // X rows; the results of a step's products (then the tree's); P0 P1; finished chunks.
+    q.n_info = (size_t)q.rows + (kMaxOps + 4) * (size_t)q.nch;
     q.off_info = take(sizeof(Info) * q.n_info);
     q.bytes = o;
     return q;
 }
 
-// Bytes before the matrices of the fixed-point stack: the largest exponents.
-static size_t stack_head(int n) { return (sizeof(int) * (size_t)n + 255) / 256 * 256; }
+// Bytes before the matrices of the fixed-point stack: the largest exponents and the row
+// norms.
+static size_t stack_head(int n) { return ((sizeof(int) + sizeof(float)) * (size_t)n + 255) / 256 * 256; }
 
 template <int S>
 static cudaError_t launch_gemm_op(const GemmArgs &a, int num_sms, cudaStream_t st, int *launches) {
@@ -733,8 +861,10 @@ static bool convert_stack(Ctx *c, const void *stack, void *dst) {
     const int d = (int)c->dim, dp = (d + 63) / 64 * 64, n = 1 + (int)c->Ke;
     int *emax = static_cast<int *>(dst);
     const C *src = static_cast<const C *>(stack);
-    if (cudaMemsetAsync(emax, 0, sizeof(int) * n, c->stream) != cudaSuccess) return false;
+    float *rnorm = reinterpret_cast<float *>(emax + n);
+    if (cudaMemsetAsync(emax, 0, (sizeof(int) + sizeof(float)) * n, c->stream) != cudaSuccess) return false;
     k_fx_stack_max<C><<<dim3(std::max(1, std::min(256, d * d / 1024)), n), 256, 0, c->stream>>>(src, (i64)d * d, emax);
+    k_fx_stack_norms<C><<<dim3(std::min(256, (d + 7) / 8), n), 256, 0, c->stream>>>(src, d, emax, rnorm);
     k_fx_stack<C><<<dim3(std::max(1, std::min(1024, dp * dp / 512)), n), 256, 0, c->stream>>>(
         src, d, dp, emax, reinterpret_cast<i64 *>(static_cast<char *>(dst) + stack_head(n)));
     return cudaGetLastError() == cudaSuccess;
@@ -785,25 +915,27 @@ static cudaError_t run_fx_t(Ctx *c, FxForm form, const void *d_carr, const Weigh
     if (e != cudaSuccess) return e;
     const size_t head = stack_head(n);
     const int *emax = static_cast<const int *>(sb);
+    const float *rnorm = reinterpret_cast<const float *>(emax + n);
     const i64 *stack = reinterpret_cast<const i64 *>(static_cast<const char *>(sb) + head);
     char *ws = static_cast<char *>(c->fx_ws.ptr);
     i64 *W = reinterpret_cast<i64 *>(ws + q.off_w), *X = reinterpret_cast<i64 *>(ws + q.off_x);
     i64 *scr = reinterpret_cast<i64 *>(ws + q.off_s), *Pb = reinterpret_cast<i64 *>(ws + q.off_p);
     i64 *chunks = reinterpret_cast<i64 *>(ws + q.off_c);
     Info *xinfo = reinterpret_cast<Info *>(ws + q.off_info), *sinfo = xinfo + q.rows;
-    Info *pinfo = sinfo + (kMaxOps + 1) * (size_t)q.nch, *cinfo = pinfo + 2 * (size_t)q.nch, *tinfo = cinfo + q.nch;
+    Info *pinfo = sinfo + (kMaxOps + 1) * (size_t)q.nch, *cinfo = pinfo + 2 * (size_t)q.nch;
     std::vector<Op> ops;
     build_program(form, M, x, c->held_norm(), ops);
     if ((int)ops.size() >= kMaxOps) return cudaErrorInvalidValue;  // orders up to 63: 62 products
     const WeightSpec w{wh.pts, wh.K, wh.amps, wh.mode, wh.magnus, wh.hfac};
     const i64 rpad = (q.rows + 63) / 64 * 64;
-    const int lgw = std::max(5, ceil_log2(2ll * q.kvalid)), lgk = ceil_log2(2ll * d);
+    const int lgw = std::max(5, ceil_log2(2ll * q.kvalid));
+    const float cap = 1.41422f * (float)d;
     const int nst = (d + kStageK - 1) / kStageK;
     auto assemble = [&](i64 i0, i64 rows, int per, Info *zero0 = nullptr, i64 n0 = 0, Info *zero1 = nullptr,
                         i64 n1 = 0) -> cudaError_t {
         const Rows r{q.ch, per, i0};
-        k_fx_weights<A><<<(unsigned)((rows + 3) / 4), 128, 0, st>>>(static_cast<const C *>(d_carr), w, Ke, emax, r,
-                                                                  rows, q.kpad, lgw, W, rpad * q.kpad, xinfo, zero0,
+        k_fx_weights<A><<<(unsigned)((rows + 3) / 4), 128, 0, st>>>(static_cast<const C *>(d_carr), w, Ke, emax,
+                                                                  rnorm, r, rows, q.kpad, lgw, W, rpad * q.kpad, xinfo, zero0,
                                                                   zero1, n0, n1);
         const AssembleArgs a{W, stack, rpad * q.kpad, X, xinfo, rows, q.item, q.kpad, q.kvalid, lgw, c->d_fault};
         const i64 units = ((rows + 63) / 64) * (q.item / 128);
@@ -812,14 +944,19 @@ static cudaError_t run_fx_t(Ctx *c, FxForm form, const void *d_carr, const Weigh
         return cudaGetLastError();
     };
     if (c->timing) cudaEventRecord(c->ev_start, st);
-    // The running product of a chunk, into kBufX of its caller: E P + E + P.
+    // The running product of a chunk, U <- U + E U, into kBufX of its caller; in the
+    // first step I + E, a second result of the step's last product.
+    const Coef one = coef(1.0, 0.0), minus = coef(-1.0, 0.0);
     Op run{kBufE, kBufP, 0, {Out{}, no_out()}};
-    const Coef one = coef(1.0, 0.0);
     run.out[0].buf = kBufX;
     run.out[0].t = one;
-    run.out[0].nterm = 2;
-    run.out[0].term[0] = Term{one, kBufE};
-    run.out[0].term[1] = Term{one, kBufP};
+    run.out[0].nterm = 1;
+    run.out[0].term[0] = Term{one, kBufP};
+    Out first{};
+    first.buf = kBufP;
+    first.t = one;
+    first.diag = one;
+    ops.back().out[1] = first;
     if (q.nt == 1) {
         StepsArgs a;
         for (size_t k = 0; k < ops.size(); ++k) a.op[k] = ops[k];
@@ -836,7 +973,7 @@ static cudaError_t run_fx_t(Ctx *c, FxForm form, const void *d_carr, const Weigh
         a.per = q.per;
         a.d = d;
         a.nst = nst;
-        a.lgk = lgk;
+        a.cap = cap;
         a.fault = c->d_fault;
         for (i64 i0 = 0; i0 < q.ch.longest(); i0 += q.per) {
             if ((e = assemble(i0, q.rows, q.per)) != cudaSuccess) return e;
@@ -852,7 +989,7 @@ static cudaError_t run_fx_t(Ctx *c, FxForm form, const void *d_carr, const Weigh
         a.dp = q.dp;
         a.d = d;
         a.nst = nst;
-        a.lgk = lgk;
+        a.cap = cap;
         a.fault = c->d_fault;
         for (i64 i = 0; i < longest; ++i) {
             const int active = i < q.ch.len ? q.nch : q.ch.nlong;
@@ -866,12 +1003,13 @@ static cudaError_t run_fx_t(Ctx *c, FxForm form, const void *d_carr, const Weigh
             const size_t results = ops.size() + 1;
             if ((e = assemble(i, active, 1, sinfo, (i64)results * q.nch, dst.info, q.nch)) != cudaSuccess) return e;
             size_t slot = 0;
-            if (i == 0) a.buf[kBufE] = dst;
+            if (i == 0) a.buf[kBufP] = dst;
             a.items = active;
             for (const Op &o : ops) {
                 a.op = o;
-                for (const Out &out : o.out)
-                    if (out.buf >= 0 && !(out.buf == kBufE && i == 0)) a.buf[out.buf].info = sinfo + slot++ * q.nch;
+                if (i > 0 && o.out[1].buf == kBufP) a.op.out[1] = no_out();
+                for (const Out &out : a.op.out)
+                    if (out.buf >= 0 && out.buf != kBufP) a.buf[out.buf].info = sinfo + slot++ * q.nch;
                 if ((e = launch_gemm_op<S>(a, c->num_sms, st, &launches)) != cudaSuccess) return e;
             }
             if (i > 0) {
@@ -895,49 +1033,82 @@ static cudaError_t run_fx_t(Ctx *c, FxForm form, const void *d_carr, const Weigh
         cinfo = pinfo + ((longest - 1) & 1) * q.nch;
     }
     if (c->timing) cudaEventRecord(c->ev_stop, st);
-    // Pairwise tree over the chunk products, later chunks on the left:
-    // E = Ea Eb + Ea + Eb; an odd leftover moves up unchanged.
-    {
+    // Pairwise tree over the chunk products, later chunks on the left: U_a U_b as U_b + E_a
+    // U_b with E = U - I, or as U_a U_b where U_a is the smaller one (a dense unitary, or a
+    // propagator that decays), both U and E for the next level.  The digits of an
+    // operand are cut at a fixed distance below its largest entry: in U alone, 64 steps of
+    // x = 0.05 at d = 64 were off by 1.5e-15 (FP64 2.7e-16), in E alone a propagator of
+    // size 1e-10 by 1e-7 of itself.
+    const i64 *res = chunks;
+    const Info *rinfo = cinfo;
+    if (q.nch > 1) {
         GemmArgs a{};
         a.nt = q.nt;
         a.dp = q.dp;
         a.d = d;
         a.nst = nst;
-        a.lgk = lgk;
+        a.cap = cap;
         a.fault = c->d_fault;
-        a.op = Op{kBufX, kBufY, 0, {Out{}, no_out()}};
-        Out &o = a.op.out[0];
-        o.buf = kBufW;
-        o.t = one;
-        o.nterm = 2;
-        o.term[0] = Term{one, kBufX};
-        o.term[1] = Term{one, kBufY};
-        i64 *cur = chunks, *nxt = scr;
-        Info *ci = cinfo, *ni = tinfo;
-        for (i64 n2 = q.nch; n2 > 1;) {
+        // Left: X as E, W as U; right: Y as U, R0 as E.  Results: U to R1, E to E.
+        auto result = [&](int buf, const Coef &dg, int term) {
+            Out o{};
+            o.buf = buf;
+            o.t = one;
+            o.diag = dg;
+            if (term >= 0) o.term[o.nterm++] = Term{one, term};
+            return o;
+        };
+        const Coef none{0, 0, 0};
+        const size_t set = (size_t)q.item * q.nch;
+        i64 *E[2] = {scr, scr + set}, *U[2] = {chunks, scr + 2 * set};
+        // Infos of E and U of each level, behind each other, zeroed at once.
+        size_t all = 0;
+        for (i64 n2 = q.nch; n2 > 1; n2 = (n2 + 1) / 2) all += (size_t)n2;
+        Info *ei = sinfo, *ui = ei + q.nch;
+        if ((e = cudaMemsetAsync(sinfo, 0, sizeof(Info) * 2 * (all + 1), st)) != cudaSuccess) return e;
+        k_fx_less_one<<<dim3(q.dp / 32, q.nch), 256, 0, st>>>(chunks, cinfo, E[0], ei, ui, d, q.dp);
+        ++launches;
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        int k = 0;
+        for (i64 n2 = q.nch; n2 > 1; k ^= 1) {
             const i64 pairs = n2 / 2;
-            if ((e = cudaMemsetAsync(ni, 0, sizeof(Info) * pairs, st)) != cudaSuccess) return e;
-            a.buf[kBufX] = Buf{cur + q.item, 2 * q.item, ci + 1, 2};
-            a.buf[kBufY] = Buf{cur, 2 * q.item, ci, 2};
-            a.buf[kBufW] = Buf{nxt, q.item, ni, 1};
+            const bool last = n2 == 2;
+            Info *en = ui + n2, *un = en + (n2 + 1) / 2;
+            a.buf[kBufX] = Buf{E[k] + q.item, 2 * q.item, ei + 1, 2};
+            a.buf[kBufR0] = Buf{E[k], 2 * q.item, ei, 2};
+            a.buf[kBufW] = Buf{U[k] + q.item, 2 * q.item, ui + 1, 2};
+            a.buf[kBufY] = Buf{U[k], 2 * q.item, ui, 2};
+            a.buf[kBufR1] = Buf{U[k ^ 1], q.item, un, 1};
+            a.buf[kBufE] = Buf{E[k ^ 1], q.item, en, 1};
             a.items = (int)pairs;
+            a.tree = 1;
+            if (last) {
+                a.op = Op{kBufX, kBufY, 0, {result(kBufR1, none, kBufY), no_out()}};
+                a.alt = Op{kBufW, kBufY, 0, {result(kBufR1, none, -1), no_out()}};
+            } else {
+                a.op = Op{kBufX, kBufY, 0, {result(kBufE, none, kBufR0), result(kBufR1, one, -1)}};
+                a.alt = Op{kBufW, kBufY, 0, {result(kBufR1, none, -1), result(kBufE, minus, -1)}};
+            }
             if ((e = launch_gemm_op<S>(a, c->num_sms, st, &launches)) != cudaSuccess) return e;
             if (n2 & 1) {
-                e = cudaMemcpyAsync(nxt + pairs * q.item, cur + 2 * pairs * q.item, sizeof(i64) * q.item,
-                                    cudaMemcpyDeviceToDevice, st);
-                if (e == cudaSuccess)
-                    e = cudaMemcpyAsync(ni + pairs, ci + 2 * pairs, sizeof(Info), cudaMemcpyDeviceToDevice, st);
-                if (e != cudaSuccess) return e;
+                const i64 o = n2 - 1;
+                k_fx_carry<<<(int)std::min<i64>(512, (q.item + 1023) / 1024), 256, 0, st>>>(
+                    E[k] + o * q.item, U[k] + o * q.item, E[k ^ 1] + pairs * q.item, U[k ^ 1] + pairs * q.item,
+                    ei + o, ui + o, en + pairs, un + pairs, q.item);
+                ++launches;
+                if ((e = cudaGetLastError()) != cudaSuccess) return e;
             }
             n2 = pairs + (n2 & 1);
-            std::swap(cur, nxt);
-            std::swap(ci, ni);
+            ei = en;
+            ui = un;
         }
-        const i64 total = (i64)d * d;
-        k_fx_out<<<(int)std::min<i64>((total + 255) / 256, 1024), 256, 0, st>>>(cur, ci, d, q.dp,
-                                                                               static_cast<C *>(d_out));
-        ++launches;
+        res = U[k];
+        rinfo = ui;
     }
+    const i64 total = (i64)d * d;
+    k_fx_out<<<(int)std::min<i64>((total + 255) / 256, 1024), 256, 0, st>>>(res, rinfo, d, q.dp,
+                                                                           static_cast<C *>(d_out));
+    ++launches;
     c->launches = launches;
     return cudaGetLastError();
 }

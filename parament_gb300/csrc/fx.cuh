@@ -4,14 +4,14 @@
 // Why: the FP64 pipe of this GPU does two fused multiply-adds per SM and clock
 // (1.2 TFLOP/s in all), so a complex128 product of 64 x 64 matrices costs an SM
 // half a million clocks there.  As integers cut into 8-bit digits the same
-// product is 34 small bf16-rate products, about ten thousand clocks, and its
-// error is smaller than that of 53-bit floating-point sums.
+// product is 34 small bf16-rate products, about ten thousand clocks.
 //
 // A matrix is an item of two planes (re, im) of dp x dp 64-bit integers (dp: d
 // rounded up to 64, padding zero) with an exponent e of its own:
 //     value = v 2^(e - 62),  |v| <= 2^62,
 // and the measured length mb of its largest |v| in bits.  An operand is
-// shifted left by 62 - mb first, so a loose exponent costs no digits.  Adding
+// shifted left by 62 - mb first, so a loose exponent costs no digits; what the sums'
+// headroom costs is kept small by measured row norms (product_of).  Adding
 // 0x8080808080808080 turns the top seven bytes into the digits of
 //     v = sum_s q_s 2^(8 (7 - s)),  q_s in [-128, 127], |q_0| <= 64,
 // (rounded at the eighth byte): byte s minus 128, which fp16 holds exactly.
@@ -26,9 +26,11 @@
 // After every 64 columns the levels are read, shifted together as integers and
 // added to the thread's 64-bit sums.  The dropped levels (6 digit pairs of
 // level 8 and on) are below 2^-58 sqrt(d) of the product of the operands'
-// maxima; with the levels up to 6 only (28 products) the error measured five
-// times that of FP64 sums, with those up to 7 a third of it.  All of this is of the
-// maxima: an entry far below its matrix's largest loses relative accuracy that FP64
+// maxima; with the levels up to 6 only (28 products) the error measured 15 times
+// as large.  Against 113-bit propagators whole calls are 0.2 to 1.5 times as far off
+// as the FP64 kernels, 2.1 times in the worst case met (d = 64, 24 steps, x = 0.5,
+// dense); a headroom of log2(2 d) bits for every sum instead took nearly diagonal
+// Hamiltonians and large steps to 3 to 13 times.  All of this is of the maxima: an entry far below its matrix's largest loses relative accuracy that FP64
 // would keep (blocks coupled by 1e-8, d = 32: their amplitudes to 3e-9; exact zeros
 // stay zero).
 //
@@ -49,8 +51,8 @@
 // stands still (its 512 columns hold one product's levels); cutting (4.5) and the
 // operands' loads (6) lie underneath.  At d <= 128 the loads' latency and the
 // epilogues (64-bit multiplies) weigh as much; with four or five digits they are
-// all of it.  Measured: d = 64 Magnus, 4096 steps, 2.04 ms; d = 96, 512 steps, 1.58
-// ms; d = 512, 16 steps, 2.96 ms on the device; complex64, d = 128, 4096 steps, 7.9
+// all of it.  Measured: d = 64 Magnus, 4096 steps, 2.07 ms; d = 96, 512 steps, 1.70
+// ms; d = 512, 16 steps, 2.96 ms on the device; complex64, d = 128, 4096 steps, 8.05
 // ms (FP32 kernel: 11.2).  With the finishers' sums spilled (136 registers) the
 // first three took 2.36, 1.71 and 3.07; with eight warps that did all but the
 // issuing 2.57, 1.80 and 3.13.  Accumulators for each half of the columns, one
@@ -95,17 +97,42 @@ constexpr int kPoison = 127;  // measured length of an item that holds infinitie
 typedef long long i64;
 typedef unsigned long long u64;
 
-// e: exponent, mb: bits of the largest magnitude (kPoison: not finite).
+// e: exponent, mb: bits of the largest magnitude (kPoison: not finite), r: a bound of
+// the row norms, max_i sum_k |a_ik|, in units of 2^e.
 struct Info {
     int e, mb;
+    float r;
 };
 __device__ __forceinline__ int headroom(Info i) { return i.mb >= 62 ? 0 : 62 - i.mb; }
+// 2^k, within FP32.
+__device__ __forceinline__ float pow2f(int k) { return __int_as_float((127 + min(max(k, -126), 127)) << 23); }
+// The row norm of a normalised operand, sqrt(2) d (`cap`) at most.
+__device__ __forceinline__ float row_norm(Info i, float cap) { return fminf(i.r * pow2f(headroom(i)), cap); }
+__device__ __forceinline__ int ceil_log2f(float q) {
+    const int b = __float_as_int(q);
+    return ((b >> 23) & 255) - 127 + ((b & 0x7FFFFF) != 0);
+}
+
+// A product of two normalised items: its values stay below 2^bits in units of the
+// operands' 2^(e - headroom), its sums are held with `head` bits above those units
+// (drain wants five at least).  The bound is the left operand's row norm: with 2 d terms
+// of the largest size instead, as for any two matrices, the sums of a nearly diagonal
+// propagator would leave up to ten bits unused, and its products were 13 times (d = 96)
+// as far off as those in FP64.
+struct Product {
+    int bits, head;
+};
+__device__ __forceinline__ Product product_of(Info a, float cap) {
+    const int b = ceil_log2f(1.4143f * row_norm(a, cap));
+    return Product{max(b, 0), max(b, 5)};
+}
 
 struct Shared {
     uint64_t full[kMaxStages], done[kMaxStages], ready[2], drained[2], finished[kFinishedBars], last;
     uint32_t tmem_base;
     uint32_t orhi[4][2], orlo[4][2];  // OR of the magnitudes of a product's results, four products in turn
     int rowmb[2][64];                 // lengths of a tile's rows, two tiles in turn
+    uint32_t rows[2][2][64];          // sums over a tile's rows of two results, two tiles in turn
 };
 
 // Where a thread sits; finishers: tensor-memory lane 32 (warp % 4) + lane, plane
@@ -386,7 +413,8 @@ __device__ __forceinline__ uint32_t split8(float f, float &r) {
 }
 
 // Adds sum_L D_L 2^(-8 L) in the units of the thread's sums, of which a product of
-// two items of scale 2^-62 has 2^(56 - sh) in level 0 (sh = 11 .. 24).
+// two items of scale 2^-62 has 2^(56 - sh) in level 0 (sh = 6 + the product's head, 11
+// .. 24).
 //
 // Levels 0 .. 2 stay within 2^22 and convert by an addition; 3 .. 5 split into a
 // multiple of 256 and a rest first (the conversion unit takes eight clocks a
@@ -489,11 +517,12 @@ __device__ __forceinline__ void cutter(Shared &s, Thread &t, const W &w, int nst
 // The finishers' loop: the levels of every group of stages into the sums, then
 // w.epilogue (false ends).
 template <int S, class W>
-__device__ __forceinline__ void finisher(Shared &s, Thread &t, const W &w, int nst, int sh) {
+__device__ __forceinline__ void finisher(Shared &s, Thread &t, const W &w, int nst) {
     using D = Digits<S>;
     uint32_t groups = 0, n = 0;
     for (typename W::At at = w.first(); w.more(at); at = w.next(at), ++n) {
         i64 T[kCols];
+        const int sh = 6 + w.head(at);
 #pragma unroll
         for (int j = 0; j < kCols; ++j) T[j] = 0;
         for (int st = 0; st < nst; st += kGroup, ++groups) {
@@ -525,7 +554,8 @@ struct Term {
 };
 constexpr int kTerms = 3;
 // One result of a product T: T itself (plain), or t T + sum terms + diag I
-// with t real (a thread holds one plane of T).
+// with t real (a thread holds one plane of T).  A second result is one of T where the
+// first is plain, else of the first result in T's place.
 struct Out {
     int buf;  // -1: none
     int plain, nterm;
@@ -546,20 +576,44 @@ struct View {
     Info info;
 };
 
-// Exponent of a result: two above the largest of up to four addends.
+// What is known of T: its units 2^eT, values below 2^(eT - h), row norms r in units of
+// 2^eT.
+struct Sum {
+    int e, h;
+    float r;
+};
+// Exponent and row norm (in its units) of a result: two above the largest of up to four
+// addends.
 template <class V>
-__device__ __forceinline__ int out_exponent(const Out &o, int eT, V view, bool &poison) {
-    if (o.plain) return eT;
+__device__ __forceinline__ int out_exponent(const Out &o, Sum T, float cap, V view, bool &poison, float &norm) {
+    if (o.plain) {
+        norm = fminf(T.r, cap);
+        return T.e;
+    }
+    auto size = [](const Coef &c) { return fabsf((float)(int)(c.m >> 32)) * 9.3132257e-10f; };  // 2^(32 - 62)
     int e = -1000000;
-    if (o.t.m) e = eT + o.t.e;
+    const int ref = T.e + o.t.e;  // r in units of 2^ref
+    float r = 0.0f;
+    if (o.t.m) {
+        e = ref - T.h;
+        r = size(o.t) * T.r;
+    }
 #pragma unroll 1
     for (int k = 0; k < o.nterm; ++k) {
         const Info i = view(o.term[k].buf).info;
+        const Coef c = o.term[k].c;
         if (i.mb == kPoison) poison = true;
-        e = max(e, i.e - headroom(i) + o.term[k].c.e);
+        const int ek = i.e - headroom(i) + c.e;
+        e = max(e, ek);
+        r += size(c) * row_norm(i, cap) * pow2f(ek - ref);
     }
-    if (o.diag.m) e = max(e, o.diag.e);
-    return e + 2;
+    if (o.diag.m) {
+        e = max(e, o.diag.e);
+        r += size(o.diag) * pow2f(o.diag.e - ref);
+    }
+    e += 2;
+    norm = fminf(1.001f * r * pow2f(ref - e), cap);
+    return e;
 }
 
 // A coefficient and the shift that its product needs, as one factor: the upper
@@ -603,16 +657,18 @@ __device__ __forceinline__ void scale_add(const Factor &f, const i64 (&x)[N], i6
 
 // One result, for this thread's columns of its row and plane: formed in place
 // of T, stored at dst (pieces qs apart, as those of the terms); returns the OR of
-// the magnitudes (ones' complement for negative values).  row, col0: global row
+// the magnitudes (ones' complement for negative values), and adds their sum in units
+// of 2^38 to `sum` (below 2^29).  row, col0: global row
 // and first column; diagonal entries below d only.  The loads of a term go out
 // together: one wait per term, not one per piece.
 template <class V>
-__device__ __forceinline__ u64 put_out(const Out &o, const Thread &t, i64 (&T)[kCols], int eT, int e, V view,
-                                       i64 plane, i64 qs, int row, int col0, int d, i64 *dst) {
+__device__ __forceinline__ u64 put_out(const Out &o, const Thread &t, i64 (&T)[kCols], Sum S, int e, V view, i64 plane,
+                                       i64 qs, int row, int col0, int d, i64 *dst,
+                                       uint32_t *sum = nullptr) {
     if (!o.plain) {
         // T times its coefficient, then the terms, a quarter of the columns at a time;
         // the first loads go out before the multiplication.
-        const Factor ft = o.t.m ? make_factor(o.t.m, e - eT - o.t.e - 2, 0) : Factor{0, 0, 0, 0};
+        const Factor ft = o.t.m ? make_factor(o.t.m, e - (S.e - S.h) - o.t.e - 2, S.h) : Factor{0, 0, 0, 0};
         constexpr int H = kCols / 4;
 #pragma unroll 1
         for (int k = 0; k < max(1, o.nterm); ++k) {
@@ -636,7 +692,7 @@ __device__ __forceinline__ u64 put_out(const Out &o, const Thread &t, i64 (&T)[k
                 if (k == 0) {
                     i64 v[H];
 #pragma unroll
-                    for (int j = 0; j < H; ++j) v[j] = T[h * H + j];
+                    for (int j = 0; j < H; ++j) v[j] = (i64)((u64)T[h * H + j] << ft.pre);
                     scale_add<H>(ft, v, T + h * H, false);
                 }
                 if (q) {
@@ -669,6 +725,15 @@ __device__ __forceinline__ u64 put_out(const Out &o, const Thread &t, i64 (&T)[k
         store4(dst + i * qs, T[4 * i], T[4 * i + 1], T[4 * i + 2], T[4 * i + 3]);
 #pragma unroll
         for (int j = 0; j < 4; ++j) m |= (u64)(T[4 * i + j] ^ (T[4 * i + j] >> 63));
+    }
+    if (sum) {
+        uint32_t u = 0;
+#pragma unroll
+        for (int j = 0; j < kCols; ++j) {
+            const int hi = (int)(T[j] >> 32);
+            u += (uint32_t)(hi ^ (hi >> 31)) >> 6;
+        }
+        atomicAdd(sum, u + kCols);
     }
     return m;
 }
@@ -705,6 +770,7 @@ __device__ __forceinline__ void setup(Shared &s, Thread &t, unsigned char *raw) 
     t.ok = true;
     if (t.tid < 8) s.orhi[t.tid >> 1][t.tid & 1] = s.orlo[t.tid >> 1][t.tid & 1] = 0;
     if (t.tid < 128) s.rowmb[t.tid >> 6][t.tid & 63] = 0;
+    if (t.tid < 256) s.rows[t.tid >> 7][(t.tid >> 6) & 1][t.tid & 63] = 0;
     if (t.warp == 0) {
         tc::tmem_alloc(&s.tmem_base, 512);
         tc::tmem_relinquish();
@@ -730,7 +796,7 @@ __device__ __forceinline__ void setup(Shared &s, Thread &t, unsigned char *raw) 
 
 // A launch: every role over the products of w (`products` of them for this CTA).
 template <int S, class W>
-__device__ __forceinline__ void run(Shared &s, Thread &t, const W &w, i64 products, int nst, int kvalid, int sh) {
+__device__ __forceinline__ void run(Shared &s, Thread &t, const W &w, i64 products, int nst, int kvalid) {
     if (t.tid >= kIssuer) {
         regs_down<kRegsIssue>();
         if (t.tid == kIssuer) t.ok = issue_products<S>(s, t.smem, products, nst);
@@ -739,7 +805,7 @@ __device__ __forceinline__ void run(Shared &s, Thread &t, const W &w, i64 produc
         cutter<S>(s, t, w, nst, kvalid);
     } else {
         regs_up<kRegsFinish>();
-        finisher<S>(s, t, w, nst, sh);
+        finisher<S>(s, t, w, nst);
     }
 }
 
