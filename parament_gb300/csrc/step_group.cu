@@ -17,7 +17,9 @@
 //
 // The chunk products meet without another launch.  The group that finds the
 // product beside its own finished goes on with the pair, the other one ends:
-// nobody waits.  In double-float (complex64) or FP64.
+// nobody waits.  In double-float (complex64) or FP64, as k_tree_df and tree_product do:
+// the nodes are products and not their distances from I, which would leave a propagator
+// of size 1e-10 good to 1e-6 of itself.
 //
 // What bounds it: latency.  A qubit's 100 steps took 71 us with host buffers, ten
 // launches (256 threads per chunk, a launch per level of the tree) between two
@@ -65,16 +67,13 @@ struct Node;
 template <>
 struct Node<float> {
     using T = float4;
-    // A chunk product minus I.
-    __device__ static T make(float2 v, bool diag) {
-        const df r = diag ? df_add_f(df{v.x, 0.f}, -1.0f) : df{v.x, 0.f};
-        return make_float4(r.hi, r.lo, v.y, 0.f);
+    __device__ static T make(float2 v, bool) { return make_float4(v.x, 0.f, v.y, 0.f); }
+    // a b as b + (a - I) b
+    __device__ static T left(T a, bool diag) {
+        const df r = diag ? df_add_f(df{a.x, a.y}, -1.0f) : df{a.x, a.y};
+        return make_float4(r.hi, r.lo, a.z, a.w);
     }
-    // a b + a + b for element sums: acc starts as a + b
-    __device__ static T add(T a, T b) {
-        const df r = df_add(df{a.x, a.y}, df{b.x, b.y}), i = df_add(df{a.z, a.w}, df{b.z, b.w});
-        return make_float4(r.hi, r.lo, i.hi, i.lo);
-    }
+    __device__ static T start(T b) { return b; }
     __device__ static void mac1(float &hi, float &lo, float xh, float xl, float yh, float yl) {
         const float p = __fmul_rn(xh, yh);
         float e = __fmaf_rn(xh, yh, -p);
@@ -95,24 +94,22 @@ struct Node<float> {
         const df r = df_norm(v.x, v.y), i = df_norm(v.z, v.w);
         return make_float4(r.hi, r.lo, i.hi, i.lo);
     }
-    // I + node, rounded once.
-    __device__ static float2 out(T v, bool diag) {
-        df r = {v.x, v.y};
-        if (diag) r = df_add_f(r, 1.0f);
-        return make_float2(__fadd_rn(r.hi, r.lo), __fadd_rn(v.z, v.w));
-    }
+    // Rounded once.
+    __device__ static float2 out(T v) { return make_float2(__fadd_rn(v.x, v.y), __fadd_rn(v.z, v.w)); }
 };
 template <>
 struct Node<double> {
     using T = double2;
-    __device__ static T make(double2 v, bool) { return v; }
-    __device__ static T add(T a, T b) { return cadd(a, b); }
-    __device__ static void mac(T &c, T a, T b) { cfma(c, a, b); }
-    __device__ static T norm(T v) { return v; }
-    __device__ static double2 out(T v, bool diag) {
+    // The chunk product from it less I.
+    __device__ static T make(double2 v, bool diag) {
         if (diag) v.x += 1.0;
         return v;
     }
+    __device__ static T left(T a, bool) { return a; }
+    __device__ static T start(T) { return make_double2(0.0, 0.0); }
+    __device__ static void mac(T &c, T a, T b) { cfma(c, a, b); }
+    __device__ static T norm(T v) { return v; }
+    __device__ static double2 out(T v) { return v; }
 };
 
 template <class R, int TM>
@@ -319,20 +316,20 @@ __global__ void __launch_bounds__(384) k_group_steps(const __grid_constant__ Gro
         if (*flag == 0) return;  // the partner's group takes the pair
         __threadfence();
         for (int e = gt; e < dd; e += NT) {
-            As[e] = __ldcg(&nodes[hi * dd + e]);
+            As[e] = N::left(__ldcg(&nodes[hi * dd + e]), e / d == e % d);
             Bs[e] = __ldcg(&nodes[lo * dd + e]);
         }
         group_sync(g);
         for (int e = gt; e < dd; e += NT) {
             const int r = e / d, c = e % d;
-            E v = N::add(As[e], Bs[e]);
+            E v = N::start(Bs[e]);
             for (int k = 0; k < d; ++k) N::mac(v, As[r * d + k], Bs[k * d + c]);
             __stcg(&nodes[lo * dd + e], N::norm(v));
         }
         first = lo;
     }
     // The root, node 0.  Each element was written by the thread that reads it.
-    for (int e = gt; e < dd; e += NT) a.out[e] = N::out(__ldcg(&nodes[e]), e / d == e % d);
+    for (int e = gt; e < dd; e += NT) a.out[e] = N::out(__ldcg(&nodes[e]));
 }
 
 // ------------------------------------------------------------------ host side

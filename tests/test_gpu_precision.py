@@ -84,7 +84,7 @@ def test_little_mixing_and_large_steps(built_lib, d, P, mixing, x):
 # (70, 6) 4.2e-13 in the fixed point and 3.6e-13 in the FP64 oracle.
 ILL = pytest.mark.xfail(reason="strongly lossy steps above x = 1: the recurrence's own conditioning")
 DECAY = [(d, P, k) if (d, P, k) not in [(14, 80, 10), (70, 6, 10)] else pytest.param(d, P, k, marks=ILL)
-         for d, P in [(14, 80), (20, 160), (36, 24), (70, 6)] for k in (3, 10)]
+         for d, P in [(2, 300), (8, 120), (14, 80), (20, 160), (36, 24), (70, 6)] for k in (3, 10)]
 
 
 @pytest.mark.parametrize("d,P,decades", DECAY)
