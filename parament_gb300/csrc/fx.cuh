@@ -30,9 +30,9 @@
 // as large.  Against 113-bit propagators whole calls are 0.2 to 1.5 times as far off
 // as the FP64 kernels, 2.1 times in the worst case met (d = 64, 24 steps, x = 0.5,
 // dense); a headroom of log2(2 d) bits for every sum instead took nearly diagonal
-// Hamiltonians and large steps to 3 to 13 times.  All of this is of the maxima: an entry far below its matrix's largest loses relative accuracy that FP64
-// would keep (blocks coupled by 1e-8, d = 32: their amplitudes to 3e-9; exact zeros
-// stay zero).
+// Hamiltonians and large steps to 3 to 13 times.  All of this is of the maxima: an
+// entry far below its matrix's largest loses relative accuracy that FP64 would keep
+// (blocks coupled by 1e-8, d = 32: their amplitudes to 3e-9; exact zeros stay zero).
 //
 // Real formulation of one K stage of 16 complex columns (M = 128 rows, K = 32):
 //     [C_r; C_i] = [[A_r, -A_i], [A_i, A_r]] [B_r; B_i].
