@@ -150,8 +150,12 @@ Parament_ErrorCode run_split_large(Ctx *c, const SplitArgs &a, double h, void *d
 // below hnorm is the norm of the stack as it is held.
 void power_coefficients(int M, double x, double hnorm, double *c0, std::vector<double> &mu);
 // The same polynomial with the FP32 coefficients of the complex64 contexts;
-// returns J_0, which c_0 = p(0) - J_0 leaves out.
+// returns J_0, which c_0 = p(0) - J_0 leaves out.  Each c_n n >= 1 is a sum over orders
+// and so no FP32 number itself.  Rounded to one, c_1 and c_2 would turn every step by the
+// same angle (0.3 x 2^-24 of x on average, adding up along the steps, where the recurrence
+// has the roundings of J_k only); kernels add the rests c - (float)c times X and X^2.
 double plain_coefficients(int M, double x, double hnorm, std::vector<double> &c);
+inline float low_part(double c) { return (float)(c - (double)(float)c); }
 
 // Exact sliced products (fx.cu): fx_prepare / fx_prepare_split convert the stack
 // (set_hamiltonian; the split form's first call), fx_ensure allocates the

@@ -65,6 +65,7 @@ static_assert(kStcXBytes % 16 == 0 && (kStcSA + kStcSB) % 1024 == 0, "plane buff
 struct SmallTcArgs {
     float2 J[kMaxOrder + 1];  // (-i)^k J_k(x) in complex64
     float c[kMaxOrder + 1];   // by powers: c_n (odd n: times i), c_0 without J_0
+    float low[2];             // what FP32 leaves of c_1 and c_2
     int powers;
     const float *xplanes;     // planes of the batch's steps, kSmallXStride floats apart
     float2 *chunks;           // nchunks products, row-major complex64
@@ -259,7 +260,9 @@ __global__ void __launch_bounds__(kTcdThreads, 1) k_small_tc(const __grid_consta
                 epilogue_f<kStcSlices - 1>(sh, t, b1);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    float v = fmaf(a.c[k + 1], b2[j], b1[j]);
+                    float v = b1[j];
+                    if (k == 0) v = fmaf(a.low[1], X[j], fmaf(a.low[0], b2[j], v));
+                    v = fmaf(a.c[k + 1], b2[j], v);
                     if (t.p == 0 && t.c0 + j == t.r) {
                         v += a.c[k];
                         if (k == 0) v += a.J[0].x;
@@ -376,6 +379,7 @@ cudaError_t launch_small_tc(const StepLaunch &l, int num_sms, float *xplanes, in
         std::vector<double> c;
         plain_coefficients(l.M, l.x, 2.0 / l.s, c);
         for (int n = 0; n <= l.M; ++n) a.c[n] = (float)c[n];
+        for (int n = 1; n <= 2; ++n) a.low[n - 1] = low_part(c[n]);
     }
     a.fault = fault;
     const WeightSpec w{l.w.pts, l.w.K, l.w.amps, l.w.mode, l.w.magnus, l.w.hfac};

@@ -44,6 +44,7 @@ constexpr int kGroupStackBytes = 96 << 10;  // largest stack kept in shared memo
 template <class R>
 struct GroupArgs {
     R c[kMaxOrder + 1];  // c_n, real for even n, imaginary for odd n; c_0 of E (complex128) or of U - J_0
+    R low[2];            // complex64: what FP32 leaves of c_1 and c_2
     R j0;                // complex64: J_0, added last
     const cplx_t<R> *stack, *carr;
     void *nodes;         // nodes of the tree, float4 (double-float) or double2
@@ -242,6 +243,10 @@ __global__ void __launch_bounds__(384) k_group_steps(const __grid_constant__ Gro
                 add_odd(r, a.c[M - 2], x[i][j]);
                 add_even(r, a.c[M - 1], y[i][j]);
                 add_odd(r, a.c[M], acc[i][j]);
+                if (kHasU && M == 3) {
+                    add_odd(r, a.low[0], x[i][j]);
+                    add_even(r, a.low[1], y[i][j]);
+                }
                 if (kHasU && M == 3 && row(i) == col(j)) r.x += a.j0;
                 acc[i][j] = r;
             }
@@ -258,6 +263,10 @@ __global__ void __launch_bounds__(384) k_group_steps(const __grid_constant__ Gro
             for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TM; ++j) {
+                    if (kHasU && k == 0) {
+                        add_odd(acc[i][j], a.low[0], x[i][j]);
+                        add_even(acc[i][j], a.low[1], y[i][j]);
+                    }
                     add_odd(acc[i][j], a.c[k + 1], x[i][j]);
                     if (row(i) == col(j)) {
                         acc[i][j].x += a.c[k];
@@ -380,7 +389,7 @@ static cudaError_t launch_group_t(const StepLaunch &l, const GroupPlan &q, doubl
                                   unsigned *arrived, unsigned turn, void *out) {
     using C = cplx_t<R>;
     GroupArgs<R> a;
-    a.j0 = (R)0;
+    a.j0 = a.low[0] = a.low[1] = (R)0;
     if (l.fp64) {
         double c0[2];
         std::vector<double> mu;
@@ -391,6 +400,7 @@ static cudaError_t launch_group_t(const StepLaunch &l, const GroupPlan &q, doubl
         std::vector<double> c;
         a.j0 = (R)plain_coefficients(l.M, x, hnorm, c);
         for (int n = 0; n <= l.M; ++n) a.c[n] = (R)c[n];
+        for (int n = 1; n <= 2; ++n) a.low[n - 1] = (R)low_part(c[n]);
     }
     a.stack = static_cast<const C *>(l.stack);
     a.carr = static_cast<const C *>(l.carr);

@@ -31,6 +31,7 @@ template <class R>
 struct SmallArgs {
     cplx_t<R> J[kMaxOrder + 1];
     R c[kMaxOrder + 1];  // by powers: c_n (odd n: times i); c_0 of E (complex128) or of U - J_0
+    R low[2];            // complex64: what FP32 leaves of c_1 and c_2
     const cplx_t<R> *stack;
     const cplx_t<R> *carr;
     cplx_t<R> *chunks;
@@ -126,6 +127,11 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_small_steps(con
                     for (int j = 0; j < TM; ++j) {
                         if (!own[i][j]) continue;
                         C r = acc[i][j];
+                        if (kHasU && k == 0) {
+                            const C y = Bs[eo[i][j]];
+                            r.x = fma(a.low[1], y.x, fma(-a.low[0], x[i][j].y, r.x));
+                            r.y = fma(a.low[1], y.y, fma(a.low[0], x[i][j].x, r.y));
+                        }
                         r.x = fma(-a.c[k + 1], x[i][j].y, r.x);
                         r.y = fma(a.c[k + 1], x[i][j].x, r.y);
                         if (diag[i][j]) {
@@ -294,6 +300,7 @@ static cudaError_t launch_small_t(const StepLaunch &l) {
         std::vector<double> c;
         plain_coefficients(l.M, l.x, 2.0 / l.s, c);
         for (int n = 0; n <= l.M; ++n) a.c[n] = (R)c[n];
+        for (int n = 1; n <= 2; ++n) a.low[n - 1] = (R)low_part(c[n]);
     }
     const void *fn = pick_small(l.fp64, l.d, powers);
     cudaError_t e = allow_smem(fn);
