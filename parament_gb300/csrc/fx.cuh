@@ -52,7 +52,7 @@
 // operands' loads (6) lie underneath.  At d <= 128 the loads' latency and the
 // epilogues (64-bit multiplies) weigh as much; with four or five digits they are
 // all of it.  Measured: d = 64 Magnus, 4096 steps, 2.07 ms; d = 96, 512 steps, 1.70
-// ms; d = 512, 16 steps, 2.96 ms on the device; complex64, d = 128, 4096 steps, 8.05
+// ms; d = 512, 16 steps, 3.24 ms a call; complex64, d = 128, 4096 steps, 8.05
 // ms (FP32 kernel: 11.2).  With the finishers' sums spilled (136 registers) the
 // first three took 2.36, 1.71 and 3.07; with eight warps that did all but the
 // issuing 2.57, 1.80 and 3.13.  Accumulators for each half of the columns, one
